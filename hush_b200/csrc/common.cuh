@@ -35,6 +35,18 @@ HD_INL float4 quant4(float4 v) {  // value after an rgba16float round trip
 }
 HD_INL float quant1(float v) { return __half2float(__float2half_rz(v)); }
 
+// One texel copied from global to shared memory without passing through registers; a thread's copies are committed as
+// groups and waited for by the number of later groups that may still fly.
+HD_INL void cp_async8(const uint2 *dst_smem, const uint2 *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src)
+               : "memory");
+}
+HD_INL void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+HD_INL void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // qf16 (hush.js:68, 99): clamp to the f16 range, drop the low 13 mantissa bits.
 HD_INL float qf16(float x) {
   return __uint_as_float(__float_as_uint(fminf(fmaxf(x, -65504.0f), 65504.0f)) & 0xffffe000u);

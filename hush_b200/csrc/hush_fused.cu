@@ -94,14 +94,6 @@ struct PixLoads {
 // A pixel's loads are issued as cp.async copies into a shared-memory slot (no registers held while they fly): slot
 // entry k of this thread at g[k * stride]: 0 normalDepth, 1 material, 2 previous par0, 3-6 key, 7-10 colour history,
 // 11-14 moments of the bilinear footprint. The caller commits the group.
-HD_INL void cp_async8(const uint2 *dst_smem, const uint2 *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(umma::smem_u32(dst_smem)), "l"(src) : "memory");
-}
-HD_INL void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-HD_INL void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 template <int STRIDE>
 HD_INL void pixel_issue_async(const HushFrame &f, int px, int py, uint2 mvr, uint2 *g) {
   const int W = f.W, H = f.H;

@@ -8,6 +8,7 @@
 #include "common.cuh"
 #include "hush.h"
 #include "hush_device.cuh"
+#include "hush_pair.cuh"
 
 using namespace hush;
 
@@ -140,161 +141,255 @@ __global__ void k_svgf_variance(const SvgfFrame f, uint2 *out) {
   sth(out, o, make_float4(scx, scy, scz, v));
 }
 
+// ATROUS iteration (svgf.js:157-216), step 1 << iter; iteration 0 also writes the colour history.
+//
+// A CTA filters 64 columns x 8 rows, the rows STEP apart (one row phase of the iteration's lattice), so its staged
+// footprint is (64 + 4 STEP) x 12 texels for every STEP: rows between two lattice rows are not loaded. A thread filters
+// four pixels: columns x and x + 32 in the two lanes of packed FP32x2 arithmetic, times two neighbouring lattice rows,
+// which share 20 of their 25 taps. The footprint is held in shared memory as the pairs of texels 32 columns apart, each
+// converted to FP32 once, so that every tap of every STEP, 1 included, is a pair without a shuffle; texels outside
+// the image are marked as sky (depth -1, colour 0), so no tap tests its position. The tap columns run as a loop (the
+// depth factors of a column's taps come from shared memory): unrolled, instruction fetch stalled the warps.
+// Bound: the FP32 pipe (the ~23 FP32 operations of a tap and pixel; packing saves issue slots, not pipe time: 61% busy
+// at 1920 x 1080) with shared-memory bandwidth next (68%). A float4 tile with a thread per pixel read 36 bytes a tap for
+// one pixel, and steps 8 and 16 loaded every tap from global memory: iterations 0-4 at 1920 x 1080 were 93 / 96 / 99 /
+// 125 / 125 us and are 65 / 66 / 68 / 71 / 76 us.
+constexpr int AT_P = 32, AT_W = 2 * AT_P, AT_H = 8, AT_NT = AT_P * AT_H / 2;
+
 // The normal weight pow(max(n . n_q, 0), sigma_n): by seven squarings for the default sigma_n = 128 (no special-function
 // unit), else as the hardware exp2(sigma_n log2 x); pow(x, 0) = 1.
-HD_INL float svgf_wn(float x, float sigma_n) {
-  if (sigma_n == 128.0f) {
+template <bool N128>
+HD_INL float2 svgf_wn2(float2 x, float sigma_n) {
+  if constexpr (N128) {
 #pragma unroll
-    for (int i = 0; i < 7; i++) x *= x;
+    for (int i = 0; i < 7; i++) x = mul2(x, x);
     return x;
+  } else {
+    return sigma_n != 0.0f ? f2(__powf(x.x, sigma_n), __powf(x.y, sigma_n)) : f2(1.0f, 1.0f);
   }
-  return sigma_n != 0.0f ? __powf(x, sigma_n) : 1.0f;
+}
+HD_INL float hi_half(uint32_t u) { return __half2float(__ushort_as_half((uint16_t)(u >> 16))); }
+
+// 1 / x to within an ulp: the hardware approximation and one Newton step, without the range checks of an IEEE division
+// (x is a sum of weights or a positive bandwidth + epsilon here).
+HD_INL float rcp1(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return fmaf(fmaf(-x, r, 1.0f), r, r);
 }
 
-// ATROUS iteration (svgf.js:157-216); iteration 0 also writes the colour history.
-__global__ void k_svgf_atrous(const SvgfFrame f, const uint2 *in, uint2 *out, int iter, int step) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= f.W || y >= f.H) return;
-  const int o = y * f.W + x;
-  const float4 nd = ldh(f.nd, y * f.p_nd + x);
-  if (nd.w < 0.0f) {
-    sth(out, o, make_float4(0.f, 0.f, 0.f, 0.f));
-    if (iter == 0) sth(f.hist, o, make_float4(0.f, 0.f, 0.f, 0.f));
-    return;
-  }
-  const float4 center = ldh(in, o);
-  const float k3[3] = {0.25f, 0.5f, 0.25f};
-  float gv = 0.f;
-#pragma unroll
-  for (int dy = -1; dy <= 1; dy++)
-#pragma unroll
-    for (int dx = -1; dx <= 1; dx++)
-      gv += k3[dx + 1] * k3[dy + 1] * ldh(in, clampi(y + dy, 0, f.H - 1) * f.W + clampi(x + dx, 0, f.W - 1)).w;
-  const float lp = lum(center);
-  const float denomL = f.sigma_l * sqrtf(fmaxf(gv, 0.0f)) + 1e-6f;
-  const float z = nd.w;
-  const float zl = ldh(f.nd, y * f.p_nd + clampi(x - 1, 0, f.W - 1)).w;
-  const float zr = ldh(f.nd, y * f.p_nd + clampi(x + 1, 0, f.W - 1)).w;
-  const float zu = ldh(f.nd, clampi(y - 1, 0, f.H - 1) * f.p_nd + x).w;
-  const float zd = ldh(f.nd, clampi(y + 1, 0, f.H - 1) * f.p_nd + x).w;
-  const float gx = fminf(zr > 0.0f ? fabsf(zr - z) : 1e9f, zl > 0.0f ? fabsf(zl - z) : 1e9f);
-  const float gy = fminf(zd > 0.0f ? fabsf(zd - z) : 1e9f, zu > 0.0f ? fabsf(zu - z) : 1e9f);
-  const float zg = fminf(fmaxf(gx, gy), z);
-  const float h[5] = {1.0f / 16.0f, 1.0f / 4.0f, 3.0f / 8.0f, 1.0f / 4.0f, 1.0f / 16.0f};
-  // the tap distances sqrt(dx^2 + dy^2) (correctly rounded: 1, sqrt 2, 2, sqrt 5, sqrt 8) and one reciprocal per
-  // distance class and for the luminance scale instead of a division per tap; the weights' exp and pow run as the
-  // hardware approximations, which WGSL's own accuracy rules allow (exp: 3 + 2|x| ULP; pow via exp2(y log2 x)). The
-  // temporal pass, whose history-length test flips on an ulp, keeps IEEE arithmetic.
-  const float dcls[5] = {1.0f, 1.41421356237f, 2.0f, 2.2360679775f, 2.82842712475f};
-  float izd[5];
-#pragma unroll
-  for (int c = 0; c < 5; c++) izd[c] = 1.0f / (f.sigma_z * zg * (dcls[c] * (float)step) + 1e-3f);
-  const float ilum = 1.0f / denomL;
-  float sw = h[2] * h[2];
-  float scx = center.x * sw, scy = center.y * sw, scz = center.z * sw;
-  float sv = center.w * sw * sw;
-#pragma unroll
-  for (int dy = -2; dy <= 2; dy++) {
-#pragma unroll
-    for (int dx = -2; dx <= 2; dx++) {
-      if (dx == 0 && dy == 0) continue;
-      const int qx = x + dx * step, qy = y + dy * step;
-      if (qx < 0 || qy < 0 || qx >= f.W || qy >= f.H) continue;
-      const float4 ndq = ldh(f.nd, qy * f.p_nd + qx);
-      if (ndq.w < 0.0f) continue;
-      const float4 cq = ldh(in, qy * f.W + qx);
-      const int d2 = dx * dx + dy * dy;  // 1, 2, 4, 5, 8
-      const int cls = d2 == 1 ? 0 : (d2 == 2 ? 1 : (d2 == 4 ? 2 : (d2 == 5 ? 3 : 4)));
-      const float wz = fabsf(ndq.w - nd.w) * izd[cls];
-      const float wn = svgf_wn(fmaxf(0.0f, dot3(ndq, nd)), f.sigma_n);
-      const float wl = fabsf(lum(cq) - lp) * ilum;
-      const float w = h[dx + 2] * h[dy + 2] * wn * __expf(-wz - wl);
-      sw += w;
-      scx += w * cq.x; scy += w * cq.y; scz += w * cq.z;
-      sv += w * w * cq.w;
+// A texel pair of the footprint: (nx, nx', ny, ny'), (nz, nz', z, z'), (r, r', g, g'), (b, b', v, v').
+struct TexelPair {
+  float4 g0, g1, c0, c1;
+};
+HD_INL TexelPair widen(uint2 na, uint2 nb, uint2 ca, uint2 cb) {
+  const float4 n0 = h4_to_f4(na), n1 = h4_to_f4(nb), c0 = h4_to_f4(ca), c1 = h4_to_f4(cb);
+  return TexelPair{make_float4(n0.x, n1.x, n0.y, n1.y), make_float4(n0.z, n1.z, n0.w, n1.w),
+                   make_float4(c0.x, c1.x, c0.y, c1.y), make_float4(c0.z, c1.z, c0.w, c1.w)};
+}
+// RAW: the pairs as stored (converted by each tap), 32 bytes instead of 64. Only STEP = 16 takes it, whose 96 x 12
+// pairs would leave two CTAs an SM.
+template <int STEP>
+struct AtrousSmem {
+  static constexpr bool RAW = STEP >= 16;
+  static constexpr int A = 2 * STEP, TC = AT_P + 2 * A, TR = AT_H + 4, N = TR * TC;
+  uint4 t[RAW ? 2 : 4][N];
+  float2 izd[2][5][AT_NT];  // log2(e) / (sigma_z zg dist + 1e-3) per tap distance 1, sqrt 2, 2, sqrt 5, sqrt 8
+  HD_INL void put(int i, uint2 na, uint2 nb, uint2 ca, uint2 cb) {
+    if constexpr (RAW) {
+      t[0][i] = make_uint4(na.x, na.y, nb.x, nb.y);
+      t[1][i] = make_uint4(ca.x, ca.y, cb.x, cb.y);
+    } else {
+      const TexelPair p = widen(na, nb, ca, cb);
+      *reinterpret_cast<float4 *>(&t[0][i]) = p.g0;
+      *reinterpret_cast<float4 *>(&t[1][i]) = p.g1;
+      *reinterpret_cast<float4 *>(&t[2][i]) = p.c0;
+      *reinterpret_cast<float4 *>(&t[3][i]) = p.c1;
     }
   }
-  const float4 r = make_float4(scx / sw, scy / sw, scz / sw, sv / (sw * sw));
-  sth(out, o, r);
-  if (iter == 0) sth(f.hist, o, make_float4(r.x, r.y, r.z, 0.f));
-}
+  HD_INL static TexelPair get(const uint4 *p) {  // p = &t[0][i]
+    if constexpr (RAW) {
+      const uint4 n = p[0], c = p[N];
+      return widen(make_uint2(n.x, n.y), make_uint2(n.z, n.w), make_uint2(c.x, c.y), make_uint2(c.z, c.w));
+    } else {
+      const float4 *q = reinterpret_cast<const float4 *>(p);
+      return TexelPair{q[0], q[N], q[2 * N], q[3 * N]};
+    }
+  }
+  HD_INL float depth(int i, int lane) const {
+    if constexpr (RAW) return hi_half((&t[0][i].y)[2 * lane]);
+    else return __uint_as_float((&t[1][i].z)[lane]);
+  }
+  HD_INL float variance(int i, int lane) const {
+    if constexpr (RAW) return hi_half((&t[1][i].y)[2 * lane]);
+    else return __uint_as_float((&t[3][i].z)[lane]);
+  }
+};
 
-// The same iteration for steps 1, 2 and 4 with the 5 x 5 footprint staged in shared memory: a 16 x 16 tile with an
-// apron of 2 step texels (clamped to the image, as the centre's 3 x 3 variance blur and depth gradient read them),
-// each texel converted once and its luminance formed once. The arithmetic per tap is the kernel's above.
-template <int STEP>
-__global__ void __launch_bounds__(256) k_svgf_atrous_tile(const SvgfFrame f, const uint2 *in, uint2 *out, int iter) {
-  constexpr int TS = 16, A = 2 * STEP, T = TS + 2 * A;
-  __shared__ float4 sC[T * T], sN[T * T];
-  __shared__ float sL[T * T];
-  const int li = threadIdx.y * TS + threadIdx.x;
-  const int bx = blockIdx.x * TS, by = blockIdx.y * TS;
-  for (int i = li; i < T * T; i += TS * TS) {
-    const int gx = clampi(bx - A + i % T, 0, f.W - 1), gy = clampi(by - A + i / T, 0, f.H - 1);
-    const float4 c = ldh(in, gy * f.W + gx);
-    sC[i] = c;
-    sN[i] = ldh(f.nd, gy * f.p_nd + gx);
-    sL[i] = lum(c);
+template <int STEP, bool N128>
+__global__ void __launch_bounds__(AT_NT, 5) k_svgf_atrous(const SvgfFrame f, const uint2 *in, uint2 *out, int iter) {
+  using Smem = AtrousSmem<STEP>;
+  constexpr int A = Smem::A, TC = Smem::TC;
+  extern __shared__ __align__(16) unsigned char at_smem[];
+  Smem &S = *reinterpret_cast<Smem *>(at_smem);
+  const int li = threadIdx.x;
+  const int bx = blockIdx.x * AT_W, phase = blockIdx.y % STEP, j0 = (blockIdx.y / STEP) * AT_H;
+  const int tx = li % AT_P, jr = (li / AT_P) * 2;  // the thread's first lattice row in the tile
+  const int x0 = bx + tx, y0 = (j0 + jr) * STEP + phase;
+  // The centre's 3 x 3 variance blur and depth gradient read the rows y +- 1, which only STEP = 1 stages; the other
+  // steps load them here (texels clamped to the image).
+  float vs[2][2], zu[2][2], zd[2][2];
+  if constexpr (STEP > 1) {
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const int y = min(y0 + k * STEP, f.H - 1);
+      const uint2 *im = in + max(y - 1, 0) * f.W, *ip = in + min(y + 1, f.H - 1) * f.W;
+      const uint2 *nm = f.nd + max(y - 1, 0) * f.p_nd, *np = f.nd + min(y + 1, f.H - 1) * f.p_nd;
+#pragma unroll
+      for (int l = 0; l < 2; l++) {
+        const int xc = min(x0 + l * AT_P, f.W - 1), xm = max(xc - 1, 0), xp = min(xc + 1, f.W - 1);
+        auto var = [](const uint2 *p) { return hi_half(__ldg(&p->y)); };
+        vs[k][l] = 0.0625f * (var(im + xm) + var(im + xp) + var(ip + xm) + var(ip + xp)) +
+                   0.125f * (var(im + xc) + var(ip + xc));
+        zu[k][l] = var(nm + xc);
+        zd[k][l] = var(np + xc);
+      }
+    }
+  }
+  // one warp a row of the footprint at a time
+  for (int r = li / 32; r < Smem::TR; r += AT_NT / 32) {
+    const int gy = (j0 - 2 + r) * STEP + phase, gx0 = bx - A + li % 32;
+    const bool iy = gy >= 0 && gy < f.H;
+    const uint2 *pn = f.nd + (gy * f.p_nd + gx0), *pc = in + (gy * f.W + gx0);
+#pragma unroll
+    for (int u = 0; u < TC; u += 32) {
+      if (u + 32 > TC && u + li % 32 >= TC) break;
+      const bool o0 = iy && gx0 + u >= 0 && gx0 + u < f.W, o1 = iy && gx0 + u + AT_P >= 0 && gx0 + u + AT_P < f.W;
+      uint2 n[2] = {make_uint2(0u, 0xbc000000u), make_uint2(0u, 0xbc000000u)}, c[2] = {};  // depth -1: sky
+      if (o0) { n[0] = __ldg(pn + u); c[0] = __ldg(pc + u); }
+      if (o1) { n[1] = __ldg(pn + u + AT_P); c[1] = __ldg(pc + u + AT_P); }
+      S.put(r * TC + u + li % 32, n[0], n[1], c[0], c[1]);
+    }
   }
   __syncthreads();
-  const int x = bx + threadIdx.x, y = by + threadIdx.y;
-  if (x >= f.W || y >= f.H) return;
-  const int o = y * f.W + x;
-  const int lx = threadIdx.x + A, ly = threadIdx.y + A, tc = ly * T + lx;
-  const float4 nd = sN[tc];
-  if (nd.w < 0.0f) {
-    sth(out, o, make_float4(0.f, 0.f, 0.f, 0.f));
-    if (iter == 0) sth(f.hist, o, make_float4(0.f, 0.f, 0.f, 0.f));
-    return;
+  if (y0 >= f.H || x0 >= f.W) return;
+  struct Centre {
+    float2 nx, ny, nz, z, lp, il, sw, sr, sg, sb, sv;
+  } C[2];
+  const int base = (jr + 2) * TC + tx + A;  // tile entry of the first row
+  constexpr float h0 = 3.0f / 8.0f, h1 = 1.0f / 4.0f, h2 = 1.0f / 16.0f;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int t = base + k * TC;
+    const TexelPair p = Smem::get(&S.t[0][t]);
+    Centre &c = C[k];
+    c.nx = lo2(p.g0); c.ny = hi2(p.g0); c.nz = lo2(p.g1); c.z = hi2(p.g1);
+    c.lp = fma2(lo2(p.c1), bc2(0.0722f), fma2(hi2(p.c0), bc2(0.7152f), mul2(lo2(p.c0), bc2(0.2126f))));
+    float il[2], izd[5][2];
+    const int y = min(y0 + k * STEP, f.H - 1);
+#pragma unroll
+    for (int l = 0; l < 2; l++) {
+      const int x = min(x0 + l * AT_P, f.W - 1);
+      const int tl = x > 0 ? t - 1 : t, tr = x + 1 < f.W ? t + 1 : t;
+      const float z = S.depth(t, l), zl = S.depth(tl, l), zr = S.depth(tr, l);
+      float up, dn, gv;
+      if constexpr (STEP > 1) {
+        gv = vs[k][l];
+        up = zu[k][l];
+        dn = zd[k][l];
+      } else {
+        const int du = y > 0 ? -TC : 0, dd = y + 1 < f.H ? TC : 0;
+        gv = 0.0625f * (S.variance(tl + du, l) + S.variance(tr + du, l) + S.variance(tl + dd, l) + S.variance(tr + dd, l)) +
+             0.125f * (S.variance(t + du, l) + S.variance(t + dd, l));
+        up = S.depth(t + du, l);
+        dn = S.depth(t + dd, l);
+      }
+      gv += 0.125f * (S.variance(tl, l) + S.variance(tr, l)) + 0.25f * S.variance(t, l);
+      const float gx = fminf(zr > 0.0f ? fabsf(zr - z) : 1e9f, zl > 0.0f ? fabsf(zl - z) : 1e9f);
+      const float gy = fminf(dn > 0.0f ? fabsf(dn - z) : 1e9f, up > 0.0f ? fabsf(up - z) : 1e9f);
+      const float zg = f.sigma_z * fminf(fmaxf(gx, gy), z);
+      il[l] = LOG2E * rcp1(f.sigma_l * sqrtf(fmaxf(gv, 0.0f)) + 1e-6f);
+      const float dcls[5] = {1.0f, 1.41421356237f, 2.0f, 2.2360679775f, 2.82842712475f};
+#pragma unroll
+      for (int d = 0; d < 5; d++) izd[d][l] = LOG2E * rcp1(zg * (dcls[d] * (float)STEP) + 1e-3f);
+    }
+    c.il = f2(il[0], il[1]);
+#pragma unroll
+    for (int d = 0; d < 5; d++) S.izd[k][d][li] = f2(izd[d][0], izd[d][1]);  // read back by this thread alone
+    c.sw = f2(h0 * h0, h0 * h0);
+    c.sr = mul2(lo2(p.c0), c.sw); c.sg = mul2(hi2(p.c0), c.sw); c.sb = mul2(lo2(p.c1), c.sw);
+    c.sv = mul2(mul2(hi2(p.c1), c.sw), c.sw);
   }
-  const float4 center = sC[tc];
-  const float k3[3] = {0.25f, 0.5f, 0.25f};
-  float gv = 0.f;
+  // One tap column at a time: its six texel pairs serve both rows' filters. The weight is
+  // h (n.n)^sigma_n 2^-(|dz| izd + |dl| il), the exponent in units of log2.
+  const uint4 *col = &S.t[0][base - 2 * STEP];
+#pragma unroll 1
+  for (int dx = -2; dx <= 2; dx++, col += STEP) {
+    const int a = dx < 0 ? -dx : dx;
+    const float hx = a == 0 ? h0 : (a == 1 ? h1 : h2);
+    const int cls[3] = {a == 2 ? 2 : 0, a == 0 ? 0 : (a == 1 ? 1 : 3), a == 0 ? 2 : (a == 1 ? 3 : 4)};  // by |dy|
+    const float2 hh[3] = {bc2(hx * h0), bc2(hx * h1), bc2(hx * h2)};
+    float2 iz[2][3];
 #pragma unroll
-  for (int dy = -1; dy <= 1; dy++)
+    for (int b = 0; b < 3; b++) { iz[0][b] = S.izd[0][cls[b]][li]; iz[1][b] = S.izd[1][cls[b]][li]; }
 #pragma unroll
-    for (int dx = -1; dx <= 1; dx++) gv += k3[dx + 1] * k3[dy + 1] * sC[tc + dy * T + dx].w;
-  const float lp = sL[tc];
-  const float denomL = f.sigma_l * sqrtf(fmaxf(gv, 0.0f)) + 1e-6f;
-  const float z = nd.w;
-  const float zl = sN[tc - 1].w, zr = sN[tc + 1].w, zu = sN[tc - T].w, zd = sN[tc + T].w;
-  const float gx = fminf(zr > 0.0f ? fabsf(zr - z) : 1e9f, zl > 0.0f ? fabsf(zl - z) : 1e9f);
-  const float gy = fminf(zd > 0.0f ? fabsf(zd - z) : 1e9f, zu > 0.0f ? fabsf(zu - z) : 1e9f);
-  const float zg = fminf(fmaxf(gx, gy), z);
-  const float h[5] = {1.0f / 16.0f, 1.0f / 4.0f, 3.0f / 8.0f, 1.0f / 4.0f, 1.0f / 16.0f};
-  const float dcls[5] = {1.0f, 1.41421356237f, 2.0f, 2.2360679775f, 2.82842712475f};
-  float izd[5];
+    for (int r = -2; r <= 3; r++) {
+      const TexelPair q = Smem::get(col + r * TC);
+      const float2 z = hi2(q.g1);
+      const float2 lq = fma2(lo2(q.c1), bc2(0.0722f), fma2(hi2(q.c0), bc2(0.7152f), mul2(lo2(q.c0), bc2(0.2126f))));
+      const bool ok0 = !(z.x < 0.0f), ok1 = !(z.y < 0.0f);
 #pragma unroll
-  for (int c = 0; c < 5; c++) izd[c] = 1.0f / (f.sigma_z * zg * (dcls[c] * (float)STEP) + 1e-3f);
-  const float ilum = 1.0f / denomL;
-  float sw = h[2] * h[2];
-  float scx = center.x * sw, scy = center.y * sw, scz = center.z * sw;
-  float sv = center.w * sw * sw;
-#pragma unroll
-  for (int dy = -2; dy <= 2; dy++) {
-#pragma unroll
-    for (int dx = -2; dx <= 2; dx++) {
-      if (dx == 0 && dy == 0) continue;
-      const int qx = x + dx * STEP, qy = y + dy * STEP;
-      if (qx < 0 || qy < 0 || qx >= f.W || qy >= f.H) continue;
-      const int t = tc + dy * STEP * T + dx * STEP;
-      const float4 ndq = sN[t];
-      if (ndq.w < 0.0f) continue;
-      const float4 cq = sC[t];
-      const int d2 = dx * dx + dy * dy;
-      const int cls = d2 == 1 ? 0 : (d2 == 2 ? 1 : (d2 == 4 ? 2 : (d2 == 5 ? 3 : 4)));
-      const float wz = fabsf(ndq.w - nd.w) * izd[cls];
-      const float wn = svgf_wn(fmaxf(0.0f, dot3(ndq, nd)), f.sigma_n);
-      const float wl = fabsf(sL[t] - lp) * ilum;
-      const float w = h[dx + 2] * h[dy + 2] * wn * __expf(-wz - wl);
-      sw += w;
-      scx += w * cq.x; scy += w * cq.y; scz += w * cq.z;
-      sv += w * w * cq.w;
+      for (int k = 0; k < 2; k++) {
+        const int dy = r - k, b = dy < 0 ? -dy : dy;
+        if (b > 2 || (b == 0 && dx == 0)) continue;
+        Centre &c = C[k];
+        const float2 dot = fma2(lo2(q.g1), c.nz, fma2(hi2(q.g0), c.ny, mul2(lo2(q.g0), c.nx)));
+        const float2 wn = svgf_wn2<N128>(f2(fmaxf(0.0f, dot.x), fmaxf(0.0f, dot.y)), f.sigma_n);
+        const float2 ez = mul2(sub2(z, c.z), iz[k][b]), el = mul2(sub2(lq, c.lp), c.il);
+        float2 w = mul2(mul2(hh[b], wn), f2(ex2_approx(-fabsf(ez.x) - fabsf(el.x)), ex2_approx(-fabsf(ez.y) - fabsf(el.y))));
+        w = f2(ok0 ? w.x : 0.0f, ok1 ? w.y : 0.0f);
+        c.sw = add2(c.sw, w);
+        c.sr = fma2(w, lo2(q.c0), c.sr);
+        c.sg = fma2(w, hi2(q.c0), c.sg);
+        c.sb = fma2(w, lo2(q.c1), c.sb);
+        c.sv = fma2(mul2(w, w), hi2(q.c1), c.sv);
+      }
     }
   }
-  const float4 r = make_float4(scx / sw, scy / sw, scz / sw, sv / (sw * sw));
-  sth(out, o, r);
-  if (iter == 0) sth(f.hist, o, make_float4(r.x, r.y, r.z, 0.f));
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int y = y0 + k * STEP;
+    if (y >= f.H) break;
+    const Centre &c = C[k];
+#pragma unroll
+    for (int l = 0; l < 2; l++) {
+      const int x = x0 + l * AT_P;
+      if (x >= f.W) break;
+      const float i = rcp1(l ? c.sw.y : c.sw.x);
+      float4 o = make_float4((l ? c.sr.y : c.sr.x) * i, (l ? c.sg.y : c.sg.x) * i, (l ? c.sb.y : c.sb.x) * i,
+                             (l ? c.sv.y : c.sv.x) * i * i);
+      if ((l ? c.z.y : c.z.x) < 0.0f) o = make_float4(0.f, 0.f, 0.f, 0.f);
+      sth(out, y * f.W + x, o);
+      if (iter == 0) sth(f.hist, y * f.W + x, make_float4(o.x, o.y, o.z, 0.f));
+    }
+  }
+}
+
+template <int STEP, bool N128>
+cudaError_t launch_atrous_n(const SvgfFrame &f, const uint2 *in, uint2 *out, int iter, cudaStream_t st) {
+  constexpr int smem = (int)sizeof(AtrousSmem<STEP>);
+  if constexpr (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k_svgf_atrous<STEP, N128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
+  const dim3 grid((f.W + AT_W - 1) / AT_W, STEP * ((f.H + AT_H * STEP - 1) / (AT_H * STEP)));
+  k_svgf_atrous<STEP, N128><<<grid, AT_NT, smem, st>>>(f, in, out, iter);
+  return cudaGetLastError();
+}
+template <int STEP>
+cudaError_t launch_atrous(const SvgfFrame &f, const uint2 *in, uint2 *out, int iter, cudaStream_t st) {
+  return f.sigma_n == 128.0f ? launch_atrous_n<STEP, true>(f, in, out, iter, st)
+                             : launch_atrous_n<STEP, false>(f, in, out, iter, st);
 }
 
 // RESOLVE (svgf.js:241-270). The reference samples the history through a hardware bilinear sampler
@@ -477,14 +572,18 @@ extern "C" int svgf_encode(svgf_t *s, const svgf_inputs *in, void *stream, const
   k_svgf_temporal<<<grd, blk, 0, st>>>(f);
   k_svgf_variance<<<grd, blk, 0, st>>>(f, s->atrous[0]);
   int src = 0;
-  const dim3 tblk(16, 16), tgrd((s->W + 15) / 16, (s->H + 15) / 16);
   for (int i = 0; i < s->o.iterations; i++) {
     const uint2 *a = s->atrous[src];
     uint2 *b = s->atrous[src ^ 1];
-    if (i == 0) k_svgf_atrous_tile<1><<<tgrd, tblk, 0, st>>>(f, a, b, i);
-    else if (i == 1) k_svgf_atrous_tile<2><<<tgrd, tblk, 0, st>>>(f, a, b, i);
-    else if (i == 2) k_svgf_atrous_tile<4><<<tgrd, tblk, 0, st>>>(f, a, b, i);
-    else k_svgf_atrous<<<grd, blk, 0, st>>>(f, a, b, i, 1 << i);
+    cudaError_t e;
+    switch (i) {
+      case 0: e = launch_atrous<1>(f, a, b, i, st); break;
+      case 1: e = launch_atrous<2>(f, a, b, i, st); break;
+      case 2: e = launch_atrous<4>(f, a, b, i, st); break;
+      case 3: e = launch_atrous<8>(f, a, b, i, st); break;
+      default: e = launch_atrous<16>(f, a, b, i, st); break;
+    }
+    if (e != cudaSuccess) return svgf_fail(s, HUSH_ERR_CUDA, std::string("SVGF: a-trous launch: ") + cudaGetErrorString(e));
     src ^= 1;
   }
   k_svgf_resolve<<<grd, blk, 0, st>>>(f, s->atrous[src]);
