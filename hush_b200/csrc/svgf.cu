@@ -24,48 +24,92 @@ struct SvgfFrame {
   uint2 *tmp, *mom, *hist, *taa;
 };
 
-HD_INL bool svgf_consistent(const SvgfFrame &f, int qx, int qy, float4 n, float zPrev, float obj) {  // svgf.js:31-39
-  if (qx < 0 || qy < 0 || qx >= f.W || qy >= f.H) return false;
-  const float4 nd = ldh(f.pnd, qy * f.p_pnd + qx);
-  if (nd.w < 0.0f) return false;
-  if (ldh(f.pmv, qy * f.p_pmv + qx).z != obj) return false;
-  if (fabsf(nd.w - zPrev) > 0.05f * zPrev + 0.01f) return false;
-  if (dot3(nd, n) < 0.9f) return false;
-  return true;
+HD_INL float hi_half(uint32_t u) { return __half2float(__ushort_as_half((uint16_t)(u >> 16))); }
+
+// 1 / x to within an ulp: the hardware approximation and one Newton step, without the range checks of an IEEE division
+// (x is a sum of weights or a positive bandwidth + epsilon here).
+HD_INL float rcp1(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return fmaf(fmaf(-x, r, 1.0f), r, r);
 }
 
-// TEMPORAL (svgf.js:41-105)
-__global__ void k_svgf_temporal(const SvgfFrame f) {
+// Quotients of one divisor: the product with rcp1 and one residual correction, which rounds as the IEEE division does but
+// for rare ties, without its range checks and branches (the divisors here are sums of weights, 1 + luminance and sizes).
+struct Divisor {
+  float d, r;
+  HD_INL explicit Divisor(float d_) : d(d_), r(rcp1(d_)) {}
+  HD_INL float operator()(float a) const {
+    const float q = a * r;
+    return fmaf(fmaf(-d, q, a), r, q);
+  }
+  HD_INL float3 operator()(float3 a) const { return make_float3((*this)(a.x), (*this)(a.y), (*this)(a.z)); }
+};
+// sqrt(x), x >= 0, rounded the same way from the hardware reciprocal square root.
+HD_INL float sqrt1(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  const float s = x * r;
+  return x > 1e-37f ? fmaf(fmaf(-s, s, x), 0.5f * r, s) : 0.0f;
+}
+
+// The history test of a previous frame's texel (guide q, object id) against this pixel's (svgf.js:31-39).
+HD_INL bool svgf_same(float4 q, float qobj, float4 n, float zPrev, float obj) {
+  return !(q.w < 0.0f) && qobj == obj && !(fabsf(q.w - zPrev) > 0.05f * zPrev + 0.01f) && !(dot3(q, n) < 0.9f);
+}
+HD_INL bool svgf_consistent(const SvgfFrame &f, int qx, int qy, float4 n, float zPrev, float obj) {
+  if (qx < 0 || qy < 0 || qx >= f.W || qy >= f.H) return false;
+  return svgf_same(ldh(f.pnd, qy * f.p_pnd + qx), ldh(f.pmv, qy * f.p_pmv + qx).z, n, zPrev, obj);
+}
+
+// TEMPORAL (svgf.js:41-105). Bound: the latency of its dependent loads (motion, then the footprint): the four texels'
+// guide, object, colour and moments are loaded together, not test by test (58 -> 47 us at 1920 x 1080).
+__global__ void __launch_bounds__(256) k_svgf_temporal(const SvgfFrame f) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= f.W || y >= f.H) return;
   const int o = y * f.W + x;
+  const float4 mv = ldh(f.mv, y * f.p_mv + x);
   const float4 nd = ldh(f.nd, y * f.p_nd + x);
+  const float ppx = (float)x + 0.5f + mv.x - 0.5f, ppy = (float)y + 0.5f + mv.y - 0.5f;
+  const float flx = floorf(ppx), fly = floorf(ppy);
+  const int bx = (int)flx, by = (int)fly;
+  const float fx = ppx - flx, fy = ppy - fly;
+  // the bilinear footprint's guide, object and history texels (clamped), all in flight before the first test
+  const bool noHistory = f.reset != 0;
+  uint2 pn[4], ph[4], pm[4];
+  uint32_t po[4];
+  if (!noHistory) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int qx = clampi(bx + (i & 1), 0, f.W - 1), qy = clampi(by + (i >> 1), 0, f.H - 1);
+      pn[i] = __ldg(f.pnd + qy * f.p_pnd + qx);
+      po[i] = __ldg(&f.pmv[qy * f.p_pmv + qx].y);
+      ph[i] = __ldg(f.hist_prev + qy * f.W + qx);
+      pm[i] = __ldg(f.mom_prev + qy * f.W + qx);
+    }
+  }
   if (nd.w < 0.0f) {
     sth(f.tmp, o, make_float4(0.f, 0.f, 0.f, 0.f));
     sth(f.mom, o, make_float4(0.f, 0.f, 0.f, 0.f));
     return;
   }
-  const float4 mv = ldh(f.mv, y * f.p_mv + x);
   const float4 alb = ldh(f.mat, y * f.p_mat + x);
   const float4 r = ldh(f.rad, y * f.p_rad + x);
-  const float ix = r.x / fmaxf(alb.x, 1e-3f), iy = r.y / fmaxf(alb.y, 1e-3f), iz = r.z / fmaxf(alb.z, 1e-3f);
+  const float ix = Divisor(fmaxf(alb.x, 1e-3f))(r.x), iy = Divisor(fmaxf(alb.y, 1e-3f))(r.y),
+              iz = Divisor(fmaxf(alb.z, 1e-3f))(r.z);
   const float l = __fadd_rn(__fadd_rn(__fmul_rn(ix, 0.2126f), __fmul_rn(iy, 0.7152f)), __fmul_rn(iz, 0.0722f));
-  const float ppx = (float)x + 0.5f + mv.x - 0.5f, ppy = (float)y + 0.5f + mv.y - 0.5f;
-  const float flx = floorf(ppx), fly = floorf(ppy);
-  const int bx = (int)flx, by = (int)fly;
-  const float fx = ppx - flx, fy = ppy - fly;
   // the history length it blends into decides the spatial / temporal variance branch (m.z >= 4), so the weighted
   // sums are rounded product by product like an unfused shader (no FMA contraction)
   float sumW = 0.f, hcx = 0.f, hcy = 0.f, hcz = 0.f, hm0 = 0.f, hm1 = 0.f, hm2 = 0.f;
   const float wts[4] = {__fmul_rn(1.0f - fx, 1.0f - fy), __fmul_rn(fx, 1.0f - fy), __fmul_rn(1.0f - fx, fy),
                         __fmul_rn(fx, fy)};
-  const bool noHistory = f.reset != 0;
   if (!noHistory) {
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       const int qx = bx + (i & 1), qy = by + (i >> 1);
-      if (svgf_consistent(f, qx, qy, nd, mv.w, mv.z) && wts[i] > 0.0f) {
-        const float4 c = ldh(f.hist_prev, qy * f.W + qx), m = ldh(f.mom_prev, qy * f.W + qx);
+      if (qx >= 0 && qy >= 0 && qx < f.W && qy < f.H && wts[i] > 0.0f &&
+          svgf_same(h4_to_f4(pn[i]), unpack2(po[i]).x, nd, mv.w, mv.z)) {
+        const float4 c = h4_to_f4(ph[i]), m = h4_to_f4(pm[i]);
         sumW += wts[i];
         hcx = __fadd_rn(hcx, __fmul_rn(wts[i], c.x)); hcy = __fadd_rn(hcy, __fmul_rn(wts[i], c.y));
         hcz = __fadd_rn(hcz, __fmul_rn(wts[i], c.z));
@@ -106,30 +150,76 @@ __global__ void k_svgf_temporal(const SvgfFrame f) {
   sth(f.mom, o, make_float4(m0, m1, len, 0.f));
 }
 
-// VARIANCE (svgf.js:114-148)
-__global__ void k_svgf_variance(const SvgfFrame f, uint2 *out) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= f.W || y >= f.H) return;
+// VARIANCE (svgf.js:114-148): temporal where the history is long enough, else from a 7 x 7 neighbourhood. Only a CTA
+// with such a pixel (a disocclusion, or the first frames) stages the neighbourhood's texels; outside the image they are
+// marked as sky. The weight's depth factor is one reciprocal per tap distance, exp and the default sigma_n = 128 run as
+// the a-trous kernel's do (seven squarings in place of a 49-fold powf): 39 -> 22 us at 1920 x 1080, 641 x 363 22.7 ->
+// 9.5 us (a sequence of eight frames, two of them without a long enough history).
+constexpr int VT_W = 32, VT_H = 8, VT_NT = VT_W * VT_H;
+template <bool N128>
+__global__ void __launch_bounds__(VT_NT) k_svgf_variance(const SvgfFrame f, uint2 *out) {
+  constexpr int TC = VT_W + 6, TR = VT_H + 6, N = TC * TR;
+  __shared__ uint2 sN[N], sC[N], sM[N];
+  const int li = threadIdx.x, tx = li % VT_W, ty = li / VT_W;
+  const int bx = blockIdx.x * VT_W, by = blockIdx.y * VT_H, x = bx + tx, y = by + ty;
+  const bool in_img = x < f.W && y < f.H;
   const int o = y * f.W + x;
-  const float4 nd = ldh(f.nd, y * f.p_nd + x);
-  if (nd.w < 0.0f) { sth(out, o, make_float4(0.f, 0.f, 0.f, 0.f)); return; }
-  const float4 c = ldh(f.tmp, o), m = ldh(f.mom, o);
-  if (m.z >= 4.0f) {
-    sth(out, o, make_float4(c.x, c.y, c.z, fmaxf(0.0f, m.y - m.x * m.x)));
+  float4 nd = make_float4(0.f, 0.f, 0.f, -1.0f), c = make_float4(0.f, 0.f, 0.f, 0.f), m = c;
+  if (in_img) {
+    nd = ldh(f.nd, y * f.p_nd + x);
+    c = ldh(f.tmp, o);
+    m = ldh(f.mom, o);
+  }
+  const bool sky = nd.w < 0.0f, spatial = !sky && !(m.z >= 4.0f);
+  if (!__syncthreads_or(spatial ? 1 : 0)) {
+    if (in_img)
+      sth(out, o, sky ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(c.x, c.y, c.z, fmaxf(0.0f, m.y - m.x * m.x)));
     return;
   }
+  for (int i = li; i < N; i += VT_NT) {
+    const int gx = bx - 3 + i % TC, gy = by - 3 + i / TC;
+    if (gx >= 0 && gy >= 0 && gx < f.W && gy < f.H) {
+      cp_async8(sN + i, f.nd + gy * f.p_nd + gx);
+      cp_async8(sC + i, f.tmp + gy * f.W + gx);
+      cp_async8(sM + i, f.mom + gy * f.W + gx);
+    } else {
+      sN[i] = make_uint2(0u, 0xbc000000u);  // depth -1: sky
+    }
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  if (!in_img) return;
+  if (!spatial) {
+    sth(out, o, sky ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(c.x, c.y, c.z, fmaxf(0.0f, m.y - m.x * m.x)));
+    return;
+  }
+  // log2(e) / (0.02 z dist + 1e-3) by |dx|, |dy| <= 3
+  float iz[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j <= i; j++) iz[i][j] = iz[j][i] = LOG2E * rcp1(0.02f * nd.w * sqrtf((float)(i * i + j * j)) + 1e-3f);
   float sw = 0.f, scx = 0.f, scy = 0.f, scz = 0.f, sm0 = 0.f, sm1 = 0.f;
+  const int t = (ty + 3) * TC + tx + 3;
+#pragma unroll
   for (int dy = -3; dy <= 3; dy++) {
+#pragma unroll
     for (int dx = -3; dx <= 3; dx++) {
-      const int qx = x + dx, qy = y + dy;
-      if (qx < 0 || qy < 0 || qx >= f.W || qy >= f.H) continue;
-      const float4 ndq = ldh(f.nd, qy * f.p_nd + qx);
+      const int q = t + dy * TC + dx;
+      const float4 ndq = h4_to_f4(sN[q]);
       if (ndq.w < 0.0f) continue;
-      const float dist = sqrtf((float)dx * (float)dx + (float)dy * (float)dy);
-      const float wz = expf(-fabsf(ndq.w - nd.w) / (0.02f * nd.w * dist + 1e-3f));
-      const float wn = powf(fmaxf(0.0f, dot3(ndq, nd)), f.sigma_n);
-      const float w = wz * wn;
-      const float4 cq = ldh(f.tmp, qy * f.W + qx), mq = ldh(f.mom, qy * f.W + qx);
+      const float dn = fmaxf(0.0f, dot3(ndq, nd));
+      float wn = dn;
+      if constexpr (N128) {
+#pragma unroll
+        for (int i = 0; i < 7; i++) wn *= wn;
+      } else {
+        wn = powf(dn, f.sigma_n);
+      }
+      const float w = wn * ex2_approx(-fabsf(ndq.w - nd.w) * iz[dy < 0 ? -dy : dy][dx < 0 ? -dx : dx]);
+      const float4 cq = h4_to_f4(sC[q]);
+      const float2 mq = unpack2(sM[q].x);
       sw += w;
       scx += w * cq.x; scy += w * cq.y; scz += w * cq.z;
       sm0 += w * mq.x; sm1 += w * mq.y;
@@ -168,16 +258,6 @@ HD_INL float2 svgf_wn2(float2 x, float sigma_n) {
     return sigma_n != 0.0f ? f2(__powf(x.x, sigma_n), __powf(x.y, sigma_n)) : f2(1.0f, 1.0f);
   }
 }
-HD_INL float hi_half(uint32_t u) { return __half2float(__ushort_as_half((uint16_t)(u >> 16))); }
-
-// 1 / x to within an ulp: the hardware approximation and one Newton step, without the range checks of an IEEE division
-// (x is a sum of weights or a positive bandwidth + epsilon here).
-HD_INL float rcp1(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return fmaf(fmaf(-x, r, 1.0f), r, r);
-}
-
 // A texel pair of the footprint: (nx, nx', ny, ny'), (nz, nz', z, z'), (r, r', g, g'), (b, b', v, v').
 struct TexelPair {
   float4 g0, g1, c0, c1;
@@ -400,57 +480,87 @@ HD_INL float3 svgf_remod(const SvgfFrame &f, const uint2 *il, int qx, int qy) {
   return make_float3(a.x * m.x + e.x, a.y * m.y + e.y, a.z * m.z + e.z);
 }
 
-__global__ void k_svgf_resolve(const SvgfFrame f, const uint2 *il) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= f.W || y >= f.H) return;
-  const int o = y * f.W + x;
-  const float3 cur = tmap(svgf_remod(f, il, x, y));
+// A 32 x 8 tile with an apron of one: each texel is remodulated, tone-mapped and converted to YCoCg once (a thread per
+// pixel did that for its nine neighbours, 27 texel loads and 27 divisions a pixel: 90 us at 1920 x 1080 where the tile
+// takes 39). The motion and the history's bilinear footprint are loaded before the tile barrier.
+HD_INL float3 svgf_tm(float3 c) { return Divisor(1.0f + lum3(c.x, c.y, c.z))(c); }
+HD_INL float3 svgf_itm(float3 c) { return Divisor(fmaxf(1.0f - lum3(c.x, c.y, c.z), 1e-4f))(c); }
+constexpr int RT_W = 32, RT_H = 8, RT_NT = RT_W * RT_H;
+__global__ void __launch_bounds__(RT_NT) k_svgf_resolve(const SvgfFrame f, const uint2 *il) {
+  constexpr int SW = RT_W + 2, SH = RT_H + 2, N = SW * SH;
+  __shared__ float sRgb[3][N], sY[3][N];
+  const int li = threadIdx.x, tx = li % RT_W, ty = li / RT_W;
+  const int x = blockIdx.x * RT_W + tx, y = blockIdx.y * RT_H + ty;
+  const bool in_img = x < f.W && y < f.H;
   if (!f.use_taa) {
-    const float3 r = itmap(cur);
-    sth(f.taa, o, make_float4(r.x, r.y, r.z, 1.0f));
+    if (!in_img) return;
+    const float3 r = svgf_itm(svgf_tm(svgf_remod(f, il, x, y)));
+    sth(f.taa, y * f.W + x, make_float4(r.x, r.y, r.z, 1.0f));
     return;
   }
+  const int cx = min(x, f.W - 1), cy = min(y, f.H - 1);
+  const float4 mv = ldh(f.mv, cy * f.p_mv + cx);
+  const float uvx = Divisor((float)f.W)((float)x + 0.5f + mv.x), uvy = Divisor((float)f.H)((float)y + 0.5f + mv.y);
+  const bool hist_in = uvx >= 0.0f && uvy >= 0.0f && uvx <= 1.0f && uvy <= 1.0f && !f.reset;
+  const float ppx = uvx * (float)f.W - 0.5f, ppy = uvy * (float)f.H - 0.5f;
+  const float bxf = floorf(ppx), byf = floorf(ppy);
+  uint2 hq[4] = {};
+  if (hist_in) {
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      hq[j] = __ldg(f.taa_prev + clampi((int)byf + (j >> 1), 0, f.H - 1) * f.W + clampi((int)bxf + (j & 1), 0, f.W - 1));
+  }
+  const int ox = blockIdx.x * RT_W - 1, oy = blockIdx.y * RT_H - 1;
+#pragma unroll
+  for (int u = 0; u < (N + RT_NT - 1) / RT_NT; u++) {
+    const int i = li + u * RT_NT;
+    if (i >= N) break;
+    const float3 c = svgf_tm(svgf_remod(f, il, ox + i % SW, oy + i / SW)), q = to_ycocg(c);
+    sRgb[0][i] = c.x; sRgb[1][i] = c.y; sRgb[2][i] = c.z;
+    sY[0][i] = q.x; sY[1][i] = q.y; sY[2][i] = q.z;
+  }
+  __syncthreads();
+  if (!in_img) return;
+  const int t = (ty + 1) * SW + tx + 1;
+  const float3 cur = make_float3(sRgb[0][t], sRgb[1][t], sRgb[2][t]);
   // E[c^2] - E[c]^2 cancels catastrophically when the neighbourhood is flat: its products are rounded separately
   // (no FMA contraction), as an unfused f32 shader computes them
   float3 m1 = make_float3(0.f, 0.f, 0.f), m2 = m1;
-  for (int dy = -1; dy <= 1; dy++)
-    for (int dx = -1; dx <= 1; dx++) {
-      const float3 c = to_ycocg(tmap(svgf_remod(f, il, x + dx, y + dy)));
-      m1.x += c.x; m1.y += c.y; m1.z += c.z;
-      m2.x = __fadd_rn(m2.x, __fmul_rn(c.x, c.x));
-      m2.y = __fadd_rn(m2.y, __fmul_rn(c.y, c.y));
-      m2.z = __fadd_rn(m2.z, __fmul_rn(c.z, c.z));
-    }
-  m1.x /= 9.0f; m1.y /= 9.0f; m1.z /= 9.0f;
-  m2.x /= 9.0f; m2.y /= 9.0f; m2.z /= 9.0f;
-  const float sdx = sqrtf(fmaxf(__fsub_rn(m2.x, __fmul_rn(m1.x, m1.x)), 0.0f)),
-              sdy = sqrtf(fmaxf(__fsub_rn(m2.y, __fmul_rn(m1.y, m1.y)), 0.0f)),
-              sdz = sqrtf(fmaxf(__fsub_rn(m2.z, __fmul_rn(m1.z, m1.z)), 0.0f));
-  const float4 mv = ldh(f.mv, y * f.p_mv + x);
-  const float uvx = ((float)x + 0.5f + mv.x) / (float)f.W, uvy = ((float)y + 0.5f + mv.y) / (float)f.H;
+#pragma unroll
+  for (int j = 0; j < 9; j++) {
+    const int q = t + (j / 3 - 1) * SW + j % 3 - 1;
+    const float3 c = make_float3(sY[0][q], sY[1][q], sY[2][q]);
+    m1.x += c.x; m1.y += c.y; m1.z += c.z;
+    m2.x = __fadd_rn(m2.x, __fmul_rn(c.x, c.x));
+    m2.y = __fadd_rn(m2.y, __fmul_rn(c.y, c.y));
+    m2.z = __fadd_rn(m2.z, __fmul_rn(c.z, c.z));
+  }
+  const Divisor nine(9.0f);
+  m1 = nine(m1);
+  m2 = nine(m2);
+  const float sdx = sqrt1(fmaxf(__fsub_rn(m2.x, __fmul_rn(m1.x, m1.x)), 0.0f)),
+              sdy = sqrt1(fmaxf(__fsub_rn(m2.y, __fmul_rn(m1.y, m1.y)), 0.0f)),
+              sdz = sqrt1(fmaxf(__fsub_rn(m2.z, __fmul_rn(m1.z, m1.z)), 0.0f));
   const float a = f.taa_alpha;
   float3 res = cur;
-  if (uvx >= 0.0f && uvy >= 0.0f && uvx <= 1.0f && uvy <= 1.0f && !f.reset) {
-    const float ppx = uvx * (float)f.W - 0.5f, ppy = uvy * (float)f.H - 0.5f;
-    const float bxf = floorf(ppx), byf = floorf(ppy);
+  if (hist_in) {
     const float fx = ppx - bxf, fy = ppy - byf;
     float3 hist = make_float3(0.f, 0.f, 0.f);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      const int ox = j & 1, oy = j >> 1;
-      const float wb = (ox == 1 ? fx : 1.0f - fx) * (oy == 1 ? fy : 1.0f - fy);
-      const float4 t = ldh(f.taa_prev, clampi((int)byf + oy, 0, f.H - 1) * f.W + clampi((int)bxf + ox, 0, f.W - 1));
-      hist.x += wb * t.x; hist.y += wb * t.y; hist.z += wb * t.z;
+      const float wb = ((j & 1) == 1 ? fx : 1.0f - fx) * ((j >> 1) == 1 ? fy : 1.0f - fy);
+      const float4 h = h4_to_f4(hq[j]);
+      hist.x += wb * h.x; hist.y += wb * h.y; hist.z += wb * h.z;
     }
-    float3 hh = to_ycocg(tmap(hist));
+    float3 hh = to_ycocg(svgf_tm(hist));
     hh.x = fminf(fmaxf(hh.x, m1.x - 1.25f * sdx), m1.x + 1.25f * sdx);
     hh.y = fminf(fmaxf(hh.y, m1.y - 1.25f * sdy), m1.y + 1.25f * sdy);
     hh.z = fminf(fmaxf(hh.z, m1.z - 1.25f * sdz), m1.z + 1.25f * sdz);
     const float3 h = from_ycocg(hh);
     res = make_float3(h.x * (1.0f - a) + cur.x * a, h.y * (1.0f - a) + cur.y * a, h.z * (1.0f - a) + cur.z * a);
   }
-  const float3 r = itmap(res);
-  sth(f.taa, o, make_float4(r.x, r.y, r.z, 1.0f));
+  const float3 r = svgf_itm(res);
+  sth(f.taa, y * f.W + x, make_float4(r.x, r.y, r.z, 1.0f));
 }
 
 thread_local std::string g_svgf_err;
@@ -568,9 +678,12 @@ extern "C" int svgf_encode(svgf_t *s, const svgf_inputs *in, void *stream, const
   f.p_rad = pt[0]; f.p_nd = pt[1]; f.p_mv = pt[2]; f.p_mat = pt[3]; f.p_emi = pt[4]; f.p_pnd = pt[5]; f.p_pmv = pt[6];
   f.hist_prev = s->hist[prev]; f.mom_prev = s->mom[prev]; f.taa_prev = s->taa[prev];
   f.tmp = s->tmp; f.mom = s->mom[cur]; f.hist = s->hist[cur]; f.taa = s->taa[cur];
-  const dim3 blk(8, 8), grd((s->W + 7) / 8, (s->H + 7) / 8);  // workgroup 8 x 8 (svgf.js:41)
+  const dim3 blk(32, 8), grd((s->W + 31) / 32, (s->H + 7) / 8);
+  const dim3 tgrd((s->W + RT_W - 1) / RT_W, (s->H + RT_H - 1) / RT_H);
   k_svgf_temporal<<<grd, blk, 0, st>>>(f);
-  k_svgf_variance<<<grd, blk, 0, st>>>(f, s->atrous[0]);
+  const dim3 vgrd((s->W + VT_W - 1) / VT_W, (s->H + VT_H - 1) / VT_H);
+  if (f.sigma_n == 128.0f) k_svgf_variance<true><<<vgrd, VT_NT, 0, st>>>(f, s->atrous[0]);
+  else k_svgf_variance<false><<<vgrd, VT_NT, 0, st>>>(f, s->atrous[0]);
   int src = 0;
   for (int i = 0; i < s->o.iterations; i++) {
     const uint2 *a = s->atrous[src];
@@ -586,7 +699,7 @@ extern "C" int svgf_encode(svgf_t *s, const svgf_inputs *in, void *stream, const
     if (e != cudaSuccess) return svgf_fail(s, HUSH_ERR_CUDA, std::string("SVGF: a-trous launch: ") + cudaGetErrorString(e));
     src ^= 1;
   }
-  k_svgf_resolve<<<grd, blk, 0, st>>>(f, s->atrous[src]);
+  k_svgf_resolve<<<tgrd, RT_NT, 0, st>>>(f, s->atrous[src]);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return svgf_fail(s, HUSH_ERR_CUDA, std::string("SVGF: kernel launch: ") + cudaGetErrorString(e));
   s->reset = false;
