@@ -72,12 +72,10 @@ HD_INL float4 f2_ac_tw(const uint4 *F2, int i) {
   const float2 a = unpack2(t.z), b = unpack2(t.w);
   return make_float4(a.x, a.y, b.x, b.y);
 }
-HD_INL void atomic_add4(float4 *p, float4 v) {
-  atomicAdd(&p->x, v.x);
-  atomicAdd(&p->y, v.y);
-  atomicAdd(&p->z, v.z);
-  atomicAdd(&p->w, v.w);
-}
+// One 16-byte vector reduction (each component added atomically by itself) in place of four scalar ones: the adjoints'
+// scatters are bound by the reductions the L2 takes.
+HD_INL void atomic_add4(float4 *p, float4 v) { atomicAdd(p, v); }
+HD_INL void atomic_add3(float4 *p, float x, float y, float z) { atomicAdd(p, make_float4(x, y, z, 0.0f)); }
 HD_INL float sgn(float x) { return x > 0.0f ? 1.0f : (x < 0.0f ? -1.0f : 0.0f); }
 
 // ------------------------------------------------------------------------------------------------ MLP
@@ -871,10 +869,7 @@ HD_INL void recomb_coarse_adj(const TwinFrame &T, int px, int py, float4 gp, flo
     const float4 cg = ldh(f.CG, q);
     if (cg.z < 0.0f) continue;
     const float k = beta * jbw(cposx - cbx, cposy - cby, j, oct_dec(cg.x, cg.y), cg.z, gp, gp.w) / swq;
-    float *d = &T.dC0[q].x;
-    atomicAdd(d, g2.x * k);
-    atomicAdd(d + 1, g2.y * k);
-    atomicAdd(d + 2, g2.z * k);
+    atomic_add3(T.dC0 + q, g2.x * k, g2.y * k, g2.z * k);
   }
 }
 
@@ -935,10 +930,8 @@ __global__ void __launch_bounds__(TW *TH) k_fine_bwd(const TwinFrame T, const fl
       for (int j = 0; j < 4; j++) {
         if (!R.vh[j]) continue;
         const float w = R.wh[j] / R.swh;
-        float *d = &T.dB3[R.qh[j]].x;  // the level's variance gets no gradient from the recombination
-        atomicAdd(d, gill.x * w);
-        atomicAdd(d + 1, gill.y * w);
-        atomicAdd(d + 2, gill.z * w);
+        // the level's variance gets no gradient from the recombination
+        atomic_add3(T.dB3 + R.qh[j], gill.x * w, gill.y * w, gill.z * w);
       }
     }
     float gv1 = 0.0f;  // the fine level's variance reaches X through nothing; only the history may seed it
@@ -1007,10 +1000,7 @@ __global__ void __launch_bounds__(TW *TH) k_fine_pyr_bwd(const TwinFrame T, cons
     for (int j = 0; j < 4; j++) {
       if (!R.vh[j]) continue;
       const float k = -p0.w * R.wh[j] / R.swh;
-      float *a = &T.dAh[R.qh[j]].x;
-      atomicAdd(a, gill.x * k);
-      atomicAdd(a + 1, gill.y * k);
-      atomicAdd(a + 2, gill.z * k);
+      atomic_add3(T.dAh + R.qh[j], gill.x * k, gill.y * k, gill.z * k);
     }
   }
 }
