@@ -18,6 +18,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstddef>
 #include <cstring>
@@ -45,7 +46,8 @@ struct TwinFrame {
   float4 *A1, *X, *out;   // full: fine level, pre-TAA colour, TAA output
   const float4 *out_prev; // full: previous frame's TAA output (temporal loss term)
   const float *clean, *clean_prev;  // full: noise-free rgb (f32, dense), previous frame's
-  float4 *gT;             // full: gradient w.r.t. the tone-mapped colour tm(X)
+  float4 *gT;             // full: the loss's gradient w.r.t. the TAA output (the per-pass pair)
+  float4 *rsave;          // full, 4 planes: the recombination's values for its adjoint (RSave), or NULL (not kept)
   float4 *dB1, *dB2, *dB3;  // half: level gradients
   const float4 *gA1;        // full: dL/d fine level through the colour history (the next frame's TEMPORAL), or NULL
   float4 *dA0;              // full: dL/d TEMPORAL's colour + variance A0 (the fine level's input), or NULL
@@ -511,60 +513,111 @@ __global__ void k_ah_to_a0(const TwinFrame T, const float4 *dah, float4 *dA0) {
 }
 
 // ------------------------------------------------------------------------------------------------ fine + final
+// The half- and quarter-resolution texels a 16 x 8 tile's recombination reads, decoded once per CTA: guides, block
+// means, mid level and coarse level (each was fetched and its guide decoded by the eight taps of every pixel: fine
+// forward at 256 x 256 8.5 -> 5.7 us; with the values it keeps for its adjoint, fine adjoint 8.7 -> 5.8 us).
+constexpr int RH_W = TW / 2 + 2, RH_H = TH / 2 + 2, RQ_W = TW / 4 + 2, RQ_H = TH / 4 + 2;
+struct RecombTile {
+  float4 hg[RH_W * RH_H], ha[RH_W * RH_H], hb[RH_W * RH_H], qg[RQ_W * RQ_H], qc[RQ_W * RQ_H];
+};
+static_assert(RH_W * RH_H <= 64 && RQ_W * RQ_H <= TW * TH - 64, "one texel per thread");
+HD_INL void recomb_stage(const TwinFrame &T, RecombTile &S, int li, int bx, int by) {
+  const HushFrame &f = T.f;
+  if (li < RH_W * RH_H) {
+    const int q = clampi(by / 2 - 1 + li / RH_W, 0, f.H2 - 1) * f.W2 + clampi(bx / 2 - 1 + li % RH_W, 0, f.W2 - 1);
+    S.hg[li] = f3_guide_tw(f.F3, q);
+    S.ha[li] = f2_ac_tw(f.F2, q);
+    S.hb[li] = T.B3[q];
+  } else if (li >= 64 && li < 64 + RQ_W * RQ_H) {
+    const int i = li - 64;
+    const int q = clampi(by / 4 - 1 + i / RQ_W, 0, f.H4 - 1) * f.W4 + clampi(bx / 4 - 1 + i % RQ_W, 0, f.W4 - 1);
+    const float4 cg = ldh(f.CG, q);
+    float4 g = oct_dec(cg.x, cg.y);
+    g.w = cg.z;
+    S.qg[i] = g;
+    S.qc[i] = ldh(f.C0, q);
+  }
+}
+
 struct Recomb {
-  float fx, fy, fz, swh, swq, uBx, uBy, uBz, uAx, uAy, uAz, uCx, uCy, uCz;
-  float wh[4], wqq[4];
-  int qh[4];
-  bool vh[4], vq[4];
+  float swh, swq, uBx, uBy, uBz, uAx, uAy, uAz, uCx, uCy, uCz;
+  float wh[4], wq[4];  // 0 for a tap outside the image or on sky
 };
 
-HD_INL void recomb_fwd(const TwinFrame &T, int px, int py, float4 A1, float4 gp, Recomb &R) {
-  const HushFrame &f = T.f;
-  R.fx = A1.x; R.fy = A1.y; R.fz = A1.z;
-  const float z = gp.w;
-  const int hsx = (f.W + 1) / 2, hsy = (f.H + 1) / 2;
-  const float hposx = ((float)px + 0.5f) / 2.0f - 0.5f, hposy = ((float)py + 0.5f) / 2.0f - 0.5f;
-  const float hbx = floorf(hposx), hby = floorf(hposy);
+// Texel (qx, qy) of tap j of the joint-bilinear footprint around pixel (px, py) at 1 / scale of its resolution.
+HD_INL int2 recomb_tap(int px, int py, float scale, int j, float &frx, float &fry) {
+  const float hx = ((float)px + 0.5f) / scale - 0.5f, hy = ((float)py + 0.5f) / scale - 0.5f;
+  const float bx = floorf(hx), by = floorf(hy);
+  frx = hx - bx;
+  fry = hy - by;
+  return make_int2((int)bx + (j & 1), (int)by + (j >> 1));
+}
+
+HD_INL void recomb_fwd(const HushFrame &f, const RecombTile &S, int px, int py, int bx, int by, float4 gp, Recomb &R) {
   R.uBx = R.uBy = R.uBz = R.uAx = R.uAy = R.uAz = R.swh = 0.f;
+#pragma unroll
   for (int j = 0; j < 4; j++) {
-    const int qx = (int)hbx + (j & 1), qy = (int)hby + (j >> 1);
-    R.vh[j] = false;
+    float frx, fry;
+    const int2 q = recomb_tap(px, py, 2.0f, j, frx, fry);
+    const int t = (q.y - (by / 2 - 1)) * RH_W + q.x - (bx / 2 - 1);
+    const float4 g = S.hg[t];
     R.wh[j] = 0.f;
-    R.qh[j] = 0;
-    if (qx < 0 || qy < 0 || qx >= hsx || qy >= hsy) continue;
-    const int q = qy * f.W2 + qx;
-    const float4 g = f3_guide_tw(f.F3, q);
-    if (g.w < 0.0f) continue;
-    const float w = jbw(hposx - hbx, hposy - hby, j, g, g.w, gp, z);
-    const float4 a = f2_ac_tw(f.F2, q), m = T.B3[q];
-    R.vh[j] = true;
+    if (q.x < 0 || q.y < 0 || q.x >= f.W2 || q.y >= f.H2 || g.w < 0.0f) continue;
+    const float w = jbw(frx, fry, j, g, g.w, gp, gp.w);
+    const float4 a = S.ha[t], m = S.hb[t];
     R.wh[j] = w;
-    R.qh[j] = q;
     R.swh += w;
     R.uBx += w * m.x; R.uBy += w * m.y; R.uBz += w * m.z;
     R.uAx += w * a.x; R.uAy += w * a.y; R.uAz += w * a.z;
   }
-  const int qsx = (f.W + 3) / 4, qsy = (f.H + 3) / 4;
-  const float cposx = ((float)px + 0.5f) / 4.0f - 0.5f, cposy = ((float)py + 0.5f) / 4.0f - 0.5f;
-  const float cbx = floorf(cposx), cby = floorf(cposy);
   R.uCx = R.uCy = R.uCz = R.swq = 0.f;
+#pragma unroll
   for (int j = 0; j < 4; j++) {
-    const int qx = (int)cbx + (j & 1), qy = (int)cby + (j >> 1);
-    if (qx < 0 || qy < 0 || qx >= qsx || qy >= qsy) continue;
-    const int q = qy * f.W4 + qx;
-    const float4 cg = ldh(f.CG, q);
-    if (cg.z < 0.0f) continue;
-    const float w = jbw(cposx - cbx, cposy - cby, j, oct_dec(cg.x, cg.y), cg.z, gp, z);
-    const float4 c = ldh(f.C0, q);
+    float frx, fry;
+    const int2 q = recomb_tap(px, py, 4.0f, j, frx, fry);
+    const int t = (q.y - (by / 4 - 1)) * RQ_W + q.x - (bx / 4 - 1);
+    const float4 g = S.qg[t];
+    R.wq[j] = 0.f;
+    if (q.x < 0 || q.y < 0 || q.x >= f.W4 || q.y >= f.H4 || g.w < 0.0f) continue;
+    const float w = jbw(frx, fry, j, g, g.w, gp, gp.w);
+    const float4 c = S.qc[t];
+    R.wq[j] = w;
     R.swq += w;
     R.uCx += w * c.x; R.uCy += w * c.y; R.uCz += w * c.z;
   }
+}
+
+// What the recombination's adjoint needs of a pixel's forward: f - uA / sum_h w (w: 1 where the mid level takes part),
+// up - ill (w: 1 where the coarse level does), and the taps' weights over their sums.
+struct RSave {
+  float4 mid, coarse, wh, wq;
+};
+// ill before the coarse level (i) from A1 and the sums; also the pixel's RSave.
+HD_INL RSave recomb_mix(const Recomb &R, float4 A1, float kappa, float &ix, float &iy, float &iz) {
+  RSave V;
+  ix = A1.x; iy = A1.y; iz = A1.z;
+  V.mid = V.coarse = V.wh = V.wq = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (R.swh > 1e-4f) {
+    V.mid = make_float4(A1.x - R.uAx / R.swh, A1.y - R.uAy / R.swh, A1.z - R.uAz / R.swh, 1.0f);
+    ix = R.uBx / R.swh + kappa * V.mid.x;
+    iy = R.uBy / R.swh + kappa * V.mid.y;
+    iz = R.uBz / R.swh + kappa * V.mid.z;
+    V.wh = make_float4(R.wh[0] / R.swh, R.wh[1] / R.swh, R.wh[2] / R.swh, R.wh[3] / R.swh);
+  }
+  float upx = ix, upy = iy, upz = iz;
+  if (R.swq > 1e-4f) { upx = R.uCx / R.swq; upy = R.uCy / R.swq; upz = R.uCz / R.swq; }
+  V.coarse = make_float4(upx - ix, upy - iy, upz - iz, R.swq > 1e-4f ? 1.0f : 0.0f);
+  if (R.swq > 1e-4f) {
+    V.wq = make_float4(R.wq[0] / R.swq, R.wq[1] / R.swq, R.wq[2] / R.swq, R.wq[3] / R.swq);
+  }
+  return V;
 }
 
 // fine level (A1, also the colour history) and recombination -> X
 __global__ void __launch_bounds__(TW *TH) k_fine_fwd(const TwinFrame T) {
   constexpr int AP = 1, SW = TW + 2, SH = TH + 2;
   __shared__ float4 sA[SW * SH], sG[SW * SH];
+  __shared__ RecombTile S;
   const HushFrame &f = T.f;
   const int li = threadIdx.y * TW + threadIdx.x;
   const int bx = blockIdx.x * TW, by = blockIdx.y * TH;
@@ -576,6 +629,7 @@ __global__ void __launch_bounds__(TW *TH) k_fine_fwd(const TwinFrame T) {
     g.w = k.z;
     sG[i] = g;
   }
+  recomb_stage(T, S, li, bx, by);
   __syncthreads();
   const int px = bx + threadIdx.x, py = by + threadIdx.y;
   if (px >= f.W || py >= f.H) return;
@@ -596,19 +650,20 @@ __global__ void __launch_bounds__(TW *TH) k_fine_fwd(const TwinFrame T) {
   T.A1[o] = A1;
   sth(f.hist, o, A1);
   Recomb R;
-  recomb_fwd(T, px, py, A1, gp, R);
-  float ix = R.fx, iy = R.fy, iz = R.fz;
-  if (R.swh > 1e-4f) {
-    ix = R.uBx / R.swh + p0.w * (R.fx - R.uAx / R.swh);
-    iy = R.uBy / R.swh + p0.w * (R.fy - R.uAy / R.swh);
-    iz = R.uBz / R.swh + p0.w * (R.fz - R.uAz / R.swh);
-  }
-  float upx = ix, upy = iy, upz = iz;
-  if (R.swq > 1e-4f) { upx = R.uCx / R.swq; upy = R.uCy / R.swq; upz = R.uCz / R.swq; }
-  ix = ix + (upx - ix) * p0.z;
-  iy = iy + (upy - iy) * p0.z;
-  iz = iz + (upz - iz) * p0.z;
+  recomb_fwd(f, S, px, py, bx, by, gp, R);
+  float ix, iy, iz;
+  const RSave V = recomb_mix(R, A1, p0.w, ix, iy, iz);
+  ix = ix + V.coarse.x * p0.z;
+  iy = iy + V.coarse.y * p0.z;
+  iz = iz + V.coarse.z * p0.z;
   T.X[o] = make_float4(ix * alb.x + emi.x, iy * alb.y + emi.y, iz * alb.z + emi.z, 0.0f);
+  if (T.rsave) {
+    const size_t n = (size_t)f.W * f.H;
+    T.rsave[o] = V.mid;
+    T.rsave[n + o] = V.coarse;
+    T.rsave[2 * n + o] = V.wh;
+    T.rsave[3 * n + o] = V.wq;
+  }
 }
 
 // ------------------------------------------------------------------------------------------------ TAA
@@ -616,20 +671,18 @@ HD_INL float3 tm3(float4 c) { return tmap(make_float3(c.x, c.y, c.z)); }
 
 struct TaaF {
   float3 y[9], m1, sd, v3, cur, hh0, hh, hr, res, out;
-  int q[9];
   bool inside, lo_act[3], hi_act[3], act_itm;
   float d;
 };
 
-HD_INL void taa_fwd(const TwinFrame &T, int px, int py, TaaF &A) {
+// y(j): the YCoCg colour of the j-th texel of the clamped 3 x 3 window
+template <class Window>
+HD_INL void taa_fwd(const TwinFrame &T, int px, int py, TaaF &A, const Window &y) {
   const HushFrame &f = T.f;
   const int o = py * f.W + px;
   A.cur = tm3(T.X[o]);
   A.inside = false;
-  for (int j = 0; j < 9; j++) {
-    A.q[j] = clampi(py + j / 3 - 1, 0, f.H - 1) * f.W + clampi(px + j % 3 - 1, 0, f.W - 1);
-    A.y[j] = to_ycocg(tm3(T.X[A.q[j]]));
-  }
+  for (int j = 0; j < 9; j++) A.y[j] = y(j);
   A.res = A.cur;
   for (int c = 0; c < 3; c++) A.lo_act[c] = A.hi_act[c] = false;
   if (!f.reset) {
@@ -681,15 +734,12 @@ HD_INL void taa_fwd(const TwinFrame &T, int px, int py, TaaF &A) {
   A.out = make_float3(A.res.x / A.d, A.res.y / A.d, A.res.z / A.d);
 }
 
-__global__ void k_taa_fwd(const TwinFrame T) {
+// The YCoCg tile of a 16 x 8 CTA, apron 1 (clamped), each texel tone-mapped once.
+constexpr int TY_W = TW + 2, TY_N = TY_W * (TH + 2);
+HD_INL void taa_stage(const TwinFrame &T, float3 *sY, int li, int bx, int by) {
   const HushFrame &f = T.f;
-  const int px = blockIdx.x * blockDim.x + threadIdx.x, py = blockIdx.y * blockDim.y + threadIdx.y;
-  if (px >= f.W || py >= f.H) return;
-  TaaF A;
-  taa_fwd(T, px, py, A);
-  const int o = py * f.W + px;
-  T.out[o] = make_float4(A.out.x, A.out.y, A.out.z, 1.0f);
-  sth(f.taa, o, make_float4(A.out.x, A.out.y, A.out.z, 1.0f));
+  for (int i = li; i < TY_N; i += TW * TH)
+    sY[i] = to_ycocg(tm3(T.X[clampi(by - 1 + i / TY_W, 0, f.H - 1) * f.W + clampi(bx - 1 + i % TY_W, 0, f.W - 1)]));
 }
 
 // ------------------------------------------------------------------------------------------------ loss
@@ -697,42 +747,57 @@ __global__ void k_taa_fwd(const TwinFrame T) {
 // (|clean| + 1e-2), 1), d = difference to the previous frame. The clip at 1 keeps the TAA's itm singularity (outputs
 // up to 1e4 where the clipped history reaches luminance 1, hush.js:636) from dominating the gradient. Writes dL/dout (into gT, as the seed of the TAA adjoint) and per-CTA FP64
 // partial sums.
-__global__ void k_loss(const TwinFrame T, int backward) {
-  const HushFrame &f = T.f;
+// One pixel's loss (times 3N) and dL/dout (times 3N) for the TAA output o.
+HD_INL double loss_pixel(const TwinFrame &T, int i, float3 o, float3 &g) {
+  const float ov[3] = {o.x, o.y, o.z};
+  float gv[3];
+  float4 op = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (T.has_prev) op = T.out_prev[i];
+  const float opv[3] = {op.x, op.y, op.z};
+  double l = 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const float cl = T.clean[3 * i + c], den = fabsf(cl) + 1e-2f;
+    const double rden = 1.0 / (double)den;
+    const float d = ov[c] - cl;
+    const double e = fabs((double)d) * rden;
+    l += e < 1.0 ? e : 1.0;
+    gv[c] = e < 1.0 ? sgn(d) / den : 0.0f;
+    if (T.has_prev) {
+      const float dd = (ov[c] - opv[c]) - (cl - T.clean_prev[3 * i + c]);
+      const double et = fabs((double)dd) * rden;
+      l += (double)T.lambda_t * (et < 1.0 ? et : 1.0);
+      gv[c] += et < 1.0 ? T.lambda_t * sgn(dd) / den : 0.0f;
+    }
+  }
+  g = make_float3(gv[0], gv[1], gv[2]);
+  return l;
+}
+
+// Sum of the CTA's l (FP64, at most 8 warps of a full CTA) into *out.
+HD_INL void block_sum_f64(double l, double *out) {
+  const int li = threadIdx.y * blockDim.x + threadIdx.x, nw = (blockDim.x * blockDim.y) >> 5;
+  for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
+  __shared__ double ws[8];
+  if ((li & 31) == 0) ws[li >> 5] = l;
+  __syncthreads();
+  if (li == 0) {
+    double v = 0.0;
+    for (int k = 0; k < nw; k++) v += ws[k];
+    *out = v;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_loss(const TwinFrame T, int backward) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double l = 0.0;
-  if (i < f.W * f.H) {
+  if (i < T.f.W * T.f.H) {
     const float4 o = T.out[i];
-    const float ov[3] = {o.x, o.y, o.z};
-    float g[3] = {0.f, 0.f, 0.f};
-    for (int c = 0; c < 3; c++) {
-      const float cl = T.clean[3 * i + c], den = fabsf(cl) + 1e-2f;
-      const float d = ov[c] - cl;
-      const double e = fabs((double)d) / den;
-      l += e < 1.0 ? e : 1.0;
-      g[c] = e < 1.0 ? sgn(d) / den : 0.0f;
-      if (T.has_prev) {
-        const float4 op = T.out_prev[i];
-        const float opv[3] = {op.x, op.y, op.z};
-        const float dd = (ov[c] - opv[c]) - (cl - T.clean_prev[3 * i + c]);
-        const double et = fabs((double)dd) / den;
-        l += (double)T.lambda_t * (et < 1.0 ? et : 1.0);
-        g[c] += et < 1.0 ? T.lambda_t * sgn(dd) / den : 0.0f;
-      }
-    }
-    l *= T.inv_n;
-    if (backward) T.gT[i] = make_float4(g[0] * T.inv_n, g[1] * T.inv_n, g[2] * T.inv_n, 0.f);
+    float3 g;
+    l = loss_pixel(T, i, make_float3(o.x, o.y, o.z), g) * T.inv_n;
+    if (backward) T.gT[i] = make_float4(g.x * T.inv_n, g.y * T.inv_n, g.z * T.inv_n, 0.f);
   }
-  // block reduction in FP64
-  for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
-  __shared__ double ws[32];
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = l;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double v = threadIdx.x < (blockDim.x >> 5) ? ws[threadIdx.x] : 0.0;
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    if (threadIdx.x == 0) T.loss_partials[blockIdx.x] = v;
-  }
+  block_sum_f64(l, T.loss_partials + blockIdx.x);
 }
 
 __global__ void k_reduce_f64(const double *partials, int n, double *out, double *acc) {
@@ -777,19 +842,15 @@ HD_INL float3 ycocg_adjoint(float3 g) {  // transpose of to_ycocg
   return make_float3(0.25f * g.x + 0.5f * g.y - 0.25f * g.z, 0.5f * g.x + 0.5f * g.z, 0.25f * g.x - 0.5f * g.y - 0.25f * g.z);
 }
 
-// coef[3p .. 3p + 2] = (gm, gcur.x), (gs, gcur.y), (m1, gcur.z)
-__global__ void k_taa_bwd_coef(const TwinFrame T, const float4 *gout, float4 *coef) {
-  const HushFrame &f = T.f;
-  const int px = blockIdx.x * blockDim.x + threadIdx.x, py = blockIdx.y * blockDim.y + threadIdx.y;
-  if (px >= f.W || py >= f.H) return;
-  const int o = py * f.W + px;
-  TaaF A;
-  taa_fwd(T, px, py, A);
-  const float4 go = gout[o];
-  const float3 gres = itm_adjoint(A, make_float3(go.x, go.y, go.z));
+// The adjoint's coefficients of one pixel from its TAA forward and dL/dout:
+// coef[3p .. 3p + 2] = (gm / 9, gcur.x), (2 gs / 9, gcur.y), (m1, gcur.z)
+HD_INL void taa_coef(const TaaF &A, float3 gout, float4 *coef) {
+  const float3 gres = itm_adjoint(A, gout);
   float3 gcur = gres;
   float gm[3] = {0.f, 0.f, 0.f}, gs[3] = {0.f, 0.f, 0.f};
+  float3 m1 = make_float3(0.f, 0.f, 0.f);
   if (A.inside) {
+    m1 = A.m1;
     gcur = make_float3(0.1f * gres.x, 0.1f * gres.y, 0.1f * gres.z);
     const float3 ghr = make_float3(0.9f * gres.x, 0.9f * gres.y, 0.9f * gres.z);
     // from_ycocg transpose
@@ -797,14 +858,59 @@ __global__ void k_taa_bwd_coef(const TwinFrame T, const float4 *gout, float4 *co
     const float v3[3] = {A.v3.x, A.v3.y, A.v3.z}, sd[3] = {A.sd.x, A.sd.y, A.sd.z};
     for (int c = 0; c < 3; c++) {
       const float glo = A.lo_act[c] ? gh[c] : 0.0f, ghi = A.hi_act[c] ? gh[c] : 0.0f;
-      gm[c] = glo + ghi;
+      gm[c] = (glo + ghi) / 9.0f;
       gs[c] = 1.25f * (ghi - glo);
-      gs[c] = v3[c] > 1e-12f ? gs[c] / (2.0f * sd[c]) : 0.0f;  // d sd / d v3
+      gs[c] = v3[c] > 1e-12f ? gs[c] / (9.0f * sd[c]) : 0.0f;  // 2 / 9 d sd / d v3
     }
   }
-  coef[3 * o] = make_float4(gm[0], gm[1], gm[2], gcur.x);
-  coef[3 * o + 1] = make_float4(gs[0], gs[1], gs[2], gcur.y);
-  coef[3 * o + 2] = make_float4(A.m1.x, A.m1.y, A.m1.z, gcur.z);
+  coef[0] = make_float4(gm[0], gm[1], gm[2], gcur.x);
+  coef[1] = make_float4(gs[0], gs[1], gs[2], gcur.y);
+  coef[2] = make_float4(m1.x, m1.y, m1.z, gcur.z);
+}
+
+__global__ void __launch_bounds__(TW *TH) k_taa_bwd_coef(const TwinFrame T, const float4 *gout, float4 *coef) {
+  __shared__ float3 sY[TY_N];
+  const HushFrame &f = T.f;
+  taa_stage(T, sY, threadIdx.y * TW + threadIdx.x, blockIdx.x * TW, blockIdx.y * TH);
+  __syncthreads();
+  const int px = blockIdx.x * TW + threadIdx.x, py = blockIdx.y * TH + threadIdx.y;
+  if (px >= f.W || py >= f.H) return;
+  const int o = py * f.W + px, t = (threadIdx.y + 1) * TY_W + threadIdx.x + 1;
+  TaaF A;
+  taa_fwd(T, px, py, A, [&](int j) { return sY[t + (j / 3 - 1) * TY_W + j % 3 - 1]; });
+  const float4 go = gout[o];
+  taa_coef(A, make_float3(go.x, go.y, go.z), coef + 3 * o);
+}
+
+// TAA's forward and, in the fused frame, the loss (TAA_LOSS) and the TAA adjoint's coefficients with it (TAA_ADJ): the
+// loss and its gradient are local to a pixel, so the window and the clip box are formed once instead of by three
+// kernels (3.3 + 4.0 + 4.2 -> 5.5 us at 256 x 256). The mode is an argument, so that the per-pass forward runs the very
+// instructions of the frame's.
+enum { TAA_FWD = 0, TAA_LOSS = 1, TAA_ADJ = 2 };
+__global__ void __launch_bounds__(TW *TH) k_taa(const TwinFrame T, int mode, float4 *coef) {
+  __shared__ float3 sY[TY_N];
+  const HushFrame &f = T.f;
+  taa_stage(T, sY, threadIdx.y * TW + threadIdx.x, blockIdx.x * TW, blockIdx.y * TH);
+  __syncthreads();
+  const int px = blockIdx.x * TW + threadIdx.x, py = blockIdx.y * TH + threadIdx.y;
+  double l = 0.0;
+  if (px < f.W && py < f.H) {
+    const int o = py * f.W + px, t = (threadIdx.y + 1) * TY_W + threadIdx.x + 1;
+    TaaF A;
+    taa_fwd(T, px, py, A, [&](int j) { return sY[t + (j / 3 - 1) * TY_W + j % 3 - 1]; });
+    T.out[o] = make_float4(A.out.x, A.out.y, A.out.z, 1.0f);
+    sth(f.taa, o, make_float4(A.out.x, A.out.y, A.out.z, 1.0f));
+    if (mode != TAA_FWD) {
+      float3 g;
+      l = loss_pixel(T, o, A.out, g) * T.inv_n;
+      if (mode == TAA_ADJ) {
+        g = make_float3(g.x * T.inv_n, g.y * T.inv_n, g.z * T.inv_n);
+        T.gT[o] = make_float4(g.x, g.y, g.z, 0.f);
+        taa_coef(A, g, coef + 3 * o);
+      }
+    }
+  }
+  if (mode != TAA_FWD) block_sum_f64(l, T.loss_partials + blockIdx.y * gridDim.x + blockIdx.x);
 }
 
 // how many of the clamped offsets p + d (d = -1, 0, 1) land on q
@@ -812,36 +918,44 @@ HD_INL int window_hits(int p, int q, int n) {
   return (clampi(p - 1, 0, n - 1) == q) + (p == q) + (clampi(p + 1, 0, n - 1) == q);
 }
 
-// gT[q] = dL/d tm(X_q) (set, not added)
-__global__ void k_taa_bwd_gather(const TwinFrame T, const float4 *coef, float4 *gT) {
+// g[q] = dL/d tm(X_q), or with TO_X dL/dX_q (the fused frame) (set, not added). ycocg_adjoint is linear: applied once.
+template <bool TO_X>
+__global__ void __launch_bounds__(TW *TH) k_taa_bwd_gather(const TwinFrame T, const float4 *coef, float4 *g) {
   const HushFrame &f = T.f;
   const int qx = blockIdx.x * blockDim.x + threadIdx.x, qy = blockIdx.y * blockDim.y + threadIdx.y;
   if (qx >= f.W || qy >= f.H) return;
   const int o = qy * f.W + qx;
-  const float3 y = to_ycocg(tm3(T.X[o]));
-  float gx = coef[3 * o].w, gyy = coef[3 * o + 1].w, gz = coef[3 * o + 2].w;
-  for (int py = max(qy - 1, 0); py <= min(qy + 1, f.H - 1); py++) {
-    const int my = window_hits(py, qy, f.H);
-    if (!my) continue;
-    for (int px = max(qx - 1, 0); px <= min(qx + 1, f.W - 1); px++) {
-      const int m = my * window_hits(px, qx, f.W);
-      if (!m) continue;
-      const int p = py * f.W + px;
-      const float4 a = coef[3 * p], b = coef[3 * p + 1], c = coef[3 * p + 2];
-      float3 g;
-      g.x = a.x / 9.0f + b.x * 2.0f * (y.x - c.x) / 9.0f;
-      g.y = a.y / 9.0f + b.y * 2.0f * (y.y - c.y) / 9.0f;
-      g.z = a.z / 9.0f + b.z * 2.0f * (y.z - c.z) / 9.0f;
-      const float3 t = ycocg_adjoint(g);
-      const float k = (float)m;
-      gx += k * t.x; gyy += k * t.y; gz += k * t.z;
-    }
+  const float4 X = T.X[o];
+  const float3 y = to_ycocg(tm3(X));
+  float3 s = make_float3(0.f, 0.f, 0.f);
+  auto add = [&](int p, float k) {
+    const float4 a = coef[3 * p], b = coef[3 * p + 1], c = coef[3 * p + 2];
+    s.x += k * (a.x + b.x * (y.x - c.x));
+    s.y += k * (a.y + b.y * (y.y - c.y));
+    s.z += k * (a.z + b.z * (y.z - c.z));
+  };
+  if (qx > 0 && qy > 0 && qx + 1 < f.W && qy + 1 < f.H) {  // every window that holds it holds it once
+#pragma unroll
+    for (int j = 0; j < 9; j++) add(o + (j / 3 - 1) * f.W + j % 3 - 1, 1.0f);
+  } else {
+    for (int py = max(qy - 1, 0); py <= min(qy + 1, f.H - 1); py++)
+      for (int px = max(qx - 1, 0); px <= min(qx + 1, f.W - 1); px++) {
+        const int m = window_hits(py, qy, f.H) * window_hits(px, qx, f.W);
+        if (m) add(py * f.W + px, (float)m);
+      }
   }
-  gT[o] = make_float4(gx, gyy, gz, 0.f);
+  const float3 t = ycocg_adjoint(s);
+  const float4 r = make_float4(coef[3 * o].w + t.x, coef[3 * o + 1].w + t.y, coef[3 * o + 2].w + t.z, 0.f);
+  if constexpr (TO_X) {
+    const float3 d = tm_adjoint(X, r);
+    g[o] = make_float4(d.x, d.y, d.z, 0.f);
+  } else {
+    g[o] = r;
+  }
 }
 
 // dX += tm adjoint of the tone-mapped-colour gradient at every pixel (the per-pass TAA adjoint's second step; the fused
-// frame folds it into k_fine_bwd, where sky pixels need no dX).
+// frame's gather applies it itself).
 __global__ void k_tm_bwd(const TwinFrame T, const float4 *gtm, float4 *dX) {
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= T.f.W * T.f.H) return;
@@ -850,31 +964,11 @@ __global__ void k_tm_bwd(const TwinFrame T, const float4 *gtm, float4 *dX) {
   dX[o] = make_float4(d.x + g.x, d.y + g.y, d.z + g.z, d.w);
 }
 
-// Pass 2 (per full pixel): dL/dX from the tm gradient; then recombination, fine-level parameter and mid-level input
-// gradients.
-// SEED_TM: the seed is the gradient w.r.t. the tone-mapped colour tm(X) (the fused frame); else w.r.t. X itself (the
-// per-pass pair, whose TAA adjoint has already applied the tm adjoint).
-// dL/dC0 of the recombination's coarse term (window sweep only): up = sum w C0 / sum w, ill2 = ill + (up - ill) beta,
-// so each quarter-res tap's colour gets g2 beta w / sum w (its variance none). The taps' weights are recomputed as
-// recomb_fwd() forms them, so the per-frame adjoint keeps no per-tap state.
-HD_INL void recomb_coarse_adj(const TwinFrame &T, int px, int py, float4 gp, float swq, float beta, float3 g2) {
-  const HushFrame &f = T.f;
-  const int qsx = (f.W + 3) / 4, qsy = (f.H + 3) / 4;
-  const float cposx = ((float)px + 0.5f) / 4.0f - 0.5f, cposy = ((float)py + 0.5f) / 4.0f - 0.5f;
-  const float cbx = floorf(cposx), cby = floorf(cposy);
-  for (int j = 0; j < 4; j++) {
-    const int qx = (int)cbx + (j & 1), qy = (int)cby + (j >> 1);
-    if (qx < 0 || qy < 0 || qx >= qsx || qy >= qsy) continue;
-    const int q = qy * f.W4 + qx;
-    const float4 cg = ldh(f.CG, q);
-    if (cg.z < 0.0f) continue;
-    const float k = beta * jbw(cposx - cbx, cposy - cby, j, oct_dec(cg.x, cg.y), cg.z, gp, gp.w) / swq;
-    atomic_add3(T.dC0 + q, g2.x * k, g2.y * k, g2.z * k);
-  }
-}
-
-template <bool SEED_TM>
-__global__ void __launch_bounds__(TW *TH) k_fine_bwd(const TwinFrame T, const float4 *gT) {
+// From dL/dX (gX): the recombination's adjoint, the fine level's parameter gradients and the mid level's input gradient.
+// SAVED: the recombination's forward values come from T.rsave (the fused frame, whose forward kernel has just
+// written them); else they are recomputed (the per-pass pair, which needs only the pass's inputs).
+template <bool SAVED>
+__global__ void __launch_bounds__(TW *TH) k_fine_bwd(const TwinFrame T, const float4 *gXp) {
   constexpr int AP = 1, SW = TW + 2, SH = TH + 2;
   __shared__ float4 sA[SW * SH], sG[SW * SH];
   const HushFrame &f = T.f;
@@ -888,6 +982,8 @@ __global__ void __launch_bounds__(TW *TH) k_fine_bwd(const TwinFrame T, const fl
     g.w = k.z;
     sG[i] = g;
   }
+  __shared__ RecombTile S;
+  if constexpr (!SAVED) recomb_stage(T, S, li, bx, by);
   __syncthreads();
   const int px = bx + threadIdx.x, py = by + threadIdx.y;
   const bool in = px < f.W && py < f.H;
@@ -897,41 +993,41 @@ __global__ void __launch_bounds__(TW *TH) k_fine_bwd(const TwinFrame T, const fl
   const float4 gp = sG[ti];
   if (in && gp.w >= 0.0f) {  // sky: X = emission, no dependence on the parameters
     const int o = py * f.W + px;
-    const float4 gt = gT[o];
-    const float3 gX = SEED_TM ? tm_adjoint(T.X[o], gt) : make_float3(gt.x, gt.y, gt.z);
+    const float4 gX = gXp[o];
     const float4 alb = ldh(f.mat, py * f.p_mat + px);
     const float4 p0 = T.par[3 * hp], p1 = T.par[3 * hp + 1], p2 = T.par[3 * hp + 2];
     Filt1<1, true, SW> F;
     F.run(sA, sG, ti, px, py, f.W, f.H, p1.x, p2.x);
-    const float4 A1 = F.out();
-    Recomb R;
-    recomb_fwd(T, px, py, A1, gp, R);
-    float ix = R.fx, iy = R.fy, iz = R.fz;
-    const bool mid = R.swh > 1e-4f;
-    if (mid) {
-      ix = R.uBx / R.swh + p0.w * (R.fx - R.uAx / R.swh);
-      iy = R.uBy / R.swh + p0.w * (R.fy - R.uAy / R.swh);
-      iz = R.uBz / R.swh + p0.w * (R.fz - R.uAz / R.swh);
+    RSave V;
+    if constexpr (SAVED) {
+      const size_t n = (size_t)f.W * f.H;
+      V.mid = T.rsave[o]; V.coarse = T.rsave[n + o]; V.wh = T.rsave[2 * n + o];
+    } else {
+      Recomb R;
+      recomb_fwd(f, S, px, py, bx, by, gp, R);
+      float ix, iy, iz;
+      V = recomb_mix(R, F.out(), p0.w, ix, iy, iz);
     }
     // X = ill2 * alb + emi, ill2 = ill + (up - ill) beta
     const float3 g2 = make_float3(gX.x * alb.x, gX.y * alb.y, gX.z * alb.z);
     float3 gill = g2;
     float gbeta = 0.0f;
-    if (R.swq > 1e-4f) {
-      const float upx = R.uCx / R.swq, upy = R.uCy / R.swq, upz = R.uCz / R.swq;
-      gbeta = g2.x * (upx - ix) + g2.y * (upy - iy) + g2.z * (upz - iz);
+    if (V.coarse.w != 0.0f) {
+      gbeta = g2.x * V.coarse.x + g2.y * V.coarse.y + g2.z * V.coarse.z;
       gill = make_float3(g2.x * (1.0f - p0.z), g2.y * (1.0f - p0.z), g2.z * (1.0f - p0.z));
     }
     float3 gf = gill;
     float gkappa = 0.0f;
-    if (mid) {
-      gkappa = gill.x * (R.fx - R.uAx / R.swh) + gill.y * (R.fy - R.uAy / R.swh) + gill.z * (R.fz - R.uAz / R.swh);
+    if (V.mid.w != 0.0f) {
+      gkappa = gill.x * V.mid.x + gill.y * V.mid.y + gill.z * V.mid.z;
       gf = make_float3(gill.x * p0.w, gill.y * p0.w, gill.z * p0.w);
+      const float wh[4] = {V.wh.x, V.wh.y, V.wh.z, V.wh.w};
+#pragma unroll
       for (int j = 0; j < 4; j++) {
-        if (!R.vh[j]) continue;
-        const float w = R.wh[j] / R.swh;
+        float frx, fry;
+        const int2 q = recomb_tap(px, py, 2.0f, j, frx, fry);
         // the level's variance gets no gradient from the recombination
-        atomic_add3(T.dB3 + R.qh[j], gill.x * w, gill.y * w, gill.z * w);
+        if (wh[j] != 0.0f) atomic_add3(T.dB3 + q.y * f.W2 + q.x, gill.x * wh[j], gill.y * wh[j], gill.z * wh[j]);
       }
     }
     float gv1 = 0.0f;  // the fine level's variance reaches X through nothing; only the history may seed it
@@ -972,35 +1068,37 @@ __global__ void __launch_bounds__(TW *TH) k_fine_bwd(const TwinFrame T, const fl
 // The recombination's adjoint into the block means and the coarse level (window sweep only; k_fine_bwd does the
 // rest): ill = uB / sum_h w + kappa (f - uA / sum_h w) and ill2 = ill + (up - ill) beta, up = sum_q w C0 / sum_q w, so
 // each half-res tap's block-mean colour gets -kappa w / sum_h w dL/d ill and each quarter-res tap's colour
-// beta w / sum_q w dL/d ill2 (X = ill2 albedo + emission). The tap weights do not depend on the levels, so nothing
-// of the fine level is recomputed.
-template <bool SEED_TM>
-__global__ void __launch_bounds__(TW *TH) k_fine_pyr_bwd(const TwinFrame T, const float4 *gT) {
+// beta w / sum_q w dL/d ill2 (X = ill2 albedo + emission). The normalised tap weights come from T.rsave.
+__global__ void __launch_bounds__(TW *TH) k_fine_pyr_bwd(const TwinFrame T, const float4 *gXp) {
   const HushFrame &f = T.f;
   const int px = blockIdx.x * TW + threadIdx.x, py = blockIdx.y * TH + threadIdx.y;
   if (px >= f.W || py >= f.H) return;
   const int o = py * f.W + px;
-  const float4 key = ldh(f.key, o);
-  if (key.z < 0.0f) return;  // sky: X = emission
-  float4 gp = oct_dec(key.x, key.y);
-  gp.w = key.z;
-  const int hp = (py >> 1) * f.W2 + (px >> 1);
-  const float4 gt = gT[o];
-  const float3 gX = SEED_TM ? tm_adjoint(T.X[o], gt) : make_float3(gt.x, gt.y, gt.z);
-  const float4 alb = ldh(f.mat, py * f.p_mat + px), p0 = T.par[3 * hp];
+  if (ldh(f.key, o).z < 0.0f) return;  // sky: X = emission
+  const size_t n = (size_t)f.W * f.H;
+  const float4 gX = gXp[o], alb = ldh(f.mat, py * f.p_mat + px), p0 = T.par[3 * ((py >> 1) * f.W2 + (px >> 1))];
+  const float4 wh4 = T.rsave[2 * n + o], wq4 = T.rsave[3 * n + o];
+  const bool mid = T.rsave[o].w != 0.0f, coarse = T.rsave[n + o].w != 0.0f;
   const float3 g2 = make_float3(gX.x * alb.x, gX.y * alb.y, gX.z * alb.z);
-  Recomb R;
-  recomb_fwd(T, px, py, make_float4(0.f, 0.f, 0.f, 0.f), gp, R);
   float3 gill = g2;
-  if (R.swq > 1e-4f) {
+  float frx, fry;
+  if (coarse) {
     gill = make_float3(g2.x * (1.0f - p0.z), g2.y * (1.0f - p0.z), g2.z * (1.0f - p0.z));
-    recomb_coarse_adj(T, px, py, gp, R.swq, p0.z, g2);
-  }
-  if (R.swh > 1e-4f) {
+    const float wq[4] = {wq4.x, wq4.y, wq4.z, wq4.w};
+#pragma unroll
     for (int j = 0; j < 4; j++) {
-      if (!R.vh[j]) continue;
-      const float k = -p0.w * R.wh[j] / R.swh;
-      atomic_add3(T.dAh + R.qh[j], gill.x * k, gill.y * k, gill.z * k);
+      const int2 q = recomb_tap(px, py, 4.0f, j, frx, fry);
+      const float k = p0.z * wq[j];
+      if (wq[j] != 0.0f) atomic_add3(T.dC0 + q.y * f.W4 + q.x, g2.x * k, g2.y * k, g2.z * k);
+    }
+  }
+  if (mid) {
+    const float wh[4] = {wh4.x, wh4.y, wh4.z, wh4.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int2 q = recomb_tap(px, py, 2.0f, j, frx, fry);
+      const float k = -p0.w * wh[j];
+      if (wh[j] != 0.0f) atomic_add3(T.dAh + q.y * f.W2 + q.x, gill.x * k, gill.y * k, gill.z * k);
     }
   }
 }
@@ -1621,7 +1719,7 @@ struct hush_trainer_s {
   float *theta = nullptr, *m = nullptr, *v = nullptr;
   double *grad = nullptr, *loss = nullptr, *loss_acc = nullptr, *loss_partials = nullptr;
   float4 *par = nullptr, *B[3] = {}, *A1 = nullptr, *X = nullptr, *out[2] = {}, *gT = nullptr, *gT2 = nullptr,
-         *dB[3] = {}, *dpar = nullptr, *dX = nullptr, *tcoef = nullptr;
+         *dB[3] = {}, *dpar = nullptr, *dX = nullptr, *tcoef = nullptr, *rsave = nullptr;
   float *partials = nullptr;
   // TEMPORAL's adjoint: seeds dA0 / dA1 (the fine level's input / output) and dmom (this frame's moments); outputs
   // dhist / dmomp (the previous frame's colour history and moments) and dag (its alpha, gamma per half-res pixel)
@@ -1687,9 +1785,10 @@ extern "C" int hush_trainer_create(hush_t *h, const float *theta, hush_trainer_t
   const size_t full = (size_t)t->W * t->H, half = (size_t)t->W2 * t->H2;
   t->n_mlp_ctas = (int)((half + MB_ROWS - 1) / MB_ROWS);
   t->n_loss_ctas = (int)((full + 255) / 256);
+  const int n_partials = std::max(t->n_loss_ctas, ((t->W + TW - 1) / TW) * ((t->H + TH - 1) / TH));
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t bytes = al(NW * 4) * 3 + al(NW * 8) + al(8) * 2 + al(t->n_loss_ctas * 8) + al(half * 48) * 2 +
-                       al(half * 16) * 6 + al(full * 16) * 12 + al(full * 48) + al((size_t)t->n_mlp_ctas * NW * 4) +
+  const size_t bytes = al(NW * 4) * 3 + al(NW * 8) + al(8) * 2 + al((size_t)n_partials * 8) + al(half * 48) * 2 +
+                       al(half * 16) * 6 + al(full * 16) * 12 + al(full * 48) + al(full * 64) + al((size_t)t->n_mlp_ctas * NW * 4) +
                        al(half * 8);
   cudaError_t e = cudaMalloc(&t->pool, bytes);
   if (e != cudaSuccess) { delete t; return hush_cuda_fail(h, e, "cudaMalloc of the trainer"); }
@@ -1698,13 +1797,14 @@ extern "C" int hush_trainer_create(hush_t *h, const float *theta, hush_trainer_t
   auto take = [&](size_t b) { char *p = t->pool + off; off += al(b); return p; };
   t->theta = (float *)take(NW * 4); t->m = (float *)take(NW * 4); t->v = (float *)take(NW * 4);
   t->grad = (double *)take(NW * 8); t->loss = (double *)take(8); t->loss_acc = (double *)take(8);
-  t->loss_partials = (double *)take(t->n_loss_ctas * 8);
+  t->loss_partials = (double *)take((size_t)n_partials * 8);
   t->par = (float4 *)take(half * 48); t->dpar = (float4 *)take(half * 48);
   for (int i = 0; i < 3; i++) { t->B[i] = (float4 *)take(half * 16); t->dB[i] = (float4 *)take(half * 16); }
   t->A1 = (float4 *)take(full * 16); t->X = (float4 *)take(full * 16);
   t->out[0] = (float4 *)take(full * 16); t->out[1] = (float4 *)take(full * 16);
   t->gT = (float4 *)take(full * 16); t->gT2 = (float4 *)take(full * 16); t->dX = (float4 *)take(full * 16);
   t->tcoef = (float4 *)take(full * 48);
+  t->rsave = (float4 *)take(full * 64);
   t->partials = (float *)take((size_t)t->n_mlp_ctas * NW * 4);
   t->dA0 = (float4 *)take(full * 16); t->dA1 = (float4 *)take(full * 16); t->dmom = (float4 *)take(full * 16);
   t->dhist = (float4 *)take(full * 16); t->dmomp = (float4 *)take(full * 16);
@@ -1828,13 +1928,12 @@ extern "C" int hush_trainer_frame(hush_trainer_t *t, const hush_inputs *in, cons
   k_mid_fwd<1><<<gh, blk, 0, st>>>(T);
   k_mid_fwd<2><<<gh, blk, 0, st>>>(T);
   k_mid_fwd<3><<<gh, blk, 0, st>>>(T);
+  T.rsave = backward ? t->rsave : nullptr;
   k_fine_fwd<<<gf, blk, 0, st>>>(T);
-  k_taa_fwd<<<gf, blk, 0, st>>>(T);
-  k_loss<<<t->n_loss_ctas, 256, 0, st>>>(T, backward);
-  k_reduce_f64<<<1, 256, 0, st>>>(t->loss_partials, t->n_loss_ctas, t->loss, t->loss_acc);
+  k_taa<<<gf, blk, 0, st>>>(T, backward ? TAA_ADJ : TAA_LOSS, t->tcoef);
+  k_reduce_f64<<<1, 256, 0, st>>>(t->loss_partials, (int)(gf.x * gf.y), t->loss, t->loss_acc);
   if (backward) {
-    k_taa_bwd_coef<<<gf, blk, 0, st>>>(T, t->gT, t->tcoef);
-    k_taa_bwd_gather<<<gf, blk, 0, st>>>(T, t->tcoef, t->gT2);
+    k_taa_bwd_gather<true><<<gf, blk, 0, st>>>(T, t->tcoef, t->gT2);
     k_fine_bwd<true><<<gf, blk, 0, st>>>(T, t->gT2);
     k_mid_bwd<3><<<gh, blk, 0, st>>>(T);
     k_mid_bwd<2><<<gh, blk, 0, st>>>(T);
@@ -2289,10 +2388,10 @@ static int run_twin_pass(hush_trainer_t *t, int pass, int backward, void *stream
       break;
     case HUSH_TWIN_TAA:
       if (!backward) {
-        k_taa_fwd<<<gf, blk, 0, st>>>(T);
+        k_taa<<<gf, blk, 0, st>>>(T, TAA_FWD, nullptr);
       } else {
         k_taa_bwd_coef<<<gf, blk, 0, st>>>(T, t->gT, t->tcoef);
-        k_taa_bwd_gather<<<gf, blk, 0, st>>>(T, t->tcoef, t->gT2);
+        k_taa_bwd_gather<false><<<gf, blk, 0, st>>>(T, t->tcoef, t->gT2);
         k_tm_bwd<<<(full + 255) / 256, 256, 0, st>>>(T, t->gT2, t->dX);
       }
       break;
@@ -2471,7 +2570,7 @@ static cudaError_t bptt_launches(hush_trainer_t *t, const hush_inputs *frames, c
     k_mid_fwd<2><<<gh, blk, 0, st>>>(T);
     k_mid_fwd<3><<<gh, blk, 0, st>>>(T);
     k_fine_fwd<<<gf, blk, 0, st>>>(T);
-    k_taa_fwd<<<gf, blk, 0, st>>>(T);
+    k_taa<<<gf, blk, 0, st>>>(T, T.zero_adj ? TAA_ADJ : TAA_LOSS, t->tcoef);
   };
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < n_frames && e == cudaSuccess; i++) {
@@ -2481,8 +2580,7 @@ static cudaError_t bptt_launches(hush_trainer_t *t, const hush_inputs *frames, c
     if (e == cudaSuccess) e = launch_pass(PASS_COARSE2, T.f, t->h->w16, st);
     if (e != cudaSuccess) break;
     forward(T);
-    k_loss<<<t->n_loss_ctas, 256, 0, st>>>(T, 0);
-    k_reduce_f64<<<1, 256, 0, st>>>(t->loss_partials, t->n_loss_ctas, t->loss, t->loss_acc);
+    k_reduce_f64<<<1, 256, 0, st>>>(t->loss_partials, (int)(gf.x * gf.y), t->loss, t->loss_acc);
   }
   int c = 0;
   for (int k = 0; k < 2 && e == cudaSuccess; k++) {
@@ -2493,11 +2591,10 @@ static cudaError_t bptt_launches(hush_trainer_t *t, const hush_inputs *frames, c
   for (int i = n_frames - 1; i >= 0 && e == cudaSuccess; i--) {
     TwinFrame T = twin(i);
     T.zero_adj = 1;
+    T.rsave = t->rsave;
     forward(T);
-    k_loss<<<t->n_loss_ctas, 256, 0, st>>>(T, 1);
     k_add_ag<<<(unsigned)((half + 255) / 256), 256, 0, st>>>(t->dpar, t->c_ag[c], (int)half);
-    k_taa_bwd_coef<<<gf, blk, 0, st>>>(T, t->gT, t->tcoef);
-    k_taa_bwd_gather<<<gf, blk, 0, st>>>(T, t->tcoef, t->gT2);
+    k_taa_bwd_gather<true><<<gf, blk, 0, st>>>(T, t->tcoef, t->gT2);
     e = cudaMemsetAsync(t->dA0, 0, full * 16, st);
     if (e == cudaSuccess && i > 0) e = cudaMemsetAsync(t->dah, 0, half * 16, st);
     if (e == cudaSuccess && i > 0) e = cudaMemsetAsync(t->dc0, 0, quarter * 16, st);
@@ -2509,7 +2606,7 @@ static cudaError_t bptt_launches(hush_trainer_t *t, const hush_inputs *frames, c
       T.dC0 = t->dc0;
     }
     k_fine_bwd<true><<<gf, blk, 0, st>>>(T, t->gT2);
-    if (i > 0) k_fine_pyr_bwd<true><<<gf, blk, 0, st>>>(T, t->gT2);
+    if (i > 0) k_fine_pyr_bwd<<<gf, blk, 0, st>>>(T, t->gT2);
     k_mid_bwd<3><<<gh, blk, 0, st>>>(T);
     k_mid_bwd<2><<<gh, blk, 0, st>>>(T);
     k_mid_bwd<1><<<gh, blk, 0, st>>>(T);
