@@ -406,7 +406,7 @@ struct Filt2 {
   }
 };
 
-// down() (hush.js:385-402) of the twin's FP32 block means ah at quarter-res texel Q, without the f16 rounding; the
+// down() (hush.js:385-402) of the twin's FP32 block means ah (NULL: the stored ones, F2.zw) at quarter-res texel Q, without the f16 rounding; the
 // weights are the blocks' pixel counts (F3), N their sum (0: the texel has no surface and holds zeros).
 HD_INL float4 down_tw(const HushFrame &f, const float4 *ah, int Qx, int Qy, float *Nout) {
   float N = 0.f, vr = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
@@ -416,7 +416,7 @@ HD_INL float4 down_tw(const HushFrame &f, const float4 *ah, int Qx, int Qy, floa
     if (hx >= f.W2 || hy >= f.H2) continue;
     const float w = unpack2(__ldg(f.F3 + hy * f.W2 + hx).y).y;
     if (w <= 0.0f) continue;
-    const float4 a = ah[hy * f.W2 + hx];
+    const float4 a = ah ? ah[hy * f.W2 + hx] : f2_ac_tw(f.F2, hy * f.W2 + hx);
     N += w;
     cx += w * a.x; cy += w * a.y; cz += w * a.z;
     vr += w * a.w;
@@ -432,7 +432,8 @@ __global__ void k_ah_fill(const TwinFrame T, float4 *ah) {
   if (o < T.f.W2 * T.f.H2) ah[o] = f2_ac_tw(T.f.F2, o);
 }
 
-// LEVEL 1: src = down(ah), output c1; LEVEL 2: src = c1, output c0. The guide is the stored coarse guide CG.
+// LEVEL 1: src = down(ah), output c1; LEVEL 2: src = c1, output c0; src NULL: the stored block means / C1 (the window
+// sweep, straight through their f16 storage). The guide is the stored coarse guide CG.
 template <int LEVEL>
 __global__ void __launch_bounds__(TW *TH) k_coarse_tw(const TwinFrame T, const float4 *src, float4 *dst,
                                                         const float4 *gout, float4 *gin) {
@@ -444,7 +445,7 @@ __global__ void __launch_bounds__(TW *TH) k_coarse_tw(const TwinFrame T, const f
   for (int i = li; i < SW * SH; i += TW * TH) {
     const int qx = clampi(bx - AP + i % SW, 0, f.W4 - 1), qy = clampi(by - AP + i / SW, 0, f.H4 - 1);
     const int q = qy * f.W4 + qx;
-    sA[i] = LEVEL == 1 ? down_tw(f, src, qx, qy, nullptr) : src[q];
+    sA[i] = LEVEL == 1 ? down_tw(f, src, qx, qy, nullptr) : (src ? src[q] : ldh(f.C1, q));
     float4 g = ldh(f.CG, q);
     float4 n = oct_dec(g.x, g.y);
     n.w = g.z;
@@ -485,12 +486,6 @@ __global__ void k_down_bwd(const TwinFrame T, const float4 *ah, const float4 *dd
   d.x += g.x * k; d.y += g.y * k; d.z += g.z * k;
   d.w += g.w * k / N;
   dah[o] = d;
-}
-
-// c1 = the stored coarse level C1 as FP32 (coarse2's input in the window sweep, straight through the f16 storage)
-__global__ void k_c1_fill(const TwinFrame T, float4 *c1) {
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o < T.f.W4 * T.f.H4) c1[o] = ldh(T.f.C1, o);
 }
 
 // The block means' adjoint into TEMPORAL's output: block() forms Ah as the mean of the f16-quantised A0 over the
@@ -1413,15 +1408,18 @@ __global__ void __launch_bounds__(MB_ROWS) k_mlp_bwd(const TwinFrame T) {
 constexpr size_t MB_SMEM = (size_t)(NW + MB_ROWS * MB_REC) * sizeof(float);
 
 // dtheta += sum over CTAs of the partials, in FP64 and in a fixed order: 32 parameters per block on the lanes, the
-// CTAs split over the 8 warps (c = w, w + 8, ...), then the 8 warp sums added in warp order.
-constexpr int RP_THREADS = 256, RP_PARAMS = 32;
+// CTAs split over the 32 warps (c = w, w + 32, ...), then the warp sums added in warp order. Bound: the latency of each
+// warp's chain of loads.
+constexpr int RP_THREADS = 1024, RP_PARAMS = 32;
 __global__ void __launch_bounds__(RP_THREADS) k_reduce_partials(const float *partials, int nparts, double *grad) {
   __shared__ double ws[RP_THREADS / 32][RP_PARAMS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int p = blockIdx.x * RP_PARAMS + lane;
   double a = 0.0;
-  if (p < NW)
+  if (p < NW) {
+#pragma unroll 4
     for (int c = w; c < nparts; c += RP_THREADS / 32) a += (double)partials[(size_t)c * NW + p];
+  }
   ws[w][lane] = a;
   __syncthreads();
   if (w == 0 && p < NW) {
@@ -1730,12 +1728,19 @@ struct hush_trainer_s {
   int W4 = 0, H4 = 0;
   float4 *ah = nullptr, *dah = nullptr, *c1 = nullptr, *dc1 = nullptr, *c0 = nullptr, *dc0 = nullptr, *ddown = nullptr;
   char *coarse_pool = nullptr;
+  size_t adj_bytes = 0, coarse_adj_bytes = 0;
   // hush_trainer_window_bptt: the window's per-frame state records and the carried gradients (ping-pong)
   struct Rec {
     uint2 *A0, *key, *mom, *hist, *taa, *par0, *C0, *C1, *CG;
     uint4 *F[4];
     float4 *out;
+    // with saved forwards, from the second frame on (frame 0 uses the trainer's own buffers): dL/dX, the
+    // recombination's values, the parameters and the mid levels the adjoints read
+    float4 *gX, *rsave, *par, *B1, *B2;
   };
+  bool rec_saved = false;       // the records hold the forwards' values (else the reverse sweep runs them again)
+  float4 *rec_tmp[4] = {};      // A1, X, B3 and dL/dout of the frame whose forward runs (saved forwards)
+  float *rec_partials = nullptr;  // per frame: the MLP adjoint's per-CTA partials, reduced once per window
   std::vector<Rec> rec;
   char *rec_pool = nullptr;
   float4 *c_hist[2] = {}, *c_mom[2] = {};
@@ -1798,15 +1803,20 @@ extern "C" int hush_trainer_create(hush_t *h, const float *theta, hush_trainer_t
   t->theta = (float *)take(NW * 4); t->m = (float *)take(NW * 4); t->v = (float *)take(NW * 4);
   t->grad = (double *)take(NW * 8); t->loss = (double *)take(8); t->loss_acc = (double *)take(8);
   t->loss_partials = (double *)take((size_t)n_partials * 8);
-  t->par = (float4 *)take(half * 48); t->dpar = (float4 *)take(half * 48);
-  for (int i = 0; i < 3; i++) { t->B[i] = (float4 *)take(half * 16); t->dB[i] = (float4 *)take(half * 16); }
+  t->par = (float4 *)take(half * 48);
+  for (int i = 0; i < 3; i++) t->B[i] = (float4 *)take(half * 16);
+  const size_t adj0 = off;  // the accumulators a window's reverse sweep clears together
+  t->dpar = (float4 *)take(half * 48);
+  for (int i = 0; i < 3; i++) t->dB[i] = (float4 *)take(half * 16);
+  t->dA0 = (float4 *)take(full * 16);
+  t->adj_bytes = off - adj0;
   t->A1 = (float4 *)take(full * 16); t->X = (float4 *)take(full * 16);
   t->out[0] = (float4 *)take(full * 16); t->out[1] = (float4 *)take(full * 16);
   t->gT = (float4 *)take(full * 16); t->gT2 = (float4 *)take(full * 16); t->dX = (float4 *)take(full * 16);
   t->tcoef = (float4 *)take(full * 48);
   t->rsave = (float4 *)take(full * 64);
   t->partials = (float *)take((size_t)t->n_mlp_ctas * NW * 4);
-  t->dA0 = (float4 *)take(full * 16); t->dA1 = (float4 *)take(full * 16); t->dmom = (float4 *)take(full * 16);
+  t->dA1 = (float4 *)take(full * 16); t->dmom = (float4 *)take(full * 16);
   t->dhist = (float4 *)take(full * 16); t->dmomp = (float4 *)take(full * 16);
   t->dag = (float2 *)take(half * 8);
   e = cudaMemcpy(t->theta, theta ? theta : h->wf.data(), NW * 4, cudaMemcpyHostToDevice);
@@ -1834,9 +1844,10 @@ static cudaError_t ensure_coarse(hush_trainer_t *t) {
   e = cudaMemset(t->coarse_pool, 0, bytes);
   size_t off = 0;
   auto take = [&](size_t b) { char *p = t->coarse_pool + off; off += al(b); return (float4 *)p; };
-  t->ah = take(half * 16); t->dah = take(half * 16);
-  t->c1 = take(quarter * 16); t->dc1 = take(quarter * 16); t->c0 = take(quarter * 16); t->dc0 = take(quarter * 16);
-  t->ddown = take(quarter * 16);
+  t->ah = take(half * 16); t->c1 = take(quarter * 16); t->c0 = take(quarter * 16);
+  const size_t adj0 = off;  // cleared together by a window's reverse sweep
+  t->dah = take(half * 16); t->dc1 = take(quarter * 16); t->dc0 = take(quarter * 16); t->ddown = take(quarter * 16);
+  t->coarse_adj_bytes = off - adj0;
   return e;
 }
 
@@ -1871,11 +1882,11 @@ static void launch_mlp_fwd(const hush_trainer_t *t, const TwinFrame &T, cudaStre
   else if (t->mlp_mode == HUSH_MLP_F16) k_mlp_fwd_tc<false><<<(half + TC_ROWS - 1) / TC_ROWS, TC_ROWS, TC_SMEM_FWD, st>>>(T);
   else k_mlp_fwd<<<(half + 127) / 128, 128, 0, st>>>(T);
 }
-static void launch_mlp_bwd(const hush_trainer_t *t, const TwinFrame &T, cudaStream_t st) {
+static void launch_mlp_bwd(const hush_trainer_t *t, const TwinFrame &T, cudaStream_t st, bool reduce = true) {
   if (t->mlp_mode == HUSH_MLP_BF16) k_mlp_bwd_tc<true><<<t->n_mlp_ctas, TC_ROWS, TC_SMEM_BWD, st>>>(T);
   else if (t->mlp_mode == HUSH_MLP_F16) k_mlp_bwd_tc<false><<<t->n_mlp_ctas, TC_ROWS, TC_SMEM_BWD, st>>>(T);
   else k_mlp_bwd<<<t->n_mlp_ctas, MB_ROWS, MB_SMEM, st>>>(T);
-  k_reduce_partials<<<RP_BLOCKS, RP_THREADS, 0, st>>>(t->partials, t->n_mlp_ctas, t->grad);
+  if (reduce) k_reduce_partials<<<RP_BLOCKS, RP_THREADS, 0, st>>>(T.partials, t->n_mlp_ctas, t->grad);
 }
 
 static TwinFrame make_twin(hush_trainer_t *t, const hush_inputs *in, const float *clean, const float *clean_prev,
@@ -2466,41 +2477,69 @@ __global__ void k_add_ag(float4 *dpar, const float2 *ag, int n) {
   dpar[3 * o].y += g.y;
 }
 
+// Bytes of one slot of the carried gradients.
+static size_t carry_bytes(const hush_trainer_t *t) {
+  const size_t full = (size_t)t->W * t->H, half = (size_t)t->W2 * t->H2;
+  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  return al(full * 16) * 2 + al(half * 8);
+}
+
 // The state of each frame of a window that the reverse sweep reads again: TEMPORAL's outputs and key, the features,
-// the coarse levels, the twin's stored history (colour, TAA, par0) and its FP32 TAA output (the next frame's temporal
-// loss term). Allocated for the longest window seen.
+// the coarse levels, the twin's stored history (colour, TAA, par0), its FP32 TAA output (the next frame's temporal loss
+// term) and, while the window's records stay under REC_SAVED_MAX, what the adjoints need of the twin's forward (27 MB
+// instead of 11 MB per frame at 384 x 384), so that the sweep does not run the forward again. Larger windows, and ones
+// whose memory is not to be had, keep the 11 MB and recompute. Allocated for the longest window seen.
+constexpr size_t REC_SAVED_MAX = (size_t)2 << 30;
 static int ensure_records(hush_trainer_t *t, int n) {
   if ((int)t->rec.size() >= n) return HUSH_OK;
   const size_t full = (size_t)t->W * t->H, half = (size_t)t->W2 * t->H2;
-  const size_t quarter = (size_t)((t->W2 + 1) / 2) * ((t->H2 + 1) / 2);
+  const size_t quarter = (size_t)((t->W2 + 1) / 2) * ((t->H2 + 1) / 2), part = (size_t)t->n_mlp_ctas * NW * 4;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t per = al(full * 8) * 5 + al(half * 8) + al(half * 16) * 4 + al(quarter * 8) * 3 + al(full * 16);
+  const size_t lean = al(full * 8) * 5 + al(half * 8) + al(half * 16) * 4 + al(quarter * 8) * 3 + al(full * 16);
+  const size_t saved = al(full * 16) + al(full * 64) + al(half * 48) + al(half * 16) * 2;
+  const size_t bytes_lean = lean * n, bytes_saved = (lean + saved) * n + al(full * 16) * 3 + al(half * 16) + al(part * n);
   drop_bptt_graph(t);  // it captured the old records' addresses
   cudaFree(t->rec_pool);
+  t->rec_pool = nullptr;
   t->rec.clear();
-  cudaError_t e = cudaMalloc(&t->rec_pool, per * n);
+  t->rec_saved = bytes_saved <= REC_SAVED_MAX && cudaMalloc(&t->rec_pool, bytes_saved) == cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  if (!t->rec_saved) {
+    cudaGetLastError();
+    e = cudaMalloc(&t->rec_pool, bytes_lean);
+  }
   if (e != cudaSuccess) { t->rec_pool = nullptr; return hush_cuda_fail(t->h, e, "cudaMalloc of the window records"); }
-  e = cudaMemset(t->rec_pool, 0, per * n);
+  e = cudaMemset(t->rec_pool, 0, t->rec_saved ? bytes_saved : bytes_lean);
   if (e != cudaSuccess) return hush_cuda_fail(t->h, e, "cudaMemset of the window records");
-  if (!t->carry_pool) {
-    const size_t cb = al(full * 16) * 4 + al(half * 8) * 2;
-    e = cudaMalloc(&t->carry_pool, cb);
+  if (!t->carry_pool) {  // per ping-pong slot: colour history, moments, alpha / gamma, cleared together
+    e = cudaMalloc(&t->carry_pool, carry_bytes(t) * 2);
     if (e != cudaSuccess) { t->carry_pool = nullptr; return hush_cuda_fail(t->h, e, "cudaMalloc of the carries"); }
     char *c = t->carry_pool;
-    for (int k = 0; k < 2; k++) { t->c_hist[k] = (float4 *)c; c += al(full * 16); }
-    for (int k = 0; k < 2; k++) { t->c_mom[k] = (float4 *)c; c += al(full * 16); }
-    for (int k = 0; k < 2; k++) { t->c_ag[k] = (float2 *)c; c += al(half * 8); }
+    for (int k = 0; k < 2; k++) {
+      t->c_hist[k] = (float4 *)c; c += al(full * 16);
+      t->c_mom[k] = (float4 *)c; c += al(full * 16);
+      t->c_ag[k] = (float2 *)c; c += al(half * 8);
+    }
   }
   char *b = t->rec_pool;
+  auto take = [&](size_t sz) { char *q = b; b += al(sz); return q; };
   for (int i = 0; i < n; i++) {
-    hush_trainer_t::Rec r;
-    auto take = [&](size_t sz) { char *q = b; b += al(sz); return q; };
+    hush_trainer_t::Rec r{};
     r.A0 = (uint2 *)take(full * 8); r.key = (uint2 *)take(full * 8); r.mom = (uint2 *)take(full * 8);
     r.hist = (uint2 *)take(full * 8); r.taa = (uint2 *)take(full * 8); r.par0 = (uint2 *)take(half * 8);
     for (int k = 0; k < 4; k++) r.F[k] = (uint4 *)take(half * 16);
     r.C0 = (uint2 *)take(quarter * 8); r.C1 = (uint2 *)take(quarter * 8); r.CG = (uint2 *)take(quarter * 8);
     r.out = (float4 *)take(full * 16);
+    if (t->rec_saved) {
+      r.gX = (float4 *)take(full * 16); r.rsave = (float4 *)take(full * 64); r.par = (float4 *)take(half * 48);
+      r.B1 = (float4 *)take(half * 16); r.B2 = (float4 *)take(half * 16);
+    }
     t->rec.push_back(r);
+  }
+  if (t->rec_saved) {
+    for (int k = 0; k < 3; k++) t->rec_tmp[k] = (float4 *)take(full * 16);
+    t->rec_tmp[3] = (float4 *)take(half * 16);
+    t->rec_partials = (float *)take(part * n);
   }
   return HUSH_OK;
 }
@@ -2519,11 +2558,20 @@ static TwinFrame rec_twin(hush_trainer_t *t, const hush_inputs *in, const float 
   T.out = r.out;
   T.out_prev = p.out;
   T.has_prev = (i > 0 && clean_prev) ? 1 : 0;
+  T.rsave = t->rsave;
+  if (t->rec_saved) {
+    T.partials = t->rec_partials + (size_t)i * t->n_mlp_ctas * NW;
+    if (i > 0) {
+      T.par = r.par; T.B1 = r.B1; T.B2 = r.B2; T.rsave = r.rsave;
+      T.A1 = t->rec_tmp[0]; T.X = t->rec_tmp[1]; T.gT = t->rec_tmp[2]; T.B3 = t->rec_tmp[3];
+    }
+  }
   return T;
 }
 
 // Backpropagation through time over one window (see include/hush.h): forward over the frames, keeping each frame's
-// state, then the reverse sweep, frame by frame from the last: the twin's forward again, the loss, TAA, fine (seeded
+// state, then the reverse sweep, frame by frame from the last: (without saved forwards) the twin's forward again with the
+// loss and dL/dX, then fine (seeded
 // with the gradient the next frame sent to this frame's colour history, and giving dL/dA0 and, from the second frame
 // on, dL/d block means and dL/dC0), mid3..mid1 (mid1 adding into dL/d block means), the MLP (whose alpha / gamma
 // seeds are the gradient the next frame sent to this frame's par0), the coarse levels' adjoints (C0 -> C1 -> down()
@@ -2558,19 +2606,22 @@ extern "C" int hush_trainer_window_bptt(hush_trainer_t *t, const hush_inputs *fr
 static cudaError_t bptt_launches(hush_trainer_t *t, const hush_inputs *frames, const float *const *cleans,
                                  int n_frames, float lambda_t, cudaStream_t st) {
   const int W = t->W, H = t->H, W2 = t->W2, H2 = t->H2;
-  const size_t full = (size_t)W * H, half = (size_t)W2 * H2, quarter = (size_t)t->W4 * t->H4;
+  const size_t full = (size_t)W * H, half = (size_t)W2 * H2;
   const dim3 blk(TW, TH), gh((W2 + TW - 1) / TW, (H2 + TH - 1) / TH), gf((W + TW - 1) / TW, (H + TH - 1) / TH);
   const dim3 gq((t->W4 + TW - 1) / TW, (t->H4 + TH - 1) / TH);
   auto twin = [&](int i) {
     return rec_twin(t, frames + i, cleans[i], i ? cleans[i - 1] : nullptr, i, lambda_t);
   };
-  auto forward = [&](const TwinFrame &T) {
+  auto gX = [&](int i) { return t->rec_saved && i > 0 ? t->rec[i].gX : t->gT2; };
+  // the twin's forward; adj: with dL/dX into gX(i) and the values its adjoint needs
+  auto forward = [&](const TwinFrame &T, int i, bool adj) {
     launch_mlp_fwd(t, T, st);
     k_mid_fwd<1><<<gh, blk, 0, st>>>(T);
     k_mid_fwd<2><<<gh, blk, 0, st>>>(T);
     k_mid_fwd<3><<<gh, blk, 0, st>>>(T);
     k_fine_fwd<<<gf, blk, 0, st>>>(T);
-    k_taa<<<gf, blk, 0, st>>>(T, T.zero_adj ? TAA_ADJ : TAA_LOSS, t->tcoef);
+    k_taa<<<gf, blk, 0, st>>>(T, adj ? TAA_ADJ : TAA_LOSS, t->tcoef);
+    if (adj) k_taa_bwd_gather<true><<<gf, blk, 0, st>>>(T, t->tcoef, gX(i));
   };
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < n_frames && e == cudaSuccess; i++) {
@@ -2579,58 +2630,46 @@ static cudaError_t bptt_launches(hush_trainer_t *t, const hush_inputs *frames, c
     if (e == cudaSuccess) e = launch_pass(PASS_COARSE1, T.f, t->h->w16, st);
     if (e == cudaSuccess) e = launch_pass(PASS_COARSE2, T.f, t->h->w16, st);
     if (e != cudaSuccess) break;
-    forward(T);
+    forward(T, i, t->rec_saved);
     k_reduce_f64<<<1, 256, 0, st>>>(t->loss_partials, (int)(gf.x * gf.y), t->loss, t->loss_acc);
   }
   int c = 0;
-  for (int k = 0; k < 2 && e == cudaSuccess; k++) {
-    e = cudaMemsetAsync(t->c_hist[k], 0, full * 16, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(t->c_mom[k], 0, full * 16, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(t->c_ag[k], 0, half * 8, st);
-  }
+  if (e == cudaSuccess) e = cudaMemsetAsync(t->c_hist[c], 0, carry_bytes(t), st);
   for (int i = n_frames - 1; i >= 0 && e == cudaSuccess; i--) {
     TwinFrame T = twin(i);
-    T.zero_adj = 1;
-    T.rsave = t->rsave;
-    forward(T);
-    k_add_ag<<<(unsigned)((half + 255) / 256), 256, 0, st>>>(t->dpar, t->c_ag[c], (int)half);
-    k_taa_bwd_gather<true><<<gf, blk, 0, st>>>(T, t->tcoef, t->gT2);
-    e = cudaMemsetAsync(t->dA0, 0, full * 16, st);
-    if (e == cudaSuccess && i > 0) e = cudaMemsetAsync(t->dah, 0, half * 16, st);
-    if (e == cudaSuccess && i > 0) e = cudaMemsetAsync(t->dc0, 0, quarter * 16, st);
+    if (!t->rec_saved) forward(T, i, true);
+    // dpar, dB1..dB3 and dA0 lie together, as do the coarse levels' gradients
+    e = cudaMemsetAsync(t->dpar, 0, t->adj_bytes, st);
+    if (e == cudaSuccess && i > 0) e = cudaMemsetAsync(t->dah, 0, t->coarse_adj_bytes, st);
     if (e != cudaSuccess) break;
+    k_add_ag<<<(unsigned)((half + 255) / 256), 256, 0, st>>>(t->dpar, t->c_ag[c], (int)half);
     T.gA1 = t->c_hist[c];
     T.dA0 = t->dA0;
     if (i > 0) {  // A0 reaches the loss also through the block means (mid1, the recombination, the coarse levels)
       T.dAh = t->dah;
       T.dC0 = t->dc0;
     }
-    k_fine_bwd<true><<<gf, blk, 0, st>>>(T, t->gT2);
-    if (i > 0) k_fine_pyr_bwd<<<gf, blk, 0, st>>>(T, t->gT2);
+    k_fine_bwd<true><<<gf, blk, 0, st>>>(T, gX(i));
+    if (i > 0) k_fine_pyr_bwd<<<gf, blk, 0, st>>>(T, gX(i));
     k_mid_bwd<3><<<gh, blk, 0, st>>>(T);
     k_mid_bwd<2><<<gh, blk, 0, st>>>(T);
     k_mid_bwd<1><<<gh, blk, 0, st>>>(T);
-    launch_mlp_bwd(t, T, st);
+    launch_mlp_bwd(t, T, st, !t->rec_saved);
     if (i > 0) {
       // the coarse levels' adjoints (C0 -> C1 -> down() -> block means), then the block means into A0
-      k_ah_fill<<<(unsigned)((half + 255) / 256), 256, 0, st>>>(T, t->ah);
-      k_c1_fill<<<(unsigned)((quarter + 255) / 256), 256, 0, st>>>(T, t->c1);
-      e = cudaMemsetAsync(t->dc1, 0, quarter * 16, st);
-      if (e == cudaSuccess) e = cudaMemsetAsync(t->ddown, 0, quarter * 16, st);
-      if (e != cudaSuccess) break;
-      k_coarse_tw<2><<<gq, blk, 0, st>>>(T, t->c1, nullptr, t->dc0, t->dc1);
-      k_coarse_tw<1><<<gq, blk, 0, st>>>(T, t->ah, nullptr, t->dc1, t->ddown);
-      k_down_bwd<<<(unsigned)((half + 255) / 256), 256, 0, st>>>(T, t->ah, t->ddown, t->dah);
+      k_coarse_tw<2><<<gq, blk, 0, st>>>(T, nullptr, nullptr, t->dc0, t->dc1);
+      k_coarse_tw<1><<<gq, blk, 0, st>>>(T, nullptr, nullptr, t->dc1, t->ddown);
+      k_down_bwd<<<(unsigned)((half + 255) / 256), 256, 0, st>>>(T, nullptr, t->ddown, t->dah);
       k_ah_to_a0<<<(unsigned)((full + 255) / 256), 256, 0, st>>>(T, t->dah, t->dA0);
       const int n = c ^ 1;
-      e = cudaMemsetAsync(t->c_hist[n], 0, full * 16, st);
-      if (e == cudaSuccess) e = cudaMemsetAsync(t->c_mom[n], 0, full * 16, st);
-      if (e == cudaSuccess) e = cudaMemsetAsync(t->c_ag[n], 0, half * 8, st);
+      e = cudaMemsetAsync(t->c_hist[n], 0, carry_bytes(t), st);
       if (e != cudaSuccess) break;
       k_temporal_bwd<<<gf, blk, 0, st>>>(T, t->dA0, t->c_mom[c], t->c_hist[n], t->c_mom[n], t->c_ag[n]);
       c = n;
     }
   }
+  if (e == cudaSuccess && t->rec_saved)
+    k_reduce_partials<<<RP_BLOCKS, RP_THREADS, 0, st>>>(t->rec_partials, t->n_mlp_ctas * n_frames, t->grad);
   return e;
 }
 

@@ -327,8 +327,9 @@ int hush_coarse2_bwd(hush_trainer_t *t, void *stream);
  * reaches the loss directly (the fine level) and through the block means (block(), hush.js:241-244), which feed mid1,
  * the recombination and the coarse levels COARSE1 / coarse2; both paths are followed. The block features and the TAA
  * history are held fixed (truncated there). Adds into the gradient and loss accumulators,
- * like hush_trainer_windows; allocates the window's per-frame records (about 11 MB per frame at 384 x 384) on first
- * use. The trainer's own Hush history is not touched. */
+ * like hush_trainer_windows; allocates the window's per-frame records on first use (about 27 MB per frame at 384 x 384
+ * while a window's stay under 2 GiB, so that the reverse sweep does not run the forward again; else 11 MB). The
+ * trainer's own Hush history is not touched. */
 int hush_trainer_window_bptt(hush_trainer_t *t, const hush_inputs *frames, const float *const *cleans, int n_frames,
                              float lambda_t, void *stream);
 

@@ -36,3 +36,31 @@ def test_fused_frame_matches_the_pass_chain_at_tile_edges(w, h):
     assert np.isfinite(g_frame).all() and np.isfinite(d_frame).all()
     assert np.abs(g_chain - g_frame).max() <= 1e-5 * np.abs(g_chain).max()
     assert np.abs(d_chain - d_frame).max() <= 1e-5 * np.abs(d_chain).max()
+
+
+def test_window_gradient_with_and_without_saved_forwards():
+    """A window's records keep the forwards' values while they fit 2 GiB; a trainer that has run a longer window keeps
+    the small records and runs the forwards again in the reverse sweep. Both give the window's gradient (the same
+    kernels on the same values; FP32 atomics in another order: 1e-5 of the largest, loss to 1e-12), in both MLP forms."""
+    from hush_b200 import Hush
+    from hush_b200.train import TrainConfig, Trainer, window, xavier_init
+
+    size, long_window = 512, 46  # 46 frames x 48 MB > 2 GiB
+    win = window(TrainConfig(size=size, frames=3), 7)
+    for mlp in ("fp32", "bf16"):
+        got = []
+        for lean in (True, False):
+            den = Hush(0, {"width": size, "height": size, "schedule": "passes"})
+            tr = Trainer(den, xavier_init(2))
+            tr.set_mlp(mlp)
+            if lean:
+                tr.window_bptt([win[i % 3] for i in range(long_window)], 0.5)
+            tr.zero_grad()
+            tr.loss_sum()
+            tr.window_bptt(win, 0.5)
+            got.append((tr.loss_sum(), tr.grad()))
+            tr.destroy()
+            den.destroy()
+        (la, ga), (lb, gb) = got
+        assert abs(la - lb) <= 1e-12 * abs(lb)
+        assert np.abs(ga - gb).max() <= 1e-5 * np.abs(gb).max()
