@@ -41,6 +41,10 @@ HD_INL void cp_async8(const uint2 *dst_smem, const uint2 *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src)
                : "memory");
 }
+HD_INL void cp_async16(const void *dst_smem, const void *src) {  // both 16-byte aligned
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src)
+               : "memory");
+}
 HD_INL void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 HD_INL void cp_async_wait() {

@@ -17,6 +17,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstring>
 #include <type_traits>
 
@@ -739,13 +740,6 @@ HD_INL bool tma_wait_or_flag(const HushFrame &f, uint32_t mb) {
   atomicOr(f.err, 8u);
   return false;
 }
-// FINE_FINAL's A0 / key tiles (8-byte texels, 2-d UINT64 maps {W, H}) on interior tiles: the copies start at
-// x = bx - 2 (even, so 16-byte aligned) with a 36 x 10 box; the tile's column c is the box's column c + 1.
-struct FineMaps {
-  CUtensorMap a0, key;
-  int ok;
-};
-
 HD_INL void tma_expect(uint32_t mbar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
 }
@@ -1065,179 +1059,278 @@ __global__ void __launch_bounds__(HT_W *HT_H) k_half_pair(const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------------------ stage 4 / 5
-constexpr int FT_W = 32, FT_H = 8;
+constexpr int FT_W = 32, FT_H = 8;  // TAA's tile
 
-// FINE_FINAL with a 32 x 8 tile. Before the barrier the CTA stages, besides the A0 / guide tile of the fine filter,
-// everything its pixels' recombination reads: the half-res footprint (guide Gd, block means Ah, mid level Bh0; 18 x 6
-// texels, decoded once), the quarter-res footprint (guide CGd, coarse level C0; 10 x 4) and the per-block filter
-// parameters (s0, c0, beta, kappa; 16 x 4). Each texel is then read from shared memory by the 16 or so taps that use
-// it instead of being fetched and decoded per tap.
-constexpr int FH_W = FT_W / 2 + 2, FH_H = FT_H / 2 + 2, FQ_W = FT_W / 4 + 2, FQ_H = FT_H / 4 + 2;
-constexpr int FB_W = FT_W + 4, FB_H = FT_H + 2;  // the TMA box of the A0 / key tiles
-__global__ void __launch_bounds__(FT_W *FT_H, 4) k_fine_final_fused(const __grid_constant__ HushFrame f,
-                                                                     const __grid_constant__ FineMaps M) {
-  constexpr int AP = 1, SW = FT_W + 2, SH = FT_H + 2;
-  constexpr int NH = FH_W * FH_H, NQ = FQ_W * FQ_H, NP = (FT_W / 2) * (FT_H / 2);
-  __shared__ float4 sA[SW * SH], sG[SW * SH];
-  __shared__ float4 sHG[NH], sHA[NH], sHB[NH], sQG[NQ], sQC[NQ], sPar[NP];
-  __shared__ alignas(128) uint2 stA[FB_W * FB_H];
-  __shared__ alignas(128) uint2 stK[FB_W * FB_H];
-  __shared__ alignas(8) uint64_t mbar;
-  const int li = threadIdx.x;
-  const int bx = blockIdx.x * FT_W, by = blockIdx.y * FT_H;
-  const bool interior = bx - 2 >= 0 && by - 1 >= 0 && bx + FT_W + 2 <= f.W && by + FT_H + 1 <= f.H;
-  const bool inner = M.ok && interior;
-  const uint32_t mb = umma::smem_u32(&mbar);
-  // this pixel's material and emission, in flight while the tiles arrive
-  const int px = bx + li % FT_W, py = by + li / FT_W;
-  const bool in_img = px < f.W && py < f.H;
-  uint2 mat_r = make_uint2(0, 0), emi_r = make_uint2(0, 0);
-  if (in_img) {
-    mat_r = __ldg(f.mat + py * f.p_mat + px);
-    emi_r = __ldg(f.emi + py * f.p_emi + px);
+// FINE_FINAL on a 32 x 16 tile, two vertically adjacent pixels of one 2 x 2 block per thread. Before the barrier the CTA
+// stages, besides the A0 / guide tile of the fine filter, everything its pixels' recombination reads: the half-res
+// footprint (guide Gd, block means Ah, mid level Bh0; 18 x 10 texels, decoded once), the quarter-res footprint (guide
+// CGd, coarse level C0; 10 x 6) and the per-block filter parameters (s0, c0, beta, kappa; 16 x 8). A thread's two pixels
+// share the loads of 10 of their 3 x 3 windows' 18 texels, one row of the half-res footprint, the whole quarter-res
+// footprint and the parameters: 52 16-byte loads of shared memory for two pixels instead of 80. With a pixel per
+// thread the kernel was at 70% of the shared-memory bandwidth and 67% of the issue slots, and with either split half of
+// the CTAs waited for their tile's texels: 70 us at 1920 x 1080 and 271 at 3840 x 2160, now 66 and 246. Three CTAs per SM
+// (80 registers, with spills) measured the same at 1920 x 1080 and 0.6 us more at 256 x 256.
+constexpr int FF_W = 32, FF_H = 16, FF_NT = FF_W * FF_H / 2;
+constexpr int FH_W = FF_W / 2 + 2, FH_H = FF_H / 2 + 2, FQ_W = FF_W / 4 + 2, FQ_H = FF_H / 4 + 2;
+constexpr int FB_W = FF_W + 4, FB_H = FF_H + 2;  // the TMA box of the A0 / key tiles
+
+// filt_x<1, 1, true> for the pixel at tile entry ti and the one below it. The taps run as pairs of one tap of each
+// pixel, on the same texel where both windows hold it: (n.n)^128, weights and their squares as packed FP32x2, lane by lane
+// the scalar arithmetic.
+template <int SW, bool CHECK>
+HD_INL void filt_v2(const float4 *sA, const float4 *sG, int ti, int qx, int qy, int w, int h, float s, float c,
+                    float4 &out0, float4 &out1) {
+  const float4 g0 = sG[ti], g1 = sG[ti + SW], a0 = sA[ti], a1 = sA[ti + SW];
+  auto v = [&](int dx, int dy) { return sA[ti + dy * SW + dx].w; };
+  auto z = [&](int dx, int dy) { return sG[ti + dy * SW + dx].w; };
+  const float vm[2] = {v(-1, 0), v(-1, 1)}, vp[2] = {v(1, 0), v(1, 1)};
+  const float gv0 = 0.0625f * (v(-1, -1) + v(1, -1) + vm[1] + vp[1]) + 0.125f * (v(0, -1) + vm[0] + vp[0] + a1.w) + 0.25f * a0.w;
+  const float gv1 = 0.0625f * (vm[0] + vp[0] + v(-1, 2) + v(1, 2)) + 0.125f * (a0.w + vm[1] + vp[1] + v(0, 2)) + 0.25f * a1.w;
+  const float lc0 = lum(a0), lc1 = lum(a1);
+  auto slope = [](float zc, float zl, float zr, float zu, float zd) {
+    const float gx = fminf(zr > 0.0f ? fabsf(zr - zc) : 1e9f, zl > 0.0f ? fabsf(zl - zc) : 1e9f);
+    const float gy = fminf(zd > 0.0f ? fabsf(zd - zc) : 1e9f, zu > 0.0f ? fabsf(zu - zc) : 1e9f);
+    return fminf(fmaxf(gx, gy), zc);
+  };
+  const float zg0 = slope(g0.w, z(-1, 0), z(1, 0), z(0, -1), g1.w), zg1 = slope(g1.w, z(-1, 1), z(1, 1), g0.w, z(0, 2));
+  const float sl0 = LOG2E * s / (sqrtf(fmaxf(gv0, 1e-12f)) + 1e-6f), sl1 = LOG2E * s / (sqrtf(fmaxf(gv1, 1e-12f)) + 1e-6f);
+  const float iz0[2] = {LOG2E / (zg0 * 1.0f + 1e-3f), LOG2E / (zg0 * 1.41421356237309515f + 1e-3f)};
+  const float iz1[2] = {LOG2E / (zg1 * 1.0f + 1e-3f), LOG2E / (zg1 * 1.41421356237309515f + 1e-3f)};
+  const float cw = 0.25f * c;
+  float sw0 = cw, sw1 = cw;
+  float x0 = a0.x * cw, y0 = a0.y * cw, b0 = a0.z * cw, v0 = a0.w * cw * cw;
+  float x1 = a1.x * cw, y1 = a1.y * cw, b1 = a1.z * cw, v1 = a1.w * cw * cw;
+  // one tap of each pixel: texel (p, cp) at offset (dx, dyp) of pixel 0, texel (q, cq) at offset (dx, dyq) of pixel 1
+  auto tap = [&](float4 p, float4 cp, int dyp, float4 q, float4 cq, int dyq, int dx) {
+    bool ok0 = p.w >= 0.0f, ok1 = q.w >= 0.0f;
+    if (CHECK) {
+      const int tx = qx + dx, t0 = qy + dyp, t1 = qy + 1 + dyq;
+      const bool ix = tx >= 0 && tx < w;
+      ok0 = ok0 && ix && t0 >= 0 && t0 < h;
+      ok1 = ok1 && ix && t1 >= 0 && t1 < h;
+    }
+    float2 pp = make_float2(fmaxf(dot3(p, g0), 0.0f), fmaxf(dot3(q, g1), 0.0f));
+#pragma unroll
+    for (int i = 0; i < 7; i++) pp = __fmul2_rn(pp, pp);  // (n.n)^128
+    const float e0 = fmaf(-fabsf(p.w - g0.w), iz0[dx != 0 && dyp != 0], fmaf(-sl0, fabsf(lum(cp) - lc0), lg_h(1, dx) + lg_h(1, dyp)));
+    const float e1 = fmaf(-fabsf(q.w - g1.w), iz1[dx != 0 && dyq != 0], fmaf(-sl1, fabsf(lum(cq) - lc1), lg_h(1, dx) + lg_h(1, dyq)));
+    const float2 wt = __fmul2_rn(pp, make_float2(ex2_approx(e0), ex2_approx(e1)));
+    const float2 ww = __fmul2_rn(wt, wt);
+    if (ok0) { sw0 += wt.x; x0 += wt.x * cp.x; y0 += wt.x * cp.y; b0 += wt.x * cp.z; v0 += ww.x * cp.w; }
+    if (ok1) { sw1 += wt.y; x1 += wt.y * cq.x; y1 += wt.y * cq.y; b1 += wt.y * cq.z; v1 += ww.y * cq.w; }
+  };
+#pragma unroll
+  for (int dx = -1; dx <= 1; dx++) tap(sG[ti - SW + dx], sA[ti - SW + dx], -1, sG[ti + 2 * SW + dx], sA[ti + 2 * SW + dx], 1, dx);
+  tap(g1, a1, 1, g0, a0, -1, 0);
+#pragma unroll
+  for (int dx = -1; dx <= 1; dx += 2) {
+    const float4 p0 = sG[ti + dx], c0 = sA[ti + dx], p1 = sG[ti + SW + dx], c1 = sA[ti + SW + dx];
+    tap(p0, c0, 0, p0, c0, -1, dx);
+    tap(p1, c1, 1, p1, c1, 0, dx);
   }
-  if (inner) {
-    if (li == 0) {
-      umma::mbar_init(mb, 1);
-      tma_expect(mb, FB_W * FB_H * 16);
-      tma_load_2d(umma::smem_u32(stA), &M.a0, bx - 2, by - 1, mb);
-      tma_load_2d(umma::smem_u32(stK), &M.key, bx - 2, by - 1, mb);
+  out0 = make_float4(x0 / sw0, y0 / sw0, b0 / sw0, v0 / (sw0 * sw0));
+  out1 = make_float4(x1 / sw1, y1 / sw1, b1 / sw1, v1 / (sw1 * sw1));
+}
+
+// The texels of one tile as they lie in memory (the copies' targets) and decoded (what the taps read).
+struct FineSmem {
+  static constexpr int SW = FF_W + 2, SH = FF_H + 2;
+  static constexpr int NH = FH_W * FH_H, NQ = FQ_W * FQ_H, NP = (FF_W / 2) * (FF_H / 2);
+  float4 a[SW * SH], g[SW * SH];                // A0 and the decoded key, apron 1
+  float4 hg[NH], ha[NH], hb[NH], qg[NQ], qc[NQ], par[NP];
+  alignas(16) uint2 ra[FB_W * FB_H], rk[FB_W * FB_H];  // A0 / key from column bx - 2
+  float4 rhg[NH], rqg[NQ];
+  uint2 rha[NH], rhb[NH], rqc[NQ], rp0[NP], rp1[NP], rp2[NP], mat[2][FF_NT], emi[2][FF_NT];
+};
+
+// Starts the copies of tile (bx, by)'s texels into the raw half of S and commits them as one group.
+HD_INL void fine_issue(const HushFrame &f, FineSmem &S, int li, int bx, int by) {
+  constexpr int SW = FineSmem::SW, NH = FineSmem::NH, NQ = FineSmem::NQ, NP = FineSmem::NP;
+  const bool interior = bx - 2 >= 0 && by - 1 >= 0 && bx + FF_W + 2 <= f.W && by + FF_H + 1 <= f.H;
+  if (interior && !(f.W & 1)) {  // even rows and columns of 8-byte texels: 16-byte copies of texel pairs
+    for (int i = li; i < FB_W / 2 * FB_H; i += FF_NT) {
+      const int r = i / (FB_W / 2), c = 2 * (i % (FB_W / 2)), q = (by - 1 + r) * f.W + bx - 2 + c;
+      cp_async16(S.ra + r * FB_W + c, f.A0 + q);
+      cp_async16(S.rk + r * FB_W + c, f.key + q);
+    }
+  } else {
+    for (int i = li; i < SW * FineSmem::SH; i += FF_NT) {
+      const int r = i / SW, c = i % SW;
+      const int q = clampi(by - 1 + r, 0, f.H - 1) * f.W + clampi(bx - 1 + c, 0, f.W - 1);
+      cp_async8(S.ra + r * FB_W + c + 1, f.A0 + q);
+      cp_async8(S.rk + r * FB_W + c + 1, f.key + q);
     }
   }
-  const int hx0 = bx / 2 - 1, hy0 = by / 2 - 1, qx0 = bx / 4 - 1, qy0 = by / 4 - 1;
   if (li < NH) {
-    const int q = clampi(hy0 + li / FH_W, 0, f.H2 - 1) * f.W2 + clampi(hx0 + li % FH_W, 0, f.W2 - 1);
-    sHG[li] = __ldg(f.Gd + q);
-    sHA[li] = ldh(f.Ah, q);
-    sHB[li] = ldh(f.Bh0, q);
+    const int q = clampi(by / 2 - 1 + li / FH_W, 0, f.H2 - 1) * f.W2 + clampi(bx / 2 - 1 + li % FH_W, 0, f.W2 - 1);
+    cp_async16(S.rhg + li, f.Gd + q);
+    cp_async8(S.rha + li, f.Ah + q);
+    cp_async8(S.rhb + li, f.Bh0 + q);
   } else if (li < NH + NQ) {
     const int i = li - NH;
-    const int r = clampi(qy0 + i / FQ_W, 0, f.H4 - 1) * f.W4 + clampi(qx0 + i % FQ_W, 0, f.W4 - 1);
-    sQG[i] = __ldg(f.CGd + r);
-    sQC[i] = ldh(f.C0, r);
-  } else if (li < NH + NQ + NP) {
-    const int i = li - NH - NQ;
-    const int hq = clampi(by / 2 + i / (FT_W / 2), 0, f.H2 - 1) * f.W2 + clampi(bx / 2 + i % (FT_W / 2), 0, f.W2 - 1);
-    const float4 p0 = ldh(f.par0, hq);
-    sPar[i] = make_float4(ldh(f.par1, hq).x, ldh(f.par2, hq).x, p0.z, p0.w);  // s0, c0, beta, kappa
+    const int r = clampi(by / 4 - 1 + i / FQ_W, 0, f.H4 - 1) * f.W4 + clampi(bx / 4 - 1 + i % FQ_W, 0, f.W4 - 1);
+    cp_async16(S.rqg + i, f.CGd + r);
+    cp_async8(S.rqc + i, f.C0 + r);
   }
-  bool staged = false;
-  if (inner) {
-    __syncthreads();  // the mbarrier's initialisation, before anyone waits on it
-    staged = tma_wait_or_flag(f, mb);
-    if (staged)
-      for (int i = li; i < SW * SH; i += FT_W * FT_H) {
-        const int t = (i / SW) * FB_W + i % SW + 1;
-        sA[i] = h4_to_f4(stA[t]);
-        const float4 k = h4_to_f4(stK[t]);
-        float4 g = oct_dec(k.x, k.y);
-        g.w = k.z;
-        sG[i] = g;
-      }
+  if (li >= FF_NT - NP) {
+    const int i = li - (FF_NT - NP);
+    const int hq = clampi(by / 2 + i / (FF_W / 2), 0, f.H2 - 1) * f.W2 + clampi(bx / 2 + i % (FF_W / 2), 0, f.W2 - 1);
+    cp_async8(S.rp0 + i, f.par0 + hq);
+    cp_async8(S.rp1 + i, f.par1 + hq);
+    cp_async8(S.rp2 + i, f.par2 + hq);
   }
-  if (!staged) {
-    for (int i = li; i < SW * SH; i += FT_W * FT_H) {
-      const int q = clampi(by - AP + i / SW, 0, f.H - 1) * f.W + clampi(bx - AP + i % SW, 0, f.W - 1);
-      sA[i] = ldh(f.A0, q);
-      const float4 k = ldh(f.key, q);
-      float4 g = oct_dec(k.x, k.y);
-      g.w = k.z;
-      sG[i] = g;
-    }
+  const int px = min(bx + li % FF_W, f.W - 1), py = by + 2 * (li / FF_W);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int y = min(py + k, f.H - 1);
+    cp_async8(&S.mat[k][li], f.mat + y * f.p_mat + px);
+    cp_async8(&S.emi[k][li], f.emi + y * f.p_emi + px);
   }
-  __syncthreads();
-  if (!in_img) return;
-  const int lx = li % FT_W + AP, ly = li / FT_W + AP;
-  const float4 alb = h4_to_f4(mat_r), emi = h4_to_f4(emi_r);
-  const float4 gp = sG[ly * SW + lx];
+  cp_async_commit();
+}
+
+// The two pixels of thread li of tile (bx, by) from the decoded half of S.
+HD_INL void fine_pixels(const HushFrame &f, const FineSmem &S, int li, int bx, int by, const uint2 *mat_r,
+                        const uint2 *emi_r) {
+  constexpr int AP = 1, SW = FineSmem::SW;
+  const bool interior = bx - 1 >= 0 && by - 1 >= 0 && bx + FF_W + 1 <= f.W && by + FF_H + 1 <= f.H;
+  const int px = bx + li % FF_W, py = by + 2 * (li / FF_W);
+  const bool in0 = px < f.W && py < f.H, in1 = in0 && py + 1 < f.H;
+  if (!in0) return;
+  const int hx0 = bx / 2 - 1, hy0 = by / 2 - 1, qx0 = bx / 4 - 1, qy0 = by / 4 - 1;
+  const int ti = (py - by + AP) * SW + px - bx + AP;
+  const float4 gp0 = S.g[ti], gp1 = S.g[ti + SW];
+  const bool live0 = gp0.w >= 0.0f, live1 = in1 && gp1.w >= 0.0f;
   const int o = py * f.W + px;
-  if (gp.w < 0.0f) {
-    sth(f.hist, o, make_float4(0.f, 0.f, 0.f, 0.f));
-    sth(f.X, o, make_float4(emi.x, emi.y, emi.z, 0.f));
-    return;
-  }
-  const float4 pr = sPar[((py - by) >> 1) * (FT_W / 2) + ((px - bx) >> 1)];
-  const float4 A1 = interior ? filt_x<1, 1, true, SW, false>(sA, sG, lx, ly, px, py, f.W, f.H, pr.x, pr.y)
-                             : filt_x<1, 1, true, SW, true>(sA, sG, lx, ly, px, py, f.W, f.H, pr.x, pr.y);
-  sth(f.hist, o, A1);
-  // recombination (hush.js:580-620) with the half-res block means (Ah) and decoded guides (Gd, CGd)
-  const float fx = qf16(A1.x), fy = qf16(A1.y), fz = qf16(A1.z);
-  const float z = gp.w;
-  const float rzl = LOG2E / (0.05f * z + 1e-3f);
-  const int hsx = (f.W + 1) / 2, hsy = (f.H + 1) / 2;
-  const float hposx = ((float)px + 0.5f) / 2.0f - 0.5f, hposy = ((float)py + 0.5f) / 2.0f - 0.5f;
-  const float hbx = floorf(hposx), hby = floorf(hposy);
-  const int qsx = (f.W + 3) / 4, qsy = (f.H + 3) / 4;
-  const float cposx = ((float)px + 0.5f) / 4.0f - 0.5f, cposy = ((float)py + 0.5f) / 4.0f - 0.5f;
-  const float cbx = floorf(cposx), cby = floorf(cposy);
-  // jbw() of two taps at a time: the (n.n)^8 and weight products as packed FP32x2, the accumulation in tap order
+  auto sky = [&](int oo, uint2 er) {
+    const float4 emi = h4_to_f4(er);
+    sth(f.hist, oo, make_float4(0.f, 0.f, 0.f, 0.f));
+    sth(f.X, oo, make_float4(emi.x, emi.y, emi.z, 0.f));
+  };
+  if (!live0) sky(o, emi_r[0]);
+  if (in1 && !live1) sky(o + f.W, emi_r[1]);
+  if (!live0 && !live1) return;
+  const float4 pr = S.par[((py - by) >> 1) * (FF_W / 2) + ((px - bx) >> 1)];
+  float4 A0v, A1v;
+  if (interior) filt_v2<SW, false>(S.a, S.g, ti, px, py, f.W, f.H, pr.x, pr.y, A0v, A1v);
+  else filt_v2<SW, true>(S.a, S.g, ti, px, py, f.W, f.H, pr.x, pr.y, A0v, A1v);
+  if (live0) sth(f.hist, o, A0v);
+  if (live1) sth(f.hist, o + f.W, A1v);
+  // recombination (hush.js:580-620) of both pixels with the half-res block means (Ah) and decoded guides (Gd, CGd)
+  const float3 f0 = make_float3(qf16(A0v.x), qf16(A0v.y), qf16(A0v.z)), f1 = make_float3(qf16(A1v.x), qf16(A1v.y), qf16(A1v.z));
+  const float2 rzl = make_float2(LOG2E / (0.05f * gp0.w + 1e-3f), LOG2E / (0.05f * gp1.w + 1e-3f));
+  // jbw() of one tap of each pixel: the (n.n)^8 and weight products as packed FP32x2
   auto jbw2 = [&](float2 wb, float4 n0, float4 n1) {
-    const float2 d = make_float2(fmaxf(dot3(n0, gp), 0.0f), fmaxf(dot3(n1, gp), 0.0f));
+    const float2 d = make_float2(fmaxf(dot3(n0, gp0), 0.0f), fmaxf(dot3(n1, gp1), 0.0f));
     const float2 d2 = __fmul2_rn(d, d), d4 = __fmul2_rn(d2, d2);
-    const float2 e = make_float2(ex2_approx(-fabsf(n0.w - z) * rzl), ex2_approx(-fabsf(n1.w - z) * rzl));
+    const float2 e = make_float2(ex2_approx(-fabsf(n0.w - gp0.w) * rzl.x), ex2_approx(-fabsf(n1.w - gp1.w) * rzl.y));
     return __fmul2_rn(__fmul2_rn(__fmul2_rn(wb, e), d4), d4);
   };
-  auto wbx = [](float fx_, float fy_, int j) {
-    return ((j & 1) == 1 ? fx_ : 1.0f - fx_) * ((j >> 1) == 1 ? fy_ : 1.0f - fy_);
+  // the bilinear phase: py is even, so pixel 0 lies 3/4 and pixel 1 1/4 of a half-res row below its base row (rows
+  // r, r + 1 and r + 1, r + 2), and both share their quarter-res rows
+  const float hposx = ((float)px + 0.5f) / 2.0f - 0.5f, hbx = floorf(hposx), hfx = hposx - hbx;
+  const float cposx = ((float)px + 0.5f) / 4.0f - 0.5f, cbx = floorf(cposx), cfx = cposx - cbx;
+  const float cpos0 = ((float)py + 0.5f) / 4.0f - 0.5f, cpos1 = ((float)py + 1.5f) / 4.0f - 0.5f, cby = floorf(cpos0);
+  struct Sum { float bx, by, bz, ax, ay, az, w; };
+  Sum u0 = {}, u1 = {};
+  auto add = [](Sum &u, float w, float4 m, float4 a) {
+    u.w += w;
+    u.bx += w * m.x; u.by += w * m.y; u.bz += w * m.z;
+    u.ax += w * a.x; u.ay += w * a.y; u.az += w * a.z;
   };
-  float uBx = 0.f, uBy = 0.f, uBz = 0.f, uAx = 0.f, uAy = 0.f, uAz = 0.f, swh = 0.f;
-  const float hfx = hposx - hbx, hfy = hposy - hby;
+  const int hr = (py >> 1) - 1, hc = (int)hbx;
 #pragma unroll
-  for (int j = 0; j < 4; j += 2) {
-    const int qy = (int)hby + (j >> 1);
-    const int qx0 = (int)hbx, qx1 = qx0 + 1;
-    const int t0 = (qy - hy0) * FH_W + (qx0 - hx0), t1 = t0 + 1;
-    const float4 g0 = sHG[t0], g1 = sHG[t1];
-    const bool iy = qy >= 0 && qy < hsy;
-    const bool ok0 = iy && qx0 >= 0 && qx0 < hsx && g0.w >= 0.0f, ok1 = iy && qx1 >= 0 && qx1 < hsx && g1.w >= 0.0f;
-    const float2 w = jbw2(make_float2(wbx(hfx, hfy, j), wbx(hfx, hfy, j + 1)), g0, g1);
-    if (ok0) {
-      const float4 a = sHA[t0], m = sHB[t0];
-      swh += w.x;
-      uBx += w.x * m.x; uBy += w.x * m.y; uBz += w.x * m.z;
-      uAx += w.x * a.x; uAy += w.x * a.y; uAz += w.x * a.z;
+  for (int j = 0; j < 2; j++) {  // columns: rows r of pixel 0 and r + 2 of pixel 1 as one pair, row r + 1 for both
+    const int t = (hr - hy0) * FH_W + hc + j - hx0;
+    const float wx = j ? hfx : 1.0f - hfx;
+    const bool ix = hc + j >= 0 && hc + j < f.W2;
+    const float4 ga = S.hg[t], gm = S.hg[t + FH_W], gb = S.hg[t + 2 * FH_W];
+    const float2 wo = jbw2(make_float2(wx * 0.25f, wx * 0.25f), ga, gb);
+    const float2 wm = jbw2(make_float2(wx * 0.75f, wx * 0.75f), gm, gm);
+    if (ix && hr >= 0 && ga.w >= 0.0f) add(u0, wo.x, S.hb[t], S.ha[t]);
+    if (ix && gm.w >= 0.0f) {
+      const float4 m = S.hb[t + FH_W], a = S.ha[t + FH_W];
+      add(u0, wm.x, m, a);
+      add(u1, wm.y, m, a);
     }
-    if (ok1) {
-      const float4 a = sHA[t1], m = sHB[t1];
-      swh += w.y;
-      uBx += w.y * m.x; uBy += w.y * m.y; uBz += w.y * m.z;
-      uAx += w.y * a.x; uAy += w.y * a.y; uAz += w.y * a.z;
-    }
+    if (ix && hr + 2 < f.H2 && gb.w >= 0.0f) add(u1, wo.y, S.hb[t + 2 * FH_W], S.ha[t + 2 * FH_W]);
   }
-  float ix = fx, iy = fy, iz = fz;
-  if (swh > 1e-4f) {
-    ix = uBx / swh + pr.w * (fx - uAx / swh);
-    iy = uBy / swh + pr.w * (fy - uAy / swh);
-    iz = uBz / swh + pr.w * (fz - uAz / swh);
-  }
-  float uCx = 0.f, uCy = 0.f, uCz = 0.f, swq = 0.f;
-  const float cfx = cposx - cbx, cfy = cposy - cby;
+  float3 i0 = f0, i1 = f1;
+  auto mix = [&](float3 fv, const Sum &u) {
+    if (!(u.w > 1e-4f)) return fv;
+    return make_float3(u.bx / u.w + pr.w * (fv.x - u.ax / u.w), u.by / u.w + pr.w * (fv.y - u.ay / u.w),
+                       u.bz / u.w + pr.w * (fv.z - u.az / u.w));
+  };
+  i0 = mix(f0, u0);
+  i1 = mix(f1, u1);
+  float c0x = 0.f, c0y = 0.f, c0z = 0.f, w0 = 0.f, c1x = 0.f, c1y = 0.f, c1z = 0.f, w1 = 0.f;
+  const float cf0 = cpos0 - cby, cf1 = cpos1 - cby;
 #pragma unroll
-  for (int j = 0; j < 4; j += 2) {
-    const int ry = (int)cby + (j >> 1);
-    const int rx0 = (int)cbx, rx1 = rx0 + 1;
-    const int t0 = (ry - qy0) * FQ_W + (rx0 - qx0), t1 = t0 + 1;
-    const float4 g0 = sQG[t0], g1 = sQG[t1];
-    const bool iy = ry >= 0 && ry < qsy;
-    const bool ok0 = iy && rx0 >= 0 && rx0 < qsx && g0.w >= 0.0f, ok1 = iy && rx1 >= 0 && rx1 < qsx && g1.w >= 0.0f;
-    const float2 w = jbw2(make_float2(wbx(cfx, cfy, j), wbx(cfx, cfy, j + 1)), g0, g1);
-    if (ok0) {
-      const float4 c = sQC[t0];
-      swq += w.x;
-      uCx += w.x * c.x; uCy += w.x * c.y; uCz += w.x * c.z;
-    }
-    if (ok1) {
-      const float4 c = sQC[t1];
-      swq += w.y;
-      uCx += w.y * c.x; uCy += w.y * c.y; uCz += w.y * c.z;
+  for (int j = 0; j < 4; j++) {
+    const int ry = (int)cby + (j >> 1), rx = (int)cbx + (j & 1);
+    const int t = (ry - qy0) * FQ_W + rx - qx0;
+    const float4 g = S.qg[t];
+    const float wx = (j & 1) ? cfx : 1.0f - cfx;
+    const float2 w = jbw2(make_float2(wx * ((j >> 1) ? cf0 : 1.0f - cf0), wx * ((j >> 1) ? cf1 : 1.0f - cf1)), g, g);
+    if (ry >= 0 && ry < f.H4 && rx >= 0 && rx < f.W4 && g.w >= 0.0f) {
+      const float4 c = S.qc[t];
+      w0 += w.x; c0x += w.x * c.x; c0y += w.x * c.y; c0z += w.x * c.z;
+      w1 += w.y; c1x += w.y * c.x; c1y += w.y * c.y; c1z += w.y * c.z;
     }
   }
-  float upx = ix, upy = iy, upz = iz;
-  if (swq > 1e-4f) { upx = uCx / swq; upy = uCy / swq; upz = uCz / swq; }
-  ix = ix + (upx - ix) * pr.z;
-  iy = iy + (upy - iy) * pr.z;
-  iz = iz + (upz - iz) * pr.z;
-  sth(f.X, o, make_float4(ix * alb.x + emi.x, iy * alb.y + emi.y, iz * alb.z + emi.z, 0.0f));
+  auto finish = [&](int oo, float3 i, float cx, float cy, float cz, float w, uint2 mr, uint2 er) {
+    const float4 alb = h4_to_f4(mr), emi = h4_to_f4(er);
+    float3 up = i;
+    if (w > 1e-4f) up = make_float3(cx / w, cy / w, cz / w);
+    i = make_float3(i.x + (up.x - i.x) * pr.z, i.y + (up.y - i.y) * pr.z, i.z + (up.z - i.z) * pr.z);
+    sth(f.X, oo, make_float4(i.x * alb.x + emi.x, i.y * alb.y + emi.y, i.z * alb.z + emi.z, 0.0f));
+  };
+  if (live0) finish(o, i0, c0x, c0y, c0z, w0, mat_r[0], emi_r[0]);
+  if (live1) finish(o + f.W, i1, c1x, c1y, c1z, w1, mat_r[1], emi_r[1]);
+}
+
+// Each CTA walks over tiles (blockIdx.x, + gridDim.x, ...): the next tile's texels fly into the raw buffers while this
+// tile's pixels are filtered, so only a CTA's first tile waits for memory.
+__global__ void __launch_bounds__(FF_NT, 2) k_fine_final_fused(const __grid_constant__ HushFrame f, int tiles_x, int tiles) {
+  constexpr int AP = 1, SW = FineSmem::SW, SH = FineSmem::SH;
+  constexpr int NH = FineSmem::NH, NQ = FineSmem::NQ, NP = FineSmem::NP;
+  static_assert(NH + NQ <= FF_NT && NP <= FF_NT, "one footprint texel and one block's parameters per thread");
+  extern __shared__ __align__(16) unsigned char ff_smem[];
+  FineSmem &S = *reinterpret_cast<FineSmem *>(ff_smem);
+  const int li = threadIdx.x;
+  int tile = blockIdx.x;
+  fine_issue(f, S, li, tile % tiles_x * FF_W, tile / tiles_x * FF_H);
+  for (; tile < tiles; tile += gridDim.x) {
+    const int bx = tile % tiles_x * FF_W, by = tile / tiles_x * FF_H;
+    cp_async_wait<0>();
+    __syncthreads();  // the tile's texels are here, and the previous tile's taps are done with the decoded half
+    for (int i = li; i < SW * SH; i += FF_NT) {
+      const int t = (i / SW) * FB_W + i % SW + 1;
+      S.a[i] = h4_to_f4(S.ra[t]);
+      const float4 k = h4_to_f4(S.rk[t]);
+      float4 g = oct_dec(k.x, k.y);
+      g.w = k.z;
+      S.g[i] = g;
+    }
+    if (li < NH) {
+      S.hg[li] = S.rhg[li];
+      S.ha[li] = h4_to_f4(S.rha[li]);
+      S.hb[li] = h4_to_f4(S.rhb[li]);
+    } else if (li < NH + NQ) {
+      S.qg[li - NH] = S.rqg[li - NH];
+      S.qc[li - NH] = h4_to_f4(S.rqc[li - NH]);
+    }
+    if (li >= FF_NT - NP) {
+      const int i = li - (FF_NT - NP);
+      const float4 p0 = h4_to_f4(S.rp0[i]);
+      S.par[i] = make_float4(h4_to_f4(S.rp1[i]).x, h4_to_f4(S.rp2[i]).x, p0.z, p0.w);  // s0, c0, beta, kappa
+    }
+    const uint2 mat_r[2] = {S.mat[0][li], S.mat[1][li]}, emi_r[2] = {S.emi[0][li], S.emi[1][li]};
+    __syncthreads();
+    const int next = tile + gridDim.x;
+    if (next < tiles) fine_issue(f, S, li, next % tiles_x * FF_W, next / tiles_x * FF_H);
+    fine_pixels(f, S, li, bx, by, mat_r, emi_r);
+  }
 }
 
 // TAA (hush.js:639-677) with a 32 x 8 tile. The pixel's motion, colour and the four history texels of its bilinear
@@ -1427,36 +1520,6 @@ static const HalfMaps &half_maps(const HushFrame &f) {
   return c.m;
 }
 
-// FINE_FINAL's maps for the frame's A0 and key (which alternates with the frame parity: two cached entries).
-static const FineMaps &fine_maps(const HushFrame &f) {
-  struct Entry {
-    const void *a0 = nullptr, *key = nullptr;
-    int w = -1, h = -1;
-    FineMaps m{};
-  };
-  static thread_local Entry c[2];
-  static thread_local int next = 0;
-  for (Entry &e : c)
-    if (e.a0 == f.A0 && e.key == f.key && e.w == f.W && e.h == f.H) return e.m;
-  Entry &e = c[next];
-  next ^= 1;
-  e.a0 = f.A0; e.key = f.key; e.w = f.W; e.h = f.H;
-  std::memset(&e.m, 0, sizeof(e.m));
-  const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-  if (!enc || (f.W & 1) || f.W < FB_W || f.H < FB_H) return e.m;
-  const cuuint32_t one[2] = {1, 1};
-  const cuuint64_t dim[2] = {(cuuint64_t)f.W, (cuuint64_t)f.H};
-  const cuuint64_t str[1] = {(cuuint64_t)f.W * 8};
-  const cuuint32_t box[2] = {(cuuint32_t)FB_W, (cuuint32_t)FB_H};
-  auto lv = [&](CUtensorMap *m, const void *p) {
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void *>(p), dim, str, box, one,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  };
-  e.m.ok = (lv(&e.m.a0, f.A0) == CUDA_SUCCESS && lv(&e.m.key, f.key) == CUDA_SUCCESS) ? 1 : 0;
-  return e.m;
-}
-
 cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const MlpConst &mc, int mlp_mode,
                                const void *mlp_tc, cudaStream_t st) {
   const int hx = (f.W2 + HT_W - 1) / HT_W, hy = (f.H2 + HT_H - 1) / HT_H;
@@ -1505,9 +1568,23 @@ cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const Ml
       if (part == HP_COARSE) break;  // no coarse level in stage 3
       k_half_pair<3, HP_MID><<<hpx * hy, HT_W * HT_H, mid_pair_smem<4>(), st>>>(f, hpx, hpx * hy, qx, half_maps(f));
       break;
-    case 4:
-      k_fine_final_fused<<<dim3((f.W + FT_W - 1) / FT_W, (f.H + FT_H - 1) / FT_H), FT_W * FT_H, 0, st>>>(f, fine_maps(f));
+    case 4: {
+      const int tx = (f.W + FF_W - 1) / FF_W, tiles = tx * ((f.H + FF_H - 1) / FF_H);
+      int dev = 0;
+      cudaGetDevice(&dev);
+      if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+      static int sms[64] = {};  // and, once it is known, the shared-memory opt-in is done
+      if (!sms[dev]) {
+        int n = 0;
+        cudaError_t e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess)
+          e = cudaFuncSetAttribute(k_fine_final_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FineSmem));
+        if (e != cudaSuccess) return e;
+        sms[dev] = n;
+      }
+      k_fine_final_fused<<<std::min(tiles, 2 * sms[dev]), FF_NT, sizeof(FineSmem), st>>>(f, tx, tiles);
       break;
+    }
     case 5: k_taa_fused<<<dim3((f.W + FT_W - 1) / FT_W, (f.H + FT_H - 1) / FT_H), FT_W * FT_H, 0, st>>>(f); break;
     default: return cudaErrorInvalidValue;
   }
@@ -1526,7 +1603,7 @@ int fused_kernel_param_count(const void *func) {
                          (const void *)k_half_pair<3, HP_MID>};
   for (const void *k : half)
     if (func == k) return 5;  // (f, nAx, nA, nBx, M)
-  if (func == (const void *)k_fine_final_fused) return 2;  // (f, M)
+  if (func == (const void *)k_fine_final_fused) return 3;  // (f, tiles_x, tiles)
   if (func == (const void *)k_taa_fused) return 1;          // (f)
   return 0;
 }
