@@ -663,6 +663,19 @@ __global__ void __launch_bounds__(TW *TH) k_fine_fwd(const TwinFrame T) {
 
 // ------------------------------------------------------------------------------------------------ TAA
 HD_INL float3 tm3(float4 c) { return tmap(make_float3(c.x, c.y, c.z)); }
+// The luminance with its roundings written out: (r, then g, then b) and (g, then r, then b). Which of the two the compiler takes
+// for lum3() depends on the code around it, and the clip flags and the signs of the loss turn on the last bit; so each use in
+// the TAA below names one, and the frame does not change with the kernels it is inlined in.
+HD_INL float lum_rgb(float3 c) { return __fmaf_rn(c.z, 0.0722f, __fmaf_rn(c.y, 0.7152f, __fmul_rn(c.x, 0.2126f))); }
+HD_INL float lum_grb(float3 c) { return __fmaf_rn(c.z, 0.0722f, __fmaf_rn(c.x, 0.2126f, __fmul_rn(c.y, 0.7152f))); }
+HD_INL float3 tmap_by(float3 c, float l) {
+  const float d = 1.0f + l;
+  return make_float3(c.x / d, c.y / d, c.z / d);
+}
+HD_INL float3 tmap_cur(float4 c) {
+  const float3 v = make_float3(c.x, c.y, c.z);
+  return tmap_by(v, lum_grb(v));
+}
 
 struct TaaF {
   float3 y[9], m1, sd, v3, cur, hh0, hh, hr, res, out;
@@ -670,12 +683,13 @@ struct TaaF {
   float d;
 };
 
-// y(j): the YCoCg colour of the j-th texel of the clamped 3 x 3 window
+// y(j): the YCoCg colour of the j-th texel of the clamped 3 x 3 window. adj: with what the adjoint takes, which has always formed
+// the clip box from differences rounded twice and the history's luminance in the other order; its flags are of those.
 template <class Window>
-HD_INL void taa_fwd(const TwinFrame &T, int px, int py, TaaF &A, const Window &y) {
+HD_INL void taa_fwd(const TwinFrame &T, int px, int py, TaaF &A, bool adj, const Window &y) {
   const HushFrame &f = T.f;
   const int o = py * f.W + px;
-  A.cur = tm3(T.X[o]);
+  A.cur = tmap_cur(T.X[o]);
   A.inside = false;
   for (int j = 0; j < 9; j++) A.y[j] = y(j);
   A.res = A.cur;
@@ -683,16 +697,28 @@ HD_INL void taa_fwd(const TwinFrame &T, int px, int py, TaaF &A, const Window &y
   if (!f.reset) {
     float3 m1 = make_float3(0.f, 0.f, 0.f);
     for (int j = 0; j < 9; j++) { m1.x += A.y[j].x; m1.y += A.y[j].y; m1.z += A.y[j].z; }
+    const float3 s1 = m1;
     m1.x /= 9.0f; m1.y /= 9.0f; m1.z /= 9.0f;
     float3 v3 = make_float3(0.f, 0.f, 0.f);
     for (int j = 0; j < 9; j++) {
-      const float dx = A.y[j].x - m1.x, dy = A.y[j].y - m1.y, dz = A.y[j].z - m1.z;
-      v3.x += dx * dx; v3.y += dy * dy; v3.z += dz * dz;
+      // y - sum / 9 as one FMA (also written out)
+      const float dx = __fmaf_rn(-s1.x, 1.0f / 9.0f, A.y[j].x), dy = __fmaf_rn(-s1.y, 1.0f / 9.0f, A.y[j].y),
+                  dz = __fmaf_rn(-s1.z, 1.0f / 9.0f, A.y[j].z);
+      v3.x = __fmaf_rn(dx, dx, v3.x); v3.y = __fmaf_rn(dy, dy, v3.y); v3.z = __fmaf_rn(dz, dz, v3.z);
     }
     v3.x /= 9.0f; v3.y /= 9.0f; v3.z /= 9.0f;
+    const float3 sd = make_float3(sqrtf(fmaxf(v3.x, 1e-12f)), sqrtf(fmaxf(v3.y, 1e-12f)), sqrtf(fmaxf(v3.z, 1e-12f)));
     A.m1 = m1;
-    A.v3 = v3;
-    A.sd = make_float3(sqrtf(fmaxf(v3.x, 1e-12f)), sqrtf(fmaxf(v3.y, 1e-12f)), sqrtf(fmaxf(v3.z, 1e-12f)));
+    if (adj) {
+      float3 va = make_float3(0.f, 0.f, 0.f);
+      for (int j = 0; j < 9; j++) {
+        const float dx = __fsub_rn(A.y[j].x, m1.x), dy = __fsub_rn(A.y[j].y, m1.y), dz = __fsub_rn(A.y[j].z, m1.z);
+        va.x = __fmaf_rn(dx, dx, va.x); va.y = __fmaf_rn(dy, dy, va.y); va.z = __fmaf_rn(dz, dz, va.z);
+      }
+      va.x /= 9.0f; va.y /= 9.0f; va.z /= 9.0f;
+      A.v3 = va;
+      A.sd = make_float3(sqrtf(fmaxf(va.x, 1e-12f)), sqrtf(fmaxf(va.y, 1e-12f)), sqrtf(fmaxf(va.z, 1e-12f)));
+    }
     const float4 mv = ldh(f.mv, py * f.p_mv + px);
     const float szx = (float)f.W, szy = (float)f.H;
     const float uvx = ((float)px + 0.5f + mv.x) / szx, uvy = ((float)py + 0.5f + mv.y) / szy;
@@ -708,14 +734,19 @@ HD_INL void taa_fwd(const TwinFrame &T, int px, int py, TaaF &A, const Window &y
         const float4 t = ldh(f.taa_prev, clampi((int)byf + oy, 0, f.H - 1) * f.W + clampi((int)bxf + ox, 0, f.W - 1));
         hist.x += wb * t.x; hist.y += wb * t.y; hist.z += wb * t.z;
       }
-      A.hh0 = to_ycocg(tmap(hist));
-      float h0[3] = {A.hh0.x, A.hh0.y, A.hh0.z}, mm[3] = {m1.x, m1.y, m1.z}, ss[3] = {A.sd.x, A.sd.y, A.sd.z}, hc[3];
-      for (int c = 0; c < 3; c++) {
-        const float lo = mm[c] - 1.25f * ss[c], hi = mm[c] + 1.25f * ss[c];
-        const float mx = fmaxf(h0[c], lo);
-        A.lo_act[c] = h0[c] < lo;
-        hc[c] = fminf(mx, hi);
-        A.hi_act[c] = mx > hi;
+      A.hh0 = to_ycocg(tmap_by(hist, lum_rgb(hist)));
+      const float h0[3] = {A.hh0.x, A.hh0.y, A.hh0.z}, mm[3] = {m1.x, m1.y, m1.z}, ss[3] = {sd.x, sd.y, sd.z};
+      float hc[3];
+      for (int c = 0; c < 3; c++)
+        hc[c] = fminf(fmaxf(h0[c], __fmaf_rn(-1.25f, ss[c], mm[c])), __fmaf_rn(1.25f, ss[c], mm[c]));
+      if (adj) {
+        const float3 ha = to_ycocg(tmap_by(hist, lum_grb(hist)));
+        const float hf[3] = {ha.x, ha.y, ha.z}, sa[3] = {A.sd.x, A.sd.y, A.sd.z};
+        for (int c = 0; c < 3; c++) {
+          const float lo = __fmaf_rn(-1.25f, sa[c], mm[c]), hi = __fmaf_rn(1.25f, sa[c], mm[c]);
+          A.lo_act[c] = hf[c] < lo;
+          A.hi_act[c] = fmaxf(hf[c], lo) > hi;
+        }
       }
       A.hh = make_float3(hc[0], hc[1], hc[2]);
       A.hr = from_ycocg(A.hh);
@@ -723,7 +754,7 @@ HD_INL void taa_fwd(const TwinFrame &T, int px, int py, TaaF &A, const Window &y
                           A.hr.z + (A.cur.z - A.hr.z) * 0.1f);
     }
   }
-  const float l = lum3(A.res.x, A.res.y, A.res.z);
+  const float l = lum_grb(A.res);
   A.act_itm = 1.0f - l > 1e-4f;
   A.d = fmaxf(1.0f - l, 1e-4f);
   A.out = make_float3(A.res.x / A.d, A.res.y / A.d, A.res.z / A.d);
@@ -734,7 +765,7 @@ constexpr int TY_W = TW + 2, TY_N = TY_W * (TH + 2);
 HD_INL void taa_stage(const TwinFrame &T, float3 *sY, int li, int bx, int by) {
   const HushFrame &f = T.f;
   for (int i = li; i < TY_N; i += TW * TH)
-    sY[i] = to_ycocg(tm3(T.X[clampi(by - 1 + i / TY_W, 0, f.H - 1) * f.W + clampi(bx - 1 + i % TY_W, 0, f.W - 1)]));
+    sY[i] = to_ycocg(tmap_cur(T.X[clampi(by - 1 + i / TY_W, 0, f.H - 1) * f.W + clampi(bx - 1 + i % TY_W, 0, f.W - 1)]));
 }
 
 // ------------------------------------------------------------------------------------------------ loss
@@ -755,14 +786,15 @@ HD_INL double loss_pixel(const TwinFrame &T, int i, float3 o, float3 &g) {
     const float cl = T.clean[3 * i + c], den = fabsf(cl) + 1e-2f;
     const double rden = 1.0 / (double)den;
     const float d = ov[c] - cl;
-    const double e = fabs((double)d) * rden;
-    l += e < 1.0 ? e : 1.0;
-    gv[c] = e < 1.0 ? sgn(d) / den : 0.0f;
+    // the clip is decided by |d| < den, which is |d| / den < 1 exactly: |d| * rden can round below 1 where |d| = den
+    const bool in = fabsf(d) < den;
+    l += in ? fabs((double)d) * rden : 1.0;
+    gv[c] = in ? sgn(d) / den : 0.0f;
     if (T.has_prev) {
       const float dd = (ov[c] - opv[c]) - (cl - T.clean_prev[3 * i + c]);
-      const double et = fabs((double)dd) * rden;
-      l += (double)T.lambda_t * (et < 1.0 ? et : 1.0);
-      gv[c] += et < 1.0 ? T.lambda_t * sgn(dd) / den : 0.0f;
+      const bool tin = fabsf(dd) < den;
+      l += (double)T.lambda_t * (tin ? fabs((double)dd) * rden : 1.0);
+      gv[c] += tin ? T.lambda_t * sgn(dd) / den : 0.0f;
     }
   }
   g = make_float3(gv[0], gv[1], gv[2]);
@@ -872,7 +904,7 @@ __global__ void __launch_bounds__(TW *TH) k_taa_bwd_coef(const TwinFrame T, cons
   if (px >= f.W || py >= f.H) return;
   const int o = py * f.W + px, t = (threadIdx.y + 1) * TY_W + threadIdx.x + 1;
   TaaF A;
-  taa_fwd(T, px, py, A, [&](int j) { return sY[t + (j / 3 - 1) * TY_W + j % 3 - 1]; });
+  taa_fwd(T, px, py, A, true, [&](int j) { return sY[t + (j / 3 - 1) * TY_W + j % 3 - 1]; });
   const float4 go = gout[o];
   taa_coef(A, make_float3(go.x, go.y, go.z), coef + 3 * o);
 }
@@ -892,7 +924,7 @@ __global__ void __launch_bounds__(TW *TH) k_taa(const TwinFrame T, int mode, flo
   if (px < f.W && py < f.H) {
     const int o = py * f.W + px, t = (threadIdx.y + 1) * TY_W + threadIdx.x + 1;
     TaaF A;
-    taa_fwd(T, px, py, A, [&](int j) { return sY[t + (j / 3 - 1) * TY_W + j % 3 - 1]; });
+    taa_fwd(T, px, py, A, mode == TAA_ADJ, [&](int j) { return sY[t + (j / 3 - 1) * TY_W + j % 3 - 1]; });
     T.out[o] = make_float4(A.out.x, A.out.y, A.out.z, 1.0f);
     sth(f.taa, o, make_float4(A.out.x, A.out.y, A.out.z, 1.0f));
     if (mode != TAA_FWD) {
