@@ -42,6 +42,8 @@ constexpr uint32_t MBAR_POLLS = 1u << 22;
 // L of a tile entry outside the image or on sky (a valid luminance is finite and far above it)
 constexpr float L_INVALID = -1e30f;
 HD_INL bool l_valid(float L) { return L > -1e29f; }
+// 1 for a valid L, else 0: 1 + 1e-20 L saturated to [0, 1] (one FMA instead of a comparison and a selection)
+HD_INL float l_counts(float L) { return __saturatef(fmaf(L, 1e-20f, 1.0f)); }
 
 // Eight values as one 16-byte operand row segment (hi), and the rounding residuals v - hi rounded again (lo): a
 // split-precision operand, hi + lo carrying 16 (bf16) or 22 (f16) significant bits of v. Two values per conversion
@@ -77,19 +79,10 @@ HD_INL void pack8_split(const float *v, uint4 &hi, uint4 &lo) {
   lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-// pixel()'s inputs to block(): P0..P4 as block() reads them and the decoded normal (Ns.w = 1 with a surface).
+// pixel()'s inputs to block() for a pixel with a surface: P0..P4 as block() reads them (P0.y, the quantised luminance, comes
+// from the tile instead) and the decoded normal.
 struct PixOut {
   float4 P0, P1, P2, P3, P4, Ns;
-};
-HD_INL PixOut pix_none() {
-  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  return PixOut{z4, z4, make_float4(0.f, 0.f, -1.0f, 0.f), z4, z4, z4};
-}
-
-// The loads of one pixel's pixel(): its G-buffer texels and the reprojection gathers of the previous frame's key,
-// colour and moments (bilinear footprint) and par0, as temporal_pixel_fast() reads them.
-struct PixLoads {
-  uint2 nd, mv, mat, k4[4], c4[4], m4[4], pq;
 };
 
 // A pixel's loads are issued as cp.async copies into a shared-memory slot (no registers held while they fly): slot
@@ -114,64 +107,47 @@ HD_INL void pixel_issue_async(const HushFrame &f, int px, int py, uint2 mvr, uin
   const int cx = __float2int_rz(floorf(ppx + 0.5f)), cy = __float2int_rz(floorf(ppy + 0.5f));
   cp_async8(g + 2 * STRIDE, f.par0_prev + (clampi(cy, 0, H - 1) >> 1) * f.W2 + (clampi(cx, 0, W - 1) >> 1));
 }
-template <int STRIDE>
-HD_INL PixLoads pixel_fetch(const uint2 *g, uint2 mvr, bool reset) {
-  PixLoads L;
-  L.nd = g[0];
-  L.mat = g[STRIDE];
-  L.mv = mvr;
-  if (!reset) {
-    L.pq = g[2 * STRIDE];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      L.k4[i] = g[(3 + i) * STRIDE];
-      L.c4[i] = g[(7 + i) * STRIDE];
-      L.m4[i] = g[(11 + i) * STRIDE];
-    }
-  }
-  return L;
+// qf16 of a value that is at most 65504 or NaN (which becomes -65504, as in qf16).
+HD_INL float qf16_low(float x) { return __uint_as_float(__float_as_uint(fmaxf(x, -65504.0f)) & 0xffffe000u); }
+
+// qf16 of feature i: all but the material means (12-15) are logarithms of FP32 values, bounded ratios or unit values.
+HD_INL float feature_qf16(int i, float x) { return i >= 12 && i < 16 ? qf16(x) : qf16_low(x); }
+
+// check_key() without normalising the decoded normal: v . n >= 0.9 |v|, tol = 0.05 zPrev + 0.01.
+HD_INL bool check_key_v(float4 k, float4 n, float zPrev, float obj, float tol) {
+  const float vz = 1.0f - fabsf(k.x) - fabsf(k.y), t = fmaxf(-vz, 0.0f);
+  const float vx = k.x - copysignf(t, k.x), vy = k.y - copysignf(t, k.y);
+  const float d = vx * n.x + vy * n.y + vz * n.z, l2 = vx * vx + vy * vy + vz * vz;
+  return k.z >= 0.0f && k.w == obj && fabsf(k.z - zPrev) <= tol && d >= 0.9f * sqrtf(l2);
 }
 
-// pixel() of hush.js:111-223 over the (r, g, b, L) tile from the preloaded texels; same arithmetic as
-// temporal_pixel(). Writes A0, mom, key and returns the pixel's inputs to block().
-template <class Tile>
-HD_INL PixOut temporal_pixel_fast(const HushFrame &f, int px, int py, const Tile &T, const PixLoads &PL) {
+// pixel() of hush.js:111-223 over the (r, g, b, L) tile from the pixel's load slot g (texel k at g[k * STRIDE]); same
+// arithmetic as temporal_pixel(). Writes A0, mom, key; returns false on sky, else the pixel's inputs to block() in o.
+template <int STRIDE, class Tile>
+HD_INL bool temporal_pixel_fast(const HushFrame &f, int px, int py, const Tile &T, const uint2 *g, uint2 mvr, PixOut &o) {
   const int W = f.W, H = f.H;
-  const float4 nd = h4_to_f4(PL.nd), mv = h4_to_f4(PL.mv);
+  const float4 nd = h4_to_f4(g[0]), mv = h4_to_f4(mvr);
   const int oi = py * W + px;
-  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
   if (nd.w < 0.0f) {
     f.A0[oi] = make_uint2(0, 0);
     f.mom[oi] = make_uint2(0, 0);
     sth(f.key, oi, make_float4(0.f, 0.f, -1.0f, mv.z));
-    return pix_none();
+    return false;
   }
-  float fx = 0.f, fy = 0.f;
-  int bix = 0, biy = 0, cx = 0, cy = 0;
-  if (!f.reset) {
-    const float ppx = (float)px + mv.x, ppy = (float)py + mv.y;
-    const float bx = floorf(ppx), by = floorf(ppy);
-    fx = ppx - bx;
-    fy = ppy - by;
-    bix = __float2int_rz(bx);
-    biy = __float2int_rz(by);
-    cx = __float2int_rz(floorf(ppx + 0.5f));
-    cy = __float2int_rz(floorf(ppy + 0.5f));
-  }
-  const uint2 *k4 = PL.k4, *c4 = PL.c4, *m4 = PL.m4;
-  const uint2 pqr = PL.pq, mrr = PL.mat;
+  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
   // 3x3 statistics of the illumination (valid neighbours), two passes
   const float4 illum = T(0, 0);
   const float l = illum.w;
   // (r, g) as one packed FP32x2 lane pair, b and (in the second pass) L as the other: the same arithmetic per lane
-  float2 s1xy = f2(0.f, 0.f);
-  float s1z = 0.f, cnt = 0.f;
+  const float4 c0 = T(-1, -1);
+  float2 s1xy = lo2(c0);
+  float s1z = c0.z, cnt = l_counts(c0.w);
 #pragma unroll
-  for (int j = 0; j < 9; j++) {
+  for (int j = 1; j < 9; j++) {
     const float4 c = T(j % 3 - 1, j / 3 - 1);
     s1xy = add2(s1xy, lo2(c));  // invalid entries hold rgb = 0
     s1z += c.z;
-    cnt += l_valid(c.w) ? 1.0f : 0.0f;
+    cnt += l_counts(c.w);
   }
   cnt = fmaxf(cnt, 1.0f);
   const float mux = s1xy.x / cnt, muy = s1xy.y / cnt, muz = s1z / cnt;
@@ -189,19 +165,29 @@ HD_INL PixOut temporal_pixel_fast(const HushFrame &f, int px, int py, const Tile
   }
   const float sdx = sqrtf(fmaxf(svxy.x / cnt, 1e-12f)), sdy = sqrtf(fmaxf(svxy.y / cnt, 1e-12f)),
               sdz = sqrtf(fmaxf(svzl.x / cnt, 1e-12f));
-  float svar = svzl.y / cnt;
+  const float svar = svzl.y / cnt;
   bool has = false;
   float hcx = 0.f, hcy = 0.f, hcz = 0.f;
   float4 hm = z4;
   float v = 0.f, alpha = 1.0f, gamma = 1.0f;
   if (!f.reset) {
+    const float ppx = (float)px + mv.x, ppy = (float)py + mv.y;
+    const float bx = floorf(ppx), by = floorf(ppy);
+    const float fx = ppx - bx, fy = ppy - by;
+    const float tol = 0.05f * mv.w + 0.01f;
+    const float wf = (float)W, hf = (float)H;
+    const bool ix[2] = {bx >= 0.0f && bx < wf, bx >= -1.0f && bx < wf - 1.0f};
+    const bool iy[2] = {by >= 0.0f && by < hf, by >= -1.0f && by < hf - 1.0f};
     float sumW = 0.f;
     const float wts[4] = {(1.0f - fx) * (1.0f - fy), fx * (1.0f - fy), (1.0f - fx) * fy, fx * fy};
+    bool ok[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      ok[i] = (wts[i] > 0.0f) & ix[i & 1] & iy[i >> 1] & check_key_v(h4_to_f4(g[(3 + i) * STRIDE]), nd, mv.w, mv.z, tol);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-      const int qx = bix + (i & 1), qy = biy + (i >> 1);
-      if (wts[i] > 0.0f && qx >= 0 && qy >= 0 && qx < W && qy < H && check_key(h4_to_f4(k4[i]), nd, mv.w, mv.z)) {
-        const float4 c = h4_to_f4(c4[i]), m = h4_to_f4(m4[i]);
+      if (ok[i]) {
+        const float4 c = h4_to_f4(g[(7 + i) * STRIDE]), m = h4_to_f4(g[(11 + i) * STRIDE]);
         const float2 w2 = bc2(wts[i]);
         sumW += wts[i];
         const float2 hxy = fma2(w2, lo2(c), f2(hcx, hcy));
@@ -217,12 +203,14 @@ HD_INL PixOut temporal_pixel_fast(const HushFrame &f, int px, int py, const Tile
       v = sumW;
       has = true;
     } else {
+      const int cx = __float2int_rz(floorf(ppx + 0.5f)), cy = __float2int_rz(floorf(ppy + 0.5f));
       float n3 = 0.f;
       hcx = hcy = hcz = 0.f;
       hm = z4;
+#pragma unroll 1
       for (int j = 0; j < 9; j++) {
         const int qx = cx + j % 3 - 1, qy = cy + j / 3 - 1;
-        if (qx >= 0 && qy >= 0 && qx < W && qy < H && check_key(ldh(f.key_prev, qy * W + qx), nd, mv.w, mv.z)) {
+        if (qx >= 0 && qy >= 0 && qx < W && qy < H && check_key_v(ldh(f.key_prev, qy * W + qx), nd, mv.w, mv.z, tol)) {
           n3 += 1.0f;
           const float4 c = ldh(f.hist_prev, qy * W + qx), m = ldh(f.mom_prev, qy * W + qx);
           hcx += c.x; hcy += c.y; hcz += c.z;
@@ -236,9 +224,9 @@ HD_INL PixOut temporal_pixel_fast(const HushFrame &f, int px, int py, const Tile
         has = true;
       }
     }
-    const float4 pq = h4_to_f4(pqr);
-    alpha = pq.x;
-    gamma = pq.y;
+    const float2 ag = unpack2(g[2 * STRIDE].x);
+    alpha = ag.x;
+    gamma = ag.y;
   }
   has = has && hm.w > 0.0f;
   float colx = illum.x, coly = illum.y, colz = illum.z;
@@ -270,16 +258,15 @@ HD_INL PixOut temporal_pixel_fast(const HushFrame &f, int px, int py, const Tile
   const float4 Aq = make_float4(qf16(A.x), qf16(A.y), qf16(A.z), qf16(A.w));
   const float m1 = E * qf16(nmx);
   const float m2 = E * E * qf16(nmy);
-  const float ox = qf16(oc.x), oy = qf16(oc.y);
-  PixOut o;
-  o.P0 = make_float4(E * lum(Aq), E * qf16(l), fmaxf(m2 - m1 * m1, 0.0f), len1);
-  o.P1 = make_float4(qf16(v), qf16(lag), E * qf16(nfast), m1);
-  o.P2 = make_float4(ox, oy, qf16(nd.w), qf16(sqrtf(mv.x * mv.x + mv.y * mv.y)));
-  o.P3 = h4_to_f4(mrr);
+  const float ox = qf16_low(oc.x), oy = qf16_low(oc.y);
+  o.P0 = make_float4(E * lum(Aq), 0.0f, fmaxf(m2 - m1 * m1, 0.0f), len1);
+  o.P1 = make_float4(qf16_low(v), qf16(lag), E * qf16(nfast), m1);
+  // (an f16 depth is its own qf16 but for infinity and NaN)
+  o.P2 = make_float4(ox, oy, fminf(fmaxf(nd.w, -65504.0f), 65504.0f), qf16(sqrtf(mv.x * mv.x + mv.y * mv.y)));
+  o.P3 = h4_to_f4(g[STRIDE]);
   o.P4 = Aq;
   o.Ns = oct_dec(ox, oy);  // block() decodes the stored oct normal (hush.js:238)
-  o.Ns.w = 1.0f;
-  return o;
+  return true;
 }
 
 HD_INL float4 scale4(float4 v, float k) { return make_float4(v.x * k, v.y * k, v.z * k, v.w * k); }
@@ -291,33 +278,43 @@ HD_INL float4 ffma4(float s, float4 w, float4 a) {  // a + s * w as two packed F
 }
 
 // ------------------------------------------------------------------------------------------------ k_temporal_block
-// One thread per 2x2 block: tile 64 x 16 pixels = 32 x 8 blocks, 256 threads. Each thread runs pixel() for its four
-// pixels in block order, accumulates block()'s sums in registers in the WGSL's order (hush.js:226-282), forms the 20
-// features once and runs the whole FP32 MLP (weights in the constant bank, a kernel parameter: each FMA takes its
-// weight as a broadcast operand), so after the tile barrier no thread waits for another. The tile is stored
-// column-parity-split (even and odd columns in separate rows of 33 entries): neighbouring threads, two pixel columns
-// apart, then read consecutive 16-byte entries. The per-pixel loads (G-buffer texels and the dependent reprojection
+// One thread per 2x2 block: tile 64 x 16 pixels = 32 x 8 blocks, 256 threads (64 x 8 and 128 for small frames). Each thread
+// runs pixel() for its four pixels in block order, accumulates block()'s sums in registers in the WGSL's order
+// (hush.js:226-282), forms the 20 features once and runs the whole FP32 MLP (weights in the constant bank, a kernel
+// parameter: each FMA takes its weight as a broadcast operand), so after the tile barrier no thread waits for another. The
+// tile is stored column-parity-split (even and odd columns in separate rows of 33 entries): neighbouring threads, two pixel
+// columns apart, then read consecutive 16-byte entries. The per-pixel loads (G-buffer texels and the dependent reprojection
 // gathers) go by cp.async into two shared-memory slots per thread, one pixel ahead: pixel q + 2's gathers are in
-// flight while pixel q + 1 computes, without holding registers. The tensor-core
-// forms instead write each block's features as one operand row and run each layer as two tcgen05 MMAs (M = 128,
+// flight while pixel q + 1 computes, without holding registers; a slot's texels are read where they are used. The
+// tensor-core forms instead write each block's features as one operand row and run each layer as two tcgen05 MMAs (M = 128,
 // N = 16) over the CTA's 256 rows, FP32 accumulators in TMEM; bias, ReLU and the heads stay FP32.
+// Bound: instruction issue and the gathers' latency at 16 warps an SM (registers and the load slots; 5 CTAs of 128 threads
+// take the L1 that the gathers hit in: 109 -> 129 us). So what is left out counts: sky pixels skip the block's sums, the
+// key test needs no normalised normal, a quantisation clamps only the sides its value can reach, a validity counts by one
+// saturating FMA. 1920x1080 FP32 119 -> 109 us (75.0 -> 71.4 M instructions), 3840x2160 bf16 530 -> 491, 256x256 16.2 -> 12.8.
 constexpr int KB_TW = 64, KB_TH = 16, KB_NT = (KB_TW / 2) * (KB_TH / 2);
-constexpr int KB_SWL = KB_TW + 2, KB_SH = KB_TH + 2, KB_HW = KB_SWL / 2;
+// Frames whose 16-row tiles fill at most the one wave of 2 x 148 CTAs an SM holds take 8-row tiles of 128 threads (4 CTAs
+// an SM) in the per-thread MLP forms, so the pixels spread over more SMs: 256x256 14.3 -> 12.8 us, 640x360 21.3 -> 18.7.
+// Beyond a wave both are even up to 1280x720 (35.8 either way at 960x540) and the larger apron share then loses
+// (1600x900 79.0 -> 82.1, 1920x1080 108.3 -> 114.4). The tensor-core forms need the CTA's 256 rows.
+constexpr int KB_HALF_CTAS = 2 * 148;
+constexpr int KB_SWL = KB_TW + 2, KB_HW = KB_SWL / 2;
 HD_INL int kb_tix(int r, int c) { return (2 * r + (c & 1)) * KB_HW + (c >> 1); }
 
 constexpr int KB_NTEX = 15;  // texels of one pixel's loads (pixel_issue_async)
+template <int TH>
 struct KbSmem {
-  float4 I[2 * KB_HW * KB_SH];   // illumination (r, g, b) and L (luminance or L_INVALID), apron 1
-  float2 Lq[2 * KB_HW * KB_SH];  // (E * qf16(L), 1) for valid entries, (0, 0) otherwise
-  uint2 G[2][KB_NTEX][KB_NT];    // two pixels' loads in flight per thread, thread-minor (conflict-free)
+  float4 I[KB_SWL * (TH + 2)];            // illumination (r, g, b) and L (luminance or L_INVALID), apron 1
+  float Lq[KB_SWL * (TH + 2)];            // E * qf16(L), or L_INVALID
+  uint2 G[2][KB_NTEX][KB_TW / 4 * TH];    // two pixels' loads in flight per thread, thread-minor (conflict-free)
 };
 // Tensor-core forms: the same tile plus the MMA operands of the CTA's 256 rows (one per block) in the K-major
 // no-swizzle layout, each as a split-precision pair (hi, lo): A1 256 x 32 (features, zero padded), A2 256 x 16
 // (hidden layers), then the weights B1 / B2 / B3 (hi, and for bf16 lo).
 // The per-pixel load slots (pixel phase) and the MMA operands (MLP phase, after a CTA barrier) share their space.
 struct KbTcSmem {
-  float4 I[2 * KB_HW * KB_SH];
-  float2 Lq[2 * KB_HW * KB_SH];
+  float4 I[KB_SWL * (KB_TH + 2)];
+  float Lq[KB_SWL * (KB_TH + 2)];
   union {
     uint2 G[2][KB_NTEX][KB_NT];
     struct {
@@ -377,12 +374,14 @@ struct ParityTile {
 
 // MODE 0: FP32 MLP per thread; 1 / 2: tensor-core MLP on split bf16 / f16 operands (dynamic shared memory);
 // 3: the reference's f16-arithmetic MLP per thread (the `f16` option).
-template <int MODE>
-__global__ void __launch_bounds__(KB_NT, 2)
+template <int MODE, int TH>
+__global__ void __launch_bounds__(KB_TW / 4 * TH, 2 * KB_TH / TH)
     k_temporal_block(const __grid_constant__ HushFrame f, const __grid_constant__ MlpConst wp,
                      const uint4 *__restrict__ blob) {
   constexpr bool TC = MODE == 1 || MODE == 2;
-  using Smem = std::conditional_t<TC, KbTcSmem, KbSmem>;
+  constexpr int NT = KB_TW / 4 * TH;
+  static_assert(!TC || TH == KB_TH, "the tensor-core forms map a CTA's blocks to 256 operand rows");
+  using Smem = std::conditional_t<TC, KbTcSmem, KbSmem<TH>>;
   extern __shared__ __align__(128) unsigned char kb_smem[];
   Smem &S = *reinterpret_cast<Smem *>(kb_smem);
   const int li = threadIdx.x;
@@ -397,12 +396,12 @@ __global__ void __launch_bounds__(KB_NT, 2)
       umma::mbar_init(umma::smem_u32(&S.mbar[1]), 1);
     }
     constexpr int NB = (MODE == 1 ? 2 : 1) * MLP_TC_BLOB_BYTES / 16;  // bf16: hi and lo weights
-    for (int i = li; i < NB; i += KB_NT) reinterpret_cast<uint4 *>(S.b)[i] = __ldg(blob + i);
+    for (int i = li; i < NB; i += NT) reinterpret_cast<uint4 *>(S.b)[i] = __ldg(blob + i);
     umma::fence_proxy_async();
     umma::fence_before_sync();
   }
   const int lbx = li % (KB_TW / 2), lby = li / (KB_TW / 2);
-  const int px0 = blockIdx.x * KB_TW + 2 * lbx, py0 = blockIdx.y * KB_TH + 2 * lby;
+  const int px0 = blockIdx.x * KB_TW + 2 * lbx, py0 = blockIdx.y * TH + 2 * lby;
   // phase 1: the four pixels' motion first (each pixel's reprojection gathers then wait for one load round trip, not
   // two), then the first pixels' loads and gathers in flight with the tile loads
   uint2 mvq[4];
@@ -411,16 +410,15 @@ __global__ void __launch_bounds__(KB_NT, 2)
     const int px = px0 + (q & 1), py = py0 + (q >> 1);
     mvq[q] = (px < f.W && py < f.H) ? __ldg(f.mv + py * f.p_mv + px) : make_uint2(0, 0);
   }
-  PixLoads PL;
-  const int ox = blockIdx.x * KB_TW - 1, oy = blockIdx.y * KB_TH - 1;
-  constexpr int N = KB_SWL * KB_SH;
+  const int ox = blockIdx.x * KB_TW - 1, oy = blockIdx.y * TH - 1;
+  constexpr int N = KB_SWL * (TH + 2);
 #pragma unroll 1
-  for (int i0 = 0; i0 < N; i0 += 2 * KB_NT) {
+  for (int i0 = 0; i0 < N; i0 += 2 * NT) {
     uint2 tn[2], tr[2], tm[2];
     bool tin[2];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
-      const int i = i0 + u * KB_NT + li;
+      const int i = i0 + u * NT + li;
       const int qx = ox + i % KB_SWL, qy = oy + i / KB_SWL;
       tin[u] = i < N && qx >= 0 && qy >= 0 && qx < f.W && qy < f.H;
       const int cx = clampi(qx, 0, f.W - 1), cy = clampi(qy, 0, f.H - 1);
@@ -432,23 +430,23 @@ __global__ void __launch_bounds__(KB_NT, 2)
 #pragma unroll
       for (int q = 0; q < 2; q++) {
         const int px = px0 + (q & 1), py = py0 + (q >> 1);
-        if (px < f.W && py < f.H) pixel_issue_async<KB_NT>(f, px, py, mvq[q], &S.G[q][0][li]);
+        if (px < f.W && py < f.H) pixel_issue_async<NT>(f, px, py, mvq[q], &S.G[q][0][li]);
         cp_async_commit();
       }
     }
 #pragma unroll
     for (int u = 0; u < 2; u++) {
-      const int i = i0 + u * KB_NT + li;
+      const int i = i0 + u * NT + li;
       if (i >= N) continue;
       float4 e = make_float4(0.f, 0.f, 0.f, L_INVALID);
-      float2 lq = make_float2(0.f, 0.f);
+      float lq = L_INVALID;
       if (tin[u] && h4_to_f4(tn[u]).w >= 0.0f) {
         const float4 r = h4_to_f4(tr[u]), m = h4_to_f4(tm[u]);
         e.x = r.x / fmaxf(m.x, 1e-3f);
         e.y = r.y / fmaxf(m.y, 1e-3f);
         e.z = r.z / fmaxf(m.z, 1e-3f);
         e.w = lum3(e.x, e.y, e.z);
-        lq = make_float2(E * qf16(e.w), 1.0f);
+        lq = E * qf16(e.w);
       }
       const int t = kb_tix(i / KB_SWL, i % KB_SWL);
       S.I[t] = e;
@@ -468,21 +466,15 @@ __global__ void __launch_bounds__(KB_NT, 2)
     const bool pin = px < f.W && py < f.H;
     if (q < 3) cp_async_wait<1>();  // this pixel's group has landed (the next pixel's may still fly)
     else cp_async_wait<0>();
-    if (pin) PL = pixel_fetch<KB_NT>(&S.G[q & 1][0][li], mvq[q], f.reset);
-    const PixOut p = pin ? temporal_pixel_fast(f, px, py, ParityTile{S.I, 2 * lby + (q >> 1) + 1, 2 * lbx + (q & 1) + 1}, PL)
-                         : pix_none();
-    if (q < 2) {  // pixel q + 2 into the slot pixel q has finished reading
-      const int qx = px0 + (q & 1), qy = py0 + 1;
-      if (qx < f.W && qy < f.H) pixel_issue_async<KB_NT>(f, qx, qy, mvq[q + 2], &S.G[q & 1][0][li]);
-      cp_async_commit();
-    }
-    okp[q] = p.Ns.w != 0.0f;
-    la[q] = p.P0.x;
-    zs[q] = p.P2.z;
-    nx4[q] = p.Ns.x; ny4[q] = p.Ns.y; nz4[q] = p.Ns.z;
+    PixOut p;
+    okp[q] = pin && temporal_pixel_fast<NT>(f, px, py, ParityTile{S.I, 2 * lby + (q >> 1) + 1, 2 * lbx + (q & 1) + 1},
+                                               &S.G[q & 1][0][li], mvq[q], p);
     if (okp[q]) {
+      la[q] = p.P0.x;
+      zs[q] = p.P2.z;
+      nx4[q] = p.Ns.x; ny4[q] = p.Ns.y; nz4[q] = p.Ns.z;
       nv += 1.0f;
-      S0.x += p.P0.x; S0.y += p.P0.y; S0.z += p.P0.z; S0.w += p.P0.w;
+      S0.x += p.P0.x; S0.z += p.P0.z; S0.w += p.P0.w;
       S1.x += p.P1.x; S1.y += p.P1.y; S1.z += p.P1.z; S1.w += p.P1.w;
       Nx += p.Ns.x; Ny += p.Ns.y; Nz += p.Ns.z;
       S3.x += p.P3.x; S3.y += p.P3.y; S3.z += p.P3.z; S3.w += p.P3.w;
@@ -490,9 +482,14 @@ __global__ void __launch_bounds__(KB_NT, 2)
       MV += p.P2.w;
       Z += p.P2.z;
     }
+    if (q < 2) {  // pixel q + 2 into the slot pixel q has finished reading
+      const int qx = px0 + (q & 1), qy = py0 + 1;
+      if (qx < f.W && qy < f.H) pixel_issue_async<NT>(f, qx, qy, mvq[q + 2], &S.G[q & 1][0][li]);
+      cp_async_commit();
+    }
   }
   // phase 3: block() (hush.js:226-282)
-  const int X = blockIdx.x * (KB_TW / 2) + lbx, Y = blockIdx.y * (KB_TH / 2) + lby;
+  const int X = blockIdx.x * (KB_TW / 2) + lbx, Y = blockIdx.y * (TH / 2) + lby;
   const bool valid = X < f.W2 && Y < f.H2;
   const bool ok = nv != 0.0f;
   float fe[N_FEAT];
@@ -509,21 +506,23 @@ __global__ void __launch_bounds__(KB_NT, 2)
     for (int q = 0; q < 4; q++)
       if (okp[q]) VA += (la[q] - Lacc) * (la[q] - Lacc);
     VA *= k;
-    // 4x4 neighbourhood (block +-1) of the quantised luminance, row-major
-    float s1 = 0.f, n4 = 0.f;
-    float2 w16[16];
+    // 4x4 neighbourhood (block +-1) of the quantised luminance, row-major; its middle entries are the block's own pixels
+    float s1 = 0.f, n4 = 0.f, lq[16], ly[16];
 #pragma unroll
     for (int e = 0; e < 16; e++) {
-      w16[e] = S.Lq[kb_tix(2 * lby + (e >> 2), 2 * lbx + (e & 3))];
-      s1 += w16[e].y * w16[e].x;
-      n4 += w16[e].y;
+      const float x = S.Lq[kb_tix(2 * lby + (e >> 2), 2 * lbx + (e & 3))];
+      ly[e] = l_counts(x);
+      lq[e] = ly[e] * x;
+      s1 += lq[e];
+      n4 += ly[e];
     }
+    S0.y = (lq[5] + lq[6] + lq[9] + lq[10]) * k;
     const float mu4 = s1 / fmaxf(n4, 1.0f);
     float var4 = 0.f;
 #pragma unroll
     for (int e = 0; e < 16; e++) {
-      const float d = w16[e].x - mu4;
-      var4 += w16[e].y * d * d;
+      const float d = lq[e] - mu4;
+      var4 += ly[e] * d * d;
     }
     var4 /= fmaxf(n4, 1.0f);
     const float nl = fmaxf(sqrtf(Nx * Nx + Ny * Ny + Nz * Nz), 1e-6f);
@@ -577,7 +576,7 @@ __global__ void __launch_bounds__(KB_NT, 2)
       float v8[8];
 #pragma unroll
       for (int e = 0; e < 8; e++)
-        v8[e] = (8 * c + e < N_FEAT && valid && ok) ? __half2float(__ushort_as_half(f2h(qf16(fe[8 * c + e])))) : 0.f;
+        v8[e] = (8 * c + e < N_FEAT && valid && ok) ? __half2float(__ushort_as_half(f2h(feature_qf16(8 * c + e, fe[8 * c + e])))) : 0.f;
       put_row(S.a1, S.a1lo, 8 * c, 4, v8);
     }
     float row[16], d[16];
@@ -632,7 +631,7 @@ __global__ void __launch_bounds__(KB_NT, 2)
     for (int p = 0; p < 8; p++) a[p] = Wh[MLP_HALF_B1 + p];
 #pragma unroll
     for (int i = 0; i < N_FEAT; i++) {
-      const uint32_t x = hdup(f2h(qf16(fe[i])));
+      const uint32_t x = hdup(f2h(feature_qf16(i, fe[i])));
 #pragma unroll
       for (int p = 0; p < 8; p++) a[p] = hadd2_rn(a[p], hmul2_rn(x, Wh[MLP_HALF_W1 + i * 8 + p]));
     }
@@ -667,7 +666,7 @@ __global__ void __launch_bounds__(KB_NT, 2)
   // phase 4: the MLP (hush.js:681-704) on the features as stored (packed f16, hush.js:278-280, 348-353); each unit
   // is its bias plus the inputs in increasing index, FP32 with packed FP32x2 FMAs
 #pragma unroll
-  for (int i = 0; i < N_FEAT; i++) fe[i] = __half2float(__ushort_as_half(f2h(qf16(fe[i]))));
+  for (int i = 0; i < N_FEAT; i++) fe[i] = __half2float(__ushort_as_half(f2h(feature_qf16(i, fe[i]))));
   const float4 *Wt;
   if constexpr (!TC) Wt = wp.w;
   float4 a[4];
@@ -1520,6 +1519,11 @@ static const HalfMaps &half_maps(const HushFrame &f) {
   return c.m;
 }
 
+// stage 0's forms: by MODE at 16 rows, then MODE 0 and MODE 3 at 8 rows
+static void (*const KB_KERN[6])(HushFrame, MlpConst, const uint4 *) = {
+    k_temporal_block<0, KB_TH>, k_temporal_block<1, KB_TH>,     k_temporal_block<2, KB_TH>,
+    k_temporal_block<3, KB_TH>, k_temporal_block<0, KB_TH / 2>, k_temporal_block<3, KB_TH / 2>};
+
 cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const MlpConst &mc, int mlp_mode,
                                const void *mlp_tc, cudaStream_t st) {
   const int hx = (f.W2 + HT_W - 1) / HT_W, hy = (f.H2 + HT_H - 1) / HT_H;
@@ -1532,20 +1536,22 @@ cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const Ml
       int dev = 0;
       cudaGetDevice(&dev);
       if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-      const dim3 g((f.W + KB_TW - 1) / KB_TW, (f.H + KB_TH - 1) / KB_TH);
-      // every form needs more than 48 KB of dynamic shared memory: opt in once per device and form
-      static bool opted[4][64] = {};
+      const int gx = (f.W + KB_TW - 1) / KB_TW;
       const int m = mlp_mode & 3;
-      void (*const kern[4])(HushFrame, MlpConst, const uint4 *) = {k_temporal_block<0>, k_temporal_block<1>,
-                                                                   k_temporal_block<2>, k_temporal_block<3>};
-      const int smem = (m == 1 || m == 2) ? (int)sizeof(KbTcSmem) : (int)sizeof(KbSmem);
-      if (!opted[m][dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(kern[m], cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      const bool tc = m == 1 || m == 2;
+      const bool half = !tc && gx * ((f.H + KB_TH - 1) / KB_TH) <= KB_HALF_CTAS;
+      const int th = half ? KB_TH / 2 : KB_TH;
+      // most forms need more than 48 KB of dynamic shared memory: opt in once per device and form
+      static bool opted[6][64] = {};
+      const int ki = !half ? m : m == 0 ? 4 : 5;
+      const int smem = tc ? (int)sizeof(KbTcSmem) : half ? (int)sizeof(KbSmem<KB_TH / 2>) : (int)sizeof(KbSmem<KB_TH>);
+      if (!opted[ki][dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(KB_KERN[ki], cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
-        opted[m][dev] = true;
+        opted[ki][dev] = true;
       }
       const uint4 *b = m == 1 ? blob + MLP_BLOB_BF16 / 16 : m == 2 ? blob + MLP_BLOB_F16 / 16 : blob;
-      kern[m]<<<g, KB_NT, smem, st>>>(f, mc, b);
+      KB_KERN[ki]<<<dim3(gx, (f.H + th - 1) / th), KB_TW / 4 * th, smem, st>>>(f, mc, b);
       break;
     }
     // stages 1 and 2: the mid tiles and the coarse tiles are separate kernels (each with its own register count);
@@ -1594,10 +1600,8 @@ cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const Ml
 size_t fused_scratch_bytes(int, int) { return 0; }
 
 int fused_kernel_param_count(const void *func) {
-  const void *three[4] = {(const void *)k_temporal_block<0>, (const void *)k_temporal_block<1>,
-                          (const void *)k_temporal_block<2>, (const void *)k_temporal_block<3>};
-  for (const void *k : three)
-    if (func == k) return 3;  // (f, wp, blob)
+  for (auto *k : KB_KERN)
+    if (func == (const void *)k) return 3;  // (f, wp, blob)
   const void *half[5] = {(const void *)k_half_stage<1, HP_MID>, (const void *)k_half_stage<1, HP_COARSE>,
                          (const void *)k_half_pair<2, HP_MID>, (const void *)k_half_pair<2, HP_COARSE>,
                          (const void *)k_half_pair<3, HP_MID>};
