@@ -27,10 +27,13 @@ struct EnvView {
   const float4 *table;
 };
 
+constexpr int MAX_DEPTH = 32;  // of a BVH, checked by the scene build
+
 size_t tex_layer_bytes();
 int fail(int code, const std::string &msg);
 SceneView scene_view(const hush_pt_scene_t *s);
 int scene_device(const hush_pt_scene_t *s);
+int scene_depth(const hush_pt_scene_t *s);  // of the deepest BVH, at most MAX_DEPTH
 bool scene_built(const hush_pt_scene_t *s);
 
 }  // namespace pt

@@ -1,15 +1,28 @@
 // The path tracer's kernel and the PathTracer instance (src/pt/pathtracer.js, pathtracer.wgsl.js).
 //
-// One thread per pixel, 8 x 8 pixel blocks (each warp covers an 8 x 4 patch, so primary rays of a warp stay
-// coherent); each thread walks the packed BVH2 with its traversal stack in shared memory, laid out stack-slot-major
-// (slot k of thread t at k * 64 + t) so that the warp's pushes and pops hit 32 distinct banks. Scene records are read
-// as float4 / uint4 through the read-only path. The arithmetic and the order of random draws follow the WGSL
-// (pathtracer.wgsl.js:75-672): PCG hash per pixel and frame, Moller-Trumbore triangles, GGX with VNDF sampling, smooth
-// glass, next-event estimation with MIS on cone lights and the importance-sampled environment map, Russian roulette
-// after two bounces. Texture and environment lookups are explicit trilinear / bilinear filters with f32 weights.
-// Mode 0 writes the five rgba16float G-buffer images (storage rounding toward zero), mode 1 accumulates.
+// A persistent kernel that alternates two phases. Shade: every thread takes the path it holds one vertex on (the direct light
+// its last shadow rays brought, then the hit's surface, the shadow rays of all its lights and the next direction; none of
+// these waits for another ray) and a thread whose path is complete takes the next pixel. Trace: the CTA's path and shadow rays
+// are one queue in shared memory, from which lanes take a ray whenever they are free, whatever pixel and kind it is of.
+//
+// What bounds it is the SIMD width: with one thread per pixel, tracing where a ray is needed, a path's end, a light that is
+// not tried, a leaf or a long ray left 7 of 32 lanes at work, and the traversal inlined at its four calls did not fit the
+// instruction cache (2.3 of 7.5 cycles between a warp's instructions). Phases keep a CTA's warps in the same code; the
+// queue and the refill keep 16 lanes at nodes and 9 at triangles (a step waits until enough lanes want it), which leaves
+// the length of a step's dependent chain. 96 threads and 72 registers (27 warps an SM): 5 CTAs of 128 threads and 96
+// registers take 3 % longer, 3 of 256 threads 4 % (a phase ends with its longest ray). 1920x1080, 32 objects, sun, a light and an
+// environment map: 3593 -> 2375 us; 320x180 612 -> 452.
+//
+// The traversal stacks are in shared memory, slot-major (slot k of thread t at k * NT + t), as deep as the scene's BVHs. Scene
+// records are read as float4 / uint4 through the read-only path. A ray's steps, the arithmetic and the order of a path's
+// random draws follow the WGSL (pathtracer.wgsl.js:75-672): PCG hash per pixel and frame, packed BVH2, Moller-Trumbore
+// triangles, GGX with VNDF sampling, smooth glass, next-event estimation with MIS on cone lights and the importance-sampled
+// environment map, Russian roulette after two bounces. Texture and environment lookups are explicit trilinear / bilinear
+// filters with f32 weights. Mode 0 writes the five rgba16float G-buffer images (storage rounding toward zero), mode 1
+// accumulates.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 
 #include "common.cuh"
@@ -24,8 +37,10 @@ namespace {
 constexpr float PI = 3.14159265358979f;
 constexpr float INF = 1e30f;
 constexpr uint32_t NONE = 0xffffffffu;
-constexpr int STACK = 32;  // >= BVH depth, checked by the scene build
-constexpr int BW = 8, BH = 8, NT = BW * BH;
+constexpr int NT = 96, CTAS = 9;  // threads of a CTA (see above), CTAs an SM
+// Lanes: finished rays that are replaced together; a warp leaves nodes for triangles (and back) when no more than these want
+// them. Half and twice these values are within 1 %.
+constexpr int WAIT = 8, NODE_LOW = 8, TRI_LOW = 6;
 constexpr uint32_t GW = HUSH_PT_ENV_GW, GH = HUSH_PT_ENV_GH;
 constexpr int TEX_S = HUSH_PT_TEX_SIZE, TEX_M = HUSH_PT_TEX_MIPS;
 
@@ -67,6 +82,18 @@ DI uint32_t pcg(uint32_t v) {
 
 struct Hit { float t; uint32_t tri; float u, v; int light; };
 
+constexpr uint32_t AT_NODE = 0u, RAY_DONE = 0xffffffffu;
+// A ray on its way through the BVHs: node r.node of BLAS r.b next, r.sp entries on the lane's stack.
+struct Ray {
+  float3 o, d, inv;
+  float t, u, v;  // of the closest hit so far (t: else the ray's length)
+  uint32_t tri, b, nodes, tris, node, sp, guard;
+  uint32_t i, e;  // the leaf's triangles still to test (or e = AT_NODE, RAY_DONE), and then:
+  uint32_t next, next_n;  // the node's other child, if its box begins at next_t < t: a leaf of next_n triangles, or inner
+  float next_t;
+  bool shadow;
+};
+
 struct Surf {
   float3 p, ng, n, base, emissive, prev_p;
   float rough, metal, transmission, ior;
@@ -81,6 +108,7 @@ struct Tracer {
   const pt::SceneView &S;
   const pt::EnvView &E;
   uint32_t *stk;  // this thread's column of the shared traversal stacks
+  uint32_t stack;  // their entries, at least the depth of the BVHs
   uint32_t rng;
 
   DI float rnd() {
@@ -89,7 +117,8 @@ struct Tracer {
   }
 
   // -------------------------------------------------------------------------------------- texture lookups
-  DI static int wrapi(int i, int n) { const int r = i % n; return r < 0 ? r + n : r; }
+  DI static int wrap1(int i, int n) { return i < 0 ? i + n : i >= n ? i - n : i; }  // of -n <= i < 2 n
+  static_assert((TEX_S & (TEX_S - 1)) == 0, "texel() wraps by masking");
   DI float4 texel(int layer, int mip, int x, int y) const {
     size_t off = 0, per = 0;
 #pragma unroll
@@ -99,7 +128,7 @@ struct Tracer {
       per += s * s * 4;
     }
     const int s = max(1, TEX_S >> mip);
-    const uchar4 t = __ldg(reinterpret_cast<const uchar4 *>(S.tex + per * layer + off) + (size_t)wrapi(y, s) * s + wrapi(x, s));
+    const uchar4 t = __ldg(reinterpret_cast<const uchar4 *>(S.tex + per * layer + off) + (size_t)(y & (s - 1)) * s + (x & (s - 1)));
     return make_float4(t.x / 255.0f, t.y / 255.0f, t.z / 255.0f, t.w / 255.0f);
   }
   DI float4 bilinear(int layer, int mip, float u, float v) const {
@@ -127,7 +156,7 @@ struct Tracer {
     const float x = u * (float)E.w - 0.5f, y = v * (float)E.h - 0.5f;
     const float x0 = floorf(x), y0 = floorf(y), fx = x - x0, fy = y - y0;
     auto at = [&](int xi, int yi) {
-      return f3(h4_to_f4(__ldg(E.texels + (size_t)min(max(yi, 0), E.h - 1) * E.w + wrapi(xi, E.w))));
+      return f3(h4_to_f4(__ldg(E.texels + (size_t)min(max(yi, 0), E.h - 1) * E.w + wrap1(xi, E.w))));
     };
     const int ix = (int)x0, iy = (int)y0;
     const float3 top = at(ix, iy) * (1.0f - fx) + at(ix + 1, iy) * fx;
@@ -181,61 +210,83 @@ struct Tracer {
     return f3(t, u, v);
   }
 
-  // closest (or, for shadow rays, any) hit over the BLAS list; packed BVH2 (both child boxes per 64-byte node)
-  DI Hit trace_bvh(float3 o, float3 d, float tmax_in, bool shadow) const {
-    Hit h{tmax_in, NONE, 0.0f, 0.0f, -1};
-    const float3 inv = f3(1.0f / (fabsf(d.x) < 1e-9f ? 1e-9f : d.x), 1.0f / (fabsf(d.y) < 1e-9f ? 1e-9f : d.y),
-                          1.0f / (fabsf(d.z) < 1e-9f ? 1e-9f : d.z));
-    for (uint32_t b = 0; b < F.counts[0]; b++) {
-      const hush_pt_blas bl = F.blas[b];
-      if (shadow && (bl.flags & 2u)) continue;
-      uint32_t sp = 0, node = 0;
-      // a BVH built by the scene visits each node at most once per ray; the cap only bounds a corrupted one
-      for (uint32_t guard = 0; guard < (1u << 24); guard++) {
-        const float4 *nd = S.nodes + (size_t)(bl.node_offset + node) * 4;
-        const float4 lmin = __ldg(nd), lmax = __ldg(nd + 1), rmin = __ldg(nd + 2), rmax = __ldg(nd + 3);
-        float tl = slab(o, inv, lmin, lmax, h.t);
-        float tr = slab(o, inv, rmin, rmax, h.t);
-        const uint32_t lc = __float_as_uint(lmax.w), rc = __float_as_uint(rmax.w);
-        if (lc > 0u && tl < INF) {
-          const uint32_t first = bl.tri_offset + __float_as_uint(lmin.w);
-          for (uint32_t i = 0; i < lc; i++) {
-            const float3 r = hit_tri(o, d, first + i, h.t);
-            if (r.x < h.t) {
-              h.t = r.x; h.u = r.y; h.v = r.z; h.tri = first + i;
-              if (shadow) return h;
-            }
-          }
-          tl = INF;
-        }
-        if (rc > 0u && tr < h.t) {
-          const uint32_t first = bl.tri_offset + __float_as_uint(rmin.w);
-          for (uint32_t i = 0; i < rc; i++) {
-            const float3 r = hit_tri(o, d, first + i, h.t);
-            if (r.x < h.t) {
-              h.t = r.x; h.u = r.y; h.v = r.z; h.tri = first + i;
-              if (shadow) return h;
-            }
-          }
-          tr = INF;
-        }
-        const uint32_t l = __float_as_uint(lmin.w), r = __float_as_uint(rmin.w);
-        if (tl < h.t && tr < h.t) {
-          const bool near_left = tl <= tr;
-          node = near_left ? l : r;
-          stk[sp * NT] = near_left ? r : l;
-          sp = min(sp + 1u, (uint32_t)STACK - 1u);
-        } else if (tl < h.t) {
-          node = l;
-        } else if (tr < h.t) {
-          node = r;
-        } else {
-          if (sp == 0u) break;
-          node = stk[--sp * NT];
-        }
+  // The ray's next BLAS (from `b` on) that it may hit, or its end.
+  DI void enter_blas(Ray &r, uint32_t b) const {
+    const uint32_t n = F.counts[0];
+    while (b < n && r.shadow && (F.blas[b].flags & 2u)) b++;
+    r.e = RAY_DONE;
+    if (b >= n) return;
+    r.b = b;
+    r.nodes = F.blas[b].node_offset;
+    r.tris = F.blas[b].tri_offset;
+    r.node = r.sp = r.guard = 0u;
+    r.e = AT_NODE;
+  }
+  DI void start_ray(Ray &r, float3 o, float3 d, float tmax, bool shadow) const {
+    r.o = o;
+    r.d = d;
+    r.inv = f3(1.0f / (fabsf(d.x) < 1e-9f ? 1e-9f : d.x), 1.0f / (fabsf(d.y) < 1e-9f ? 1e-9f : d.y),
+               1.0f / (fabsf(d.z) < 1e-9f ? 1e-9f : d.z));
+    r.t = tmax;
+    r.tri = NONE;
+    r.u = r.v = 0.0f;
+    r.shadow = shadow;
+    r.b = 0u;
+    enter_blas(r, 0u);
+  }
+  // The traversal to the closest (or, for shadow rays, any) hit, one step at a time: a packed BVH2 node (both child boxes per
+  // 64-byte node), or one triangle of a leaf. A node's leaf children come first, left before right, then the nearer inner
+  // child or the stack.
+  DI void pop(Ray &r) const {
+    if (r.sp > 0u) r.node = stk[--r.sp * NT];
+    else enter_blas(r, r.b + 1u);
+  }
+  DI void node_step(Ray &r) const {
+    const float4 *nd = S.nodes + (size_t)(r.nodes + r.node) * 4;
+    const float4 lmin = __ldg(nd), lmax = __ldg(nd + 1), rmin = __ldg(nd + 2), rmax = __ldg(nd + 3);
+    const float tl = slab(r.o, r.inv, lmin, lmax, r.t);  // INF if the box is missed or begins at or beyond r.t
+    const float tr = slab(r.o, r.inv, rmin, rmax, r.t);
+    const uint32_t lc = __float_as_uint(lmax.w), rc = __float_as_uint(rmax.w);
+    const uint32_t lref = __float_as_uint(lmin.w), rref = __float_as_uint(rmin.w);
+    const bool left_leaf = lc > 0u && tl < INF, right_leaf = rc > 0u && tr < INF, leaf = left_leaf || right_leaf;
+    // the child that comes first, and the other one
+    const bool right_first = leaf ? !left_leaf : !(tl <= tr);
+    const uint32_t ref = right_first ? rref : lref;
+    r.next = right_first ? lref : rref;
+    r.next_n = right_first ? lc : rc;
+    r.next_t = right_first ? tl : tr;
+    r.node = ref;
+    if (leaf) {
+      r.i = r.tris + ref;
+      r.e = r.i + (right_first ? rc : lc);
+    } else if (r.next_t < INF) {
+      stk[r.sp * NT] = r.next;
+      r.sp = min(r.sp + 1u, stack - 1u);
+    } else if (!((right_first ? tr : tl) < INF)) {
+      pop(r);
+    }
+    // a BVH built by the scene visits each node at most once per ray; the cap only bounds a corrupted one
+    if (++r.guard == 1u << 24) enter_blas(r, r.b + 1u);
+  }
+  DI void tri_step(Ray &r) const {
+    const float3 q = hit_tri(r.o, r.d, r.i, r.t);
+    if (q.x < r.t) {
+      r.t = q.x; r.u = q.y; r.v = q.z; r.tri = r.i;
+      if (r.shadow) {
+        r.e = RAY_DONE;
+        return;
       }
     }
-    return h;
+    if (++r.i < r.e) return;
+    r.e = AT_NODE;
+    r.node = r.next;
+    if (!(r.next_t < r.t)) {
+      pop(r);
+    } else if (r.next_n > 0u) {  // the right leaf
+      r.i = r.tris + r.next;
+      r.e = r.i + r.next_n;
+      r.next_t = INF;
+    }
   }
 
   DI static float sphere_t(float3 o, float3 d, float3 c, float r) {
@@ -249,8 +300,8 @@ struct Tracer {
     return t < 1e-4f ? INF : t;
   }
 
-  DI Hit trace_scene(float3 o, float3 d) const {
-    Hit h = trace_bvh(o, d, INF, false);
+  // The closest hit among the triangles' (h) and the spherical lights.
+  DI Hit closest(float3 o, float3 d, Hit h) const {
     for (uint32_t i = 0; i < F.counts[1]; i++) {
       const hush_pt_light &L = F.lights[i];
       if (L.params[0] != 1.0f) continue;
@@ -259,8 +310,6 @@ struct Tracer {
     }
     return h;
   }
-
-  DI bool visible(float3 o, float3 d, float tmax) const { return trace_bvh(o, d, tmax, true).tri == NONE; }
 
   // -------------------------------------------------------------------------------------- environment
   DI float3 env_local(float3 d) const { return f3(F.env[1] * d.x - F.env[2] * d.z, d.y, F.env[2] * d.x + F.env[1] * d.z); }
@@ -436,10 +485,15 @@ struct Tracer {
   DI static float cone_pdf(float cos_max) { return 1.0f / (2.0f * PI * fmaxf(1.0f - cos_max, 1e-7f)); }
   DI static float mis(float a, float b) { const float a2 = a * a; return a2 / fmaxf(a2 + b * b, 1e-20f); }
 
-  DI float3 direct_light(const Surf &s, const Basis &frame, float3 v, float3 tp, bool all) {
-    float3 acc = f3(0.f, 0.f, 0.f), pick_c = acc, pick_d = acc;
+  // The shadow rays of the surface's direct light (pathtracer.wgsl.js's directLight): put(k, direction, length, what it adds if
+  // nothing is hit), k = light, lights for the environment map. all: one ray per light; otherwise one light (k = 0), picked
+  // by its contribution. No random draw depends on a ray's outcome.
+  template <class Put>
+  DI void light_rays(const Surf &s, const Basis &frame, float3 v, float3 tp, bool all, const Put &put) {
+    const uint32_t nl = F.counts[1];
     float w_sum = 0.0f, pick_w = 0.0f, pick_t = 0.0f;
-    for (uint32_t i = 0; i < F.counts[1]; i++) {
+    float3 pick_c = f3(0.f, 0.f, 0.f), pick_d = pick_c;
+    for (uint32_t i = 0; i < nl; i++) {
       const hush_pt_light &L = F.lights[i];
       const float4 ax = cone_axis(L, s.p);
       if (ax.w < -1.0f) continue;
@@ -456,8 +510,7 @@ struct Tracer {
       const float lp = cone_pdf(ax.w);
       const float3 c = f * f3(L.radiance) / lp * mis(lp, pdf);
       if (all) {
-        if (!visible(s.p + s.ng * 1e-3f, dir, tmax)) continue;
-        acc = acc + c;
+        put(i, dir, tmax, c);
       } else {
         const float wl = lum(tp * c);
         if (wl <= 0.0f) continue;
@@ -467,7 +520,7 @@ struct Tracer {
     }
     if (!all && w_sum > 0.0f) {
       const float q = fminf(1.0f, w_sum / F.shadow_tau);
-      if (rnd() < q && visible(s.p + s.ng * 1e-3f, pick_d, pick_t)) acc = pick_c * (w_sum / (pick_w * q));
+      if (rnd() < q) put(0u, pick_d, pick_t, pick_c * (w_sum / (pick_w * q)));
     }
     if (F.env[3] > 0.5f) {
       const float4 es = sample_env_dir();
@@ -476,10 +529,9 @@ struct Tracer {
       if (es.w > 0.0f && ll.z > 0.0f && dot(ed, s.ng) > 0.0f) {
         float3 f;
         const float pdf = eval_bsdf(s, v, ll, f).w;
-        if (lum(f) > 0.0f && visible(s.p + s.ng * 1e-3f, ed, INF)) acc = acc + f * sky(ed) / es.w * mis(es.w, pdf);
+        if (lum(f) > 0.0f) put(nl, ed, INF, f * sky(ed) / es.w * mis(es.w, pdf));
       }
     }
-    return acc;
   }
 
   DI float2 project_pix(const float *m, float px, float py, float pz, float pw) const {
@@ -490,171 +542,324 @@ struct Tracer {
     return make_float2((nx * 0.5f + 0.5f) * (float)F.size[0], (0.5f - ny * 0.5f) * (float)F.size[1]);
   }
 
-  // tracePath (pathtracer.wgsl.js:511-646); with write_g the primary hit's G-buffer values go to g[0..11]
-  DI void trace_path(float pix_x, float pix_y, bool write_g, float3 &radiance, float3 &prim_emission, float *g) {
-    radiance = f3(0.f, 0.f, 0.f);
-    prim_emission = radiance;
+  DI float3 primary_dir(float pix_x, float pix_y) const {
     const float ndx = (pix_x / (float)F.size[0]) * 2.0f - 1.0f, ndy = (pix_y / (float)F.size[1]) * 2.0f - 1.0f;
-    float3 o = f3(F.cam_pos);
-    float3 d = normalize(f3(F.cam_fwd) + f3(F.cam_right) * ndx - f3(F.cam_up) * ndy);
-    float3 tp = f3(1.f, 1.f, 1.f);
-    float last_pdf = 0.0f, lod_base = 1.0f;
-    uint32_t bounces = 0, delta_chain = 0;
-    for (uint32_t depth = 0; depth < 12u; depth++) {
-      const Hit h = trace_scene(o, d);
-      const bool primary = depth == 0u;
-      if (h.tri == NONE && h.light < 0) {  // sky
-        float3 e = sky(d);
-        if (F.env[3] > 0.5f && last_pdf > 0.0f) e = e * mis(last_pdf, env_pdf(d));
-        for (uint32_t i = 0; i < F.counts[1]; i++) {  // sun disks reached by BSDF sampling
-          const hush_pt_light &L = F.lights[i];
-          if (L.params[0] == 0.0f && dot(d, f3(L.pos)) >= L.params[1])
-            e = e + f3(L.radiance) * (last_pdf > 0.0f ? mis(last_pdf, cone_pdf(L.params[1])) : 1.0f);
-        }
-        if (primary) {
-          prim_emission = e;
-          if (write_g) {
-            const float2 a = project_pix(F.prev_view_proj, d.x, d.y, d.z, 0.0f);
-            const float2 b = project_pix(F.view_proj, d.x, d.y, d.z, 0.0f);
-            const float gv[12] = {-d.x, -d.y, -d.z, -1.0f, a.x - b.x, a.y - b.y, 65535.0f, -1.0f, 1.f, 1.f, 1.f, 1.f};
-#pragma unroll
-            for (int k = 0; k < 12; k++) g[k] = gv[k];
-          }
-        } else {
-          float3 c = tp * e;
-          const float lc = lum(c);
-          if (lc > F.clamp_lum) c = c * (F.clamp_lum / lc);
-          radiance = radiance + c;
-        }
-        break;
-      }
-      const Surf s = fetch_surf(h, o, d, lod_base);
-      if (lum(s.emissive) > 0.0f) {
-        float3 e = s.emissive;
-        if (h.light >= 0 && last_pdf > 0.0f) e = e * mis(last_pdf, cone_pdf(cone_axis(F.lights[h.light], o).w));
-        if (primary) {
-          prim_emission = e;
-        } else {
-          float3 c = tp * e;
-          const float lc = lum(c);
-          if (lc > F.clamp_lum) c = c * (F.clamp_lum / lc);
-          radiance = radiance + c;
-        }
-      }
-      const bool glass = s.transmission > 0.5f;
-      if (primary && write_g) {
-        const bool white = glass || h.light >= 0;
-        const float3 alb = s.base * (1.0f - s.metal) + lerp3(f3(0.04f, 0.04f, 0.04f), s.base, s.metal) * s.metal;
-        const float2 a = project_pix(F.prev_view_proj, s.prev_p.x, s.prev_p.y, s.prev_p.z, 1.0f);
-        const float2 b = project_pix(F.view_proj, s.p.x, s.p.y, s.p.z, 1.0f);
-        const float *pm = F.prev_view_proj;
-        const float prev_w = pm[3] * s.prev_p.x + pm[7] * s.prev_p.y + pm[11] * s.prev_p.z + pm[15];
-        g[0] = s.n.x; g[1] = s.n.y; g[2] = s.n.z;
-        g[3] = dot(s.p - f3(F.cam_pos), f3(F.cam_fwd));
-        g[4] = a.x - b.x; g[5] = a.y - b.y;
-        g[6] = (float)s.obj;
-        g[7] = prev_w;
-        g[8] = white ? 1.0f : fmaxf(alb.x, 0.02f);
-        g[9] = white ? 1.0f : fmaxf(alb.y, 0.02f);
-        g[10] = white ? 1.0f : fmaxf(alb.z, 0.02f);
-        g[11] = glass ? 0.0f : s.rough;
-      }
-      if (h.light >= 0) break;
-      if (glass) {  // smooth dielectric: Fresnel-weighted reflect / refract
-        if (++delta_chain > 8u) break;
-        const float eta = s.front ? 1.0f / s.ior : s.ior;
-        const float3 n = s.ng;
-        const float c = -dot(d, n);
-        const float k = 1.0f - eta * eta * (1.0f - c * c);
-        float R = 1.0f;
-        if (k > 0.0f) {
-          const float ct = sqrtf(k);
-          const float rs = (eta * c - ct) / (eta * c + ct), rp = (c - eta * ct) / (c + eta * ct);
-          R = 0.5f * (rs * rs + rp * rp);
-        }
-        if (rnd() < R) {
-          d = reflect(d, n);
-          o = s.p + n * 1e-3f;
-        } else {
-          d = normalize(d * eta + n * (eta * c - sqrtf(k)));
-          o = s.p - n * 1e-3f;
-          tp = tp * s.base;
-        }
-        last_pdf = 0.0f;
-        continue;
-      }
-      if (bounces >= F.max_bounces) break;
-      bounces++;
-      const Basis frame = onb(s.n);
-      const float3 v = to_local(frame, -d);
-      if (v.z <= 0.0f) break;
-      float3 dl = tp * direct_light(s, frame, v, tp, primary || F.shadow_tau <= 0.0f);
-      const float cl = primary ? (F.clamp_direct > 0.0f ? F.clamp_direct : INF) : F.clamp_lum;
-      const float ld = lum(dl);
-      if (ld > cl) dl = dl * (cl / ld);
-      radiance = radiance + dl;
-      const float ps = spec_prob(s, v.z);
-      float3 l;
-      if (rnd() < ps) {
-        const float a = fmaxf(s.rough * s.rough, 0.0025f);
-        const float u1 = rnd();
-        const float u2 = rnd();
-        l = reflect(-v, sample_vndf(v, a, u1, u2));
-      } else {
-        const float r = sqrtf(rnd());
-        const float ph = 2.0f * PI * rnd();
-        l = f3(r * cosf(ph), r * sinf(ph), sqrtf(fmaxf(0.0f, 1.0f - r * r)));
-      }
-      if (l.z <= 0.0f) break;
-      float3 f;
-      const float pdf = eval_bsdf(s, v, l, f).w;
-      if (pdf <= 0.0f) break;
-      tp = tp * f / pdf;
-      last_pdf = pdf;
-      d = normalize(to_world(frame, l));
-      if (dot(d, s.ng) <= 0.0f) break;
-      o = s.p + s.ng * 1e-3f;
-      lod_base = 4.0f;
-      if (bounces >= 2u) {  // Russian roulette
-        const float q = clampf(fmaxf(tp.x, fmaxf(tp.y, tp.z)), 0.05f, 0.95f);
-        if (rnd() > q) break;
-        tp = tp / q;
-      }
-    }
+    return normalize(f3(F.cam_fwd) + f3(F.cam_right) * ndx - f3(F.cam_up) * ndy);
+  }
+  DI float3 clamped(float3 c) const {
+    const float lc = lum(c);
+    return lc > F.clamp_lum ? c * (F.clamp_lum / lc) : c;
   }
 };
 
-// main() of pathtracer.wgsl.js:648-672
-__global__ void __launch_bounds__(NT, 8) k_pathtrace(const __grid_constant__ hush_pt_frame F, const pt::SceneView S,
-                                                   const pt::EnvView E, const GBuf G, float4 *__restrict__ accum) {
-  __shared__ uint32_t stacks[STACK * NT];
-  const uint32_t t = threadIdx.y * BW + threadIdx.x;
-  const uint32_t x = blockIdx.x * BW + threadIdx.x, y = blockIdx.y * BH + threadIdx.y;
-  if (x >= F.size[0] || y >= F.size[1]) return;  // no block-wide barrier below
-  Tracer T{F, S, E, stacks + t, 0u};
-  const uint32_t idx = y * F.size[0] + x;
-  if (F.mode == 0u) {
-    T.rng = pcg(idx ^ pcg(F.frame * 0x9E3779B9u + 17u));
-    float3 rad, pe;
-    float g[12];
-    T.trace_path((float)x + 0.5f + F.jitter[0], (float)y + 0.5f + F.jitter[1], true, rad, pe, g);
-    G.rad[idx] = f4_to_h4(make_float4(rad.x, rad.y, rad.z, 1.0f));
-    G.nd[idx] = f4_to_h4(make_float4(g[0], g[1], g[2], g[3]));
-    G.mv[idx] = f4_to_h4(make_float4(g[4], g[5], g[6], g[7]));
-    G.mat[idx] = f4_to_h4(make_float4(g[8], g[9], g[10], g[11]));
-    G.emi[idx] = f4_to_h4(make_float4(pe.x, pe.y, pe.z, 0.0f));
-  } else {
-    float3 sum = f3(0.f, 0.f, 0.f);
-    for (uint32_t sp = 0; sp < F.spp; sp++) {
-      T.rng = pcg(idx ^ pcg((F.counts[2] + sp) * 0x9E3779B9u + F.frame * 7919u + 1u));
-      const float jx = T.rnd();
-      const float jy = T.rnd();
-      float3 rad, pe;
-      T.trace_path((float)x + jx, (float)y + jy, false, rad, pe, nullptr);
-      sum = sum + rad + pe;
+// Shared memory of a CTA, in words: the thread's path ray (origin, direction) and its hit, then 7 words per shadow ray, each
+// thread-minor, the traversal stacks and the queue of rays to trace (entry k * NT + thread: k = 0 the path ray, else shadow
+// ray k - 1; 16 bits).
+enum : uint32_t { W_O = 0, W_D = 3, W_T = 6, W_U, W_V, W_TRI, W_LIGHT, W_CLAMP = W_LIGHT + 3, W_SHADOW, W_PER_SHADOW = 7 };
+constexpr uint32_t words_per_thread(uint32_t shadows) { return W_SHADOW + W_PER_SHADOW * shadows; }
+constexpr size_t pt_smem(uint32_t shadows, uint32_t stack) {
+  return (size_t)NT * 4 * (words_per_thread(shadows) + stack) + (size_t)NT * 2 * (shadows + 1);
+}
+
+// main() and tracePath (pathtracer.wgsl.js:511-672). CTAs walk the image's 8 x 4 tiles (tile blockIdx.x, + gridDim.x, ...) and
+// hand out their pixels one by one. In mode 0 the primary hit's G-buffer values are stored when they are known, the radiance
+// when the path is complete.
+template <bool ACCUM>
+__global__ void __launch_bounds__(NT, CTAS) k_pathtrace(const __grid_constant__ hush_pt_frame F, const pt::SceneView S,
+                                                        const pt::EnvView E, const GBuf G, float4 *__restrict__ accum,
+                                                        uint32_t tiles_x, uint32_t tiles, uint32_t shadows, uint32_t stack) {
+  extern __shared__ uint32_t pt_words[];
+  __shared__ uint32_t next_px, filled[2], taken[2];  // pixels handed out; rays in the queue and taken from it, by turn
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  uint32_t *const W = pt_words;
+  float *const Wf = reinterpret_cast<float *>(pt_words);
+  uint32_t *const stk = pt_words + NT * words_per_thread(shadows) + tid;
+  uint16_t *const queue = reinterpret_cast<uint16_t *>(pt_words + NT * (words_per_thread(shadows) + stack));
+  if (tid == 0) next_px = filled[0] = taken[0] = 0u;
+  __syncthreads();
+  Tracer T{F, S, E, stk, stack, 0u};
+  const uint32_t my_px = (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x * 32u;
+  bool idle = false, fresh = true, ended = false, lit = false;
+  uint32_t x = 0u, y = 0u, sample = 0u, depth = 0u, bounces = 0u, delta_chain = 0u, turn = 0u;
+  uint32_t mask = 0u;  // the thread's rays of this turn (bit k: queue entry k)
+  float3 rad = f3(0.f, 0.f, 0.f), pe = rad, sum = rad, tp = rad;
+  float last_pdf = 0.0f;
+  auto put3 = [&](uint32_t w, float3 v) {
+    Wf[w * NT + tid] = v.x;
+    Wf[(w + 1u) * NT + tid] = v.y;
+    Wf[(w + 2u) * NT + tid] = v.z;
+  };
+  auto get3 = [&](uint32_t w, uint32_t t) { return f3(Wf[w * NT + t], Wf[(w + 1u) * NT + t], Wf[(w + 2u) * NT + t]); };
+  for (;;) {
+    // ---- shade: every thread takes its path one vertex on
+    if (tid == 0) filled[turn ^ 1u] = taken[turn ^ 1u] = 0u;  // last used in the turn before this one's barriers
+    if (lit) {  // the direct light of the last vertex
+      float3 acc = f3(0.f, 0.f, 0.f);
+      for (uint32_t k = 0; k < shadows; k++) {
+        const uint32_t w = W_SHADOW + W_PER_SHADOW * k;
+        if ((mask >> (k + 1u) & 1u) && Wf[(w + 3u) * NT + tid] >= 0.0f) acc = acc + get3(w + 4u, tid);
+      }
+      // (tp moved on with the path; the vertex's own is kept beside the hit while its shadow rays are out)
+      float3 dl = get3(W_LIGHT, tid) * acc;
+      const float cl = Wf[W_CLAMP * NT + tid];
+      const float ld = lum(dl);
+      if (ld > cl) dl = dl * (cl / ld);
+      rad = rad + dl;
+      lit = false;
     }
-    const float4 a = accum[idx];
-    accum[idx] = make_float4(a.x + sum.x, a.y + sum.y, a.z + sum.z, a.w + (float)F.spp);
+    const bool vertex = !idle && !fresh && !ended;
+    mask = 0u;
+    if (vertex) {
+      const float3 o = get3(W_O, tid), d = get3(W_D, tid);
+      const Hit h = T.closest(o, d, Hit{Wf[W_T * NT + tid], W[W_TRI * NT + tid], Wf[W_U * NT + tid], Wf[W_V * NT + tid], -1});
+      const bool primary = depth == 0u;
+      const uint32_t idx = y * F.size[0] + x;
+      float3 no = o, nd = d;
+      bool emit = false;
+      if (h.tri == NONE && h.light < 0) {  // sky
+        float3 e = T.sky(d);
+        if (F.env[3] > 0.5f && last_pdf > 0.0f) e = e * T.mis(last_pdf, T.env_pdf(d));
+        for (uint32_t i = 0; i < F.counts[1]; i++) {  // sun disks reached by BSDF sampling
+          const hush_pt_light &L = F.lights[i];
+          if (L.params[0] == 0.0f && dot(d, f3(L.pos)) >= L.params[1])
+            e = e + f3(L.radiance) * (last_pdf > 0.0f ? T.mis(last_pdf, T.cone_pdf(L.params[1])) : 1.0f);
+        }
+        if (!primary) {
+          rad = rad + T.clamped(tp * e);
+        } else if (ACCUM) {
+          pe = e;
+        } else {
+          const float2 a = T.project_pix(F.prev_view_proj, d.x, d.y, d.z, 0.0f);
+          const float2 b = T.project_pix(F.view_proj, d.x, d.y, d.z, 0.0f);
+          G.nd[idx] = f4_to_h4(make_float4(-d.x, -d.y, -d.z, -1.0f));
+          G.mv[idx] = f4_to_h4(make_float4(a.x - b.x, a.y - b.y, 65535.0f, -1.0f));
+          G.mat[idx] = f4_to_h4(make_float4(1.f, 1.f, 1.f, 1.f));
+          G.emi[idx] = f4_to_h4(make_float4(e.x, e.y, e.z, 0.0f));
+        }
+      } else {
+        const Surf s = T.fetch_surf(h, o, d, bounces > 0u ? 4.0f : 1.0f);
+        float3 pem = f3(0.f, 0.f, 0.f);
+        if (lum(s.emissive) > 0.0f) {
+          float3 e = s.emissive;
+          if (h.light >= 0 && last_pdf > 0.0f) e = e * T.mis(last_pdf, T.cone_pdf(T.cone_axis(F.lights[h.light], o).w));
+          if (primary) pem = e;
+          else rad = rad + T.clamped(tp * e);
+        }
+        const bool glass = s.transmission > 0.5f;
+        if (primary && ACCUM) pe = pem;
+        if (primary && !ACCUM) {
+          const bool white = glass || h.light >= 0;
+          const float3 alb = s.base * (1.0f - s.metal) + lerp3(f3(0.04f, 0.04f, 0.04f), s.base, s.metal) * s.metal;
+          const float2 a = T.project_pix(F.prev_view_proj, s.prev_p.x, s.prev_p.y, s.prev_p.z, 1.0f);
+          const float2 b = T.project_pix(F.view_proj, s.p.x, s.p.y, s.p.z, 1.0f);
+          const float *pm = F.prev_view_proj;
+          const float prev_w = pm[3] * s.prev_p.x + pm[7] * s.prev_p.y + pm[11] * s.prev_p.z + pm[15];
+          G.nd[idx] = f4_to_h4(make_float4(s.n.x, s.n.y, s.n.z, dot(s.p - f3(F.cam_pos), f3(F.cam_fwd))));
+          G.mv[idx] = f4_to_h4(make_float4(a.x - b.x, a.y - b.y, (float)s.obj, prev_w));
+          G.mat[idx] = f4_to_h4(make_float4(white ? 1.0f : fmaxf(alb.x, 0.02f), white ? 1.0f : fmaxf(alb.y, 0.02f),
+                                            white ? 1.0f : fmaxf(alb.z, 0.02f), glass ? 0.0f : s.rough));
+          G.emi[idx] = f4_to_h4(make_float4(pem.x, pem.y, pem.z, 0.0f));
+        }
+        if (h.light < 0 && glass) {  // smooth dielectric: Fresnel-weighted reflect / refract
+          if (++delta_chain <= 8u) {
+            const float eta = s.front ? 1.0f / s.ior : s.ior;
+            const float3 n = s.ng;
+            const float c = -dot(d, n);
+            const float k = 1.0f - eta * eta * (1.0f - c * c);
+            float R = 1.0f;
+            if (k > 0.0f) {
+              const float ct = sqrtf(k);
+              const float rs = (eta * c - ct) / (eta * c + ct), rp = (c - eta * ct) / (c + eta * ct);
+              R = 0.5f * (rs * rs + rp * rp);
+            }
+            if (T.rnd() < R) {
+              nd = reflect(d, n);
+              no = s.p + n * 1e-3f;
+            } else {
+              nd = normalize(d * eta + n * (eta * c - sqrtf(k)));
+              no = s.p - n * 1e-3f;
+              tp = tp * s.base;
+            }
+            last_pdf = 0.0f;
+            emit = true;
+          }
+        } else if (h.light < 0 && bounces < F.max_bounces) {
+          bounces++;
+          const Basis frame = onb(s.n);
+          const float3 v = to_local(frame, -d);
+          if (!(v.z <= 0.0f)) {
+            lit = true;
+            put3(W_LIGHT, tp);
+            Wf[W_CLAMP * NT + tid] = primary ? (F.clamp_direct > 0.0f ? F.clamp_direct : INF) : F.clamp_lum;
+            no = s.p + s.ng * 1e-3f;
+            T.light_rays(s, frame, v, tp, primary || F.shadow_tau <= 0.0f, [&](uint32_t k, float3 dir, float tmax, float3 c) {
+              const uint32_t w = W_SHADOW + W_PER_SHADOW * k;
+              put3(w, dir);
+              Wf[(w + 3u) * NT + tid] = tmax;
+              put3(w + 4u, c);
+              mask |= 2u << k;
+            });
+            const float ps = T.spec_prob(s, v.z);
+            float3 l;
+            if (T.rnd() < ps) {
+              const float a = fmaxf(s.rough * s.rough, 0.0025f);
+              const float u1 = T.rnd();
+              const float u2 = T.rnd();
+              l = reflect(-v, T.sample_vndf(v, a, u1, u2));
+            } else {
+              const float r = sqrtf(T.rnd());
+              const float ph = 2.0f * PI * T.rnd();
+              l = f3(r * cosf(ph), r * sinf(ph), sqrtf(fmaxf(0.0f, 1.0f - r * r)));
+            }
+            if (!(l.z <= 0.0f)) {
+              float3 f;
+              const float pdf = T.eval_bsdf(s, v, l, f).w;
+              if (!(pdf <= 0.0f)) {
+                tp = tp * f / pdf;
+                last_pdf = pdf;
+                nd = normalize(to_world(frame, l));
+                emit = !(dot(nd, s.ng) <= 0.0f);
+                if (emit && bounces >= 2u) {  // Russian roulette
+                  const float q = clampf(fmaxf(tp.x, fmaxf(tp.y, tp.z)), 0.05f, 0.95f);
+                  if (T.rnd() > q) emit = false;
+                  tp = tp / q;
+                }
+              }
+            }
+          }
+        }
+      }
+      if (++depth == 12u) emit = false;
+      ended = !emit;
+      if (emit || mask) put3(W_O, no);
+      if (emit) {
+        put3(W_D, nd);
+        mask |= 1u;
+      }
+    }
+    // ---- a path that is complete gives its thread to the next pixel (or the pixel's next sample)
+    if (ended && !lit) {
+      const uint32_t idx = y * F.size[0] + x;
+      ended = false;
+      fresh = true;
+      if (ACCUM) {
+        sum = sum + rad + pe;
+        if (++sample >= F.spp) {
+          const float4 a = accum[idx];
+          accum[idx] = make_float4(a.x + sum.x, a.y + sum.y, a.z + sum.z, a.w + (float)F.spp);
+          sample = 0u;
+        }
+      } else {
+        G.rad[idx] = f4_to_h4(make_float4(rad.x, rad.y, rad.z, 1.0f));
+      }
+    }
+    bool start = fresh && ACCUM && sample > 0u;
+    for (;;) {
+      const bool ask = fresh && !start && !idle;
+      const uint32_t want = __ballot_sync(0xffffffffu, ask);
+      if (want == 0u) break;
+      uint32_t base = 0u;
+      if (lane == 0u) base = atomicAdd(&next_px, (uint32_t)__popc(want));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (ask) {
+        const uint32_t n = base + __popc(want & ((1u << lane) - 1u)), tile = blockIdx.x + (n >> 5u) * gridDim.x;
+        x = tile % tiles_x * 8u + (n & 7u);
+        y = tile / tiles_x * 4u + ((n >> 3u) & 3u);
+        if (n >= my_px) idle = true;
+        else start = x < F.size[0] && y < F.size[1] && (!ACCUM || F.spp > 0u);  // (else it asks again)
+        sum = f3(0.f, 0.f, 0.f);
+      }
+    }
+    if (start) {
+      const uint32_t idx = y * F.size[0] + x;
+      float px = (float)x, py = (float)y;
+      if (ACCUM) {
+        T.rng = pcg(idx ^ pcg((F.counts[2] + sample) * 0x9E3779B9u + F.frame * 7919u + 1u));
+        const float jx = T.rnd();
+        const float jy = T.rnd();
+        px = px + jx;
+        py = py + jy;
+      } else {
+        T.rng = pcg(idx ^ pcg(F.frame * 0x9E3779B9u + 17u));
+        px = px + 0.5f + F.jitter[0];
+        py = py + 0.5f + F.jitter[1];
+      }
+      rad = pe = f3(0.f, 0.f, 0.f);
+      tp = f3(1.f, 1.f, 1.f);
+      last_pdf = 0.0f;
+      depth = bounces = delta_chain = 0u;
+      put3(W_O, f3(F.cam_pos));
+      put3(W_D, T.primary_dir(px, py));
+      mask = 1u;
+      fresh = false;
+    }
+    // ---- the rays into the queue
+    for (uint32_t k = 0; k <= shadows; k++) {
+      const uint32_t m = __ballot_sync(0xffffffffu, mask >> k & 1u);
+      if (m == 0u) continue;
+      uint32_t base = 0u;
+      if (lane == 0u) base = atomicAdd(&filled[turn], (uint32_t)__popc(m));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (mask >> k & 1u) queue[base + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(k * NT + tid);
+    }
+    if (!__syncthreads_or(!idle)) break;
+    // ---- trace: lanes take rays as they become free
+    const uint32_t total = filled[turn];
+    Ray r;
+    r.e = RAY_DONE;
+    uint32_t entry = 0u;
+    bool more = true, held = false;
+    for (;;) {
+      if (held && r.e == RAY_DONE) {  // the ray's result
+        const uint32_t k = entry / NT, t = entry % NT;
+        if (k == 0u) {
+          Wf[W_T * NT + t] = r.t;
+          Wf[W_U * NT + t] = r.u;
+          Wf[W_V * NT + t] = r.v;
+          W[W_TRI * NT + t] = r.tri;
+        } else if (r.tri != NONE) {
+          Wf[(W_SHADOW + W_PER_SHADOW * (k - 1u) + 3u) * NT + t] = -1.0f;
+        }
+        held = false;
+      }
+      const uint32_t want = __ballot_sync(0xffffffffu, more && !held);
+      if (want) {
+        uint32_t base = 0u;
+        if (lane == 0u) base = atomicAdd(&taken[turn], (uint32_t)__popc(want));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (more && !held) {
+          const uint32_t n = base + __popc(want & ((1u << lane) - 1u));
+          more = n < total;
+          if (more) {
+            entry = queue[n];
+            held = true;
+            const uint32_t k = entry / NT, t = entry % NT, w = W_SHADOW + W_PER_SHADOW * (k - 1u);
+            T.start_ray(r, get3(W_O, t), get3(k ? w : (uint32_t)W_D, t), k ? Wf[(w + 3u) * NT + t] : INF, k > 0u);
+          }
+        }
+      }
+      const int rays = __popc(__ballot_sync(0xffffffffu, held));
+      if (rays == 0) break;
+      const int enough = __any_sync(0xffffffffu, more) ? rays - WAIT : 0;  // rays left when the finished ones are replaced
+      do {
+        int at = __popc(__ballot_sync(0xffffffffu, r.e == AT_NODE));
+        if (at > 0) {
+          do {
+            if (r.e == AT_NODE) T.node_step(r);
+            at = __popc(__ballot_sync(0xffffffffu, r.e == AT_NODE));
+          } while (at > NODE_LOW);
+        }
+        at = __popc(__ballot_sync(0xffffffffu, r.e - 1u < RAY_DONE - 1u));
+        if (at > 0) {
+          do {
+            if (r.e - 1u < RAY_DONE - 1u) T.tri_step(r);
+            at = __popc(__ballot_sync(0xffffffffu, r.e - 1u < RAY_DONE - 1u));
+          } while (at > TRI_LOW);
+        }
+      } while (__popc(__ballot_sync(0xffffffffu, r.e != RAY_DONE)) > max(enough, 0));
+    }
+    turn ^= 1u;
+    __syncthreads();
   }
 }
 
@@ -765,8 +970,23 @@ extern "C" int hush_pt_encode(hush_pt_t *p, const hush_pt_frame *f, int slot, vo
     return pt::fail(HUSH_ERR_ARG, "PathTracer.encode: env.w = 1 but no environment map is bound");
   cudaSetDevice(p->dev);
   const GBuf G{p->gbuf[slot][0], p->gbuf[slot][1], p->gbuf[slot][2], p->gbuf[slot][3], p->gbuf[slot][4]};
-  const dim3 grid((p->W + BW - 1) / BW, (p->H + BH - 1) / BH), blk(BW, BH);
-  k_pathtrace<<<grid, blk, 0, (cudaStream_t)stream>>>(*f, pt::scene_view(p->scene), p->env, G, p->accum);
+  const uint32_t tx = ((uint32_t)p->W + 7u) / 8u, tiles = tx * (((uint32_t)p->H + 3u) / 4u);
+  const uint32_t grid = std::min((tiles + NT / 32 - 1) / (NT / 32), 148u * CTAS);
+  const uint32_t shadows = f->counts[1] + (f->env[3] > 0.5f ? 1u : 0u);
+  const uint32_t stack = (uint32_t)pt::scene_depth(p->scene) + 1u;
+  const size_t smem = pt_smem(shadows, stack);
+  const int accum = f->mode == 0u ? 0 : 1;
+  void (*const kern[2])(hush_pt_frame, pt::SceneView, pt::EnvView, GBuf, float4 *, uint32_t, uint32_t, uint32_t, uint32_t) = {
+      k_pathtrace<false>, k_pathtrace<true>};
+  static bool opted[2][64] = {};  // dynamic shared memory above 48 KB, once per device and form
+  if (p->dev >= 64) return pt::fail(HUSH_ERR_ARG, "PathTracer.encode: device ordinal above 63");
+  if (!opted[accum][p->dev]) {
+    const cudaError_t oe = cudaFuncSetAttribute(kern[accum], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)pt_smem(HUSH_PT_MAX_LIGHTS + 1, pt::MAX_DEPTH + 1));
+    if (oe != cudaSuccess) return pt::fail(HUSH_ERR_CUDA, std::string("PathTracer.encode: ") + cudaGetErrorString(oe));
+    opted[accum][p->dev] = true;
+  }
+  kern[accum]<<<grid, NT, smem, (cudaStream_t)stream>>>(*f, pt::scene_view(p->scene), p->env, G, p->accum, tx, tiles, shadows, stack);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? HUSH_OK : pt::fail(HUSH_ERR_CUDA, std::string("PathTracer.encode: ") + cudaGetErrorString(e));
 }

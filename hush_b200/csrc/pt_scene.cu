@@ -542,7 +542,7 @@ extern "C" int hush_pt_scene_build(hush_pt_scene_t *s) {
       std::memcpy(&s->tri_idx[(size_t)(g.tri_offset + i) * 4], &g.local_idx[(size_t)src * 4], 16);
     }
   }
-  if (s->max_depth > 32)
+  if (s->max_depth > pt::MAX_DEPTH)
     return pt::fail(HUSH_ERR_ARG, "SceneGPU.build: BVH depth " + std::to_string(s->max_depth) +
                                       " exceeds the traversal stack (32)");
   s->nodes.assign((size_t)node_off * 16, 0.0f);
@@ -662,6 +662,7 @@ SceneView scene_view(const hush_pt_scene_t *s) {
   return v;
 }
 int scene_device(const hush_pt_scene_t *s) { return s->dev; }
+int scene_depth(const hush_pt_scene_t *s) { return s->max_depth; }
 bool scene_built(const hush_pt_scene_t *s) { return s && s->built; }
 }  // namespace pt
 
