@@ -5,7 +5,7 @@ import ctypes as C
 from typing import Optional
 
 from . import _lib as L
-from .hush import HushError, _FIELD, _stream_handle, device_view
+from .hush import HushError, OutputViews, _FIELD, _stream_handle, device_view
 
 SVGF_INPUTS = ["radiance", "normalDepth", "motion", "material", "emission", "prevNormalDepth", "prevMotion"]
 _OPT_FIELDS = {"iterations": "iterations", "sigmaL": "sigma_l", "sigmaN": "sigma_n", "sigmaZ": "sigma_z",
@@ -32,6 +32,7 @@ class SVGF:
         self._h = h
         self._w, self._hgt = int(width), int(height)
         self._inp = L.SvgfInputs()
+        self._out_views = OutputViews()
 
     @property
     def width(self) -> int:
@@ -42,22 +43,24 @@ class SVGF:
         return self._hgt
 
     def encode(self, inputs: dict, timer=None, stream=None):
+        inp, pitch = self._inp, self._inp.pitch
         for k, name in enumerate(SVGF_INPUTS):
             t = inputs.get(name)
             if t is None:
                 raise HushError(f"SVGF.encode: missing input '{name}'")
-            if not t.is_cuda or t.dtype.itemsize != 2 or t.dim() != 3 or t.shape[2] != 4:
+            shape = t.shape
+            if not t.is_cuda or t.dtype.itemsize != 2 or len(shape) != 3 or shape[2] != 4:
                 raise HushError(f"SVGF.encode: '{name}' must be a CUDA (H, W, 4) float16 tensor")
-            if t.shape[0] != self._hgt or t.shape[1] != self._w:
-                raise HushError(f"SVGF.encode: '{name}' is {t.shape[1]}x{t.shape[0]}, the denoiser "
+            if shape[0] != self._hgt or shape[1] != self._w:
+                raise HushError(f"SVGF.encode: '{name}' is {shape[1]}x{shape[0]}, the denoiser "
                                 f"{self._w}x{self._hgt} (call resize)")
-            setattr(self._inp, _FIELD[name], t.data_ptr())
-            self._inp.pitch[k] = t.stride(0) * 2
+            setattr(inp, _FIELD[name], t.data_ptr())
+            pitch[k] = t.stride(0) * 2
         out = C.c_void_p()
-        rc = L.lib().svgf_encode(self._h, C.byref(self._inp), C.c_void_p(_stream_handle(stream)), C.byref(out))
+        rc = L.lib().svgf_encode(self._h, C.byref(inp), C.c_void_p(_stream_handle(stream)), C.byref(out))
         if rc != L.HUSH_OK:
             raise HushError(L.lib().svgf_last_error(self._h).decode())
-        return device_view(out.value, self._hgt, self._w)
+        return self._out_views.get(out.value, self._hgt, self._w)
 
     denoise = encode
 
