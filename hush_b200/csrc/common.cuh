@@ -2,6 +2,7 @@
 // (src/denoise/hush.js:28-49, 67-74, 98-108).
 #pragma once
 #include <cuda_fp16.h>
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 #define HD_INL __device__ __forceinline__
@@ -91,5 +92,28 @@ constexpr float HMAX = 32.0f;
 constexpr float COARSE_S = 0.25f;  // hush.js:26
 constexpr int N_FEAT = 20;
 constexpr int N_OUT = 12;
+
+// A chain of short kernels, each launched as the next one's programmatic predecessor: a kernel's CTAs are set up while the one
+// before runs, and pass_begin(), the first thing that every kernel of the chain but the first does, waits for the end of that
+// one (which has waited for the end of its own predecessor, and so on). The first kernel waits for whatever the stream did
+// before, as any kernel; so does the first kernel after the chain.
+__device__ __forceinline__ void pass_begin(bool last = false) {
+  if (!last) asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t launch_pass(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, bool first, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = first ? 0 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
 
 }  // namespace hush

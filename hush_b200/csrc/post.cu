@@ -95,13 +95,6 @@ HD_INL float sub_texel(float u, int n) {  // the sampler's weight of a coordinat
   return x - floorf(x);
 }
 
-// The start of every pass but the first: the next pass may be set up, and this one waits until the one before has ended. (The
-// first pass does not say so: its 8100 short CTAs took 9.6 instead of 7.2 us with it, and the frame no less.)
-HD_INL void pass_begin(bool last = false) {
-  if (!last) asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 HD_INL uint2 pack_rgb1(float3 c, float a) { return f4_to_h4(make_float4(c.x, c.y, c.z, a)); }
 
 // COMPOSITE (post.js:27-38): left | mid | right at split / split2, times exposure; same = each third shows the
@@ -439,22 +432,13 @@ static int post_resize(hush_post_t *p, int W, int H) {
   return HUSH_OK;
 }
 
-// The passes are a chain of short kernels, so each is launched as the next one's programmatic predecessor: a pass's CTAs are
-// set up while the one before runs and wait for its end (pass_begin). The 12 gaps between the 13 passes of 1920x1080 took 22
-// us; with the small levels' passes begun early the frame is as long as its passes are (86.8 us). (The small levels in one
-// cluster of 16 CTAs took as long as their launches: 38 us from 240x135 on, 17.7 from 120x67 on.)
+// The passes are a chain of short kernels, each set up while the one before runs (launch_pass). The 12 gaps between the 13
+// passes of 1920x1080 took 22 us; with the small levels' passes begun early the frame is as long as its passes are (86.8
+// us). (The small levels in one cluster of 16 CTAs took as long as their launches: 38 us from 240x135 on, 17.7 from 120x67
+// on.) COMPOSITE does not let its successor in early: with 8100 short CTAs that made it 9.6 instead of 7.2 us long.
 template <class... P, class... A>
-static cudaError_t launch_pass(void (*kern)(P...), dim3 grid, bool first, cudaStream_t st, A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(BX, BY);
-  cfg.stream = st;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = first ? 0 : 1;  // the first pass waits for whatever the stream did before, as any kernel
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+static cudaError_t run_pass(void (*kern)(P...), dim3 grid, bool first, cudaStream_t st, A... args) {
+  return launch_pass(kern, grid, dim3(BX, BY), 0, first, st, args...);
 }
 
 // Post.encode (post.js:191-210).
@@ -482,24 +466,24 @@ extern "C" int hush_post_encode(hush_post_t *p, const hush_post_inputs *in, void
   auto half = [&](int sw, int sh, int dw, int dh) { return sw == 2 * dw && sh == 2 * dh; };
   const bool half0 = half(W, H, p->lw[0], p->lh[0]);
   const int *lw = p->lw, *lh = p->lh;
-  cudaError_t e = launch_pass(k_post_composite, grid_for(W, H), true, st, L, R, M, W, H, in->split, in->split2, in->exposure,
+  cudaError_t e = run_pass(k_post_composite, grid_for(W, H), true, st, L, R, M, W, H, in->split, in->split2, in->exposure,
                               in->same, p->hdr);
   if (e == cudaSuccess)
-    e = launch_pass(half0 ? k_post_down<true, true> : k_post_down<true, false>, grid_for(lw[0], lh[0]), false, st, p->hdr, W,
+    e = run_pass(half0 ? k_post_down<true, true> : k_post_down<true, false>, grid_for(lw[0], lh[0]), false, st, p->hdr, W,
                     H, p->lev[0], lw[0], lh[0]);
   for (int i = 1; i < LEVELS && e == cudaSuccess; i++)
-    e = launch_pass(half(lw[i - 1], lh[i - 1], lw[i], lh[i]) ? k_post_down<false, true> : k_post_down<false, false>,
+    e = run_pass(half(lw[i - 1], lh[i - 1], lw[i], lh[i]) ? k_post_down<false, true> : k_post_down<false, false>,
                     grid_for(lw[i], lh[i]), false, st, p->lev[i - 1], lw[i - 1], lh[i - 1], p->lev[i], lw[i], lh[i]);
   for (int i = LEVELS - 1; i > 0 && e == cudaSuccess; i--)
-    e = launch_pass(half(lw[i - 1], lh[i - 1], lw[i], lh[i]) ? k_post_up<true> : k_post_up<false>,
+    e = run_pass(half(lw[i - 1], lh[i - 1], lw[i], lh[i]) ? k_post_up<true> : k_post_up<false>,
                     grid_for(lw[i - 1], lh[i - 1]), false, st, p->lev[i], lw[i], lh[i], p->lev[i - 1], lw[i - 1], lh[i - 1]);
   FinalArgs fa{in->split, in->split2, in->line, p->d.bloom, p->d.vignette, p->d.format};
   if (e == cudaSuccess) {
     if (target_width == W && target_height == H && half0)
-      e = launch_pass(k_post_final_half, grid_for(lw[0], lh[0]), false, st, p->hdr, W, H, p->lev[0], lw[0], lh[0], target,
+      e = run_pass(k_post_final_half, grid_for(lw[0], lh[0]), false, st, p->hdr, W, H, p->lev[0], lw[0], lh[0], target,
                       pitch, fa);
     else
-      e = launch_pass(k_post_final, grid_for(target_width, target_height), false, st, p->hdr, W, H, p->lev[0], lw[0], lh[0],
+      e = run_pass(k_post_final, grid_for(target_width, target_height), false, st, p->hdr, W, H, p->lev[0], lw[0], lh[0],
                       target, target_width, target_height, pitch, fa);
   }
   return e == cudaSuccess ? HUSH_OK : post_fail(p, HUSH_ERR_CUDA, std::string("Post.encode: ") + cudaGetErrorString(e));
