@@ -1,6 +1,6 @@
 // The path tracer's kernel and the PathTracer instance (src/pt/pathtracer.js, pathtracer.wgsl.js).
 //
-// A persistent kernel that alternates two phases. Shade: every thread takes the path it holds one vertex on (the direct light
+// With an environment map, a persistent kernel that alternates two phases (without one, k_pathtrace_pixel). Shade: every thread takes the path it holds one vertex on (the direct light
 // its last shadow rays brought, then the hit's surface, the shadow rays of all its lights and the next direction; none of
 // these waits for another ray) and a thread whose path is complete takes the next pixel. Trace: the CTA's path and shadow rays
 // are one queue in shared memory, from which lanes take a ray whenever they are free, whatever pixel and kind it is of.
@@ -339,11 +339,11 @@ struct Tracer {
     const float pdf = st > 1e-5f ? __ldg(E.table + i).z * (float)N / (2.0f * PI * PI * st) : 0.0f;
     return make_float4(F.env[1] * l.x + F.env[2] * l.z, l.y, -F.env[2] * l.x + F.env[1] * l.z, pdf);
   }
-  DI float3 sky(float3 d) const {
-    if (F.env[3] > 0.5f) {
-      const float2 uv = env_uv(env_local(d));
-      return sample_env(uv.x, uv.y) * F.env[0];
-    }
+  DI float3 sky_map(float3 d) const {
+    const float2 uv = env_uv(env_local(d));
+    return sample_env(uv.x, uv.y) * F.env[0];
+  }
+  DI float3 sky_gradient(float3 d) const {  // without a map
     float3 c;
     if (d.y >= 0.0f) c = lerp3(f3(F.sky_horizon), f3(F.sky_zenith), powf(clampf(d.y, 0.0f, 1.0f), 0.6f));
     else c = lerp3(f3(F.sky_horizon), f3(F.ground), clampf(-d.y * 4.0f, 0.0f, 1.0f));
@@ -522,15 +522,13 @@ struct Tracer {
       const float q = fminf(1.0f, w_sum / F.shadow_tau);
       if (rnd() < q) put(0u, pick_d, pick_t, pick_c * (w_sum / (pick_w * q)));
     }
-    if (F.env[3] > 0.5f) {
-      const float4 es = sample_env_dir();
-      const float3 ed = f3(es);
-      const float3 ll = to_local(frame, ed);
-      if (es.w > 0.0f && ll.z > 0.0f && dot(ed, s.ng) > 0.0f) {
-        float3 f;
-        const float pdf = eval_bsdf(s, v, ll, f).w;
-        if (lum(f) > 0.0f) put(nl, ed, INF, f * sky(ed) / es.w * mis(es.w, pdf));
-      }
+    const float4 es = sample_env_dir();
+    const float3 ed = f3(es);
+    const float3 ll = to_local(frame, ed);
+    if (es.w > 0.0f && ll.z > 0.0f && dot(ed, s.ng) > 0.0f) {
+      float3 f;
+      const float pdf = eval_bsdf(s, v, ll, f).w;
+      if (lum(f) > 0.0f) put(nl, ed, INF, f * sky_map(ed) / es.w * mis(es.w, pdf));
     }
   }
 
@@ -552,6 +550,276 @@ struct Tracer {
   }
 };
 
+// Without an environment map a vertex has a shadow ray fewer and half the shading, and one thread per pixel, tracing where a
+// ray is needed, is faster: 1920x1080, 32 objects of three seeds, 2236 / 1965 / 1747 us (2312 / 2012 / 1825 with the map's code
+// in the kernel) against 2301 / 2063 / 1958 in phases; with the map 4102 / 3559 / 3379 against 2706 / 2386 / 2327. 8 x 8 pixel
+// blocks, a warp an 8 x 4 patch; traversal stacks in shared memory, slot-major.
+constexpr int PIXEL_NT = 64;
+struct PixelTracer : Tracer {
+  // closest (or, for shadow rays, any) hit over the BLAS list; packed BVH2 (both child boxes per 64-byte node)
+  DI Hit trace_bvh(float3 o, float3 d, float tmax_in, bool shadow) const {
+    Hit h{tmax_in, NONE, 0.0f, 0.0f, -1};
+    const float3 inv = f3(1.0f / (fabsf(d.x) < 1e-9f ? 1e-9f : d.x), 1.0f / (fabsf(d.y) < 1e-9f ? 1e-9f : d.y),
+                          1.0f / (fabsf(d.z) < 1e-9f ? 1e-9f : d.z));
+    for (uint32_t b = 0; b < F.counts[0]; b++) {
+      const hush_pt_blas bl = F.blas[b];
+      if (shadow && (bl.flags & 2u)) continue;
+      uint32_t sp = 0, node = 0;
+      // a BVH built by the scene visits each node at most once per ray; the cap only bounds a corrupted one
+      for (uint32_t guard = 0; guard < (1u << 24); guard++) {
+        const float4 *nd = S.nodes + (size_t)(bl.node_offset + node) * 4;
+        const float4 lmin = __ldg(nd), lmax = __ldg(nd + 1), rmin = __ldg(nd + 2), rmax = __ldg(nd + 3);
+        float tl = slab(o, inv, lmin, lmax, h.t);
+        float tr = slab(o, inv, rmin, rmax, h.t);
+        const uint32_t lc = __float_as_uint(lmax.w), rc = __float_as_uint(rmax.w);
+        if (lc > 0u && tl < INF) {
+          const uint32_t first = bl.tri_offset + __float_as_uint(lmin.w);
+          for (uint32_t i = 0; i < lc; i++) {
+            const float3 r = hit_tri(o, d, first + i, h.t);
+            if (r.x < h.t) {
+              h.t = r.x; h.u = r.y; h.v = r.z; h.tri = first + i;
+              if (shadow) return h;
+            }
+          }
+          tl = INF;
+        }
+        if (rc > 0u && tr < h.t) {
+          const uint32_t first = bl.tri_offset + __float_as_uint(rmin.w);
+          for (uint32_t i = 0; i < rc; i++) {
+            const float3 r = hit_tri(o, d, first + i, h.t);
+            if (r.x < h.t) {
+              h.t = r.x; h.u = r.y; h.v = r.z; h.tri = first + i;
+              if (shadow) return h;
+            }
+          }
+          tr = INF;
+        }
+        const uint32_t l = __float_as_uint(lmin.w), r = __float_as_uint(rmin.w);
+        if (tl < h.t && tr < h.t) {
+          const bool near_left = tl <= tr;
+          node = near_left ? l : r;
+          stk[sp * PIXEL_NT] = near_left ? r : l;
+          sp = min(sp + 1u, (uint32_t)pt::MAX_DEPTH - 1u);
+        } else if (tl < h.t) {
+          node = l;
+        } else if (tr < h.t) {
+          node = r;
+        } else {
+          if (sp == 0u) break;
+          node = stk[--sp * PIXEL_NT];
+        }
+      }
+    }
+    return h;
+  }
+
+  DI Hit trace_scene(float3 o, float3 d) const { return closest(o, d, trace_bvh(o, d, INF, false)); }
+
+  DI bool visible(float3 o, float3 d, float tmax) const { return trace_bvh(o, d, tmax, true).tri == NONE; }
+
+
+  DI float3 direct_light(const Surf &s, const Basis &frame, float3 v, float3 tp, bool all) {
+    float3 acc = f3(0.f, 0.f, 0.f), pick_c = acc, pick_d = acc;
+    float w_sum = 0.0f, pick_w = 0.0f, pick_t = 0.0f;
+    for (uint32_t i = 0; i < F.counts[1]; i++) {
+      const hush_pt_light &L = F.lights[i];
+      const float4 ax = cone_axis(L, s.p);
+      if (ax.w < -1.0f) continue;
+      const float ct = 1.0f - rnd() * (1.0f - ax.w);
+      const float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
+      const float ph = 2.0f * PI * rnd();
+      const float3 dir = normalize(to_world(onb(f3(ax)), f3(cosf(ph) * st, sinf(ph) * st, ct)));
+      const float3 ll = to_local(frame, dir);
+      if (ll.z <= 0.0f || dot(dir, s.ng) <= 0.0f) continue;
+      float3 f;
+      const float pdf = eval_bsdf(s, v, ll, f).w;
+      if (pdf <= 0.0f && lum(f) <= 0.0f) continue;
+      const float tmax = L.params[0] == 1.0f ? sphere_t(s.p, dir, f3(L.pos), L.pos[3]) : INF;
+      const float lp = cone_pdf(ax.w);
+      const float3 c = f * f3(L.radiance) / lp * mis(lp, pdf);
+      if (all) {
+        if (!visible(s.p + s.ng * 1e-3f, dir, tmax)) continue;
+        acc = acc + c;
+      } else {
+        const float wl = lum(tp * c);
+        if (wl <= 0.0f) continue;
+        w_sum += wl;
+        if (rnd() * w_sum < wl) { pick_d = dir; pick_t = tmax; pick_c = c; pick_w = wl; }
+      }
+    }
+    if (!all && w_sum > 0.0f) {
+      const float q = fminf(1.0f, w_sum / F.shadow_tau);
+      if (rnd() < q && visible(s.p + s.ng * 1e-3f, pick_d, pick_t)) acc = pick_c * (w_sum / (pick_w * q));
+    }
+    return acc;
+  }
+
+  // tracePath (pathtracer.wgsl.js:511-646); with write_g the primary hit's G-buffer values go to g[0..11]
+  DI void trace_path(float pix_x, float pix_y, bool write_g, float3 &radiance, float3 &prim_emission, float *g) {
+    radiance = f3(0.f, 0.f, 0.f);
+    prim_emission = radiance;
+    const float ndx = (pix_x / (float)F.size[0]) * 2.0f - 1.0f, ndy = (pix_y / (float)F.size[1]) * 2.0f - 1.0f;
+    float3 o = f3(F.cam_pos);
+    float3 d = normalize(f3(F.cam_fwd) + f3(F.cam_right) * ndx - f3(F.cam_up) * ndy);
+    float3 tp = f3(1.f, 1.f, 1.f);
+    float last_pdf = 0.0f, lod_base = 1.0f;
+    uint32_t bounces = 0, delta_chain = 0;
+    for (uint32_t depth = 0; depth < 12u; depth++) {
+      const Hit h = trace_scene(o, d);
+      const bool primary = depth == 0u;
+      if (h.tri == NONE && h.light < 0) {  // sky
+        float3 e = sky_gradient(d);
+        for (uint32_t i = 0; i < F.counts[1]; i++) {  // sun disks reached by BSDF sampling
+          const hush_pt_light &L = F.lights[i];
+          if (L.params[0] == 0.0f && dot(d, f3(L.pos)) >= L.params[1])
+            e = e + f3(L.radiance) * (last_pdf > 0.0f ? mis(last_pdf, cone_pdf(L.params[1])) : 1.0f);
+        }
+        if (primary) {
+          prim_emission = e;
+          if (write_g) {
+            const float2 a = project_pix(F.prev_view_proj, d.x, d.y, d.z, 0.0f);
+            const float2 b = project_pix(F.view_proj, d.x, d.y, d.z, 0.0f);
+            const float gv[12] = {-d.x, -d.y, -d.z, -1.0f, a.x - b.x, a.y - b.y, 65535.0f, -1.0f, 1.f, 1.f, 1.f, 1.f};
+#pragma unroll
+            for (int k = 0; k < 12; k++) g[k] = gv[k];
+          }
+        } else {
+          float3 c = tp * e;
+          const float lc = lum(c);
+          if (lc > F.clamp_lum) c = c * (F.clamp_lum / lc);
+          radiance = radiance + c;
+        }
+        break;
+      }
+      const Surf s = fetch_surf(h, o, d, lod_base);
+      if (lum(s.emissive) > 0.0f) {
+        float3 e = s.emissive;
+        if (h.light >= 0 && last_pdf > 0.0f) e = e * mis(last_pdf, cone_pdf(cone_axis(F.lights[h.light], o).w));
+        if (primary) {
+          prim_emission = e;
+        } else {
+          float3 c = tp * e;
+          const float lc = lum(c);
+          if (lc > F.clamp_lum) c = c * (F.clamp_lum / lc);
+          radiance = radiance + c;
+        }
+      }
+      const bool glass = s.transmission > 0.5f;
+      if (primary && write_g) {
+        const bool white = glass || h.light >= 0;
+        const float3 alb = s.base * (1.0f - s.metal) + lerp3(f3(0.04f, 0.04f, 0.04f), s.base, s.metal) * s.metal;
+        const float2 a = project_pix(F.prev_view_proj, s.prev_p.x, s.prev_p.y, s.prev_p.z, 1.0f);
+        const float2 b = project_pix(F.view_proj, s.p.x, s.p.y, s.p.z, 1.0f);
+        const float *pm = F.prev_view_proj;
+        const float prev_w = pm[3] * s.prev_p.x + pm[7] * s.prev_p.y + pm[11] * s.prev_p.z + pm[15];
+        g[0] = s.n.x; g[1] = s.n.y; g[2] = s.n.z;
+        g[3] = dot(s.p - f3(F.cam_pos), f3(F.cam_fwd));
+        g[4] = a.x - b.x; g[5] = a.y - b.y;
+        g[6] = (float)s.obj;
+        g[7] = prev_w;
+        g[8] = white ? 1.0f : fmaxf(alb.x, 0.02f);
+        g[9] = white ? 1.0f : fmaxf(alb.y, 0.02f);
+        g[10] = white ? 1.0f : fmaxf(alb.z, 0.02f);
+        g[11] = glass ? 0.0f : s.rough;
+      }
+      if (h.light >= 0) break;
+      if (glass) {  // smooth dielectric: Fresnel-weighted reflect / refract
+        if (++delta_chain > 8u) break;
+        const float eta = s.front ? 1.0f / s.ior : s.ior;
+        const float3 n = s.ng;
+        const float c = -dot(d, n);
+        const float k = 1.0f - eta * eta * (1.0f - c * c);
+        float R = 1.0f;
+        if (k > 0.0f) {
+          const float ct = sqrtf(k);
+          const float rs = (eta * c - ct) / (eta * c + ct), rp = (c - eta * ct) / (c + eta * ct);
+          R = 0.5f * (rs * rs + rp * rp);
+        }
+        if (rnd() < R) {
+          d = reflect(d, n);
+          o = s.p + n * 1e-3f;
+        } else {
+          d = normalize(d * eta + n * (eta * c - sqrtf(k)));
+          o = s.p - n * 1e-3f;
+          tp = tp * s.base;
+        }
+        last_pdf = 0.0f;
+        continue;
+      }
+      if (bounces >= F.max_bounces) break;
+      bounces++;
+      const Basis frame = onb(s.n);
+      const float3 v = to_local(frame, -d);
+      if (v.z <= 0.0f) break;
+      float3 dl = tp * direct_light(s, frame, v, tp, primary || F.shadow_tau <= 0.0f);
+      const float cl = primary ? (F.clamp_direct > 0.0f ? F.clamp_direct : INF) : F.clamp_lum;
+      const float ld = lum(dl);
+      if (ld > cl) dl = dl * (cl / ld);
+      radiance = radiance + dl;
+      const float ps = spec_prob(s, v.z);
+      float3 l;
+      if (rnd() < ps) {
+        const float a = fmaxf(s.rough * s.rough, 0.0025f);
+        const float u1 = rnd();
+        const float u2 = rnd();
+        l = reflect(-v, sample_vndf(v, a, u1, u2));
+      } else {
+        const float r = sqrtf(rnd());
+        const float ph = 2.0f * PI * rnd();
+        l = f3(r * cosf(ph), r * sinf(ph), sqrtf(fmaxf(0.0f, 1.0f - r * r)));
+      }
+      if (l.z <= 0.0f) break;
+      float3 f;
+      const float pdf = eval_bsdf(s, v, l, f).w;
+      if (pdf <= 0.0f) break;
+      tp = tp * f / pdf;
+      last_pdf = pdf;
+      d = normalize(to_world(frame, l));
+      if (dot(d, s.ng) <= 0.0f) break;
+      o = s.p + s.ng * 1e-3f;
+      lod_base = 4.0f;
+      if (bounces >= 2u) {  // Russian roulette
+        const float q = clampf(fmaxf(tp.x, fmaxf(tp.y, tp.z)), 0.05f, 0.95f);
+        if (rnd() > q) break;
+        tp = tp / q;
+      }
+    }
+  }
+};
+
+__global__ void __launch_bounds__(PIXEL_NT, 8) k_pathtrace_pixel(const __grid_constant__ hush_pt_frame F, const pt::SceneView S,
+                                                   const pt::EnvView E, const GBuf G, float4 *__restrict__ accum) {
+  __shared__ uint32_t stacks[pt::MAX_DEPTH * PIXEL_NT];
+  const uint32_t t = threadIdx.y * 8 + threadIdx.x;
+  const uint32_t x = blockIdx.x * 8 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+  if (x >= F.size[0] || y >= F.size[1]) return;  // no block-wide barrier below
+  PixelTracer T{{F, S, E, stacks + t, (uint32_t)pt::MAX_DEPTH, 0u}};
+  const uint32_t idx = y * F.size[0] + x;
+  if (F.mode == 0u) {
+    T.rng = pcg(idx ^ pcg(F.frame * 0x9E3779B9u + 17u));
+    float3 rad, pe;
+    float g[12];
+    T.trace_path((float)x + 0.5f + F.jitter[0], (float)y + 0.5f + F.jitter[1], true, rad, pe, g);
+    G.rad[idx] = f4_to_h4(make_float4(rad.x, rad.y, rad.z, 1.0f));
+    G.nd[idx] = f4_to_h4(make_float4(g[0], g[1], g[2], g[3]));
+    G.mv[idx] = f4_to_h4(make_float4(g[4], g[5], g[6], g[7]));
+    G.mat[idx] = f4_to_h4(make_float4(g[8], g[9], g[10], g[11]));
+    G.emi[idx] = f4_to_h4(make_float4(pe.x, pe.y, pe.z, 0.0f));
+  } else {
+    float3 sum = f3(0.f, 0.f, 0.f);
+    for (uint32_t sp = 0; sp < F.spp; sp++) {
+      T.rng = pcg(idx ^ pcg((F.counts[2] + sp) * 0x9E3779B9u + F.frame * 7919u + 1u));
+      const float jx = T.rnd();
+      const float jy = T.rnd();
+      float3 rad, pe;
+      T.trace_path((float)x + jx, (float)y + jy, false, rad, pe, nullptr);
+      sum = sum + rad + pe;
+    }
+    const float4 a = accum[idx];
+    accum[idx] = make_float4(a.x + sum.x, a.y + sum.y, a.z + sum.z, a.w + (float)F.spp);
+  }
+}
+
 // Shared memory of a CTA, in words: the thread's path ray (origin, direction) and its hit, then 7 words per shadow ray, each
 // thread-minor, the traversal stacks and the queue of rays to trace (entry k * NT + thread: k = 0 the path ray, else shadow
 // ray k - 1; 16 bits).
@@ -561,7 +829,7 @@ constexpr size_t pt_smem(uint32_t shadows, uint32_t stack) {
   return (size_t)NT * 4 * (words_per_thread(shadows) + stack) + (size_t)NT * 2 * (shadows + 1);
 }
 
-// main() and tracePath (pathtracer.wgsl.js:511-672). CTAs walk the image's 8 x 4 tiles (tile blockIdx.x, + gridDim.x, ...) and
+// main() and tracePath (pathtracer.wgsl.js:511-672) with an environment map. CTAs walk the image's 8 x 4 tiles (tile blockIdx.x, + gridDim.x, ...) and
 // hand out their pixels one by one. In mode 0 the primary hit's G-buffer values are stored when they are known, the radiance
 // when the path is complete.
 template <bool ACCUM>
@@ -617,8 +885,8 @@ __global__ void __launch_bounds__(NT, CTAS) k_pathtrace(const __grid_constant__ 
       float3 no = o, nd = d;
       bool emit = false;
       if (h.tri == NONE && h.light < 0) {  // sky
-        float3 e = T.sky(d);
-        if (F.env[3] > 0.5f && last_pdf > 0.0f) e = e * T.mis(last_pdf, T.env_pdf(d));
+        float3 e = T.sky_map(d);
+        if (last_pdf > 0.0f) e = e * T.mis(last_pdf, T.env_pdf(d));
         for (uint32_t i = 0; i < F.counts[1]; i++) {  // sun disks reached by BSDF sampling
           const hush_pt_light &L = F.lights[i];
           if (L.params[0] == 0.0f && dot(d, f3(L.pos)) >= L.params[1])
@@ -970,23 +1238,18 @@ extern "C" int hush_pt_encode(hush_pt_t *p, const hush_pt_frame *f, int slot, vo
     return pt::fail(HUSH_ERR_ARG, "PathTracer.encode: env.w = 1 but no environment map is bound");
   cudaSetDevice(p->dev);
   const GBuf G{p->gbuf[slot][0], p->gbuf[slot][1], p->gbuf[slot][2], p->gbuf[slot][3], p->gbuf[slot][4]};
-  const uint32_t tx = ((uint32_t)p->W + 7u) / 8u, tiles = tx * (((uint32_t)p->H + 3u) / 4u);
-  const uint32_t grid = std::min((tiles + NT / 32 - 1) / (NT / 32), 148u * CTAS);
-  const uint32_t shadows = f->counts[1] + (f->env[3] > 0.5f ? 1u : 0u);
-  const uint32_t stack = (uint32_t)pt::scene_depth(p->scene) + 1u;
-  const size_t smem = pt_smem(shadows, stack);
-  const int accum = f->mode == 0u ? 0 : 1;
-  void (*const kern[2])(hush_pt_frame, pt::SceneView, pt::EnvView, GBuf, float4 *, uint32_t, uint32_t, uint32_t, uint32_t) = {
-      k_pathtrace<false>, k_pathtrace<true>};
-  static bool opted[2][64] = {};  // dynamic shared memory above 48 KB, once per device and form
-  if (p->dev >= 64) return pt::fail(HUSH_ERR_ARG, "PathTracer.encode: device ordinal above 63");
-  if (!opted[accum][p->dev]) {
-    const cudaError_t oe = cudaFuncSetAttribute(kern[accum], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)pt_smem(HUSH_PT_MAX_LIGHTS + 1, pt::MAX_DEPTH + 1));
-    if (oe != cudaSuccess) return pt::fail(HUSH_ERR_CUDA, std::string("PathTracer.encode: ") + cudaGetErrorString(oe));
-    opted[accum][p->dev] = true;
+  const pt::SceneView scene = pt::scene_view(p->scene);
+  if (f->env[3] > 0.5f) {
+    const uint32_t tx = ((uint32_t)p->W + 7u) / 8u, tiles = tx * (((uint32_t)p->H + 3u) / 4u);
+    const uint32_t grid = std::min((tiles + NT / 32 - 1) / (NT / 32), 148u * CTAS);
+    const uint32_t shadows = f->counts[1] + 1u, stack = (uint32_t)pt::scene_depth(p->scene) + 1u;
+    static_assert(pt_smem(HUSH_PT_MAX_LIGHTS + 1, pt::MAX_DEPTH + 1) <= 48 * 1024, "else opt in to larger shared memory");
+    (f->mode == 0u ? k_pathtrace<false> : k_pathtrace<true>)<<<grid, NT, pt_smem(shadows, stack), (cudaStream_t)stream>>>(
+        *f, scene, p->env, G, p->accum, tx, tiles, shadows, stack);
+  } else {
+    k_pathtrace_pixel<<<dim3((p->W + 7) / 8, (p->H + 7) / 8), dim3(8, 8), 0, (cudaStream_t)stream>>>(*f, scene, p->env, G,
+                                                                                                  p->accum);
   }
-  kern[accum]<<<grid, NT, smem, (cudaStream_t)stream>>>(*f, pt::scene_view(p->scene), p->env, G, p->accum, tx, tiles, shadows, stack);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? HUSH_OK : pt::fail(HUSH_ERR_CUDA, std::string("PathTracer.encode: ") + cudaGetErrorString(e));
 }
