@@ -1042,9 +1042,10 @@ __global__ void __launch_bounds__(HT_W *HT_H) k_half_stage(const __grid_constant
 
 // stages 2 and 3 with the two-pixel mid tiles: 32 x 8 mid2 / mid3 tiles (HP_MID), or stage 2's coarse2 tiles (16 x 8,
 // quarter resolution; HP_COARSE). Dynamic shared memory: the pair tile, or coarse2's two float4 tiles.
-template <int STAGE, int PART>
+template <int STAGE, int PART, bool NEXT>
 __global__ void __launch_bounds__(HT_W *HT_H) k_half_pair(const __grid_constant__ HushFrame f, int nAx, int nA,
                                                           int nBx, const __grid_constant__ HalfMaps M) {
+  if constexpr (NEXT) pass_begin(true);
   extern __shared__ __align__(128) float4 hp_smem[];  // 128-byte aligned: coarse2 stages its guide by TMA
   const int b = (int)blockIdx.x;
   if (PART == HP_MID) {
@@ -1337,7 +1338,9 @@ __global__ void __launch_bounds__(FF_NT, 2) k_fine_final_fused(const __grid_cons
 // YCoCg tile is held as (Y, Co) pairs beside a Cg plane, so the 3x3 statistics, the history sum, the clip bounds and
 // the blend run (Y, Co) as one packed FP32x2 operation and Cg as a scalar one, lane by lane the same arithmetic
 // (40 registers: six CTAs per SM).
+template <bool NEXT>  // launched as FINE_FINAL's programmatic successor
 __global__ void __launch_bounds__(FT_W *FT_H) k_taa_fused(const __grid_constant__ HushFrame f) {
+  if constexpr (NEXT) pass_begin(true);
   constexpr int SW = FT_W + 2, SH = FT_H + 2, NT = FT_W * FT_H, NIT = (SW * SH + NT - 1) / NT;
   __shared__ float2 sXY[SW * SH];
   __shared__ float sXZ[SW * SH];
@@ -1524,11 +1527,20 @@ static void (*const KB_KERN[6])(HushFrame, MlpConst, const uint4 *) = {
     k_temporal_block<0, KB_TH>, k_temporal_block<1, KB_TH>,     k_temporal_block<2, KB_TH>,
     k_temporal_block<3, KB_TH>, k_temporal_block<0, KB_TH / 2>, k_temporal_block<3, KB_TH / 2>};
 
+// The kernels that directly follow another one of the frame on their stream (mid2, mid3, coarse2, TAA) are set up while that
+// one runs: directly launched frames 256x256 43.2 -> 39.7 us, 640x360 60.5 -> 55.0, 1283x717 144.5 -> 142.0. Captured frames
+// keep plain launches: replayed they are no faster (1920x1080 247 -> 249 us), and their kernel nodes' parameters are rewritten.
+static bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
+}
+
 cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const MlpConst &mc, int mlp_mode,
                                const void *mlp_tc, cudaStream_t st) {
   const int hx = (f.W2 + HT_W - 1) / HT_W, hy = (f.H2 + HT_H - 1) / HT_H;
   const int qx = (f.W4 + HT_W - 1) / HT_W, qy = (f.H4 + HT_H - 1) / HT_H;
   const int hpx = (f.W2 + MP_W - 1) / MP_W;  // two-pixel mid tiles per row
+  const bool full = (stage == 2 || stage == 3 || stage == 5) && capturing(st);  // plain launches
   switch (stage) {
     case 0: {
       // blob: the tensor-core forms' bf16 hi / lo operands and f16 operands; mc: the weights as a kernel parameter
@@ -1564,15 +1576,21 @@ cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const Ml
       break;
     case 2: {
       constexpr int smc = 2 * (HT_W + 8) * (HT_H + 8) * 16;  // coarse2's two float4 tiles
+      cudaError_t e = cudaSuccess;
       if (part != HP_COARSE)
-        k_half_pair<2, HP_MID><<<hpx * hy, HT_W * HT_H, mid_pair_smem<2>(), st>>>(f, hpx, hpx * hy, qx, half_maps(f));
-      if (part != HP_MID)
-        k_half_pair<2, HP_COARSE><<<qx * qy, HT_W * HT_H, smc, st>>>(f, hpx, hpx * hy, qx, half_maps(f));
+        e = launch_pass(full ? k_half_pair<2, HP_MID, false> : k_half_pair<2, HP_MID, true>, dim3(hpx * hy), dim3(HT_W * HT_H), (size_t)mid_pair_smem<2>(), full, st, f, hpx,
+                        hpx * hy, qx, half_maps(f));
+      if (part != HP_MID && e == cudaSuccess)
+        e = launch_pass(full ? k_half_pair<2, HP_COARSE, false> : k_half_pair<2, HP_COARSE, true>, dim3(qx * qy), dim3(HT_W * HT_H), (size_t)smc, full, st, f, hpx, hpx * hy, qx,
+                        half_maps(f));
+      if (e != cudaSuccess) return e;
       break;
     }
     case 3:
       if (part == HP_COARSE) break;  // no coarse level in stage 3
-      k_half_pair<3, HP_MID><<<hpx * hy, HT_W * HT_H, mid_pair_smem<4>(), st>>>(f, hpx, hpx * hy, qx, half_maps(f));
+      if (const cudaError_t e = launch_pass(full ? k_half_pair<3, HP_MID, false> : k_half_pair<3, HP_MID, true>,
+                                            dim3(hpx * hy), dim3(HT_W * HT_H), (size_t)mid_pair_smem<4>(), full, st, f, hpx, hpx * hy, qx, half_maps(f)))
+        return e;
       break;
     case 4: {
       const int tx = (f.W + FF_W - 1) / FF_W, tiles = tx * ((f.H + FF_H - 1) / FF_H);
@@ -1591,7 +1609,11 @@ cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const Ml
       k_fine_final_fused<<<std::min(tiles, 2 * sms[dev]), FF_NT, sizeof(FineSmem), st>>>(f, tx, tiles);
       break;
     }
-    case 5: k_taa_fused<<<dim3((f.W + FT_W - 1) / FT_W, (f.H + FT_H - 1) / FT_H), FT_W * FT_H, 0, st>>>(f); break;
+    case 5:
+      if (const cudaError_t e = launch_pass(full ? k_taa_fused<false> : k_taa_fused<true>, dim3((f.W + FT_W - 1) / FT_W, (f.H + FT_H - 1) / FT_H),
+                                            dim3(FT_W * FT_H), 0, full, st, f))
+        return e;
+      break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -1603,12 +1625,12 @@ int fused_kernel_param_count(const void *func) {
   for (auto *k : KB_KERN)
     if (func == (const void *)k) return 3;  // (f, wp, blob)
   const void *half[5] = {(const void *)k_half_stage<1, HP_MID>, (const void *)k_half_stage<1, HP_COARSE>,
-                         (const void *)k_half_pair<2, HP_MID>, (const void *)k_half_pair<2, HP_COARSE>,
-                         (const void *)k_half_pair<3, HP_MID>};
+                         (const void *)k_half_pair<2, HP_MID, false>, (const void *)k_half_pair<2, HP_COARSE, false>,
+                         (const void *)k_half_pair<3, HP_MID, false>};
   for (const void *k : half)
     if (func == k) return 5;  // (f, nAx, nA, nBx, M)
   if (func == (const void *)k_fine_final_fused) return 3;  // (f, tiles_x, tiles)
-  if (func == (const void *)k_taa_fused) return 1;          // (f)
+  if (func == (const void *)k_taa_fused<false>) return 1;          // (f)
   return 0;
 }
 
