@@ -30,6 +30,12 @@ HD_INL float2 unpack2(uint32_t u) {
   return __half22float2(h);
 }
 HD_INL float4 ldh(const uint2 *__restrict__ p, int idx) { return h4_to_f4(__ldg(p + idx)); }
+// A texel that an earlier kernel of a programmatic chain (pass_begin(), below) writes: by an ordinary load. __ldg's
+// ld.global.nc is for memory that nobody writes while the kernel is resident, and a kernel of such a chain is resident
+// before its predecessor has written, so that no wait orders it.
+template <class T>
+HD_INL T ld_pass(const T *p) { return *p; }
+HD_INL float4 ldh_pass(const uint2 *p, int idx) { return h4_to_f4(ld_pass(p + idx)); }
 HD_INL void sth(uint2 *__restrict__ p, int idx, float4 v) { p[idx] = f4_to_h4(v); }
 HD_INL float4 quant4(float4 v) {  // value after an rgba16float round trip
   return h4_to_f4(f4_to_h4(v));
@@ -96,7 +102,9 @@ constexpr int N_OUT = 12;
 // A chain of short kernels, each launched as the next one's programmatic predecessor: a kernel's CTAs are set up while the one
 // before runs, and pass_begin(), the first thing that every kernel of the chain but the first does, waits for the end of that
 // one (which has waited for the end of its own predecessor, and so on). The first kernel waits for whatever the stream did
-// before, as any kernel; so does the first kernel after the chain.
+// before, as any kernel; so does the first kernel after the chain. What a kernel of the chain writes is read in it by ld_pass() and
+// ldh_pass() and never through a `const __restrict__` parameter; the caller's inputs and former frames' images, which no
+// kernel of the chain writes, may take the read-only path.
 __device__ __forceinline__ void pass_begin(bool last = false) {
   if (!last) asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -931,8 +931,8 @@ HD_INL void tile_coarse2(const HushFrame &f, int tileX, int tileY, float4 *sA, f
   if (!staged) {
     for (int i = li; i < SW * SH; i += HT_W * HT_H) {
       const int q = clampi(by - AP + i / SW, 0, f.H4 - 1) * f.W4 + clampi(bx - AP + i % SW, 0, f.W4 - 1);
-      sA[i] = ldh(f.C1, q);
-      sG[i] = __ldg(f.CGd + q);
+      sA[i] = ldh_pass(f.C1, q);
+      sG[i] = ld_pass(f.CGd + q);
     }
   }
   __syncthreads();
@@ -981,9 +981,9 @@ HD_INL void tile_mid_pair(const HushFrame &f, int tileX, int tileY, const uint2 
     const int x0 = clampi(gx, 0, f.W2 - 1), x1 = clampi(gx + 1, 0, f.W2 - 1);
     if (e < NE) {
       if (even_w && gx >= 0 && gx + 1 < f.W2) {
-        lv[i] = __ldg(reinterpret_cast<const uint4 *>(src + gy * f.W2 + gx));
+        lv[i] = ld_pass(reinterpret_cast<const uint4 *>(src + gy * f.W2 + gx));
       } else {
-        const uint2 a = __ldg(src + gy * f.W2 + x0), b = __ldg(src + gy * f.W2 + x1);
+        const uint2 a = ld_pass(src + gy * f.W2 + x0), b = ld_pass(src + gy * f.W2 + x1);
         lv[i] = make_uint4(a.x, a.y, b.x, b.y);
       }
       qa[i] = __ldg(f.Gd + gy * f.W2 + x0);
@@ -1354,9 +1354,9 @@ __global__ void __launch_bounds__(FT_W *FT_H) k_taa_fused(const __grid_constant_
 #pragma unroll
   for (int it = 0; it < NIT; it++) {
     const int i = min(li + it * NT, SW * SH - 1);
-    tl[it] = __ldg(f.X + clampi(oy + i / SW, 0, f.H - 1) * f.W + clampi(ox + i % SW, 0, f.W - 1));
+    tl[it] = ld_pass(f.X + clampi(oy + i / SW, 0, f.H - 1) * f.W + clampi(ox + i % SW, 0, f.W - 1));
   }
-  const uint2 xr = __ldg(f.X + cpy * f.W + cpx);
+  const uint2 xr = ld_pass(f.X + cpy * f.W + cpx);
   // the history footprint (clamped loads; used only when the reprojected position lies inside the image)
   const float4 mv = h4_to_f4(mvr);
   const float szx = (float)f.W, szy = (float)f.H;

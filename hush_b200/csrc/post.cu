@@ -26,8 +26,8 @@ namespace {
 constexpr int LEVELS = HUSH_POST_LEVELS;  // post.js:135
 constexpr int BX = 32, BY = 8;
 
-HD_INL float3 ld3(const uint2 *__restrict__ img, int w, int x, int y) {
-  const float4 t = h4_to_f4(__ldg(img + y * w + x));
+HD_INL float3 ld3(const uint2 *img, int w, int x, int y) {  // of the HDR image or a bloom level
+  const float4 t = ldh_pass(img, y * w + x);
   return make_float3(t.x, t.y, t.z);
 }
 HD_INL float3 operator+(float3 a, float3 b) { return make_float3(a.x + b.x, a.y + b.y, a.z + b.z); }
@@ -38,7 +38,7 @@ HD_INL float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z
 HD_INL float3 mix3(float3 a, float3 b, float t) { return a * (1.0f - t) + b * t; }  // WGSL mix
 
 // textureSampleLevel(tex, clamp-to-edge linear sampler, uv, 0)
-HD_INL float3 sample(const uint2 *__restrict__ img, int w, int h, float u, float v) {
+HD_INL float3 sample(const uint2 *img, int w, int h, float u, float v) {
   const float x = u * (float)w - 0.5f, y = v * (float)h - 0.5f;
   const float x0 = floorf(x), y0 = floorf(y);
   const float fx = x - x0, fy = y - y0;
@@ -55,7 +55,7 @@ HD_INL float3 sample(const uint2 *__restrict__ img, int w, int h, float u, float
 template <int COLS, int ROWS>
 struct Taps {
   float3 t[ROWS][COLS];
-  HD_INL void load(const uint2 *__restrict__ img, int w, int h, int x0, int y0) {
+  HD_INL void load(const uint2 *img, int w, int h, int x0, int y0) {
     int xs[COLS];
 #pragma unroll
     for (int i = 0; i < COLS; i++) xs[i] = clampi(x0 + i, 0, w - 1);
@@ -67,7 +67,7 @@ struct Taps {
     }
   }
   // the same from x0 = 2 p - 2 of an even width, two texels per load
-  HD_INL void load_pairs(const uint2 *__restrict__ img, int w, int h, int p, int y0) {
+  HD_INL void load_pairs(const uint2 *img, int w, int h, int p, int y0) {
     const int n = w >> 1;
 #pragma unroll
     for (int j = 0; j < ROWS; j++) {
@@ -75,7 +75,7 @@ struct Taps {
 #pragma unroll
       for (int i = 0; i < COLS; i += 2) {
         const int q = p - 1 + i / 2;
-        uint4 v = __ldg(row + clampi(q, 0, n - 1));
+        uint4 v = ld_pass(row + clampi(q, 0, n - 1));
         if (q < 0) { v.z = v.x; v.w = v.y; }
         if (q >= n) { v.x = v.z; v.y = v.w; }
         const float4 a = h4_to_f4(make_uint2(v.x, v.y)), b = h4_to_f4(make_uint2(v.z, v.w));
@@ -108,7 +108,8 @@ __global__ void k_post_composite(const uint2 *__restrict__ left, const uint2 *__
   int px = x;
   if (same) px = px - (min(px * 3 / W, 2) - 1) * (W / 3);
   const uint2 *src = u < split ? left : (u < split2 ? mid : right);
-  float3 c = ld3(src, W, px, y);
+  const float4 t = ldh(src, y * W + px);
+  float3 c = make_float3(t.x, t.y, t.z);
   c = make_float3(fmaxf(c.x, 0.0f) * exposure, fmaxf(c.y, 0.0f) * exposure, fmaxf(c.z, 0.0f) * exposure);
   hdr[y * W + x] = pack_rgb1(c, 1.0f);
 }
@@ -133,7 +134,7 @@ HD_INL uint2 down_sum(const S &s) {
   return pack_rgb1(o, 1.0f);
 }
 template <bool KARIS>
-HD_INL void down_texel(const uint2 *__restrict__ src, int sw, int sh, uint2 *dst, int dw, int dh, int x, int y) {
+HD_INL void down_texel(const uint2 *src, int sw, int sh, uint2 *dst, int dw, int dh, int x, int y) {
   const float u = ((float)x + 0.5f) / (float)dw, v = ((float)y + 0.5f) / (float)dh;
   const float tx = 1.0f / (float)sw, ty = 1.0f / (float)sh;
   dst[y * dw + x] = down_sum<KARIS>([&](int ox, int oy) {
@@ -151,7 +152,7 @@ HD_INL uint2 up_sum(const S &t, float4 d) {
   o = o / 16.0f;
   return f4_to_h4(make_float4(d.x + o.x, d.y + o.y, d.z + o.z, d.w + 1.0f));
 }
-HD_INL void up_texel(const uint2 *__restrict__ src, int sw, int sh, uint2 *dst, int dw, int dh, int x, int y) {
+HD_INL void up_texel(const uint2 *src, int sw, int sh, uint2 *dst, int dw, int dh, int x, int y) {
   const float u = ((float)x + 0.5f) / (float)dw, v = ((float)y + 0.5f) / (float)dh;
   const float tx = 1.0f / (float)sw, ty = 1.0f / (float)sh;
   const float4 d = h4_to_f4(dst[y * dw + x]);
@@ -165,8 +166,7 @@ HD_INL void up_texel(const uint2 *__restrict__ src, int sw, int sh, uint2 *dst, 
 // one clamp per axis, instead of 52 with four each. Bound by instructions issued. First level of 1920x1080 18.9 -> 15.0 us, the
 // next two 11.3 -> 7.9.
 template <bool KARIS, bool HALF>
-__global__ void __launch_bounds__(BX *BY) k_post_down(const uint2 *__restrict__ src, int sw, int sh,
-                                                      uint2 *__restrict__ dst, int dw, int dh) {
+__global__ void __launch_bounds__(BX *BY) k_post_down(const uint2 *src, int sw, int sh, uint2 *dst, int dw, int dh) {
   pass_begin();
   const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y;
   if (x >= dw || y >= dh) return;
@@ -190,8 +190,7 @@ __global__ void __launch_bounds__(BX *BY) k_post_down(const uint2 *__restrict__ 
 // HALF: src is exactly half of dst: the nine samples share 4 x 4 texels (from (x - 1) / 2 - 1 on), a quarter texel from where
 // rounding could move them: 16 loads instead of 36. 960x540 and 480x270 17.6 -> 12.8 us.
 template <bool HALF>
-__global__ void __launch_bounds__(BX *BY) k_post_up(const uint2 *__restrict__ src, int sw, int sh, uint2 *__restrict__ dst,
-                                                    int dw, int dh) {
+__global__ void __launch_bounds__(BX *BY) k_post_up(const uint2 *src, int sw, int sh, uint2 *dst, int dw, int dh) {
   pass_begin();
   const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y;
   if (x >= dw || y >= dh) return;
@@ -281,8 +280,8 @@ HD_INL void final_pixel(float u, float v, float3 c, float3 b, void *target, int 
 }
 
 // The fragment positions below are by IEEE division: the divider line compares them against a pixel threshold.
-__global__ void k_post_final(const uint2 *__restrict__ hdr, int W, int H, const uint2 *__restrict__ bl, int bw, int bh,
-                             void *__restrict__ target, int OW, int OH, size_t pitch, FinalArgs a) {
+__global__ void k_post_final(const uint2 *hdr, int W, int H, const uint2 *bl, int bw, int bh, void *target, int OW,
+                             int OH, size_t pitch, FinalArgs a) {
   pass_begin(true);
   const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y;
   if (x >= OW || y >= OH) return;
@@ -304,9 +303,8 @@ __global__ void k_post_final(const uint2 *__restrict__ hdr, int W, int H, const 
 // out exactly. The four pixels' kernels cover 5 x 5 texels, and a row's sum is that of both pixels above one another: 25
 // loads and 120 + 48 multiply-adds for four pixels instead of 64 and 192 + 48. Bound by instructions issued: 1920x1080
 // 36.7 -> 24.4 us.
-__global__ void __launch_bounds__(BX *BY) k_post_final_half(const uint2 *__restrict__ hdr, int W, int H,
-                                                            const uint2 *__restrict__ bl, int bw, int bh,
-                                                            void *__restrict__ target, size_t pitch, FinalArgs a) {
+__global__ void __launch_bounds__(BX *BY) k_post_final_half(const uint2 *hdr, int W, int H, const uint2 *bl, int bw,
+                                                            int bh, void *target, size_t pitch, FinalArgs a) {
   pass_begin(true);
   const int mx = blockIdx.x * BX + threadIdx.x, my = blockIdx.y * BY + threadIdx.y;
   if (mx >= bw || my >= bh) return;

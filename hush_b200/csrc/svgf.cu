@@ -168,8 +168,8 @@ __global__ void __launch_bounds__(VT_NT) k_svgf_variance(const SvgfFrame f, uint
   float4 nd = make_float4(0.f, 0.f, 0.f, -1.0f), c = make_float4(0.f, 0.f, 0.f, 0.f), m = c;
   if (in_img) {
     nd = ldh(f.nd, y * f.p_nd + x);
-    c = ldh(f.tmp, o);
-    m = ldh(f.mom, o);
+    c = ldh_pass(f.tmp, o);
+    m = ldh_pass(f.mom, o);
   }
   const bool sky = nd.w < 0.0f, spatial = !sky && !(m.z >= 4.0f);
   if (!__syncthreads_or(spatial ? 1 : 0)) {
@@ -330,11 +330,11 @@ __global__ void __launch_bounds__(AT_NT, 5) k_svgf_atrous(const SvgfFrame f, con
 #pragma unroll
       for (int l = 0; l < 2; l++) {
         const int xc = min(x0 + l * AT_P, f.W - 1), xm = max(xc - 1, 0), xp = min(xc + 1, f.W - 1);
-        auto var = [](const uint2 *p) { return hi_half(__ldg(&p->y)); };
+        auto var = [](const uint2 *p) { return hi_half(ld_pass(&p->y)); };
         vs[k][l] = 0.0625f * (var(im + xm) + var(im + xp) + var(ip + xm) + var(ip + xp)) +
                    0.125f * (var(im + xc) + var(ip + xc));
-        zu[k][l] = var(nm + xc);
-        zd[k][l] = var(np + xc);
+        zu[k][l] = hi_half(__ldg(&nm[xc].y));
+        zd[k][l] = hi_half(__ldg(&np[xc].y));
       }
     }
   }
@@ -348,8 +348,8 @@ __global__ void __launch_bounds__(AT_NT, 5) k_svgf_atrous(const SvgfFrame f, con
       if (u + 32 > TC && u + li % 32 >= TC) break;
       const bool o0 = iy && gx0 + u >= 0 && gx0 + u < f.W, o1 = iy && gx0 + u + AT_P >= 0 && gx0 + u + AT_P < f.W;
       uint2 n[2] = {make_uint2(0u, 0xbc000000u), make_uint2(0u, 0xbc000000u)}, c[2] = {};  // depth -1: sky
-      if (o0) { n[0] = __ldg(pn + u); c[0] = __ldg(pc + u); }
-      if (o1) { n[1] = __ldg(pn + u + AT_P); c[1] = __ldg(pc + u + AT_P); }
+      if (o0) { n[0] = __ldg(pn + u); c[0] = ld_pass(pc + u); }
+      if (o1) { n[1] = __ldg(pn + u + AT_P); c[1] = ld_pass(pc + u + AT_P); }
       S.put(r * TC + u + li % 32, n[0], n[1], c[0], c[1]);
     }
   }
@@ -477,7 +477,7 @@ cudaError_t launch_atrous(const SvgfFrame &f, const uint2 *in, uint2 *out, int i
 // (clamp-to-edge); here the same texel footprint is weighted exactly in f32.
 HD_INL float3 svgf_remod(const SvgfFrame &f, const uint2 *il, int qx, int qy) {
   const int cx = clampi(qx, 0, f.W - 1), cy = clampi(qy, 0, f.H - 1);
-  const float4 a = ldh(il, cy * f.W + cx), m = ldh(f.mat, cy * f.p_mat + cx), e = ldh(f.emi, cy * f.p_emi + cx);
+  const float4 a = ldh_pass(il, cy * f.W + cx), m = ldh(f.mat, cy * f.p_mat + cx), e = ldh(f.emi, cy * f.p_emi + cx);
   return make_float3(a.x * m.x + e.x, a.y * m.y + e.y, a.z * m.z + e.z);
 }
 
