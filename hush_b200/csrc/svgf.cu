@@ -4,11 +4,13 @@
 
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "common.cuh"
 #include "hush.h"
 #include "hush_device.cuh"
 #include "hush_pair.cuh"
+#include "quotient.cuh"
 
 using namespace hush;
 
@@ -26,33 +28,6 @@ struct SvgfFrame {
 
 HD_INL float hi_half(uint32_t u) { return __half2float(__ushort_as_half((uint16_t)(u >> 16))); }
 
-// 1 / x to within an ulp: the hardware approximation and one Newton step, without the range checks of an IEEE division
-// (x is a sum of weights or a positive bandwidth + epsilon here).
-HD_INL float rcp1(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return fmaf(fmaf(-x, r, 1.0f), r, r);
-}
-
-// Quotients of one divisor: the product with rcp1 and one residual correction, which rounds as the IEEE division does but
-// for rare ties, without its range checks and branches (the divisors here are sums of weights, 1 + luminance and sizes).
-struct Divisor {
-  float d, r;
-  HD_INL explicit Divisor(float d_) : d(d_), r(rcp1(d_)) {}
-  HD_INL float operator()(float a) const {
-    const float q = a * r;
-    return fmaf(fmaf(-d, q, a), r, q);
-  }
-  HD_INL float3 operator()(float3 a) const { return make_float3((*this)(a.x), (*this)(a.y), (*this)(a.z)); }
-};
-// sqrt(x), x >= 0, rounded the same way from the hardware reciprocal square root.
-HD_INL float sqrt1(float x) {
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  const float s = x * r;
-  return x > 1e-37f ? fmaf(fmaf(-s, s, x), 0.5f * r, s) : 0.0f;
-}
-
 // The history test of a previous frame's texel (guide q, object id) against this pixel's (svgf.js:31-39).
 HD_INL bool svgf_same(float4 q, float qobj, float4 n, float zPrev, float obj) {
   return !(q.w < 0.0f) && qobj == obj && !(fabsf(q.w - zPrev) > 0.05f * zPrev + 0.01f) && !(dot3(q, n) < 0.9f);
@@ -63,7 +38,8 @@ HD_INL bool svgf_consistent(const SvgfFrame &f, int qx, int qy, float4 n, float 
 }
 
 // TEMPORAL (svgf.js:41-105). Bound: the latency of its dependent loads (motion, then the footprint): the four texels'
-// guide, object, colour and moments are loaded together, not test by test (58 -> 47 us at 1920 x 1080).
+// guide, object, colour and moments are loaded together, not test by test (58 -> 53 us at 1920 x 1080). Its quotients round as
+// the IEEE ones do: an ulp in the history length flips the variance pass's branch.
 __global__ void __launch_bounds__(256) k_svgf_temporal(const SvgfFrame f) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= f.W || y >= f.H) return;
@@ -95,9 +71,6 @@ __global__ void __launch_bounds__(256) k_svgf_temporal(const SvgfFrame f) {
   }
   const float4 alb = ldh(f.mat, y * f.p_mat + x);
   const float4 r = ldh(f.rad, y * f.p_rad + x);
-  const float ix = Divisor(fmaxf(alb.x, 1e-3f))(r.x), iy = Divisor(fmaxf(alb.y, 1e-3f))(r.y),
-              iz = Divisor(fmaxf(alb.z, 1e-3f))(r.z);
-  const float l = __fadd_rn(__fadd_rn(__fmul_rn(ix, 0.2126f), __fmul_rn(iy, 0.7152f)), __fmul_rn(iz, 0.0722f));
   // the history length it blends into decides the spatial / temporal variance branch (m.z >= 4), so the weighted
   // sums are rounded product by product like an unfused shader (no FMA contraction)
   float sumW = 0.f, hcx = 0.f, hcy = 0.f, hcz = 0.f, hm0 = 0.f, hm1 = 0.f, hm2 = 0.f;
@@ -132,6 +105,13 @@ __global__ void __launch_bounds__(256) k_svgf_temporal(const SvgfFrame f) {
       }
     }
   }
+  // (last: the test below would hold the footprint's loads back)
+  const float ax = fmaxf(alb.x, 1e-3f), ay = fmaxf(alb.y, 1e-3f), az = fmaxf(alb.z, 1e-3f);
+  float ix = quot_rn(r.x, ax, rcp_rn(ax)), iy = quot_rn(r.y, ay, rcp_rn(ay)), iz = quot_rn(r.z, az, rcp_rn(az));
+  if (!all_finite(ix + iy + iz)) {
+    ix = quot_any(r.x, ax); iy = quot_any(r.y, ay); iz = quot_any(r.z, az);
+  }
+  const float l = __fadd_rn(__fadd_rn(__fmul_rn(ix, 0.2126f), __fmul_rn(iy, 0.7152f)), __fmul_rn(iz, 0.0722f));
   float len, cx = ix, cy = iy, cz = iz, m0 = l, m1 = __fmul_rn(l, l);
   if (sumW >= 0.01f) {
     hcx /= sumW; hcy /= sumW; hcz /= sumW;
@@ -152,11 +132,16 @@ __global__ void __launch_bounds__(256) k_svgf_temporal(const SvgfFrame f) {
 
 // VARIANCE (svgf.js:114-148): temporal where the history is long enough, else from a 7 x 7 neighbourhood. Only a CTA
 // with such a pixel (a disocclusion, or the first frames) stages the neighbourhood's texels; outside the image they are
-// marked as sky. The weight's depth factor is one reciprocal per tap distance, exp and the default sigma_n = 128 run as
-// the a-trous kernel's do (seven squarings in place of a 49-fold powf): 39 -> 22 us at 1920 x 1080, 641 x 363 22.7 ->
-// 9.5 us (a sequence of eight frames, two of them without a long enough history).
+// marked as sky. Taps, weights and sums are the reference's in its order (exp and pow with their full accuracy, quotients rounded
+// as IEEE ones); the tap distances and a row's divisors are formed once. Bound: the 49 pow of such a pixel. 1920 x 1080
+// 39 -> 32 us, 641 x 363 22.7 -> 15.7 us with the set-up beside the pass before (a sequence of eight frames, two of them
+// without a long enough history).
 constexpr int VT_W = 32, VT_H = 8, VT_NT = VT_W * VT_H;
-template <bool N128>
+// sqrt(i^2 + j^2), correctly rounded
+__constant__ const float VT_DIST[4][4] = {{0.0f, 1.0f, 2.0f, 3.0f},
+                                          {1.0f, 1.41421356237f, 2.2360679775f, 3.16227766017f},
+                                          {2.0f, 2.2360679775f, 2.82842712475f, 3.60555127546f},
+                                          {3.0f, 3.16227766017f, 3.60555127546f, 4.24264068712f}};
 __global__ void __launch_bounds__(VT_NT) k_svgf_variance(const SvgfFrame f, uint2 *out) {
   pass_begin();
   constexpr int TC = VT_W + 6, TR = VT_H + 6, N = TC * TR;
@@ -195,30 +180,27 @@ __global__ void __launch_bounds__(VT_NT) k_svgf_variance(const SvgfFrame f, uint
     sth(out, o, sky ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(c.x, c.y, c.z, fmaxf(0.0f, m.y - m.x * m.x)));
     return;
   }
-  // log2(e) / (0.02 z dist + 1e-3) by |dx|, |dy| <= 3
-  float iz[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j <= i; j++) iz[i][j] = iz[j][i] = LOG2E * rcp1(0.02f * nd.w * sqrtf((float)(i * i + j * j)) + 1e-3f);
   float sw = 0.f, scx = 0.f, scy = 0.f, scz = 0.f, sm0 = 0.f, sm1 = 0.f;
   const int t = (ty + 3) * TC + tx + 3;
-#pragma unroll
+#pragma unroll 1
   for (int dy = -3; dy <= 3; dy++) {
+    float den[4], rcp[4];  // of a row's depth weights, by |dx|
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      den[i] = 0.02f * nd.w * VT_DIST[dy < 0 ? -dy : dy][i] + 1e-3f;
+      rcp[i] = rcp_rn(den[i]);
+    }
 #pragma unroll
     for (int dx = -3; dx <= 3; dx++) {
-      const int q = t + dy * TC + dx;
+      const int q = t + dy * TC + dx, i = dx < 0 ? -dx : dx;
       const float4 ndq = h4_to_f4(sN[q]);
       if (ndq.w < 0.0f) continue;
-      const float dn = fmaxf(0.0f, dot3(ndq, nd));
-      float wn = dn;
-      if constexpr (N128) {
-#pragma unroll
-        for (int i = 0; i < 7; i++) wn *= wn;
-      } else {
-        wn = powf(dn, f.sigma_n);
-      }
-      const float w = wn * ex2_approx(-fabsf(ndq.w - nd.w) * iz[dy < 0 ? -dy : dy][dx < 0 ? -dx : dx]);
+      const float dz = -fabsf(ndq.w - nd.w);
+      float x = quot_rn(dz, den[i], rcp[i]);
+      if (!all_finite(x)) x = quot_any(dz, den[i]);
+      const float wz = expf(x);
+      const float wn = powf(fmaxf(0.0f, dot3(ndq, nd)), f.sigma_n);
+      const float w = wz * wn;
       const float4 cq = h4_to_f4(sC[q]);
       const float2 mq = unpack2(sM[q].x);
       sw += w;
@@ -239,14 +221,19 @@ __global__ void __launch_bounds__(VT_NT) k_svgf_variance(const SvgfFrame f, uint
 // four pixels: columns x and x + 32 in the two lanes of packed FP32x2 arithmetic, times two neighbouring lattice rows,
 // which share 20 of their 25 taps. The footprint is held in shared memory as the pairs of texels 32 columns apart, each
 // converted to FP32 once, so that every tap of every STEP, 1 included, is a pair without a shuffle; texels outside
-// the image are marked as sky (depth -1, colour 0), so no tap tests its position. The tap columns run as a loop (the
-// depth factors of a column's taps come from shared memory): unrolled, instruction fetch stalled the warps.
-// Bound: the FP32 pipe (the ~23 FP32 operations of a tap and pixel; packing saves issue slots, not pipe time: 61% busy
-// at 1920 x 1080) with shared-memory bandwidth next (68%). A float4 tile with a thread per pixel read 36 bytes a tap for
-// one pixel, and steps 8 and 16 loaded every tap from global memory: iterations 0-4 at 1920 x 1080 were 93 / 96 / 99 /
-// 125 / 125 us and are 65 / 66 / 68 / 71 / 76 us.
+// the image are marked as sky (depth -1, colour 0), so no tap tests its position. The tap rows run as a loop over the rows that
+// both pixels share, between one row of the upper and one of the lower alone (a row's depth factors come from shared memory):
+// all unrolled, instruction fetch stalled the warps; with a test per pixel and row in one loop the pass took 8 % longer. A
+// pixel's taps are summed in the order of their rows and every quotient is rounded as the IEEE one, so the frame is the one of a
+// thread per pixel bit for bit (column by column, with quotients by a product, iterations 0-4 took 71 / 69 / 76 / 78 / 82 us).
+// Bound: the FP32 pipe (the ~25 FP32 operations of a tap and pixel; packing saves issue slots, not pipe time). A float4 tile
+// with a thread per pixel read 36 bytes a tap for one pixel, and steps 8 and 16 loaded every tap from global memory: iterations
+// 0-4 at 1920 x 1080 were 93 / 96 / 99 / 125 / 125 us and are 81 / 72 / 81 / 85 / 86 us with the set-up beside the pass before.
 constexpr int AT_P = 32, AT_W = 2 * AT_P, AT_H = 8, AT_NT = AT_P * AT_H / 2;
 
+HD_INL float2 neg_abs2(float2 a) {
+  return f2(__uint_as_float(__float_as_uint(a.x) | 0x80000000u), __uint_as_float(__float_as_uint(a.y) | 0x80000000u));
+}
 // The normal weight pow(max(n . n_q, 0), sigma_n): by seven squarings for the default sigma_n = 128 (no special-function
 // unit), else as the hardware exp2(sigma_n log2 x); pow(x, 0) = 1.
 template <bool N128>
@@ -268,6 +255,9 @@ HD_INL TexelPair widen(uint2 na, uint2 nb, uint2 ca, uint2 cb) {
   return TexelPair{make_float4(n0.x, n1.x, n0.y, n1.y), make_float4(n0.z, n1.z, n0.w, n1.w),
                    make_float4(c0.x, c1.x, c0.y, c1.y), make_float4(c0.z, c1.z, c0.w, c1.w)};
 }
+HD_INL float2 lum2(const TexelPair &p) {
+  return fma2(lo2(p.c1), bc2(0.0722f), fma2(lo2(p.c0), bc2(0.2126f), mul2(hi2(p.c0), bc2(0.7152f))));
+}
 // RAW: the pairs as stored (converted by each tap), 32 bytes instead of 64. Only STEP = 16 takes it, whose 96 x 12
 // pairs would leave two CTAs an SM.
 template <int STEP>
@@ -275,7 +265,7 @@ struct AtrousSmem {
   static constexpr bool RAW = STEP >= 16;
   static constexpr int A = 2 * STEP, TC = AT_P + 2 * A, TR = AT_H + 4, N = TR * TC;
   uint4 t[RAW ? 2 : 4][N];
-  float2 izd[2][5][AT_NT];  // log2(e) / (sigma_z zg dist + 1e-3) per tap distance 1, sqrt 2, 2, sqrt 5, sqrt 8
+  float2 izd[2][5][AT_NT];  // 1 / (sigma_z zg dist + 1e-3) per tap distance 1, sqrt 2, 2, sqrt 5, sqrt 8
   HD_INL void put(int i, uint2 na, uint2 nb, uint2 ca, uint2 cb) {
     if constexpr (RAW) {
       t[0][i] = make_uint4(na.x, na.y, nb.x, nb.y);
@@ -320,7 +310,7 @@ __global__ void __launch_bounds__(AT_NT, 5) k_svgf_atrous(const SvgfFrame f, con
   const int x0 = bx + tx, y0 = (j0 + jr) * STEP + phase;
   // The centre's 3 x 3 variance blur and depth gradient read the rows y +- 1, which only STEP = 1 stages; the other
   // steps load them here (texels clamped to the image).
-  float vs[2][2], zu[2][2], zd[2][2];
+  float vu[2][2], vd[2][2][3], zu[2][2], zd[2][2];
   if constexpr (STEP > 1) {
 #pragma unroll
     for (int k = 0; k < 2; k++) {
@@ -331,8 +321,8 @@ __global__ void __launch_bounds__(AT_NT, 5) k_svgf_atrous(const SvgfFrame f, con
       for (int l = 0; l < 2; l++) {
         const int xc = min(x0 + l * AT_P, f.W - 1), xm = max(xc - 1, 0), xp = min(xc + 1, f.W - 1);
         auto var = [](const uint2 *p) { return hi_half(ld_pass(&p->y)); };
-        vs[k][l] = 0.0625f * (var(im + xm) + var(im + xp) + var(ip + xm) + var(ip + xp)) +
-                   0.125f * (var(im + xc) + var(ip + xc));
+        vu[k][l] = 0.0625f * var(im + xm) + 0.125f * var(im + xc) + 0.0625f * var(im + xp);
+        vd[k][l][0] = var(ip + xm); vd[k][l][1] = var(ip + xc); vd[k][l][2] = var(ip + xp);
         zu[k][l] = hi_half(__ldg(&nm[xc].y));
         zd[k][l] = hi_half(__ldg(&np[xc].y));
       }
@@ -366,69 +356,83 @@ __global__ void __launch_bounds__(AT_NT, 5) k_svgf_atrous(const SvgfFrame f, con
     const TexelPair p = Smem::get(&S.t[0][t]);
     Centre &c = C[k];
     c.nx = lo2(p.g0); c.ny = hi2(p.g0); c.nz = lo2(p.g1); c.z = hi2(p.g1);
-    c.lp = fma2(lo2(p.c1), bc2(0.0722f), fma2(hi2(p.c0), bc2(0.7152f), mul2(lo2(p.c0), bc2(0.2126f))));
-    float il[2], izd[5][2];
+    c.lp = lum2(p);
+    float den[6][2];  // of the luminance weight, then of the depth weight by tap distance
     const int y = min(y0 + k * STEP, f.H - 1);
 #pragma unroll
     for (int l = 0; l < 2; l++) {
       const int x = min(x0 + l * AT_P, f.W - 1);
       const int tl = x > 0 ? t - 1 : t, tr = x + 1 < f.W ? t + 1 : t;
       const float z = S.depth(t, l), zl = S.depth(tl, l), zr = S.depth(tr, l);
-      float up, dn, gv;
+      // the blur's sums in the order of its rows
+      float up, dn, gv, v0, v1, v2;
       if constexpr (STEP > 1) {
-        gv = vs[k][l];
+        gv = vu[k][l];
+        v0 = vd[k][l][0]; v1 = vd[k][l][1]; v2 = vd[k][l][2];
         up = zu[k][l];
         dn = zd[k][l];
       } else {
         const int du = y > 0 ? -TC : 0, dd = y + 1 < f.H ? TC : 0;
-        gv = 0.0625f * (S.variance(tl + du, l) + S.variance(tr + du, l) + S.variance(tl + dd, l) + S.variance(tr + dd, l)) +
-             0.125f * (S.variance(t + du, l) + S.variance(t + dd, l));
+        gv = 0.0625f * S.variance(tl + du, l) + 0.125f * S.variance(t + du, l) + 0.0625f * S.variance(tr + du, l);
+        v0 = S.variance(tl + dd, l); v1 = S.variance(t + dd, l); v2 = S.variance(tr + dd, l);
         up = S.depth(t + du, l);
         dn = S.depth(t + dd, l);
       }
-      gv += 0.125f * (S.variance(tl, l) + S.variance(tr, l)) + 0.25f * S.variance(t, l);
+      gv = gv + 0.125f * S.variance(tl, l) + 0.25f * S.variance(t, l) + 0.125f * S.variance(tr, l);
+      gv = gv + 0.0625f * v0 + 0.125f * v1 + 0.0625f * v2;
       const float gx = fminf(zr > 0.0f ? fabsf(zr - z) : 1e9f, zl > 0.0f ? fabsf(zl - z) : 1e9f);
       const float gy = fminf(dn > 0.0f ? fabsf(dn - z) : 1e9f, up > 0.0f ? fabsf(up - z) : 1e9f);
       const float zg = f.sigma_z * fminf(fmaxf(gx, gy), z);
-      il[l] = LOG2E * rcp1(f.sigma_l * sqrtf(fmaxf(gv, 0.0f)) + 1e-6f);
+      den[5][l] = f.sigma_l * sqrt_rn(fmaxf(gv, 0.0f)) + 1e-6f;
       const float dcls[5] = {1.0f, 1.41421356237f, 2.0f, 2.2360679775f, 2.82842712475f};
 #pragma unroll
-      for (int d = 0; d < 5; d++) izd[d][l] = LOG2E * rcp1(zg * (dcls[d] * (float)STEP) + 1e-3f);
+      for (int d = 0; d < 5; d++) den[d][l] = zg * (dcls[d] * (float)STEP) + 1e-3f;
     }
-    c.il = f2(il[0], il[1]);
+    float2 rcp[6], sum = f2(0.0f, 0.0f);
 #pragma unroll
-    for (int d = 0; d < 5; d++) S.izd[k][d][li] = f2(izd[d][0], izd[d][1]);  // read back by this thread alone
+    for (int d = 0; d < 6; d++) {
+      rcp[d] = f2(rcp_rn(den[d][0]), rcp_rn(den[d][1]));
+      sum = add2(sum, rcp[d]);
+    }
+    if (!all_finite(sum.x + sum.y)) {
+#pragma unroll
+      for (int d = 0; d < 6; d++) rcp[d] = f2(quot_any(1.0f, den[d][0]), quot_any(1.0f, den[d][1]));
+    }
+    c.il = rcp[5];
+#pragma unroll
+    for (int d = 0; d < 5; d++) S.izd[k][d][li] = rcp[d];  // read back by this thread alone
     c.sw = f2(h0 * h0, h0 * h0);
     c.sr = mul2(lo2(p.c0), c.sw); c.sg = mul2(hi2(p.c0), c.sw); c.sb = mul2(lo2(p.c1), c.sw);
     c.sv = mul2(mul2(hi2(p.c1), c.sw), c.sw);
   }
-  // One tap column at a time: its six texel pairs serve both rows' filters. The weight is
-  // h (n.n)^sigma_n 2^-(|dz| izd + |dl| il), the exponent in units of log2.
-  const uint4 *col = &S.t[0][base - 2 * STEP];
-#pragma unroll 1
-  for (int dx = -2; dx <= 2; dx++, col += STEP) {
-    const int a = dx < 0 ? -dx : dx;
-    const float hx = a == 0 ? h0 : (a == 1 ? h1 : h2);
-    const int cls[3] = {a == 2 ? 2 : 0, a == 0 ? 0 : (a == 1 ? 1 : 3), a == 0 ? 2 : (a == 1 ? 3 : 4)};  // by |dy|
-    const float2 hh[3] = {bc2(hx * h0), bc2(hx * h1), bc2(hx * h2)};
-    float2 iz[2][3];
+  // One row of taps at a time: its five texel pairs serve both rows' filters.
+  const uint4 *row = &S.t[0][base - 2 * TC];
+  auto taps = [&](int r, auto first, auto last) {  // for the pixels first .. last
+    float2 hh[2][3], iz[2][3];  // by row and |dx|
 #pragma unroll
-    for (int b = 0; b < 3; b++) { iz[0][b] = S.izd[0][cls[b]][li]; iz[1][b] = S.izd[1][cls[b]][li]; }
+    for (int k = first; k <= last; k++) {
+      const int b = r < k ? k - r : r - k;
+      const float hy = b == 0 ? h0 : (b == 1 ? h1 : h2);
+      const int cls[3] = {b == 2 ? 2 : 0, b == 0 ? 0 : (b == 1 ? 1 : 3), b == 0 ? 2 : (b == 1 ? 3 : 4)};
+      hh[k][0] = bc2(h0 * hy); hh[k][1] = bc2(h1 * hy); hh[k][2] = bc2(h2 * hy);
 #pragma unroll
-    for (int r = -2; r <= 3; r++) {
-      const TexelPair q = Smem::get(col + r * TC);
-      const float2 z = hi2(q.g1);
-      const float2 lq = fma2(lo2(q.c1), bc2(0.0722f), fma2(hi2(q.c0), bc2(0.7152f), mul2(lo2(q.c0), bc2(0.2126f))));
+      for (int a = 0; a < 3; a++) iz[k][a] = S.izd[k][cls[a]][li];
+    }
+#pragma unroll
+    for (int dx = -2; dx <= 2; dx++) {
+      const TexelPair q = Smem::get(row + dx * STEP);
+      const float2 z = hi2(q.g1), lq = lum2(q);
       const bool ok0 = !(z.x < 0.0f), ok1 = !(z.y < 0.0f);
 #pragma unroll
-      for (int k = 0; k < 2; k++) {
-        const int dy = r - k, b = dy < 0 ? -dy : dy;
-        if (b > 2 || (b == 0 && dx == 0)) continue;
+      for (int k = first; k <= last; k++) {
+        const int a = dx < 0 ? -dx : dx;
+        if (dx == 0 && r == k) continue;
         Centre &c = C[k];
         const float2 dot = fma2(lo2(q.g1), c.nz, fma2(hi2(q.g0), c.ny, mul2(lo2(q.g0), c.nx)));
         const float2 wn = svgf_wn2<N128>(f2(fmaxf(0.0f, dot.x), fmaxf(0.0f, dot.y)), f.sigma_n);
-        const float2 ez = mul2(sub2(z, c.z), iz[k][b]), el = mul2(sub2(lq, c.lp), c.il);
-        float2 w = mul2(mul2(hh[b], wn), f2(ex2_approx(-fabsf(ez.x) - fabsf(el.x)), ex2_approx(-fabsf(ez.y) - fabsf(el.y))));
+        const float2 dz = sub2(z, c.z), dl = sub2(lq, c.lp);
+        const float2 e = mul2(fma2(neg_abs2(dz), iz[k][a], mul2(neg_abs2(dl), c.il)), bc2(LOG2E));
+        float2 w = mul2(mul2(hh[k][a], wn), f2(ex2_approx(e.x), ex2_approx(e.y)));
         w = f2(ok0 ? w.x : 0.0f, ok1 ? w.y : 0.0f);
         c.sw = add2(c.sw, w);
         c.sr = fma2(w, lo2(q.c0), c.sr);
@@ -437,7 +441,17 @@ __global__ void __launch_bounds__(AT_NT, 5) k_svgf_atrous(const SvgfFrame f, con
         c.sv = fma2(mul2(w, w), hi2(q.c1), c.sv);
       }
     }
+  };
+  const std::integral_constant<int, 0> k0;
+  const std::integral_constant<int, 1> k1;
+  taps(-2, k0, k0);
+#pragma unroll 1
+  for (int r = -1; r <= 2; r++) {
+    row += TC;
+    taps(r, k0, k1);
   }
+  row += TC;
+  taps(3, k1, k1);
 #pragma unroll
   for (int k = 0; k < 2; k++) {
     const int y = y0 + k * STEP;
@@ -447,9 +461,11 @@ __global__ void __launch_bounds__(AT_NT, 5) k_svgf_atrous(const SvgfFrame f, con
     for (int l = 0; l < 2; l++) {
       const int x = x0 + l * AT_P;
       if (x >= f.W) break;
-      const float i = rcp1(l ? c.sw.y : c.sw.x);
-      float4 o = make_float4((l ? c.sr.y : c.sr.x) * i, (l ? c.sg.y : c.sg.x) * i, (l ? c.sb.y : c.sb.x) * i,
-                             (l ? c.sv.y : c.sv.x) * i * i);
+      const float sw = l ? c.sw.y : c.sw.x, sw2 = sw * sw, sr = l ? c.sr.y : c.sr.x, sg = l ? c.sg.y : c.sg.x,
+                  sb = l ? c.sb.y : c.sb.x, sv = l ? c.sv.y : c.sv.x, rw = rcp_rn(sw);
+      float4 o = make_float4(quot_rn(sr, sw, rw), quot_rn(sg, sw, rw), quot_rn(sb, sw, rw), quot_rn(sv, sw2, rcp_rn(sw2)));
+      if (!all_finite(o.x + o.y + o.z + o.w))
+        o = make_float4(quot_any(sr, sw), quot_any(sg, sw), quot_any(sb, sw), quot_any(sv, sw2));
       if ((l ? c.z.y : c.z.x) < 0.0f) o = make_float4(0.f, 0.f, 0.f, 0.f);
       sth(out, y * f.W + x, o);
       if (iter == 0) sth(f.hist, y * f.W + x, make_float4(o.x, o.y, o.z, 0.f));
@@ -483,9 +499,13 @@ HD_INL float3 svgf_remod(const SvgfFrame &f, const uint2 *il, int qx, int qy) {
 
 // A 32 x 8 tile with an apron of one: each texel is remodulated, tone-mapped and converted to YCoCg once (a thread per
 // pixel did that for its nine neighbours, 27 texel loads and 27 divisions a pixel: 90 us at 1920 x 1080 where the tile
-// takes 39). The motion and the history's bilinear footprint are loaded before the tile barrier.
-HD_INL float3 svgf_tm(float3 c) { return Divisor(1.0f + lum3(c.x, c.y, c.z))(c); }
-HD_INL float3 svgf_itm(float3 c) { return Divisor(fmaxf(1.0f - lum3(c.x, c.y, c.z), 1e-4f))(c); }
+// takes 53 with its set-up beside the pass before, 65 with the IEEE operators' branches). The motion and the history's bilinear
+// footprint are loaded before the tile barrier.
+// The luminance's two roundings and the blend's are written out: the compiler's choice of FMAs depends on the code around it.
+HD_INL float lum_grb(float3 c) { return __fmaf_rn(c.z, 0.0722f, __fmaf_rn(c.x, 0.2126f, __fmul_rn(c.y, 0.7152f))); }
+HD_INL float lum_rgb(float3 c) { return __fmaf_rn(c.z, 0.0722f, __fmaf_rn(c.y, 0.7152f, __fmul_rn(c.x, 0.2126f))); }
+HD_INL float3 svgf_tm(float3 c) { return div3(c, 1.0f + lum_grb(c)); }
+HD_INL float3 svgf_itm(float3 c) { return div3(c, fmaxf(1.0f - lum_grb(c), 1e-4f)); }
 constexpr int RT_W = 32, RT_H = 8, RT_NT = RT_W * RT_H;
 __global__ void __launch_bounds__(RT_NT) k_svgf_resolve(const SvgfFrame f, const uint2 *il) {
   pass_begin(true);
@@ -502,7 +522,9 @@ __global__ void __launch_bounds__(RT_NT) k_svgf_resolve(const SvgfFrame f, const
   }
   const int cx = min(x, f.W - 1), cy = min(y, f.H - 1);
   const float4 mv = ldh(f.mv, cy * f.p_mv + cx);
-  const float uvx = Divisor((float)f.W)((float)x + 0.5f + mv.x), uvy = Divisor((float)f.H)((float)y + 0.5f + mv.y);
+  // (a motion that is not finite gives a position that is not, outside the image either way)
+  const float wf = (float)f.W, hf = (float)f.H;
+  const float uvx = quot_rn((float)x + 0.5f + mv.x, wf, rcp_rn(wf)), uvy = quot_rn((float)y + 0.5f + mv.y, hf, rcp_rn(hf));
   const bool hist_in = uvx >= 0.0f && uvy >= 0.0f && uvx <= 1.0f && uvy <= 1.0f && !f.reset;
   const float ppx = uvx * (float)f.W - 0.5f, ppy = uvy * (float)f.H - 0.5f;
   const float bxf = floorf(ppx), byf = floorf(ppy);
@@ -513,11 +535,18 @@ __global__ void __launch_bounds__(RT_NT) k_svgf_resolve(const SvgfFrame f, const
       hq[j] = __ldg(f.taa_prev + clampi((int)byf + (j >> 1), 0, f.H - 1) * f.W + clampi((int)bxf + (j & 1), 0, f.W - 1));
   }
   const int ox = blockIdx.x * RT_W - 1, oy = blockIdx.y * RT_H - 1;
+  constexpr int NU = (N + RT_NT - 1) / RT_NT;
+  float3 tl[NU];
 #pragma unroll
-  for (int u = 0; u < (N + RT_NT - 1) / RT_NT; u++) {
+  for (int u = 0; u < NU; u++) {
+    const int i = min(li + u * RT_NT, N - 1);
+    tl[u] = svgf_remod(f, il, ox + i % SW, oy + i / SW);
+  }
+#pragma unroll
+  for (int u = 0; u < NU; u++) {
     const int i = li + u * RT_NT;
     if (i >= N) break;
-    const float3 c = svgf_tm(svgf_remod(f, il, ox + i % SW, oy + i / SW)), q = to_ycocg(c);
+    const float3 c = svgf_tm(tl[u]), q = to_ycocg(c);
     sRgb[0][i] = c.x; sRgb[1][i] = c.y; sRgb[2][i] = c.z;
     sY[0][i] = q.x; sY[1][i] = q.y; sY[2][i] = q.z;
   }
@@ -537,12 +566,11 @@ __global__ void __launch_bounds__(RT_NT) k_svgf_resolve(const SvgfFrame f, const
     m2.y = __fadd_rn(m2.y, __fmul_rn(c.y, c.y));
     m2.z = __fadd_rn(m2.z, __fmul_rn(c.z, c.z));
   }
-  const Divisor nine(9.0f);
-  m1 = nine(m1);
-  m2 = nine(m2);
-  const float sdx = sqrt1(fmaxf(__fsub_rn(m2.x, __fmul_rn(m1.x, m1.x)), 0.0f)),
-              sdy = sqrt1(fmaxf(__fsub_rn(m2.y, __fmul_rn(m1.y, m1.y)), 0.0f)),
-              sdz = sqrt1(fmaxf(__fsub_rn(m2.z, __fmul_rn(m1.z, m1.z)), 0.0f));
+  m1 = div3(m1, 9.0f);
+  m2 = div3(m2, 9.0f);
+  const float sdx = sqrt_rn(fmaxf(__fsub_rn(m2.x, __fmul_rn(m1.x, m1.x)), 0.0f)),
+              sdy = sqrt_rn(fmaxf(__fsub_rn(m2.y, __fmul_rn(m1.y, m1.y)), 0.0f)),
+              sdz = sqrt_rn(fmaxf(__fsub_rn(m2.z, __fmul_rn(m1.z, m1.z)), 0.0f));
   const float a = f.taa_alpha;
   float3 res = cur;
   if (hist_in) {
@@ -554,12 +582,14 @@ __global__ void __launch_bounds__(RT_NT) k_svgf_resolve(const SvgfFrame f, const
       const float4 h = h4_to_f4(hq[j]);
       hist.x += wb * h.x; hist.y += wb * h.y; hist.z += wb * h.z;
     }
-    float3 hh = to_ycocg(svgf_tm(hist));
+    float3 hh = to_ycocg(div3(hist, 1.0f + lum_rgb(hist)));
     hh.x = fminf(fmaxf(hh.x, m1.x - 1.25f * sdx), m1.x + 1.25f * sdx);
     hh.y = fminf(fmaxf(hh.y, m1.y - 1.25f * sdy), m1.y + 1.25f * sdy);
     hh.z = fminf(fmaxf(hh.z, m1.z - 1.25f * sdz), m1.z + 1.25f * sdz);
     const float3 h = from_ycocg(hh);
-    res = make_float3(h.x * (1.0f - a) + cur.x * a, h.y * (1.0f - a) + cur.y * a, h.z * (1.0f - a) + cur.z * a);
+    const float b = 1.0f - a;
+    res = make_float3(__fmaf_rn(cur.x, a, __fmul_rn(h.x, b)), __fmaf_rn(cur.y, a, __fmul_rn(h.y, b)),
+                      __fmaf_rn(cur.z, a, __fmul_rn(h.z, b)));
   }
   const float3 r = svgf_itm(res);
   sth(f.taa, y * f.W + x, make_float4(r.x, r.y, r.z, 1.0f));
@@ -685,7 +715,7 @@ extern "C" int svgf_encode(svgf_t *s, const svgf_inputs *in, void *stream, const
   k_svgf_temporal<<<grd, blk, 0, st>>>(f);
   const dim3 vgrd((s->W + VT_W - 1) / VT_W, (s->H + VT_H - 1) / VT_H);
   // each pass is set up while the one before runs: 641x363 with 3 iterations 68.9 -> 62.4 us, 1920x1080 with 5 462.6 -> 451.1
-  cudaError_t e = launch_pass(f.sigma_n == 128.0f ? k_svgf_variance<true> : k_svgf_variance<false>, vgrd, dim3(VT_NT), 0, false,
+  cudaError_t e = launch_pass(k_svgf_variance, vgrd, dim3(VT_NT), 0, false,
                               st, f, s->atrous[0]);
   int src = 0;
   for (int i = 0; i < s->o.iterations; i++) {
