@@ -90,9 +90,10 @@ def device_view(ptr: int, h: int, w: int, c: int = 4, typestr: str = "<f2"):
 
 
 class OutputViews:
-    """Views of an instance's own output images, one per buffer: making a tensor of a device pointer takes 6 us, an alias of
-    one 1 us. Entries are of buffers the instance has handed out as its output; those of sizes it no longer has go when
-    there are more than a few."""
+    """Views of an instance's own output images, one per buffer: making a tensor of a device pointer takes 6 us, another one
+    of the same storage (a tensor of its own, with a version counter of its own) 1 us. Entries are of buffers the instance has
+    handed out as its output; those of sizes it no longer has go when there are more than a few. Under inference mode the
+    outputs are inference tensors, from a view of their own."""
 
     def __init__(self):
         self._views = {}
@@ -100,13 +101,13 @@ class OutputViews:
     def get(self, ptr: int, h: int, w: int):
         import torch
 
-        key = (ptr, h, w, torch.cuda.current_device())
+        key = (ptr, h, w, torch.cuda.current_device(), torch.is_inference_mode_enabled())
         v = self._views.get(key)
         if v is None:
             if len(self._views) >= 8:
                 self._views.clear()
             v = self._views[key] = device_view(ptr, h, w)
-        return v.detach()
+        return v.data
 
 
 def _fill_inputs(inp: "L.HushInputs", tensors: dict, names=INPUTS):
