@@ -121,7 +121,9 @@ inline cudaError_t launch_pass(void (*kern)(P...), dim3 grid, dim3 block, size_t
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = first ? 0 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // it is returned, not left for the next call that asks
+  return e;
 }
 
 }  // namespace hush

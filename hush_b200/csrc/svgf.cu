@@ -732,7 +732,8 @@ extern "C" int svgf_encode(svgf_t *s, const svgf_inputs *in, void *stream, const
     src ^= 1;
   }
   if (e == cudaSuccess) e = launch_pass(k_svgf_resolve, tgrd, dim3(RT_NT), 0, false, st, f, s->atrous[src]);
-  if (e == cudaSuccess) e = cudaGetLastError();
+  const cudaError_t last = cudaGetLastError();  // (the first pass's; asked for in any case, so that none is left behind)
+  if (e == cudaSuccess) e = last;
   if (e != cudaSuccess) return svgf_fail(s, HUSH_ERR_CUDA, std::string("SVGF: kernel launch: ") + cudaGetErrorString(e));
   s->reset = false;
   s->frame++;

@@ -1,0 +1,32 @@
+"""A launch that the runtime refuses (an image of more rows of 8 texels than a grid has, 65535) is that call's error alone: the next
+calls, of the same class or another, go through."""
+import pytest
+
+from hush_b200 import SVGF, Hush, Post, scene
+from hush_b200.hush import HushError
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+TALL = 600000
+
+
+def _images(w, h):
+    f = {k: torch.ones((h, w, 4), dtype=torch.float16, device="cuda") for k in scene.NAMES}
+    return dict(f, prevNormalDepth=f["normalDepth"], prevMotion=f["motion"])
+
+
+@pytest.mark.parametrize("refused", ["svgf", "post"])
+def test_a_refused_launch_is_not_reported_twice(refused):
+    f, tall = _images(40, 24), _images(1, TALL)
+    calls = {"svgf": SVGF(0, 40, 24).encode, "hush": Hush(0, {"width": 40, "height": 24}).denoise}
+    post = Post(0, "rgba8unorm")
+    for other in ("svgf", "hush", "post"):
+        with pytest.raises(HushError):
+            if refused == "svgf":
+                SVGF(0, 1, TALL).encode(tall)
+            else:
+                Post(0, "rgba8unorm").encode(tall["radiance"], tall["radiance"])
+        out = post.encode(f["radiance"], f["radiance"]) if other == "post" else calls[other](f)
+        torch.cuda.synchronize()
+        assert tuple(out.shape) == (24, 40, 4)
