@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(AT_NT, 5) k_svgf_atrous(const SvgfFrame f, con
   extern __shared__ __align__(16) unsigned char at_smem[];
   Smem &S = *reinterpret_cast<Smem *>(at_smem);
   const int li = threadIdx.x;
-  const int bx = blockIdx.x * AT_W, phase = blockIdx.y % STEP, j0 = (blockIdx.y / STEP) * AT_H;
+  const int bx = blockIdx.x * AT_W, phase = blockIdx.y, j0 = blockIdx.z * AT_H;
   const int tx = li % AT_P, jr = (li / AT_P) * 2;  // the thread's first lattice row in the tile
   const int x0 = bx + tx, y0 = (j0 + jr) * STEP + phase;
   // The centre's 3 x 3 variance blur and depth gradient read the rows y +- 1, which only STEP = 1 stages; the other
@@ -480,7 +480,8 @@ cudaError_t launch_atrous_n(const SvgfFrame &f, const uint2 *in, uint2 *out, int
     const cudaError_t e = cudaFuncSetAttribute(k_svgf_atrous<STEP, N128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
   }
-  const dim3 grid((f.W + AT_W - 1) / AT_W, STEP * ((f.H + AT_H * STEP - 1) / (AT_H * STEP)));
+  // phases and their tiles in two dimensions: their product may be more than a grid's 65535 where no other pass's rows are
+  const dim3 grid((f.W + AT_W - 1) / AT_W, STEP, (f.H + AT_H * STEP - 1) / (AT_H * STEP));
   return launch_pass(k_svgf_atrous<STEP, N128>, grid, dim3(AT_NT), smem, false, st, f, in, out, iter);
 }
 template <int STEP>
