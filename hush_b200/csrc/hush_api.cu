@@ -414,6 +414,11 @@ static int encode_frame(hush_t *h, const HushFrame &f, cudaStream_t st, bool tim
     // register count. Timed frames keep one stream and run each stage's mid and coarse kernels one after the other,
     // so that the stage times add up to the frame.
     const bool fork = !timed && h->side;
+    // Captured frames keep plain launches: replayed they are no faster chained (1920x1080 247 -> 249 us), and their kernel nodes'
+    // parameters are rewritten. So do timed frames, which record an event between the stages and so time the kernels
+    // that a replayed frame runs.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool chained = !timed && cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
     const MlpConst &mc = h->mconst[h->mlp_mode];
     const int ns = fused_stage_count();
     for (int s = 0; s < ns && e == cudaSuccess; s++) {
@@ -422,13 +427,13 @@ static int encode_frame(hush_t *h, const HushFrame &f, cudaStream_t st, bool tim
         e = cudaEventRecord(h->ev_fork, st);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
         for (int c = 1; c <= 2 && e == cudaSuccess; c++)
-          e = launch_fused_stage(c, HP_COARSE, f, mc, h->mlp_mode, h->tc_blob_dev, h->side);
+          e = launch_fused_stage(c, HP_COARSE, f, mc, h->mlp_mode, h->tc_blob_dev, chained, h->side);
         if (e == cudaSuccess) e = cudaEventRecord(h->ev_join, h->side);
       }
       if (fork && s == 4 && e == cudaSuccess) e = cudaStreamWaitEvent(st, h->ev_join, 0);
       if (e != cudaSuccess) break;
       const int part = (s == 1 || s == 2) && fork ? HP_MID : HP_BOTH;
-      e = launch_fused_stage(s, part, f, mc, h->mlp_mode, h->tc_blob_dev, st);
+      e = launch_fused_stage(s, part, f, mc, h->mlp_mode, h->tc_blob_dev, chained, st);
     }
   }
   if (timed) {

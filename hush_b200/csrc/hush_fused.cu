@@ -1527,20 +1527,14 @@ static void (*const KB_KERN[6])(HushFrame, MlpConst, const uint4 *) = {
     k_temporal_block<0, KB_TH>, k_temporal_block<1, KB_TH>,     k_temporal_block<2, KB_TH>,
     k_temporal_block<3, KB_TH>, k_temporal_block<0, KB_TH / 2>, k_temporal_block<3, KB_TH / 2>};
 
-// The kernels that directly follow another one of the frame on their stream (mid2, mid3, coarse2, TAA) are set up while that
-// one runs: directly launched frames 256x256 43.2 -> 39.7 us, 640x360 60.5 -> 55.0, 1283x717 144.5 -> 142.0. Captured frames
-// keep plain launches: replayed they are no faster (1920x1080 247 -> 249 us), and their kernel nodes' parameters are rewritten.
-static bool capturing(cudaStream_t st) {
-  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
-}
-
+// chained: the kernels that directly follow another one of the frame on their stream (mid2, mid3, coarse2, TAA) are set up while
+// that one runs: directly launched frames 256x256 43.2 -> 39.7 us, 640x360 60.5 -> 55.0, 1283x717 144.5 -> 142.0.
 cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const MlpConst &mc, int mlp_mode,
-                               const void *mlp_tc, cudaStream_t st) {
+                               const void *mlp_tc, bool chained, cudaStream_t st) {
   const int hx = (f.W2 + HT_W - 1) / HT_W, hy = (f.H2 + HT_H - 1) / HT_H;
   const int qx = (f.W4 + HT_W - 1) / HT_W, qy = (f.H4 + HT_H - 1) / HT_H;
   const int hpx = (f.W2 + MP_W - 1) / MP_W;  // two-pixel mid tiles per row
-  const bool full = (stage == 2 || stage == 3 || stage == 5) && capturing(st);  // plain launches
+  const bool plain = !chained;
   switch (stage) {
     case 0: {
       // blob: the tensor-core forms' bf16 hi / lo operands and f16 operands; mc: the weights as a kernel parameter
@@ -1578,18 +1572,19 @@ cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const Ml
       constexpr int smc = 2 * (HT_W + 8) * (HT_H + 8) * 16;  // coarse2's two float4 tiles
       cudaError_t e = cudaSuccess;
       if (part != HP_COARSE)
-        e = launch_pass(full ? k_half_pair<2, HP_MID, false> : k_half_pair<2, HP_MID, true>, dim3(hpx * hy), dim3(HT_W * HT_H), (size_t)mid_pair_smem<2>(), full, st, f, hpx,
-                        hpx * hy, qx, half_maps(f));
+        e = launch_pass(plain ? k_half_pair<2, HP_MID, false> : k_half_pair<2, HP_MID, true>, dim3(hpx * hy),
+                        dim3(HT_W * HT_H), (size_t)mid_pair_smem<2>(), plain, st, f, hpx, hpx * hy, qx, half_maps(f));
       if (part != HP_MID && e == cudaSuccess)
-        e = launch_pass(full ? k_half_pair<2, HP_COARSE, false> : k_half_pair<2, HP_COARSE, true>, dim3(qx * qy), dim3(HT_W * HT_H), (size_t)smc, full, st, f, hpx, hpx * hy, qx,
-                        half_maps(f));
+        e = launch_pass(plain ? k_half_pair<2, HP_COARSE, false> : k_half_pair<2, HP_COARSE, true>, dim3(qx * qy),
+                        dim3(HT_W * HT_H), (size_t)smc, plain, st, f, hpx, hpx * hy, qx, half_maps(f));
       if (e != cudaSuccess) return e;
       break;
     }
     case 3:
       if (part == HP_COARSE) break;  // no coarse level in stage 3
-      if (const cudaError_t e = launch_pass(full ? k_half_pair<3, HP_MID, false> : k_half_pair<3, HP_MID, true>,
-                                            dim3(hpx * hy), dim3(HT_W * HT_H), (size_t)mid_pair_smem<4>(), full, st, f, hpx, hpx * hy, qx, half_maps(f)))
+      if (const cudaError_t e = launch_pass(plain ? k_half_pair<3, HP_MID, false> : k_half_pair<3, HP_MID, true>,
+                                            dim3(hpx * hy), dim3(HT_W * HT_H), (size_t)mid_pair_smem<4>(), plain, st, f, hpx,
+                                            hpx * hy, qx, half_maps(f)))
         return e;
       break;
     case 4: {
@@ -1610,8 +1605,9 @@ cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const Ml
       break;
     }
     case 5:
-      if (const cudaError_t e = launch_pass(full ? k_taa_fused<false> : k_taa_fused<true>, dim3((f.W + FT_W - 1) / FT_W, (f.H + FT_H - 1) / FT_H),
-                                            dim3(FT_W * FT_H), 0, full, st, f))
+      if (const cudaError_t e = launch_pass(plain ? k_taa_fused<false> : k_taa_fused<true>,
+                                            dim3((f.W + FT_W - 1) / FT_W, (f.H + FT_H - 1) / FT_H), dim3(FT_W * FT_H), 0,
+                                            plain, st, f))
         return e;
       break;
     default: return cudaErrorInvalidValue;

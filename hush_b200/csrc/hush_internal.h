@@ -26,9 +26,10 @@ struct MlpConst;
 // kernel keeps its own register count; HP_BOTH runs the stage's two kernels one after the other.
 enum HalfPart { HP_BOTH = 0, HP_MID = 1, HP_COARSE = 2 };
 // One stage of the fused frame on `st`; part (a HalfPart) selects the tiles of stages 1 and 2, the half-res levels
-// with a coarse level beside them (stage 3 has no coarse tiles, the other stages ignore it).
+// with a coarse level beside them (stage 3 has no coarse tiles, the other stages ignore it). chained: a kernel that directly
+// follows another one of the frame is launched as its programmatic successor.
 cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const MlpConst &mc, int mlp_mode,
-                               const void *mlp_tc, cudaStream_t st);
+                               const void *mlp_tc, bool chained, cudaStream_t st);
 int fused_stage_count();
 const char *fused_stage_label(int stage);
 size_t fused_scratch_bytes(int W, int H);
