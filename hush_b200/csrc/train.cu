@@ -46,8 +46,9 @@ struct TwinFrame {
   float4 *A1, *X, *out;   // full: fine level, pre-TAA colour, TAA output
   const float4 *out_prev; // full: previous frame's TAA output (temporal loss term)
   const float *clean, *clean_prev;  // full: noise-free rgb (f32, dense), previous frame's
-  float4 *gT;             // full: the loss's gradient w.r.t. the TAA output (the per-pass pair)
-  float4 *rsave;          // full, 4 planes: the recombination's values for its adjoint (RSave), or NULL (not kept)
+  float4 *gT;             // full: the loss's gradient w.r.t. the TAA output (the per-pass pair), or NULL (not kept)
+  float4 *rsave;          // full, 3 planes: the recombination's values for its adjoint (RSave), or NULL (not kept)
+  float4 *rwq;            // full: its quarter-res weights (RSave::wq), which the window sweep alone reads, or NULL
   float4 *dB1, *dB2, *dB3;  // half: level gradients
   const float4 *gA1;        // full: dL/d fine level through the colour history (the next frame's TEMPORAL), or NULL
   float4 *dA0;              // full: dL/d TEMPORAL's colour + variance A0 (the fine level's input), or NULL
@@ -588,7 +589,7 @@ struct RSave {
   float4 mid, coarse, wh, wq;
 };
 // ill before the coarse level (i) from A1 and the sums; also the pixel's RSave.
-HD_INL RSave recomb_mix(const Recomb &R, float4 A1, float kappa, float &ix, float &iy, float &iz) {
+HD_INL RSave recomb_mix(const Recomb &R, float4 A1, float kappa, float &ix, float &iy, float &iz, bool want_wq) {
   RSave V;
   ix = A1.x; iy = A1.y; iz = A1.z;
   V.mid = V.coarse = V.wh = V.wq = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -602,7 +603,7 @@ HD_INL RSave recomb_mix(const Recomb &R, float4 A1, float kappa, float &ix, floa
   float upx = ix, upy = iy, upz = iz;
   if (R.swq > 1e-4f) { upx = R.uCx / R.swq; upy = R.uCy / R.swq; upz = R.uCz / R.swq; }
   V.coarse = make_float4(upx - ix, upy - iy, upz - iz, R.swq > 1e-4f ? 1.0f : 0.0f);
-  if (R.swq > 1e-4f) {
+  if (want_wq && R.swq > 1e-4f) {
     V.wq = make_float4(R.wq[0] / R.swq, R.wq[1] / R.swq, R.wq[2] / R.swq, R.wq[3] / R.swq);
   }
   return V;
@@ -647,7 +648,7 @@ __global__ void __launch_bounds__(TW *TH) k_fine_fwd(const TwinFrame T) {
   Recomb R;
   recomb_fwd(f, S, px, py, bx, by, gp, R);
   float ix, iy, iz;
-  const RSave V = recomb_mix(R, A1, p0.w, ix, iy, iz);
+  const RSave V = recomb_mix(R, A1, p0.w, ix, iy, iz, T.rwq != nullptr);
   ix = ix + V.coarse.x * p0.z;
   iy = iy + V.coarse.y * p0.z;
   iz = iz + V.coarse.z * p0.z;
@@ -657,7 +658,7 @@ __global__ void __launch_bounds__(TW *TH) k_fine_fwd(const TwinFrame T) {
     T.rsave[o] = V.mid;
     T.rsave[n + o] = V.coarse;
     T.rsave[2 * n + o] = V.wh;
-    T.rsave[3 * n + o] = V.wq;
+    if (T.rwq) T.rwq[o] = V.wq;
   }
 }
 
@@ -932,7 +933,7 @@ __global__ void __launch_bounds__(TW *TH) k_taa(const TwinFrame T, int mode, flo
       l = loss_pixel(T, o, A.out, g) * T.inv_n;
       if (mode == TAA_ADJ) {
         g = make_float3(g.x * T.inv_n, g.y * T.inv_n, g.z * T.inv_n);
-        T.gT[o] = make_float4(g.x, g.y, g.z, 0.f);
+        if (T.gT) T.gT[o] = make_float4(g.x, g.y, g.z, 0.f);
         taa_coef(A, g, coef + 3 * o);
       }
     }
@@ -1033,7 +1034,7 @@ __global__ void __launch_bounds__(TW *TH) k_fine_bwd(const TwinFrame T, const fl
       Recomb R;
       recomb_fwd(f, S, px, py, bx, by, gp, R);
       float ix, iy, iz;
-      V = recomb_mix(R, F.out(), p0.w, ix, iy, iz);
+      V = recomb_mix(R, F.out(), p0.w, ix, iy, iz, false);
     }
     // X = ill2 * alb + emi, ill2 = ill + (up - ill) beta
     const float3 g2 = make_float3(gX.x * alb.x, gX.y * alb.y, gX.z * alb.z);
@@ -1095,7 +1096,7 @@ __global__ void __launch_bounds__(TW *TH) k_fine_bwd(const TwinFrame T, const fl
 // The recombination's adjoint into the block means and the coarse level (window sweep only; k_fine_bwd does the
 // rest): ill = uB / sum_h w + kappa (f - uA / sum_h w) and ill2 = ill + (up - ill) beta, up = sum_q w C0 / sum_q w, so
 // each half-res tap's block-mean colour gets -kappa w / sum_h w dL/d ill and each quarter-res tap's colour
-// beta w / sum_q w dL/d ill2 (X = ill2 albedo + emission). The normalised tap weights come from T.rsave.
+// beta w / sum_q w dL/d ill2 (X = ill2 albedo + emission). The normalised tap weights come from T.rsave and T.rwq.
 __global__ void __launch_bounds__(TW *TH) k_fine_pyr_bwd(const TwinFrame T, const float4 *gXp) {
   const HushFrame &f = T.f;
   const int px = blockIdx.x * TW + threadIdx.x, py = blockIdx.y * TH + threadIdx.y;
@@ -1104,7 +1105,7 @@ __global__ void __launch_bounds__(TW *TH) k_fine_pyr_bwd(const TwinFrame T, cons
   if (ldh(f.key, o).z < 0.0f) return;  // sky: X = emission
   const size_t n = (size_t)f.W * f.H;
   const float4 gX = gXp[o], alb = ldh(f.mat, py * f.p_mat + px), p0 = T.par[3 * ((py >> 1) * f.W2 + (px >> 1))];
-  const float4 wh4 = T.rsave[2 * n + o], wq4 = T.rsave[3 * n + o];
+  const float4 wh4 = T.rsave[2 * n + o], wq4 = T.rwq[o];
   const bool mid = T.rsave[o].w != 0.0f, coarse = T.rsave[n + o].w != 0.0f;
   const float3 g2 = make_float3(gX.x * alb.x, gX.y * alb.y, gX.z * alb.z);
   float3 gill = g2;
@@ -1768,10 +1769,11 @@ struct hush_trainer_s {
     float4 *out;
     // with saved forwards, from the second frame on (frame 0 uses the trainer's own buffers): dL/dX, the
     // recombination's values, the parameters and the mid levels the adjoints read
-    float4 *gX, *rsave, *par, *B1, *B2;
+    float4 *gX, *rsave, *rwq, *par, *B1, *B2;
   };
   bool rec_saved = false;       // the records hold the forwards' values (else the reverse sweep runs them again)
-  float4 *rec_tmp[4] = {};      // A1, X, B3 and dL/dout of the frame whose forward runs (saved forwards)
+  float4 *rec_tmp[3] = {};      // A1, X and B3 of the frame whose forward runs (saved forwards)
+  float4 *rec_wq = nullptr;     // the quarter-res weights of the frame whose forward the sweep runs again (else)
   float *rec_partials = nullptr;  // per frame: the MLP adjoint's per-CTA partials, reduced once per window
   std::vector<Rec> rec;
   char *rec_pool = nullptr;
@@ -1825,7 +1827,7 @@ extern "C" int hush_trainer_create(hush_t *h, const float *theta, hush_trainer_t
   const int n_partials = std::max(t->n_loss_ctas, ((t->W + TW - 1) / TW) * ((t->H + TH - 1) / TH));
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t bytes = al(NW * 4) * 3 + al(NW * 8) + al(8) * 2 + al((size_t)n_partials * 8) + al(half * 48) * 2 +
-                       al(half * 16) * 6 + al(full * 16) * 12 + al(full * 48) + al(full * 64) + al((size_t)t->n_mlp_ctas * NW * 4) +
+                       al(half * 16) * 6 + al(full * 16) * 12 + al(full * 48) * 2 + al((size_t)t->n_mlp_ctas * NW * 4) +
                        al(half * 8);
   cudaError_t e = cudaMalloc(&t->pool, bytes);
   if (e != cudaSuccess) { delete t; return hush_cuda_fail(h, e, "cudaMalloc of the trainer"); }
@@ -1846,7 +1848,7 @@ extern "C" int hush_trainer_create(hush_t *h, const float *theta, hush_trainer_t
   t->out[0] = (float4 *)take(full * 16); t->out[1] = (float4 *)take(full * 16);
   t->gT = (float4 *)take(full * 16); t->gT2 = (float4 *)take(full * 16); t->dX = (float4 *)take(full * 16);
   t->tcoef = (float4 *)take(full * 48);
-  t->rsave = (float4 *)take(full * 64);
+  t->rsave = (float4 *)take(full * 48);
   t->partials = (float *)take((size_t)t->n_mlp_ctas * NW * 4);
   t->dA1 = (float4 *)take(full * 16); t->dmom = (float4 *)take(full * 16);
   t->dhist = (float4 *)take(full * 16); t->dmomp = (float4 *)take(full * 16);
@@ -2528,8 +2530,9 @@ static int ensure_records(hush_trainer_t *t, int n) {
   const size_t quarter = (size_t)((t->W2 + 1) / 2) * ((t->H2 + 1) / 2), part = (size_t)t->n_mlp_ctas * NW * 4;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t lean = al(full * 8) * 5 + al(half * 8) + al(half * 16) * 4 + al(quarter * 8) * 3 + al(full * 16);
-  const size_t saved = al(full * 16) + al(full * 64) + al(half * 48) + al(half * 16) * 2;
-  const size_t bytes_lean = lean * n, bytes_saved = (lean + saved) * n + al(full * 16) * 3 + al(half * 16) + al(part * n);
+  const size_t saved = al(full * 16) * 2 + al(full * 48) + al(half * 48) + al(half * 16) * 2;
+  const size_t bytes_lean = lean * n + al(full * 16),
+               bytes_saved = (lean + saved) * n + al(full * 16) * 2 + al(half * 16) + al(part * n);
   drop_bptt_graph(t);  // it captured the old records' addresses
   cudaFree(t->rec_pool);
   t->rec_pool = nullptr;
@@ -2563,15 +2566,18 @@ static int ensure_records(hush_trainer_t *t, int n) {
     r.C0 = (uint2 *)take(quarter * 8); r.C1 = (uint2 *)take(quarter * 8); r.CG = (uint2 *)take(quarter * 8);
     r.out = (float4 *)take(full * 16);
     if (t->rec_saved) {
-      r.gX = (float4 *)take(full * 16); r.rsave = (float4 *)take(full * 64); r.par = (float4 *)take(half * 48);
+      r.gX = (float4 *)take(full * 16); r.rsave = (float4 *)take(full * 48); r.rwq = (float4 *)take(full * 16);
+      r.par = (float4 *)take(half * 48);
       r.B1 = (float4 *)take(half * 16); r.B2 = (float4 *)take(half * 16);
     }
     t->rec.push_back(r);
   }
   if (t->rec_saved) {
-    for (int k = 0; k < 3; k++) t->rec_tmp[k] = (float4 *)take(full * 16);
-    t->rec_tmp[3] = (float4 *)take(half * 16);
+    for (int k = 0; k < 2; k++) t->rec_tmp[k] = (float4 *)take(full * 16);
+    t->rec_tmp[2] = (float4 *)take(half * 16);
     t->rec_partials = (float *)take(part * n);
+  } else {
+    t->rec_wq = (float4 *)take(full * 16);
   }
   return HUSH_OK;
 }
@@ -2591,11 +2597,12 @@ static TwinFrame rec_twin(hush_trainer_t *t, const hush_inputs *in, const float 
   T.out_prev = p.out;
   T.has_prev = (i > 0 && clean_prev) ? 1 : 0;
   T.rsave = t->rsave;
+  if (!t->rec_saved) T.rwq = i > 0 ? t->rec_wq : nullptr;  // (frame 0 sends nothing to block means or coarse levels)
   if (t->rec_saved) {
     T.partials = t->rec_partials + (size_t)i * t->n_mlp_ctas * NW;
     if (i > 0) {
-      T.par = r.par; T.B1 = r.B1; T.B2 = r.B2; T.rsave = r.rsave;
-      T.A1 = t->rec_tmp[0]; T.X = t->rec_tmp[1]; T.gT = t->rec_tmp[2]; T.B3 = t->rec_tmp[3];
+      T.par = r.par; T.B1 = r.B1; T.B2 = r.B2; T.rsave = r.rsave; T.rwq = r.rwq;
+      T.A1 = t->rec_tmp[0]; T.X = t->rec_tmp[1]; T.gT = nullptr; T.B3 = t->rec_tmp[2];
     }
   }
   return T;
@@ -2657,7 +2664,8 @@ static cudaError_t bptt_launches(hush_trainer_t *t, const hush_inputs *frames, c
   };
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < n_frames && e == cudaSuccess; i++) {
-    const TwinFrame T = twin(i);
+    TwinFrame T = twin(i);
+    if (!t->rec_saved) T.rsave = T.rwq = nullptr;  // kept when the sweep runs the forward again
     e = launch_pass(PASS_TEMPORAL, T.f, t->h->w16, st);
     if (e == cudaSuccess) e = launch_pass(PASS_COARSE1, T.f, t->h->w16, st);
     if (e == cudaSuccess) e = launch_pass(PASS_COARSE2, T.f, t->h->w16, st);
