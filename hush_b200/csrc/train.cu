@@ -1777,6 +1777,7 @@ struct hush_trainer_s {
   float *rec_partials = nullptr;  // per frame: the MLP adjoint's per-CTA partials, reduced once per window
   std::vector<Rec> rec;
   char *rec_pool = nullptr;
+  size_t rec_bytes = 0;  // of rec_pool
   float4 *c_hist[2] = {}, *c_mom[2] = {};
   float2 *c_ag[2] = {};
   char *carry_pool = nullptr;
@@ -2275,7 +2276,7 @@ static int make_lanes(hush_trainer_t *t, int n) {
 }
 
 static int windows_serial_bptt(hush_trainer_t *t, const hush_scene *sc, const uint32_t *seeds, int n_windows,
-                               int stride, int n_frames, float lambda_t, cudaStream_t st);
+                               int lanes, int n_frames, float lambda_t, cudaStream_t st);
 
 // Windows of the analytic scene generator, trained in place (hush_trainer_windows: per-frame gradient by
 // windows_serial; hush_trainer_windows_bptt: through time by windows_serial_bptt): for each seed, the window's frames
@@ -2520,32 +2521,55 @@ static size_t carry_bytes(const hush_trainer_t *t) {
 
 // The state of each frame of a window that the reverse sweep reads again: TEMPORAL's outputs and key, the features,
 // the coarse levels, the twin's stored history (colour, TAA, par0), its FP32 TAA output (the next frame's temporal loss
-// term) and, while the window's records stay under REC_SAVED_MAX, what the adjoints need of the twin's forward (27 MB
-// instead of 11 MB per frame at 384 x 384), so that the sweep does not run the forward again. Larger windows, and ones
-// whose memory is not to be had, keep the 11 MB and recompute. Allocated for the longest window seen.
+// term) and, while the window's records stay under REC_SAVED_MAX / lanes (the lanes that run windows at the same time share
+// that), what the adjoints need of the twin's forward (26 MB instead of 11 MB per frame at 384 x 384), so that the sweep
+// does not run the forward again (a step through time of 16 windows x 8 frames 13.8 -> 11.5 ms). Larger windows, and ones
+// that would take more than half of the device's free memory, keep the 11 MB and recompute. A window's form does not
+// depend on the windows before it; the pool is kept for the largest.
 constexpr size_t REC_SAVED_MAX = (size_t)2 << 30;
-static int ensure_records(hush_trainer_t *t, int n) {
-  if ((int)t->rec.size() >= n) return HUSH_OK;
+static int ensure_records(hush_trainer_t *t, int n, int lanes) {
   const size_t full = (size_t)t->W * t->H, half = (size_t)t->W2 * t->H2;
   const size_t quarter = (size_t)((t->W2 + 1) / 2) * ((t->H2 + 1) / 2), part = (size_t)t->n_mlp_ctas * NW * 4;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t lean = al(full * 8) * 5 + al(half * 8) + al(half * 16) * 4 + al(quarter * 8) * 3 + al(full * 16);
-  const size_t saved = al(full * 16) * 2 + al(full * 48) + al(half * 48) + al(half * 16) * 2;
+  const size_t more = al(full * 16) * 2 + al(full * 48) + al(half * 48) + al(half * 16) * 2;
   const size_t bytes_lean = lean * n + al(full * 16),
-               bytes_saved = (lean + saved) * n + al(full * 16) * 2 + al(half * 16) + al(part * n);
-  drop_bptt_graph(t);  // it captured the old records' addresses
-  cudaFree(t->rec_pool);
-  t->rec_pool = nullptr;
-  t->rec.clear();
-  t->rec_saved = bytes_saved <= REC_SAVED_MAX && cudaMalloc(&t->rec_pool, bytes_saved) == cudaSuccess;
-  cudaError_t e = cudaSuccess;
-  if (!t->rec_saved) {
-    cudaGetLastError();
-    e = cudaMalloc(&t->rec_pool, bytes_lean);
+               bytes_saved = (lean + more) * n + al(full * 16) * 2 + al(half * 16) + al(part * n);
+  const bool laid_out = (int)t->rec.size() >= n;
+  if (laid_out && t->rec_saved) return HUSH_OK;
+  bool saved = bytes_saved <= REC_SAVED_MAX / lanes;
+  if (saved && bytes_saved > t->rec_bytes) {
+    size_t free_bytes = 0, total = 0;
+    saved = cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && bytes_saved <= (free_bytes + t->rec_bytes) / 2;
   }
-  if (e != cudaSuccess) { t->rec_pool = nullptr; return hush_cuda_fail(t->h, e, "cudaMalloc of the window records"); }
-  e = cudaMemset(t->rec_pool, 0, t->rec_saved ? bytes_saved : bytes_lean);
-  if (e != cudaSuccess) return hush_cuda_fail(t->h, e, "cudaMemset of the window records");
+  if (laid_out && !saved) return HUSH_OK;
+  drop_bptt_graph(t);  // it captured the old records' addresses
+  t->rec.clear();
+  cudaError_t e = cudaSuccess;
+  const size_t bytes = saved ? bytes_saved : bytes_lean;
+  if (bytes > t->rec_bytes) {
+    cudaFree(t->rec_pool);
+    t->rec_pool = nullptr;
+    t->rec_bytes = 0;
+    e = cudaMalloc(&t->rec_pool, bytes);
+    if (e == cudaSuccess) {
+      t->rec_bytes = bytes;
+      e = cudaMemset(t->rec_pool, 0, bytes);
+    } else if (saved) {  // (free memory in pieces, or taken meanwhile)
+      cudaGetLastError();
+      saved = false;
+      e = cudaMalloc(&t->rec_pool, bytes_lean);
+      if (e == cudaSuccess) {
+        t->rec_bytes = bytes_lean;
+        e = cudaMemset(t->rec_pool, 0, bytes_lean);
+      }
+    }
+    if (e != cudaSuccess) {
+      if (!t->rec_bytes) t->rec_pool = nullptr;
+      return hush_cuda_fail(t->h, e, "memory of the window records");
+    }
+  }
+  t->rec_saved = saved;
   if (!t->carry_pool) {  // per ping-pong slot: colour history, moments, alpha / gamma, cleared together
     e = cudaMalloc(&t->carry_pool, carry_bytes(t) * 2);
     if (e != cudaSuccess) { t->carry_pool = nullptr; return hush_cuda_fail(t->h, e, "cudaMalloc of the carries"); }
@@ -2631,7 +2655,7 @@ extern "C" int hush_trainer_window_bptt(hush_trainer_t *t, const hush_inputs *fr
     if (rc != HUSH_OK) return rc;
   }
   cudaSetDevice(t->h->dev);
-  int rc = ensure_records(t, n_frames);
+  int rc = ensure_records(t, n_frames, 1);
   if (rc != HUSH_OK) return rc;
   cudaError_t e = ensure_coarse(t);  // the coarse levels' adjoint buffers
   if (e != cudaSuccess) return hush_cuda_fail(t->h, e, "cudaMalloc of the coarse-level buffers");
@@ -2713,16 +2737,16 @@ static cudaError_t bptt_launches(hush_trainer_t *t, const hush_inputs *frames, c
   return e;
 }
 
-// The windows seeds[0], seeds[stride], ... through time, in order on one trainer and stream: each window generated
+// The windows seeds[0], seeds[lanes], ... through time, in order on one trainer and stream: each window generated
 // into win_pool on `st`, then its forward + reverse sweep (bptt_launches) replayed as one CUDA graph, captured at the
 // first window and kept while the frame count, lambda, the exposure and the MLP form stay the same (the buffers it
 // names are the trainer's and stay put; reallocating them drops it). Where capture is not possible the launches run
 // directly.
 static int windows_serial_bptt(hush_trainer_t *t, const hush_scene *sc, const uint32_t *seeds, int n_windows,
-                               int stride, int n_frames, float lambda_t, cudaStream_t st) {
+                               int lanes, int n_frames, float lambda_t, cudaStream_t st) {
   size_t img = 0, per = 0;
   int rc = ensure_win_pool(t, n_frames, img, per);
-  if (rc == HUSH_OK) rc = ensure_records(t, n_frames);
+  if (rc == HUSH_OK) rc = ensure_records(t, n_frames, lanes);
   if (rc != HUSH_OK) return rc;
   const cudaError_t ec = ensure_coarse(t);  // the coarse levels' adjoint buffers
   if (ec != cudaSuccess) return hush_cuda_fail(t->h, ec, "cudaMalloc of the coarse-level buffers");
@@ -2747,7 +2771,7 @@ static int windows_serial_bptt(hush_trainer_t *t, const hush_scene *sc, const ui
     in[i].emission = b + 4 * img;
     cl[i] = (const float *)(b + 5 * img);
   }
-  for (int k = 0; k < n_windows; k += stride) {
+  for (int k = 0; k < n_windows; k += lanes) {
     rc = generate_window(t, sc, seeds[k], n_frames, img, per, st);
     if (rc != HUSH_OK) return rc;
     if (!t->bptt_graph) {  // capture on the trainer's own stream (the caller's may be the legacy default stream)

@@ -327,18 +327,18 @@ int hush_coarse2_bwd(hush_trainer_t *t, void *stream);
  * reaches the loss directly (the fine level) and through the block means (block(), hush.js:241-244), which feed mid1,
  * the recombination and the coarse levels COARSE1 / coarse2; both paths are followed. The block features and the TAA
  * history are held fixed (truncated there). Adds into the gradient and loss accumulators,
- * like hush_trainer_windows; allocates the window's per-frame records on first use (about 27 MB per frame at 384 x 384
- * while a window's stay under 2 GiB, so that the reverse sweep does not run the forward again; else 11 MB). The
- * trainer's own Hush history is not touched. */
+ * like hush_trainer_windows; allocates the window's per-frame records on first use: about 26 MB per frame at 384 x 384
+ * where the window's stay under 2 GiB and half of the device's free memory, so that the reverse sweep does not run the
+ * forward again; else 11 MB. The trainer's own Hush history is not touched. */
 int hush_trainer_window_bptt(hush_trainer_t *t, const hush_inputs *frames, const float *const *cleans, int n_frames,
                              float lambda_t, void *stream);
 
 /* hush_trainer_window_bptt over the training windows of the analytic scene generator, as hush_trainer_windows runs
  * them: for each of n_windows seeds the n_frames frames of *sc are generated on the device into trainer-owned buffers
  * and the window runs forward and backward through time. Up to eight windows run concurrently on the same lanes
- * (each lane its own records), summed into this trainer's accumulators in lane order; each window's forward + reverse
- * sweep replays as a cached CUDA graph. No optimiser step; sc's size must be the trainer's. The trainer's own Hush
- * history is not touched. */
+ * (each lane its own records, the lanes sharing the 2 GiB within which they take the larger form), summed into this
+ * trainer's accumulators in lane order; each window's forward + reverse sweep replays as a cached CUDA graph. No
+ * optimiser step; sc's size must be the trainer's. The trainer's own Hush history is not touched. */
 int hush_trainer_windows_bptt(hush_trainer_t *t, const struct hush_scene_s *sc, const uint32_t *seeds, int n_windows,
                               int n_frames, float lambda_t, void *stream);
 
