@@ -501,7 +501,14 @@ def _extras_ms(frames, stream, n=32, warmup=4):
             tracer.encode(i & 1, stream=stream)
 
         out["pt_ms_per_frame"] = timed(pt_step)
-        out["pt_config"] = "demo scene, 32 objects, 1 spp, 3 bounces, NEE + MIS, env map"
+        # the same scene under an environment map (a vertical gradient, 512 x 256), which the tracer's other kernel runs
+        import numpy as np
+
+        img = np.ones((256, 512, 4), np.float32)
+        img[..., :3] = np.linspace(1.0, 0.2, 256, dtype=np.float32)[:, None, None] * np.array([0.6, 0.8, 1.0], np.float32)
+        env = dict(env, map=pt.prepare_env_map(img, sun=False))
+        out["pt_envmap_ms_per_frame"] = timed(pt_step)
+        out["pt_config"] = "demo scene, 32 objects, 1 spp, 3 bounces, NEE + MIS, gradient sky / environment map"
         tracer.destroy()
     except Exception as e:  # pragma: no cover
         out["pt_ms_per_frame"] = f"failed: {e}"

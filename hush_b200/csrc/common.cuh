@@ -102,15 +102,15 @@ constexpr int N_OUT = 12;
 // A chain of short kernels, each launched as the next one's programmatic predecessor: a kernel's CTAs are set up while the one
 // before runs, and pass_begin(), the first thing that every kernel of the chain but the first does, waits for the end of that
 // one (which has waited for the end of its own predecessor, and so on). The first kernel waits for whatever the stream did
-// before, as any kernel; so does the first kernel after the chain. What a kernel of the chain writes is read in it by ld_pass() and
-// ldh_pass() and never through a `const __restrict__` parameter; the caller's inputs and former frames' images, which no
+// before, as any kernel; so does the first kernel after the chain. What a kernel of the chain writes is read in it by ld_pass()
+// and ldh_pass() and never through a `const __restrict__` parameter; the caller's inputs and former frames' images, which no
 // kernel of the chain writes, may take the read-only path.
 __device__ __forceinline__ void pass_begin(bool last = false) {
   if (!last) asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 template <class... P, class... A>
-inline cudaError_t launch_pass(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, bool first, cudaStream_t st, A... args) {
+inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, bool first, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;

@@ -1067,12 +1067,13 @@ constexpr int FT_W = 32, FT_H = 8;  // TAA's tile
 // CGd, coarse level C0; 10 x 6) and the per-block filter parameters (s0, c0, beta, kappa; 16 x 8). A thread's two pixels
 // share the loads of 10 of their 3 x 3 windows' 18 texels, one row of the half-res footprint, the whole quarter-res
 // footprint and the parameters: 52 16-byte loads of shared memory for two pixels instead of 80. With a pixel per
-// thread the kernel was at 70% of the shared-memory bandwidth and 67% of the issue slots, and with either split half of
-// the CTAs waited for their tile's texels: 70 us at 1920 x 1080 and 271 at 3840 x 2160, now 66 and 246. Three CTAs per SM
-// (80 registers, with spills) measured the same at 1920 x 1080 and 0.6 us more at 256 x 256.
+// thread the kernel was at 70% of the shared-memory bandwidth and 67% of the issue slots, and half of its CTAs waited for their
+// tile's texels (so they did with two pixels per thread and a CTA per tile): 70 us at 1920 x 1080 and 271 at 3840 x 2160,
+// now 66 and 246. Three CTAs per SM (80 registers, with spills) measured the same at 1920 x 1080 and 0.6 us more at
+// 256 x 256.
 constexpr int FF_W = 32, FF_H = 16, FF_NT = FF_W * FF_H / 2;
 constexpr int FH_W = FF_W / 2 + 2, FH_H = FF_H / 2 + 2, FQ_W = FF_W / 4 + 2, FQ_H = FF_H / 4 + 2;
-constexpr int FB_W = FF_W + 4, FB_H = FF_H + 2;  // the TMA box of the A0 / key tiles
+constexpr int FB_W = FF_W + 4, FB_H = FF_H + 2;  // A0 / key texels as copied, from column -2 on
 
 // filt_x<1, 1, true> for the pixel at tile entry ti and the one below it. The taps run as pairs of one tap of each
 // pixel, on the same texel where both windows hold it: (n.n)^128, weights and their squares as packed FP32x2, lane by lane
@@ -1572,19 +1573,19 @@ cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const Ml
       constexpr int smc = 2 * (HT_W + 8) * (HT_H + 8) * 16;  // coarse2's two float4 tiles
       cudaError_t e = cudaSuccess;
       if (part != HP_COARSE)
-        e = launch_pass(plain ? k_half_pair<2, HP_MID, false> : k_half_pair<2, HP_MID, true>, dim3(hpx * hy),
-                        dim3(HT_W * HT_H), (size_t)mid_pair_smem<2>(), plain, st, f, hpx, hpx * hy, qx, half_maps(f));
+        e = launch_chained(plain ? k_half_pair<2, HP_MID, false> : k_half_pair<2, HP_MID, true>, dim3(hpx * hy),
+                           dim3(HT_W * HT_H), (size_t)mid_pair_smem<2>(), plain, st, f, hpx, hpx * hy, qx, half_maps(f));
       if (part != HP_MID && e == cudaSuccess)
-        e = launch_pass(plain ? k_half_pair<2, HP_COARSE, false> : k_half_pair<2, HP_COARSE, true>, dim3(qx * qy),
-                        dim3(HT_W * HT_H), (size_t)smc, plain, st, f, hpx, hpx * hy, qx, half_maps(f));
+        e = launch_chained(plain ? k_half_pair<2, HP_COARSE, false> : k_half_pair<2, HP_COARSE, true>, dim3(qx * qy),
+                           dim3(HT_W * HT_H), (size_t)smc, plain, st, f, hpx, hpx * hy, qx, half_maps(f));
       if (e != cudaSuccess) return e;
       break;
     }
     case 3:
       if (part == HP_COARSE) break;  // no coarse level in stage 3
-      if (const cudaError_t e = launch_pass(plain ? k_half_pair<3, HP_MID, false> : k_half_pair<3, HP_MID, true>,
-                                            dim3(hpx * hy), dim3(HT_W * HT_H), (size_t)mid_pair_smem<4>(), plain, st, f, hpx,
-                                            hpx * hy, qx, half_maps(f)))
+      if (const cudaError_t e = launch_chained(plain ? k_half_pair<3, HP_MID, false> : k_half_pair<3, HP_MID, true>,
+                                               dim3(hpx * hy), dim3(HT_W * HT_H), (size_t)mid_pair_smem<4>(), plain, st, f, hpx,
+                                               hpx * hy, qx, half_maps(f)))
         return e;
       break;
     case 4: {
@@ -1605,9 +1606,9 @@ cudaError_t launch_fused_stage(int stage, int part, const HushFrame &f, const Ml
       break;
     }
     case 5:
-      if (const cudaError_t e = launch_pass(plain ? k_taa_fused<false> : k_taa_fused<true>,
-                                            dim3((f.W + FT_W - 1) / FT_W, (f.H + FT_H - 1) / FT_H), dim3(FT_W * FT_H), 0,
-                                            plain, st, f))
+      if (const cudaError_t e = launch_chained(plain ? k_taa_fused<false> : k_taa_fused<true>,
+                                               dim3((f.W + FT_W - 1) / FT_W, (f.H + FT_H - 1) / FT_H), dim3(FT_W * FT_H), 0,
+                                               plain, st, f))
         return e;
       break;
     default: return cudaErrorInvalidValue;

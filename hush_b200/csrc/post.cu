@@ -430,13 +430,13 @@ static int post_resize(hush_post_t *p, int W, int H) {
   return HUSH_OK;
 }
 
-// The passes are a chain of short kernels, each set up while the one before runs (launch_pass). The 12 gaps between the 13
+// The passes are a chain of short kernels, each set up while the one before runs (launch_chained). The 12 gaps between the 13
 // passes of 1920x1080 took 22 us; with the small levels' passes begun early the frame is as long as its passes are (86.8
 // us). (The small levels in one cluster of 16 CTAs took as long as their launches: 38 us from 240x135 on, 17.7 from 120x67
 // on.) COMPOSITE does not let its successor in early: with 8100 short CTAs that made it 9.6 instead of 7.2 us long.
 template <class... P, class... A>
 static cudaError_t run_pass(void (*kern)(P...), dim3 grid, bool first, cudaStream_t st, A... args) {
-  return launch_pass(kern, grid, dim3(BX, BY), 0, first, st, args...);
+  return launch_chained(kern, grid, dim3(BX, BY), 0, first, st, args...);
 }
 
 // Post.encode (post.js:191-210).
@@ -465,7 +465,7 @@ extern "C" int hush_post_encode(hush_post_t *p, const hush_post_inputs *in, void
   const bool half0 = half(W, H, p->lw[0], p->lh[0]);
   const int *lw = p->lw, *lh = p->lh;
   cudaError_t e = run_pass(k_post_composite, grid_for(W, H), true, st, L, R, M, W, H, in->split, in->split2, in->exposure,
-                              in->same, p->hdr);
+                           in->same, p->hdr);
   if (e == cudaSuccess)
     e = run_pass(half0 ? k_post_down<true, true> : k_post_down<true, false>, grid_for(lw[0], lh[0]), false, st, p->hdr, W,
                     H, p->lev[0], lw[0], lh[0]);

@@ -1,9 +1,10 @@
 // The path tracer's kernel and the PathTracer instance (src/pt/pathtracer.js, pathtracer.wgsl.js).
 //
-// With an environment map, a persistent kernel that alternates two phases (without one, k_pathtrace_pixel). Shade: every thread takes the path it holds one vertex on (the direct light
-// its last shadow rays brought, then the hit's surface, the shadow rays of all its lights and the next direction; none of
-// these waits for another ray) and a thread whose path is complete takes the next pixel. Trace: the CTA's path and shadow rays
-// are one queue in shared memory, from which lanes take a ray whenever they are free, whatever pixel and kind it is of.
+// With an environment map, a persistent kernel that alternates two phases (without one, k_pathtrace_pixel). Shade: every thread
+// takes the path it holds one vertex on (the direct light its last shadow rays brought, then the hit's surface, the shadow rays
+// of all its lights and the next direction; none of these waits for another ray) and a thread whose path is complete takes
+// the next pixel. Trace: the CTA's path and shadow rays are one queue in shared memory, from which lanes take a ray whenever
+// they are free, whatever pixel and kind it is of.
 //
 // What bounds it is the SIMD width: with one thread per pixel, tracing where a ray is needed, a path's end, a light that is
 // not tried, a leaf or a long ray left 7 of 32 lanes at work, and the traversal inlined at its four calls did not fit the
@@ -829,9 +830,9 @@ constexpr size_t pt_smem(uint32_t shadows, uint32_t stack) {
   return (size_t)NT * 4 * (words_per_thread(shadows) + stack) + (size_t)NT * 2 * (shadows + 1);
 }
 
-// main() and tracePath (pathtracer.wgsl.js:511-672) with an environment map. CTAs walk the image's 8 x 4 tiles (tile blockIdx.x, + gridDim.x, ...) and
-// hand out their pixels one by one. In mode 0 the primary hit's G-buffer values are stored when they are known, the radiance
-// when the path is complete.
+// main() and tracePath (pathtracer.wgsl.js:511-672) with an environment map. CTAs walk the image's 8 x 4 tiles (tile blockIdx.x,
+// + gridDim.x, ...) and hand out their pixels one by one. In mode 0 the primary hit's G-buffer values are stored when they are
+// known, the radiance when the path is complete.
 template <bool ACCUM>
 __global__ void __launch_bounds__(NT, CTAS) k_pathtrace(const __grid_constant__ hush_pt_frame F, const pt::SceneView S,
                                                         const pt::EnvView E, const GBuf G, float4 *__restrict__ accum,
@@ -1135,7 +1136,7 @@ __global__ void __launch_bounds__(NT, CTAS) k_pathtrace(const __grid_constant__ 
 
 struct hush_pt_s {
   hush_pt_scene_t *scene = nullptr;
-  int dev = 0, W = 0, H = 0;
+  int dev = 0, sms = 0, W = 0, H = 0;
   void *pool = nullptr;
   uint2 *gbuf[2][5] = {};
   float4 *accum = nullptr;
@@ -1172,6 +1173,7 @@ extern "C" int hush_pt_create(hush_pt_scene_t *scene, int W, int H, hush_pt_t **
   hush_pt_t *p = new hush_pt_t();
   p->scene = scene;
   p->dev = pt::scene_device(scene);
+  if (cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->dev) != cudaSuccess) p->sms = 148;
   if (int rc = pt_alloc(p, W, H)) {
     delete p;
     return rc;
@@ -1241,7 +1243,7 @@ extern "C" int hush_pt_encode(hush_pt_t *p, const hush_pt_frame *f, int slot, vo
   const pt::SceneView scene = pt::scene_view(p->scene);
   if (f->env[3] > 0.5f) {
     const uint32_t tx = ((uint32_t)p->W + 7u) / 8u, tiles = tx * (((uint32_t)p->H + 3u) / 4u);
-    const uint32_t grid = std::min((tiles + NT / 32 - 1) / (NT / 32), 148u * CTAS);
+    const uint32_t grid = std::min((tiles + NT / 32 - 1) / (NT / 32), (uint32_t)p->sms * CTAS);
     const uint32_t shadows = f->counts[1] + 1u, stack = (uint32_t)pt::scene_depth(p->scene) + 1u;
     static_assert(pt_smem(HUSH_PT_MAX_LIGHTS + 1, pt::MAX_DEPTH + 1) <= 48 * 1024, "else opt in to larger shared memory");
     (f->mode == 0u ? k_pathtrace<false> : k_pathtrace<true>)<<<grid, NT, pt_smem(shadows, stack), (cudaStream_t)stream>>>(
