@@ -1243,7 +1243,11 @@ extern "C" int hush_pt_encode(hush_pt_t *p, const hush_pt_frame *f, int slot, vo
   const pt::SceneView scene = pt::scene_view(p->scene);
   if (f->env[3] > 0.5f) {
     const uint32_t tx = ((uint32_t)p->W + 7u) / 8u, tiles = tx * (((uint32_t)p->H + 3u) / 4u);
-    const uint32_t grid = std::min((tiles + NT / 32 - 1) / (NT / 32), (uint32_t)p->sms * CTAS);
+    // A tile per CTA until all that fit the device have one, although three tiles would give each of its threads a pixel: the
+    // threads without one trace the others' rays. Three tiles per CTA were slower than one thread per pixel on some small
+    // images (240 x 135, one light picked per vertex: 310 us, three tiles 364, one 313; 48 x 27: 270, 297, 248; 320 x 180, a
+    // ray per light: 483, 369, 364).
+    const uint32_t grid = std::min(tiles, (uint32_t)p->sms * CTAS);
     const uint32_t shadows = f->counts[1] + 1u, stack = (uint32_t)pt::scene_depth(p->scene) + 1u;
     static_assert(pt_smem(HUSH_PT_MAX_LIGHTS + 1, pt::MAX_DEPTH + 1) <= 48 * 1024, "else opt in to larger shared memory");
     (f->mode == 0u ? k_pathtrace<false> : k_pathtrace<true>)<<<grid, NT, pt_smem(shadows, stack), (cudaStream_t)stream>>>(
