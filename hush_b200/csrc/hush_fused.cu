@@ -110,8 +110,9 @@ HD_INL void pixel_issue_async(const HushFrame &f, int px, int py, uint2 mvr, uin
 // qf16 of a value that is at most 65504 or NaN (which becomes -65504, as in qf16).
 HD_INL float qf16_low(float x) { return __uint_as_float(__float_as_uint(fmaxf(x, -65504.0f)) & 0xffffe000u); }
 
-// qf16 of feature i: all but the material means (12-15) are logarithms of FP32 values, bounded ratios or unit values.
-HD_INL float feature_qf16(int i, float x) { return i >= 12 && i < 16 ? qf16(x) : qf16_low(x); }
+// qf16 of feature i: all but the material means (12-15) and the logarithm of a quotient (7), which a zero divisor makes
+// infinite, are logarithms of finite values, bounded ratios or unit values.
+HD_INL float feature_qf16(int i, float x) { return i == 7 || (i >= 12 && i < 16) ? qf16(x) : qf16_low(x); }
 
 // check_key() without normalising the decoded normal: v . n >= 0.9 |v|, tol = 0.05 zPrev + 0.01.
 HD_INL bool check_key_v(float4 k, float4 n, float zPrev, float obj, float tol) {
@@ -258,7 +259,7 @@ HD_INL bool temporal_pixel_fast(const HushFrame &f, int px, int py, const Tile &
   const float4 Aq = make_float4(qf16(A.x), qf16(A.y), qf16(A.z), qf16(A.w));
   const float m1 = E * qf16(nmx);
   const float m2 = E * E * qf16(nmy);
-  const float ox = qf16_low(oc.x), oy = qf16_low(oc.y);
+  const float ox = qf16(oc.x), oy = qf16(oc.y);  // (beside a NaN component the others leave the unit square)
   o.P0 = make_float4(E * lum(Aq), 0.0f, fmaxf(m2 - m1 * m1, 0.0f), len1);
   o.P1 = make_float4(qf16_low(v), qf16(lag), E * qf16(nfast), m1);
   // (an f16 depth is its own qf16 but for infinity and NaN)
