@@ -508,16 +508,20 @@ __global__ void __launch_bounds__(KB_TW / 4 * TH, 2 * KB_TH / TH)
       if (okp[q]) VA += (la[q] - Lacc) * (la[q] - Lacc);
     VA *= k;
     // 4x4 neighbourhood (block +-1) of the quantised luminance, row-major; its middle entries are the block's own pixels
+    // (a pixel of NaN depth is one of them but no valid neighbour: its luminance counts as the lowest)
     float s1 = 0.f, n4 = 0.f, lq[16], ly[16];
+    float own[4];
 #pragma unroll
     for (int e = 0; e < 16; e++) {
       const float x = S.Lq[kb_tix(2 * lby + (e >> 2), 2 * lbx + (e & 3))];
+      const int q = (e >> 2) * 2 + (e & 3) - 3;  // of a middle entry
+      if (((e >> 2) == 1 || (e >> 2) == 2) && ((e & 3) == 1 || (e & 3) == 2)) own[q] = okp[q] ? fmaxf(x, E * -65504.0f) : 0.0f;
       ly[e] = l_counts(x);
       lq[e] = ly[e] * x;
       s1 += lq[e];
       n4 += ly[e];
     }
-    S0.y = (lq[5] + lq[6] + lq[9] + lq[10]) * k;
+    S0.y = (own[0] + own[1] + own[2] + own[3]) * k;
     const float mu4 = s1 / fmaxf(n4, 1.0f);
     float var4 = 0.f;
 #pragma unroll
@@ -1202,7 +1206,7 @@ HD_INL void fine_pixels(const HushFrame &f, const FineSmem &S, int li, int bx, i
   const int hx0 = bx / 2 - 1, hy0 = by / 2 - 1, qx0 = bx / 4 - 1, qy0 = by / 4 - 1;
   const int ti = (py - by + AP) * SW + px - bx + AP;
   const float4 gp0 = S.g[ti], gp1 = S.g[ti + SW];
-  const bool live0 = gp0.w >= 0.0f, live1 = in1 && gp1.w >= 0.0f;
+  const bool live0 = !(gp0.w < 0.0f), live1 = in1 && !(gp1.w < 0.0f);
   const int o = py * f.W + px;
   auto sky = [&](int oo, uint2 er) {
     const float4 emi = h4_to_f4(er);
